@@ -132,7 +132,11 @@ void setConstants(dev::Args<T>& a, const lfm_solver_desc* d) {
     const double RpsiRef = pRef / d->rhoInf;
     const double gh = d->gamma / (d->gamma - 1.0);
     a.pRef = pRef;
+    a.RpsiRef = RpsiRef;
     a.gh = gh;
+    a.gm1Inv = 1.0 / a.gm1;
+    a.RTInv = a.Rinv / d->TInf;
+    a.keInf = 0.5 * u2;
     a.mu23 = d->mu * 2.0 / 3.0;
     a.ref.rho = (float)d->rhoInf;
     for (int k = 0; k < 3; ++k) {

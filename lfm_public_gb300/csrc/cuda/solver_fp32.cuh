@@ -105,7 +105,7 @@ __device__ __forceinline__ void ghost32(const Args<float>& a, int g, const doubl
     const int t = a.nc + g;
     double qv[NQ];
     ghost_bc<float, D>(a, g, qi, qv);
-    const double rinv = 1.0 / qv[0];
+    const double rinv = rcp64(qv[0]);
     double ke = 0.0;
     dst[(size_t)P::r * nt + t] = (float)(qv[0] - a.qRef[0]);
 #pragma unroll
@@ -115,7 +115,7 @@ __device__ __forceinline__ void ghost32(const Args<float>& a, int g, const doubl
         ke += qv[k + 1] * qv[k + 1];
     }
     const double p = a.gm1 * (qv[D + 1] - 0.5 * ke * rinv);
-    const float Rpsi = (float)(p * rinv - a.pRef / a.qRef[0]);
+    const float Rpsi = (float)(p * rinv - a.RpsiRef);
     dst[(size_t)P::Rpsi * nt + t] = Rpsi;
     dst[(size_t)P::c * nt + t] = sqrtf(a.ref.gamma * (a.ref.Rpsi + Rpsi));
 }
@@ -168,12 +168,7 @@ __device__ __forceinline__ void ghosts_of32(const Args<float>& a, int c, const d
     double qa[NQ];
 #pragma unroll
     for (int v = 0; v < NQ; ++v) qa[v] = qp[v] + a.qRef[v];
-    for (int e = a.cfOff[c]; e < a.cfOff[c + 1]; ++e) {
-        const int code = a.cfList[e];
-        if (code < 0) continue;
-        const int j = a.fN[code];
-        if (j >= a.nc && j < a.nc + a.ng) ghost32<D>(a, j - a.nc, qa, dst);
-    }
+    for_ghosts<float, D>(a, c, [&](int j) { ghost32<D>(a, j - a.nc, qa, dst); });
 }
 
 // gather32: the face rhs sum of cell c (ascending face order).

@@ -119,11 +119,14 @@ struct Args {
     // constants
     double gamma, gm1, Rinv, rhoInf, EInf, pInf, TInf, UInf[3], mu, kcond;
     double gh;                // gamma / (gamma - 1): enthalpy per unit R psi
+    double gm1Inv;            // boundary states: 1 / (gamma - 1), 1 / (R T_inf), |U_inf|^2 / 2
+    double RTInv, keInf;
     double mu23;              // 2/3 mu (the trace term of the deviatoric stress)
     // FP32-bulk: conservative reference state q_ref = (rho_inf, rho_inf U_inf,
     // rho_inf E_inf) in FP64 (index = variable) and its derived FP32 constants
     double qRef[5];
     double pRef;              // (gamma - 1)(rho_inf E_inf - rho_inf |U_inf|^2 / 2)
+    double RpsiRef;           // p_ref / rho_inf
     RefState32 ref;
     // FP64 path: the primitives include the sound speed (read by M2AUSM only)
     int primC;
