@@ -143,6 +143,7 @@ int upload(lfm_solver* s, X** out, const X* src, size_t n) {
 // Converts an FP64 host array to T and uploads it.
 template <typename T>
 int uploadAs(lfm_solver* s, T** out, const double* src, size_t n) {
+    if constexpr (sizeof(T) == sizeof(double)) return upload(s, out, src, n);
     std::vector<T> tmp(n);
     for (size_t k = 0; k < n; ++k) tmp[k] = (T)src[k];
     int rc = upload(s, out, tmp.data(), n);
@@ -180,9 +181,12 @@ int buildArgs(lfm_solver* s, const lfm_solver_desc* d, Args<T>& a, const int* fP
     a.fOwn = nullptr;
     a.smagC = nullptr;
     a.wN = nullptr;
+    a.mS = a.mK = a.mT = a.mSK = a.kK = a.ml = a.kl = nullptr;
+    a.smag = a.d = a.K = a.lapc = a.dmag = nullptr;
     a.cfSoN = nullptr;
     a.cellSoW = nullptr;
     a.primC = s->scheme == LFM_SOLVER_M2AUSM ? 1 : 0;
+    constexpr bool fp64 = sizeof(T) == sizeof(double);
     const size_t nt = (size_t)s->nt, nf = (size_t)s->nf, D = (size_t)s->D;
     int rc;
     if ((rc = devAlloc(s, &a.dq, (size_t)s->nq * s->nc))) return rc;
@@ -196,20 +200,18 @@ int buildArgs(lfm_solver* s, const lfm_solver_desc* d, Args<T>& a, const int* fP
     T* p;
     if ((rc = uploadAs<T>(s, &p, d->S, D * nf))) return rc;
     a.S = p;
-    if ((rc = uploadAs<T>(s, &p, d->d, D * nf))) return rc;
-    a.d = p;
     if ((rc = uploadAs<T>(s, &p, d->w, nf))) return rc;
     a.w = p;
-    if ((rc = uploadAs<T>(s, &p, d->smag, nf))) return rc;
-    a.smag = p;
     if ((rc = uploadAs<T>(s, &p, d->dmag_inv, nf))) return rc;
     a.dinv = p;
     if ((rc = uploadAs<T>(s, &p, d->dnorm, D * nf))) return rc;
     a.dnorm = p;
-    if ((rc = uploadAs<T>(s, &p, d->delta_mag, nf))) return rc;
-    a.dmag = p;
-    if ((rc = uploadAs<T>(s, &p, d->K, D * nf))) return rc;
-    a.K = p;
+    if (s->scheme == LFM_SOLVER_M2AUSM) {   // read by its reconstruction only
+        if ((rc = uploadAs<T>(s, &p, d->d, D * nf))) return rc;
+        a.d = p;
+        if ((rc = uploadAs<T>(s, &p, d->smag, nf))) return rc;
+        a.smag = p;
+    }
     if ((rc = uploadAs<T>(s, &p, d->sponge, (size_t)s->nc))) return rc;
     a.sponge = p;
     if (d->smag_c) {
@@ -224,44 +226,44 @@ int buildArgs(lfm_solver* s, const lfm_solver_desc* d, Args<T>& a, const int* fP
             cf[(size_t)c] = d->smag_c[e1 > e0 ? d->face_p[d->cell_faces[e1 - 1]] : c];
         }
         if ((rc = uploadAs<T>(s, &p, cf.data(), cf.size()))) return rc;
+        LFM_CUDA(cudaStreamSynchronize(s->stream));   // cf dies here
         a.smagC = p;
     }
-    {
+    if (sizeof(T) == sizeof(float)) {
+        if ((rc = uploadAs<T>(s, &p, d->K, D * nf))) return rc;
+        a.K = p;
         std::vector<double> lapc(nf);
         for (size_t f = 0; f < nf; ++f) lapc[f] = d->delta_mag[f] * d->dmag_inv[f];
         if ((rc = uploadAs<T>(s, &p, lapc.data(), nf))) return rc;
         a.lapc = p;
+    } else if (d->mu != 0.0) {
+        // viscous face constants, formed on the device (launch_fp64_constants)
+        T* rows[7];
+        for (int k = 0; k < 7; ++k)
+            if ((rc = devAlloc(s, &rows[k], k < 5 ? D * nf : nf))) return rc;
+        a.mS = rows[0];
+        a.mK = rows[1];
+        a.mT = rows[2];
+        a.mSK = rows[3];
+        a.kK = rows[4];
+        a.ml = rows[5];
+        a.kl = rows[6];
+        if ((rc = uploadAs<T>(s, &p, d->K, D * nf))) return rc;
+        a.K = p;
+        if ((rc = uploadAs<T>(s, &p, d->delta_mag, nf))) return rc;
+        a.dmag = p;
     }
     if (sizeof(T) == sizeof(double)) {
-        // FP64 face, face-entry and cell constants, each the value the kernels
-        // would otherwise compute per face visit: 1 - w per face; for the
-        // Gauss gradients, with the face value v_f = w v_P + (1 - w) v_N and
-        // so_e = S/V of entry e's face seen from its cell c,
-        //   sum_e v_f so_e = v_c sum_e w_own so_e + sum_e v_across w_across so_e,
-        // the first sum a cell constant, w_across so_e an entry constant
-        // (w_own = w where c is P, 1 - w where c is N)
-        std::vector<double> wN(nf);
-        for (size_t f = 0; f < nf; ++f) wN[f] = 1.0 - d->w[f];
-        if ((rc = uploadAs<T>(s, &p, wN.data(), nf))) return rc;
-        a.wN = p;
+        // face, entry and cell constants, formed on the device
         const size_t ne = (size_t)d->cell_face_offsets[s->nc], nc = (size_t)s->nc;
-        std::vector<double> soN(D * ne), soW(D * nc, 0.0);
-        for (size_t c = 0; c < nc; ++c)
-            for (int64_t e = d->cell_face_offsets[c]; e < d->cell_face_offsets[c + 1]; ++e) {
-                const int64_t f = d->cell_faces[e];
-                const bool isP = d->cell_face_sign[e] > 0;
-                const double wOwn = isP ? d->w[f] : wN[(size_t)f], wAcross = isP ? wN[(size_t)f] : d->w[f];
-                for (size_t k = 0; k < D; ++k) {
-                    const double Sk = d->S[k * nf + (size_t)f];
-                    const double so = isP ? Sk * d->vol_inv[c] : -Sk * d->vol_inv[c];
-                    soN[(size_t)e * D + k] = wAcross * so;   // entry-major: one entry's D values together
-                    soW[c * D + k] += wOwn * so;
-                }
-            }
-        if ((rc = uploadAs<T>(s, &p, soN.data(), soN.size()))) return rc;
-        a.cfSoN = p;
-        if ((rc = uploadAs<T>(s, &p, soW.data(), soW.size()))) return rc;
-        a.cellSoW = p;
+        T *wN, *soN, *soW;
+        if ((rc = devAlloc(s, &wN, nf)) || (rc = devAlloc(s, &soN, D * ne)) || (rc = devAlloc(s, &soW, D * nc)))
+            return rc;
+        a.wN = wN;
+        a.cfSoN = soN;
+        a.cellSoW = soW;
+        if constexpr (fp64) lfm::dev::launch_fp64_constants(a, s->stream);
+        LFM_CUDA(cudaGetLastError());
     }
     a.volInv32 = nullptr;
     if (sizeof(T) == sizeof(float)) {

@@ -105,8 +105,8 @@ __global__ void __launch_bounds__(256) k_vis(Args<T> a) {
 #pragma unroll
         for (int l = 0; l < D; ++l) g[k][l] = T(0);
     }
-    // Gauss gradients of u and of R psi (T = R psi / R: the 1/R factor is
-    // applied once to the sum). With the face value v_f = w v_P + (1 - w) v_N
+    // Gauss gradients of u and of R psi (T = R psi / R: the flux's face
+    // constant kK carries the 1/R). With the face value v_f = w v_P + (1 - w) v_N
     // and so = S/V seen from c, sum_f v_f so = v_c cellSoW_c + sum_e v_j
     // cfSoN_e: the cell's own share through one cell constant, each
     // neighbour's through an entry constant (the other cell j = cfNbr[e]).
@@ -136,9 +136,6 @@ __global__ void __launch_bounds__(256) k_vis(Args<T> a) {
             gT[x] += fR * so[x];
         }
     }
-    const T Rinv = (T)a.Rinv;
-#pragma unroll
-    for (int x = 0; x < D; ++x) gT[x] *= Rinv;
     const T mu = (T)a.mu;
     T tau[D][D];
     stress<T, D>(g, mu, tau);
@@ -175,12 +172,9 @@ __global__ void __launch_bounds__(128) k_flux(Args<T> a) {
     const int i = a.fP[f], j = a.fN[f];
     const bool ghost = a.fGhost[f] != 0;
     const T w = a.w[f], wN = a.wN[f];
-    T S[D], Kf[D];
+    T S[D];
 #pragma unroll
-    for (int k = 0; k < D; ++k) {
-        S[k] = a.S[k * nf + f];
-        Kf[k] = a.K[k * nf + f];
-    }
+    for (int k = 0; k < D; ++k) S[k] = a.S[k * nf + f];
     T qi[NQ], qj[NQ];
 #pragma unroll
     for (int v = 0; v < NQ; ++v) {
@@ -195,8 +189,7 @@ __global__ void __launch_bounds__(128) k_flux(Args<T> a) {
         aU[k] = a.prim[(1 + k) * nt + j];
     }
     const T cRpsi = a.prim[(D + 1) * nt + i], aRpsi = a.prim[(D + 1) * nt + j];
-    const T Rinv = (T)a.Rinv;
-    const T dT = (aRpsi - cRpsi) * Rinv;   // T_N - T_P
+    const T dR = aRpsi - cRpsi;
     T rhs[NQ];
 
     if (SCH == kSchemeM1) {
@@ -215,7 +208,7 @@ __global__ void __launch_bounds__(128) k_flux(Args<T> a) {
         T m[D];
 #pragma unroll
         for (int k = 0; k < D; ++k) m[k] = interp2(w, wN, qi[k + 1], qj[k + 1]);
-        const T Rpsi = interp2(w, wN, cRpsi, aRpsi);
+        const T Rpsi = aRpsi - w * dR;   // the same interpolation from the difference
         const T rinv = rcp64(rho);
         T mS = T(0), u2 = T(0);
 #pragma unroll
@@ -231,13 +224,17 @@ __global__ void __launch_bounds__(128) k_flux(Args<T> a) {
         rhs[D + 1] = -mS * ((T)a.gh * Rpsi + T(0.5) * u2 * (rinv * rinv));
     } else {
         // Pirozzoli kinetic-energy-preserving mid-point flux (src/cfd_v0.cpp:1966-2023)
-        const T rhoavg = T(0.5) * (qi[0] + qj[0]);
-        const T rhoavg_inv = rcp64(rhoavg);
-        T rhoUavg[D];
+        // on the sums of the two sides: rho u.S = (m_P + m_N).S / 2 and
+        // u = (m_P + m_N) / (rho_P + rho_N), the halves left to the products
+        const T rho2 = qi[0] + qj[0];
+        T m2[D], mS2 = T(0);
 #pragma unroll
-        for (int k = 0; k < D; ++k) rhoUavg[k] = T(0.5) * (qi[k + 1] + qj[k + 1]);
-        T pavg = rhoavg * (T(0.5) * (cRpsi + aRpsi));
-        const T Havg = T(0.5) * ((qi[D + 1] * cri + cRpsi) + (qj[D + 1] * ari + aRpsi));
+        for (int k = 0; k < D; ++k) {
+            m2[k] = qi[k + 1] + qj[k + 1];
+            mS2 = k ? mS2 + m2[k] * S[k] : m2[0] * S[0];
+        }
+        T pavg = (T(0.25) * rho2) * (cRpsi + aRpsi);
+        const T H2 = (qi[D + 1] * cri + cRpsi) + (qj[D + 1] * ari + aRpsi);
         if (SCH == kSchemeAUSM) {
             // shock sensor, minmod reconstructions and AUSM+ pressure
             // dissipation (src/cfd_v0.cpp:2288-2339)
@@ -245,8 +242,7 @@ __global__ void __launch_bounds__(128) k_flux(Args<T> a) {
             T d[D];
 #pragma unroll
             for (int k = 0; k < D; ++k) d[k] = a.d[k * nf + f];
-            T cdiv = T(0), ndiv = T(0), ccurl = T(0), ncurl = T(0), cv2 = T(0), nv2 = T(0), unPos = T(0),
-              unNeg = T(0), norm = T(0);
+            T cdiv = T(0), ndiv = T(0), ccurl = T(0), ncurl = T(0), unPos = T(0), unNeg = T(0);
 #pragma unroll
             for (int x = 0; x < D; ++x) {
                 cdiv += a.V[(x * D + x) * nt + i];
@@ -258,27 +254,23 @@ __global__ void __launch_bounds__(128) k_flux(Args<T> a) {
                     ccurl += cc * cc;
                     ncurl += nn * nn;
                 }
-                cv2 += cU[x] * cU[x];
-                nv2 += aU[x] * aU[x];
                 T gi[D], gj[D];
 #pragma unroll
                 for (int y = 0; y < D; ++y) {
                     gi[y] = a.grad[(2 * D + x * D + y) * nt + i];
                     gj[y] = a.grad[(2 * D + x * D + y) * nt + j];
                 }
-                const T uP = minmod_interp<T, D>(cU[x], aU[x], gi, d, w, T(1));
-                const T uN = minmod_interp<T, D>(cU[x], aU[x], gj, d, w, T(-1));
+                T uP, uN;
+                minmod_pair<D>(cU[x], aU[x], gi, gj, d, w, wN, uP, uN);
                 unPos += uP * S[x];
                 unNeg += uN * S[x];
-                norm += S[x] * S[x];
             }
-            T ct = -(cdiv / sqrt(cdiv * cdiv + ccurl + T(4e-2)));
+            T ct = -cdiv * rsqrt(cdiv * cdiv + ccurl + T(4e-2));
             ct = (ct < T(0)) ? T(0) : ct;
-            T nt_ = -(ndiv / sqrt(ndiv * ndiv + ncurl + T(4e-2)));
+            T nt_ = -ndiv * rsqrt(ndiv * ndiv + ncurl + T(4e-2));
             nt_ = (nt_ < T(0)) ? T(0) : nt_;
             const T theta = T(0.5) * (ct + nt_);
-            const T cp = qi[0] * (T)a.gm1 * (qi[D + 1] * cri - T(0.5) * cv2);
-            const T np = qj[0] * (T)a.gm1 * (qj[D + 1] * ari - T(0.5) * nv2);
+            const T cp = qi[0] * cRpsi, np = qj[0] * aRpsi;   // p = rho R psi
             T gri[D], grj[D], gpi[D], gpj[D];
 #pragma unroll
             for (int y = 0; y < D; ++y) {
@@ -287,86 +279,103 @@ __global__ void __launch_bounds__(128) k_flux(Args<T> a) {
                 gpi[y] = a.grad[(D + y) * nt + i];
                 gpj[y] = a.grad[(D + y) * nt + j];
             }
-            const T rhoPos = minmod_interp<T, D>(qi[0], qj[0], gri, d, w, T(1));
-            const T rhoNeg = minmod_interp<T, D>(qi[0], qj[0], grj, d, w, T(-1));
-            const T pPos = minmod_interp<T, D>(cp, np, gpi, d, w, T(1));
-            const T pNeg = minmod_interp<T, D>(cp, np, gpj, d, w, T(-1));
-            const T Msq = (unPos * unPos + unNeg * unNeg) / (T(2) * cavg * cavg * norm);
-            const T snorm = sqrt(norm);
-            const T MPos = unPos / (snorm * cavg);
-            const T MNeg = unNeg / (snorm * cavg);
+            T rhoPos, rhoNeg, pPos, pNeg;
+            minmod_pair<D>(qi[0], qj[0], gri, grj, d, w, wN, rhoPos, rhoNeg);
+            minmod_pair<D>(cp, np, gpi, gpj, d, w, wN, pPos, pNeg);
+            const T sc = rcp64(a.smag[f] * cavg);
+            const T MPos = unPos * sc, MNeg = unNeg * sc;
+            const T Msq = T(0.5) * (MPos * MPos + MNeg * MNeg);
             const T Minf = T(0.2);
             T m = (Msq < Minf * Minf) ? Minf * Minf : Msq;
             m = (m < T(1)) ? m : T(1);
             const T M0 = sqrt(m);
             const T fa = M0 * (T(2) - M0);
-            const T alpha = T(3) * (T(5) * fa * fa - T(4)) / T(16);
-            const T phalf = pNeg * (p5pos(MNeg, alpha) - p5neg(MNeg, alpha)) -
-                            pPos * (p5pos(MPos, alpha) - p5neg(MPos, alpha));
-            const T pu = T(-0.75) * p5pos(MPos, alpha) * p5neg(MNeg, alpha) * (rhoPos + rhoNeg) * cavg * fa *
-                         (unNeg - unPos);
+            const T alpha = T(3.0 / 16.0) * (T(5) * fa * fa - T(4));
+            const T ppP = p5pos(MPos, alpha), pnP = p5neg(MPos, alpha);
+            const T ppN = p5pos(MNeg, alpha), pnN = p5neg(MNeg, alpha);
+            const T phalf = pNeg * (ppN - pnN) - pPos * (ppP - pnP);
+            const T pu = T(-0.75) * ppP * pnN * (rhoPos + rhoNeg) * cavg * fa * (unNeg - unPos);
             pavg += theta * (pu - T(0.5) * phalf);
         }
-        T phiavg = T(0);
+        const T hphi = T(0.5) * mS2 * rcp64(rho2);   // u_f . S / 2
+        const T mS = T(0.5) * mS2;
+        rhs[0] = -mS;
 #pragma unroll
-        for (int k = 0; k < D; ++k) phiavg += (rhoUavg[k] * rhoavg_inv) * S[k];
-        rhs[0] = -rhoavg * phiavg;
-#pragma unroll
-        for (int k = 0; k < D; ++k) rhs[k + 1] = -(rhoUavg[k] * phiavg + pavg * S[k]);
-        rhs[D + 1] = -(rhoavg * Havg * phiavg);
+        for (int k = 0; k < D; ++k) rhs[k + 1] = -(m2[k] * hphi + pavg * S[k]);
+        rhs[D + 1] = -(T(0.5) * mS) * H2;
     }
 
     // Viscous face terms (src/cfd_v0.cpp:2682-2796). With mu == 0 every term
     // is an exact zero and the block is skipped.
+    // Each is linear in the face's velocity gradient g, in its R psi gradient
+    // gR and in the differences across the face, with per-face constants that
+    // carry mu, the conductivity and 1/R (solver_kernels.cuh: mS .. kl):
+    //   div tauMC + the Laplacian split, component x:
+    //     sum_y g[y][x] mu S_y - (2/3) mu tr(g) S_x + mu (K.g[x] + |delta|/|d| du_x)
+    //     (the face tauMC, which the reference interpolates from the cells' or
+    //     applies to the boundary's two-point gradient, is linear in g)
+    //   heat: k/R (K.gR + |delta|/|d| d(R psi)) + sigmaU . S
+    // The heat flux and sigmaU.S of each side are summed before they are
+    // interpolated (10 instead of 12 operations in 2D). The kernel is bound by
+    // the FP64 pipe, and loads are not: seven constants more per face and 14
+    // operations less took the flux of the 768 x 512 M1 cylinder from 583 to
+    // 459 us a step, of the 97 x 61 x 23 M2 wake from 484 to 390 (GB300).
     const T mu = (T)a.mu;
     if (mu != T(0)) {
-        const T lapc = a.lapc[f];   // |delta| / |d|
-        T g[D][D], gT[D], sU[D];
+        T g[D][D], eV;
         if (!ghost) {
+            T ei = T(0), ej = T(0);
 #pragma unroll
             for (int x = 0; x < D; ++x) {
 #pragma unroll
                 for (int y = 0; y < D; ++y)
                     g[x][y] = interp2(w, wN, a.V[(x * D + y) * nt + i], a.V[(x * D + y) * nt + j]);
-                gT[x] = interp2(w, wN, a.V[(D * D + x) * nt + i], a.V[(D * D + x) * nt + j]);
-                sU[x] = interp2(w, wN, a.V[(D * D + D + x) * nt + i], a.V[(D * D + D + x) * nt + j]);
+                const T kK = a.kK[x * nf + f];
+                ei = x ? ei + a.V[(D * D + x) * nt + i] * kK : a.V[(D * D) * nt + i] * kK;
+                ej = x ? ej + a.V[(D * D + x) * nt + j] * kK : a.V[(D * D) * nt + j] * kK;
+                ei += a.V[(D * D + D + x) * nt + i] * S[x];
+                ej += a.V[(D * D + D + x) * nt + j] * S[x];
             }
+            eV = interp2(w, wN, ei, ej);
         } else {
             // explicit two-point gradients on physical boundaries
             const T dinv = a.dinv[f];
             T dn[D], tau[D][D], Uf[D];
+            eV = T(0);
 #pragma unroll
-            for (int k = 0; k < D; ++k) dn[k] = a.dnorm[k * nf + f];
+            for (int k = 0; k < D; ++k) {
+                dn[k] = a.dnorm[k * nf + f] * dinv;
+                eV += dR * dn[k] * a.kK[k * nf + f];
+            }
 #pragma unroll
             for (int x = 0; x < D; ++x) {
 #pragma unroll
-                for (int y = 0; y < D; ++y) g[x][y] = (aU[x] - cU[x]) * dn[y] * dinv;
-                gT[x] = dT * dn[x] * dinv;
+                for (int y = 0; y < D; ++y) g[x][y] = (aU[x] - cU[x]) * dn[y];
                 Uf[x] = interp(w, cU[x], aU[x]);
             }
             stress<T, D>(g, mu, tau);
 #pragma unroll
-            for (int x = 0; x < D; ++x) sU[x] = dotv<T, D>(Uf, tau[x]);
+            for (int x = 0; x < D; ++x) eV += dotv<T, D>(Uf, tau[x]) * S[x];
         }
-        // The face tauMC: the reference interpolates the cells' tauMC =
-        // mu dudx^T - (2/3) mu tr(dudx) I (and on boundary faces applies the
-        // same expression to the two-point gradient); it is linear in dudx,
-        // so it is rebuilt here from the face gradient g.
-        T tr = g[0][0];
-#pragma unroll
-        for (int x = 1; x < D; ++x) tr += g[x][x];
-        const T dsum = -(T)a.mu23 * tr;
-        const T kc = (T)a.kcond;
+        const T ml = a.ml[f];
 #pragma unroll
         for (int x = 0; x < D; ++x) {
-            T gtS = g[0][x] * S[0];
+            T r = rhs[x + 1] + g[x][x] * a.mSK[x * nf + f];
+            T off = T(0);   // the trace without g[x][x]
+            bool any = false;
 #pragma unroll
-            for (int y = 1; y < D; ++y) gtS += g[y][x] * S[y];
-            // div tauMC + the Laplacian split: mu (g^T S + |delta|/|d| du + K.g) + dsum S
-            rhs[x + 1] += mu * (gtS + lapc * (aU[x] - cU[x]) + dotv<T, D>(Kf, g[x])) + dsum * S[x];
+            for (int y = 0; y < D; ++y) {
+                if (y == x) continue;
+                r += g[y][x] * a.mS[y * nf + f];
+                r += g[x][y] * a.mK[y * nf + f];
+                off = any ? off + g[y][y] : g[y][y];
+                any = true;
+            }
+            r += off * a.mT[x * nf + f];
+            rhs[x + 1] = r + ml * (aU[x] - cU[x]);
         }
-        const T lapT = kc * (lapc * dT + dotv<T, D>(Kf, gT));
-        rhs[D + 1] += dotv<T, D>(sU, S) + lapT;
+        rhs[D + 1] += eV;
+        rhs[D + 1] += a.kl[f] * dR;
         // Smagorinsky LES: the face tauMC also interpolates the cells' SGS
         // stress (boundary faces keep the laminar two-point one, as in the
         // reference)
@@ -559,6 +568,70 @@ void launch_res_sum(const double* res, int nc, double* partial, double* out, cud
     const unsigned nb = blocks(nc, 256);
     k_res_sq<<<nb, 256, 0, st>>>(res, nc, partial);
     k_reduce_final<<<1, 256, 0, st>>>(partial, (int)nb, 2, out);
+}
+
+// The constants of the FP64 path, each the value its kernels would otherwise
+// form on every visit. Formed here because a mesh's geometry is uploaded once
+// while its host loops would double the set-up time of a case.
+template <int D>
+__global__ void __launch_bounds__(256) k_fp64_face_constants(const Args<double> a, double* wN, double* mS, double* mK,
+                                                             double* mT, double* mSK, double* kK, double* ml,
+                                                             double* kl) {
+    const int f = LFM_GLOBAL_ID();
+    if (f >= a.nf) return;
+    wN[f] = 1.0 - a.w[f];
+    if (!mS) return;
+    const double kR = a.kcond * a.Rinv, lap = a.dmag[f] * a.dinv[f];
+#pragma unroll
+    for (int k = 0; k < D; ++k) {
+        const size_t at = (size_t)k * a.nf + f;
+        const double S = a.S[at], K = a.K[at];
+        mS[at] = a.mu * S;
+        mK[at] = a.mu * K;
+        mT[at] = -a.mu23 * S;
+        mSK[at] = a.mu * (S * (1.0 / 3.0) + K);
+        kK[at] = kR * K;
+    }
+    ml[f] = a.mu * lap;
+    kl[f] = kR * lap;
+}
+
+// With the face value v_f = w v_P + (1 - w) v_N and so_e = S/V of entry e's
+// face seen from its cell c, the Gauss gradient is
+//   sum_e v_f so_e = v_c sum_e w_own so_e + sum_e v_across w_across so_e,
+// the first sum a cell constant, w_across so_e an entry constant (w_own = w
+// where c is P, 1 - w where c is N).
+template <int D>
+__global__ void __launch_bounds__(256) k_fp64_cell_constants(const Args<double> a, double* soN, double* soW) {
+    const int c = LFM_GLOBAL_ID();
+    if (c >= a.nc) return;
+    double own[D];
+#pragma unroll
+    for (int k = 0; k < D; ++k) own[k] = 0.0;
+    for (int e = a.cfOff[c]; e < a.cfOff[c + 1]; ++e) {
+        const int code = a.cfList[e], f = code >= 0 ? code : ~code;
+        const double w = a.w[f], wOwn = code >= 0 ? w : 1.0 - w, wAcross = code >= 0 ? 1.0 - w : w;
+#pragma unroll
+        for (int k = 0; k < D; ++k) {
+            const double Sv = a.S[(size_t)k * a.nf + f] * a.volInv[c], so = code >= 0 ? Sv : -Sv;
+            soN[(size_t)e * D + k] = wAcross * so;   // entry-major: one entry's D values together
+            own[k] += wOwn * so;
+        }
+    }
+#pragma unroll
+    for (int k = 0; k < D; ++k) soW[(size_t)c * D + k] = own[k];
+}
+
+template <int D>
+static void fp64_constants(const Args<double>& a, cudaStream_t st) {
+    auto w = [](const double* p) { return const_cast<double*>(p); };
+    k_fp64_face_constants<D><<<blocks(a.nf, 256), 256, 0, st>>>(a, w(a.wN), w(a.mS), w(a.mK), w(a.mT), w(a.mSK), w(a.kK),
+                                                               w(a.ml), w(a.kl));
+    k_fp64_cell_constants<D><<<blocks(a.nc, 256), 256, 0, st>>>(a, w(a.cfSoN), w(a.cellSoW));
+}
+
+void launch_fp64_constants(const Args<double>& a, cudaStream_t st) {
+    a.D == 2 ? fp64_constants<2>(a, st) : fp64_constants<3>(a, st);
 }
 
 void launch_set_flag(int* flag, int v, cudaStream_t st) { k_set_flag<<<1, 1, 0, st>>>(flag, v); }

@@ -88,6 +88,14 @@ struct Args {
     const T* K;               // D x nf
     const T* lapc;            // |delta| / |d| per face
     const T* wN;              // FP64 path: 1 - w per face (the linear weight of N)
+    // FP64 path, mu != 0: the viscous face constants (D x nf, ml and kl nf)
+    const T* mS;              // mu S
+    const T* mK;              // mu K
+    const T* mT;              // -(2/3) mu S: the trace term
+    const T* mSK;             // mu S + mu K - (2/3) mu S: the diagonal's three terms together
+    const T* kK;              // (k / R) K
+    const T* ml;              // mu |delta| / |d|
+    const T* kl;              // (k / R) |delta| / |d|
     // cells
     const double* volInv;
     const float* volInv32;    // FP32 copy (FP32-bulk gradient kernels)

@@ -74,6 +74,9 @@ constexpr int primRows(int D) {
 struct QOffset {
     double v[5];
 };
+// FP64 path, at set-up: the face, entry and cell constants of a (wN, cfSoN,
+// cellSoW and, where allocated, mS .. kl) from its geometry.
+void launch_fp64_constants(const Args<double>& a, cudaStream_t st);
 // mode 0: max CFL, mode 1: min dt
 void launch_cfl(int D, const double* q, QOffset qo, int nt, int nc, const double* volInv, const int* sOff, const double* cellS,
                 double dt, int mode, double maxCo, double* partial, double* out, cudaStream_t st);
