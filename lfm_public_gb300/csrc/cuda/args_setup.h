@@ -8,6 +8,7 @@
 #include <vector>
 
 #include "../host/capi_internal.h"
+#include "face_pack.h"
 #include "lfm_gpu.h"
 #include "solver_kernels.cuh"
 
@@ -97,6 +98,33 @@ struct DescIndex {
     }
 };
 
+// Whether every cell's faces fit the fixed-width tables (kEllWidth).
+inline bool ellFits(const lfm_solver_desc* d) {
+    const int64_t W = d->dim == 2 ? dev::kEllWidth<2> : dev::kEllWidth<3>;
+    for (int64_t c = 0; c < d->n_cells; ++c)
+        if (d->cell_face_offsets[c + 1] - d->cell_face_offsets[c] > W) return false;
+    return true;
+}
+
+// Fixed-width tables of the face entries and the cells across them
+// (Args::cfEll, cfEllN), [n_cells][W] each.
+inline void packEll(const lfm_solver_desc* d, int* ell, int* ellN) {
+    const size_t W = (size_t)(d->dim == 2 ? dev::kEllWidth<2> : dev::kEllWidth<3>);
+    for (size_t c = 0; c < (size_t)d->n_cells; ++c) {
+        size_t at = c * W;
+        for (int64_t e = d->cell_face_offsets[c]; e < d->cell_face_offsets[c + 1]; ++e, ++at) {
+            const int64_t f = d->cell_faces[e];
+            const bool own = d->cell_face_sign[e] > 0;
+            ell[at] = own ? (int)f : ~(int)f;
+            ellN[at] = (int)(own ? d->face_n[f] : d->face_p[f]);
+        }
+        for (; at < (c + 1) * W; ++at) {
+            ell[at] = dev::kEllPad;
+            ellN[at] = -1;
+        }
+    }
+}
+
 // Scalar constants of the kernel arguments (counts, gas constants, free
 // stream, and the reference state of the FP32-bulk perturbation form).
 template <typename T>
@@ -131,6 +159,7 @@ void setConstants(dev::Args<T>& a, const lfm_solver_desc* d) {
     const double pRef = (d->gamma - 1.0) * (a.qRef[D + 1] - 0.5 * d->rhoInf * u2);
     const double RpsiRef = pRef / d->rhoInf;
     const double gh = d->gamma / (d->gamma - 1.0);
+    a.primC = d->solver == LFM_SOLVER_M2AUSM ? 1 : 0;
     a.pRef = pRef;
     a.RpsiRef = RpsiRef;
     a.gh = gh;

@@ -79,8 +79,8 @@ private:
 // Byte offsets of every array of one case inside its arena block.
 struct CaseLayout {
     size_t total = 0;
-    size_t q, dq, res, prim, V, grad, flux, S, d, w, dinv, dnorm, K, lapc, fP, fN, fGhost, volInv, volInv32,
-        sponge, cfOff, cfList, cfNbr, cfEll, cellGhosts, gCell, gKind, gFace;
+    size_t q, dq, res, prim, V, grad, flux, fG0, fG1, d, dinv, dnorm, fP, fN, volInv32, sponge, cfOff, cfList,
+        cfNbr, cfEll, cfEllN, cellGhosts, gCell, gKind, gFace;
 
     explicit CaseLayout(const lfm_solver_desc* d) {
         const size_t D = (size_t)d->dim, nq = (size_t)d->nq, nc = (size_t)d->n_cells, ng = (size_t)d->n_ghosts;
@@ -90,31 +90,27 @@ struct CaseLayout {
         dq = add(nq * nc * 4);
         res = d->residuals ? add(nq * nc * 8) : npos();
         prim = add((size_t)lfm::dev::primRows<float>(d->dim) * nt * 4);
-        V = lfm::setup::needVis(d) ? add((D * D + 2 * D) * nt * 4) : npos();
-        grad = ausm ? add((2 * D + D * D) * nt * 4) : npos();
+        V = lfm::setup::needVis(d) ? add((size_t)lfm::dev::visStride32(d->dim, false) * nt * 4) : npos();
+        grad = ausm ? add((size_t)lfm::dev::gradStride32(d->dim) * nt * 4) : npos();
         flux = add(nq * nf * 4);
-        S = add(D * nf * 4);
-        this->d = add(D * nf * 4);
-        w = add(nf * 4);
+        fG0 = add(nf * 16);
+        fG1 = add(nf * 16);
+        this->d = ausm ? add(D * nf * 4) : npos();
         dinv = add(nf * 4);
         dnorm = add(D * nf * 4);
-        K = add(D * nf * 4);
-        lapc = add(nf * 4);
-        fP = add(nf * 4);
-        fN = add(nf * 4);
-        fGhost = add(nf);
-        volInv = add(nc * 8);
+        fP = D == 3 ? add(nf * 4) : npos();   // 2D: in fG1
+        fN = D == 3 ? add(nf * 4) : npos();
         volInv32 = add(nc * 4);
         sponge = add(nc * 4);
-        cfOff = add((nc + 1) * 4);
-        cfList = add(ne * 4);
-        cfNbr = add(ne * 4);
-        // the update's fixed-width cell -> face table, when every cell fits it
+        // the fixed-width cell -> face tables when every cell fits them, else
+        // the face lists
+        const bool fits = lfm::setup::ellFits(d);
+        cfOff = fits ? npos() : add((nc + 1) * 4);
+        cfList = fits ? npos() : add(ne * 4);
+        cfNbr = fits ? npos() : add(ne * 4);
         const size_t W = (size_t)(D == 2 ? lfm::dev::kEllWidth<2> : lfm::dev::kEllWidth<3>);
-        bool fits = true;
-        for (size_t c = 0; c < nc && fits; ++c)
-            fits = (size_t)(d->cell_face_offsets[c + 1] - d->cell_face_offsets[c]) <= W;
         cfEll = fits ? add(W * nc * 4) : npos();
+        cfEllN = fits ? add(W * nc * 4) : npos();
         cellGhosts = add(nc);
         gCell = add(ng * 4);
         gKind = add(ng * 4);

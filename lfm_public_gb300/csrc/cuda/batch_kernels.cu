@@ -64,8 +64,14 @@ __device__ __forceinline__ void item(const BatchCase& bc, int stage, int i) {
         prep32<D>(a, i);
     } else if (PH == 1) {
         if (FULL) {
-            if (bc.needGrad) grad32<D>(a, i);
-            if (bc.needVis) vis32<D>(a, i);
+            if (bc.needGrad) {
+                if (a.cfEll) grad32<D, true>(a, i);
+                else grad32<D, false>(a, i);
+            }
+            if (bc.needVis) {
+                if (a.cfEll) vis32<D, false, true>(a, i);
+                else vis32<D, false, false>(a, i);
+            }
         }
     } else if (PH == 2) {
         if (bc.scheme == kSchemeM1)

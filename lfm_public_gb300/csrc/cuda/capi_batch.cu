@@ -66,30 +66,24 @@ std::vector<unsigned char> packCase(const lfm_solver_desc* d, const CaseLayout& 
         double* row = f64(L.q) + v * nt;
         for (size_t c = 0; c < nc; ++c) row[c] = (d->q0 ? d->q0[v * nc + c] : 0.0) - qRef[v];
     }
-    conv(L.S, d->S, D * nf);
-    conv(L.d, d->d, D * nf);
-    conv(L.w, d->w, nf);
+    if (L.d != CaseLayout::npos()) conv(L.d, d->d, D * nf);
     conv(L.dinv, d->dmag_inv, nf);
     conv(L.dnorm, d->dnorm, D * nf);
-    conv(L.K, d->K, D * nf);
     lfm::setup::DescIndex ix(d);
-    conv(L.lapc, ix.lapc.data(), nf);
-    std::memcpy(i32(L.fP), ix.fP.data(), nf * 4);
-    std::memcpy(i32(L.fN), ix.fN.data(), nf * 4);
-    std::memcpy(img.data() + L.fGhost, d->face_ghost, nf);
-    std::memcpy(f64(L.volInv), d->vol_inv, nc * 8);
+    for (size_t f = 0; f < nf; ++f) {
+        const int n = lfm::setup::flaggedN(d, f);
+        lfm::setup::packFace32(d, f, ix.fP[f], n, f32(L.fG0) + 4 * f, f32(L.fG1) + 4 * f);
+        if (L.fN != CaseLayout::npos()) i32(L.fN)[f] = n;
+    }
+    if (L.fP != CaseLayout::npos()) std::memcpy(i32(L.fP), ix.fP.data(), nf * 4);
     conv(L.volInv32, d->vol_inv, nc);
     conv(L.sponge, d->sponge, nc);
-    std::memcpy(i32(L.cfOff), ix.cfOff.data(), (nc + 1) * 4);
-    std::memcpy(i32(L.cfList), ix.cfList.data(), ix.cfList.size() * 4);
-    std::memcpy(i32(L.cfNbr), ix.cfNbr.data(), ix.cfNbr.size() * 4);
-    if (L.cfEll != CaseLayout::npos()) {   // entry k of cell c at k * nc + c, padded
-        const size_t W = (size_t)(D == 2 ? lfm::dev::kEllWidth<2> : lfm::dev::kEllWidth<3>);
-        int* ell = i32(L.cfEll);
-        for (size_t k = 0; k < W * nc; ++k) ell[k] = lfm::dev::kEllPad;
-        for (size_t c = 0; c < nc; ++c)
-            for (int e = ix.cfOff[c]; e < ix.cfOff[c + 1]; ++e)
-                ell[(size_t)(e - ix.cfOff[c]) * nc + c] = ix.cfList[(size_t)e];
+    if (L.cfEll != CaseLayout::npos()) {
+        lfm::setup::packEll(d, i32(L.cfEll), i32(L.cfEllN));
+    } else {
+        std::memcpy(i32(L.cfOff), ix.cfOff.data(), (nc + 1) * 4);
+        std::memcpy(i32(L.cfList), ix.cfList.data(), ix.cfList.size() * 4);
+        std::memcpy(i32(L.cfNbr), ix.cfNbr.data(), ix.cfNbr.size() * 4);
     }
     unsigned char* cg = img.data() + L.cellGhosts;   // cells whose update writes ghosts
     for (size_t f = 0; f < nf; ++f)
@@ -387,17 +381,13 @@ int commitCase(lfm_batch* b, const PreparedCase& pc, int* slot) {
     a.V = reinterpret_cast<float*>(P(L.V));
     a.grad = reinterpret_cast<float*>(P(L.grad));
     a.flux = reinterpret_cast<float*>(P(L.flux));
-    a.S = reinterpret_cast<const float*>(P(L.S));
+    a.fG0 = reinterpret_cast<const float4*>(P(L.fG0));
+    a.fG1 = reinterpret_cast<const float4*>(P(L.fG1));
     a.d = reinterpret_cast<const float*>(P(L.d));
-    a.w = reinterpret_cast<const float*>(P(L.w));
     a.dinv = reinterpret_cast<const float*>(P(L.dinv));
     a.dnorm = reinterpret_cast<const float*>(P(L.dnorm));
-    a.K = reinterpret_cast<const float*>(P(L.K));
-    a.lapc = reinterpret_cast<const float*>(P(L.lapc));
     a.fP = reinterpret_cast<const int*>(P(L.fP));
     a.fN = reinterpret_cast<const int*>(P(L.fN));
-    a.fGhost = reinterpret_cast<const uint8_t*>(P(L.fGhost));
-    a.volInv = reinterpret_cast<const double*>(P(L.volInv));
     a.volInv32 = reinterpret_cast<const float*>(P(L.volInv32));
     a.sponge = reinterpret_cast<const float*>(P(L.sponge));
     a.cfOff = reinterpret_cast<const int*>(P(L.cfOff));
@@ -405,6 +395,7 @@ int commitCase(lfm_batch* b, const PreparedCase& pc, int* slot) {
     a.cfNbr = reinterpret_cast<const int*>(P(L.cfNbr));
     a.cellGhosts = reinterpret_cast<const uint8_t*>(P(L.cellGhosts));
     a.cfEll = reinterpret_cast<const int*>(P(L.cfEll));
+    a.cfEllN = reinterpret_cast<const int*>(P(L.cfEllN));
     a.smagC = nullptr;
     a.gCell = reinterpret_cast<const int*>(P(L.gCell));
     a.gKind = reinterpret_cast<const int*>(P(L.gKind));

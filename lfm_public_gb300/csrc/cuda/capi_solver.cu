@@ -178,30 +178,43 @@ int buildArgs(lfm_solver* s, const lfm_solver_desc* d, Args<T>& a, const int* fP
     a.flag = s->flag;
     a.cellGhosts = nullptr;
     a.cfEll = nullptr;
+    a.cfEllN = nullptr;
+    a.fG0 = a.fG1 = nullptr;
     a.fOwn = nullptr;
     a.smagC = nullptr;
     a.wN = nullptr;
     a.mS = a.mK = a.mT = a.mSK = a.kK = a.ml = a.kl = nullptr;
-    a.smag = a.d = a.K = a.lapc = a.dmag = nullptr;
+    a.S = a.w = a.smag = a.d = a.K = a.lapc = a.dmag = nullptr;
     a.cfSoN = nullptr;
     a.cellSoW = nullptr;
-    a.primC = s->scheme == LFM_SOLVER_M2AUSM ? 1 : 0;
     constexpr bool fp64 = sizeof(T) == sizeof(double);
     const size_t nt = (size_t)s->nt, nf = (size_t)s->nf, D = (size_t)s->D;
     int rc;
     if ((rc = devAlloc(s, &a.dq, (size_t)s->nq * s->nc))) return rc;
     if ((rc = devAlloc(s, &a.prim, (size_t)lfm::dev::primRows<T>(s->D) * nt))) return rc;
     a.primW = a.prim;
-    if ((rc = devAlloc(s, &a.V, (D * D + 2 * D + (d->smag_c ? D * D : 0)) * nt))) return rc;
+    if ((rc = devAlloc(s, &a.V, lfm::dev::visWords<T>(s->D, d->smag_c != nullptr) * nt))) return rc;
     // M2AUSM always reads the gradients (all zero when minmod is off, as in the
     // reference, whose prepare_for_RKstep zeroes them every stage).
-    if ((rc = devAlloc(s, &a.grad, (2 * D + D * D) * (s->scheme == LFM_SOLVER_M2AUSM ? nt : 1)))) return rc;
+    if ((rc = devAlloc(s, &a.grad, s->scheme == LFM_SOLVER_M2AUSM ? lfm::dev::gradWords<T>(s->D) * nt : 1))) return rc;
     if ((rc = devAlloc(s, &a.flux, (size_t)s->nq * nf))) return rc;
     T* p;
-    if ((rc = uploadAs<T>(s, &p, d->S, D * nf))) return rc;
-    a.S = p;
-    if ((rc = uploadAs<T>(s, &p, d->w, nf))) return rc;
-    a.w = p;
+    if (fp64) {
+        if ((rc = uploadAs<T>(s, &p, d->S, D * nf))) return rc;
+        a.S = p;
+        if ((rc = uploadAs<T>(s, &p, d->w, nf))) return rc;
+        a.w = p;
+    } else {   // face geometry in 16-byte parts
+        std::vector<float> g0(4 * nf), g1(4 * nf);
+        for (size_t f = 0; f < nf; ++f)
+            lfm::setup::packFace32(d, f, (int)d->face_p[f], lfm::setup::flaggedN(d, f), &g0[4 * f], &g1[4 * f]);
+        float *d0, *d1;
+        if ((rc = upload(s, &d0, g0.data(), 4 * nf))) return rc;
+        if ((rc = upload(s, &d1, g1.data(), 4 * nf))) return rc;
+        if (cudaStreamSynchronize(s->stream) != cudaSuccess) return cudaFail(cudaGetLastError(), "upload");
+        a.fG0 = reinterpret_cast<const float4*>(d0);
+        a.fG1 = reinterpret_cast<const float4*>(d1);
+    }
     if ((rc = uploadAs<T>(s, &p, d->dmag_inv, nf))) return rc;
     a.dinv = p;
     if ((rc = uploadAs<T>(s, &p, d->dnorm, D * nf))) return rc;
@@ -229,14 +242,7 @@ int buildArgs(lfm_solver* s, const lfm_solver_desc* d, Args<T>& a, const int* fP
         LFM_CUDA(cudaStreamSynchronize(s->stream));   // cf dies here
         a.smagC = p;
     }
-    if (sizeof(T) == sizeof(float)) {
-        if ((rc = uploadAs<T>(s, &p, d->K, D * nf))) return rc;
-        a.K = p;
-        std::vector<double> lapc(nf);
-        for (size_t f = 0; f < nf; ++f) lapc[f] = d->delta_mag[f] * d->dmag_inv[f];
-        if ((rc = uploadAs<T>(s, &p, lapc.data(), nf))) return rc;
-        a.lapc = p;
-    } else if (d->mu != 0.0) {
+    if (fp64 && d->mu != 0.0) {
         // viscous face constants, formed on the device (launch_fp64_constants)
         T* rows[7];
         for (int k = 0; k < 7; ++k)
@@ -638,10 +644,15 @@ int createSolver(const lfm_solver_desc* d, const lfm_solver_opts* opts, cudaStre
         if (fN[(size_t)f] >= s->nc && fN[(size_t)f] < s->nc + s->ng) gFace[(size_t)(fN[(size_t)f] - s->nc)] = f;
     std::vector<int> sOff = toInt(d->cell_s_offsets, nc + 1);
     int *dP, *dN, *dOff, *dList, *dNbr, *dGC, *dGK, *dGF;
-    uint8_t* dG;
+    uint8_t* dG = nullptr;
     if ((rc = upload(s, &dP, fP.data(), nf))) return fail(rc);
-    if ((rc = upload(s, &dN, fN.data(), nf))) return fail(rc);
-    if ((rc = upload(s, &dG, d->face_ghost, nf))) return fail(rc);
+    std::vector<int> fNf;   // FP32-bulk: with the boundary flag in the top bit
+    if (s->precision == LFM_FP32_BULK) {
+        fNf.resize(nf);
+        for (size_t f = 0; f < nf; ++f) fNf[f] = lfm::setup::flaggedN(d, f);
+    }
+    if ((rc = upload(s, &dN, fNf.empty() ? fN.data() : fNf.data(), nf))) return fail(rc);
+    if (s->precision == LFM_FP64 && (rc = upload(s, &dG, d->face_ghost, nf))) return fail(rc);
     if ((rc = upload(s, &dOff, cfOff.data(), nc + 1))) return fail(rc);
     if ((rc = upload(s, &dList, cfList.data(), ne))) return fail(rc);
     if ((rc = upload(s, &dNbr, cfNbr.data(), ne))) return fail(rc);
@@ -685,22 +696,16 @@ int createSolver(const lfm_solver_desc* d, const lfm_solver_opts* opts, cudaStre
         if (s->precision == LFM_FP32_BULK) s->a32.cellGhosts = dCG;
         else s->a64.cellGhosts = dCG;
     }
-    if (s->precision == LFM_FP32_BULK && !tiled && (s->D == 3 || s->nc > kFuseGhostCells2D)) {
-        // the update's fixed-width cell -> face table, when every cell fits it:
-        // cases whose gathers come from HBM (3D; 2D beyond 1M cells, 0.263 ->
-        // 0.255 ms per step on a 1.57M-cell cylinder); a 2D case that L2 holds
-        // loses more L2 hits to the extra table than the shorter gather saves
+    if (s->precision == LFM_FP32_BULK && !tiled && lfm::setup::ellFits(d)) {
+        // the fixed-width tables of a cell's faces and the cells across them
         const size_t W = (size_t)(s->D == 2 ? lfm::dev::kEllWidth<2> : lfm::dev::kEllWidth<3>);
-        bool fits = true;
-        for (size_t c = 0; c < nc && fits; ++c) fits = (size_t)(cfOff[c + 1] - cfOff[c]) <= W;
-        if (fits) {
-            std::vector<int> ell(W * nc, lfm::dev::kEllPad);
-            for (size_t c = 0; c < nc; ++c)
-                for (int e = cfOff[c]; e < cfOff[c + 1]; ++e) ell[(size_t)(e - cfOff[c]) * nc + c] = cfList[(size_t)e];
-            int* dEll = nullptr;
-            if ((rc = upload(s, &dEll, ell.data(), W * nc))) return fail(rc);
-            s->a32.cfEll = dEll;
-        }
+        std::vector<int> ell(W * nc), ellN(W * nc);
+        lfm::setup::packEll(d, ell.data(), ellN.data());
+        int *dEll = nullptr, *dEllN = nullptr;
+        if ((rc = upload(s, &dEll, ell.data(), W * nc))) return fail(rc);
+        if ((rc = upload(s, &dEllN, ellN.data(), W * nc))) return fail(rc);
+        s->a32.cfEll = dEll;
+        s->a32.cfEllN = dEllN;
     }
     {   // ghost face geometry in FP64 and patch ids (post-processing)
         const size_t ng = (size_t)s->ng, D = (size_t)s->D;
@@ -722,16 +727,13 @@ int createSolver(const lfm_solver_desc* d, const lfm_solver_opts* opts, cudaStre
         lfm::TileDesc* dT = nullptr;
         int* dI = nullptr;
         float* dF = nullptr;
-        uint8_t* dB = nullptr;
         if ((rc = upload(s, &dT, tiles.tiles.data(), tiles.tiles.size()))) return fail(rc);
         if ((rc = upload(s, &dI, tiles.ints.data(), tiles.ints.size()))) return fail(rc);
         if ((rc = upload(s, &dF, tiles.floats.data(), tiles.floats.size()))) return fail(rc);
-        if ((rc = upload(s, &dB, tiles.bytes.data(), tiles.bytes.size()))) return fail(rc);
         if ((rc = devAlloc(s, &s->prim1, (size_t)lfm::dev::primRows<float>(s->D) * nt))) return fail(rc);
         s->tile.tiles = dT;
         s->tile.ints = dI;
         s->tile.floats = dF;
-        s->tile.bytes = dB;
         s->tile.nTiles = (int)tiles.tiles.size();
         s->tile.smemBytes = lfm::dev::tile_smem_bytes(s->D, tiles.maxL, tiles.maxLF, tileHaveV(s), tileHaveGrad(s));
         s->tile.needGrad = s->needGrad ? 1 : 0;
@@ -1061,6 +1063,8 @@ int noallocScratch(int device, unsigned char** out) {
     return LFM_OK;
 }
 
+// Residual of cell c: its faces' rhs summed in ascending face order (FP64:
+// flux is [nq][nf]; FP32-bulk: [nf][4], then in 3D the fifth value's row).
 template <typename T, int D>
 __global__ void __launch_bounds__(256) k_gather_residual(const T* flux, int nf, int nc, const int* cfOff,
                                                          const int* cfList, double* res) {
@@ -1072,12 +1076,25 @@ __global__ void __launch_bounds__(256) k_gather_residual(const T* flux, int nf, 
     for (int v = 0; v < NQ; ++v) sum[v] = T(0);
     for (int e = cfOff[c]; e < cfOff[c + 1]; ++e) {
         const int code = cfList[e];
-        if (code >= 0) {
-#pragma unroll
-            for (int v = 0; v < NQ; ++v) sum[v] += flux[(size_t)v * nf + code];
+        const size_t f = (size_t)(code >= 0 ? code : ~code);
+        T x[NQ];
+        if constexpr (sizeof(T) == sizeof(float)) {
+            const float4 x4 = reinterpret_cast<const float4*>(flux)[f];
+            x[0] = x4.x;
+            x[1] = x4.y;
+            x[2] = x4.z;
+            x[3] = x4.w;
+            if constexpr (D == 3) x[4] = flux[4 * (size_t)nf + f];
         } else {
 #pragma unroll
-            for (int v = 0; v < NQ; ++v) sum[v] -= flux[(size_t)v * nf + ~code];
+            for (int v = 0; v < NQ; ++v) x[v] = flux[(size_t)v * nf + f];
+        }
+        if (code >= 0) {
+#pragma unroll
+            for (int v = 0; v < NQ; ++v) sum[v] += x[v];
+        } else {
+#pragma unroll
+            for (int v = 0; v < NQ; ++v) sum[v] -= x[v];
         }
     }
 #pragma unroll
@@ -1095,6 +1112,7 @@ int residualNoalloc(const lfm_solver* s, const Args<T>& base, const double* q, i
     const size_t bV = round((D * D + 2 * D + (base.smagC ? D * D : 0)) * nt * sizeof(T));
     const size_t bGrad = ausm ? round((2 * D + D * D) * nt * sizeof(T)) : 0;
     const size_t bFlux = round(nq * nf * sizeof(T));
+    // the limit a case is held to: the scratch of these arrays without padding
     const size_t need = bq + bPrim + bV + bGrad + bFlux;
     if (need > LFM_NOALLOC_SCRATCH_BYTES)
         return lfm::setError(LFM_ERR_UNSUPPORTED, "the case needs " + std::to_string(need) +
@@ -1104,18 +1122,27 @@ int residualNoalloc(const lfm_solver* s, const Args<T>& base, const double* q, i
     int rc = noallocScratch(s->device, &scratch);
     if (rc) return rc;
     Args<T> a = base;
+    // FP32-bulk: the padded viscous and gradient rows take 4 bytes a cell each
+    // more in 3D, the space of q' (at least 32 bytes a cell) holds the face rhs:
+    // the fluxes read the primitives alone, so q' is dead by then.
+    constexpr bool fp32 = sizeof(T) == sizeof(float);
+    const size_t pV = round(lfm::dev::visWords<T>(s->D, base.smagC != nullptr) * nt * sizeof(T));
+    const size_t pGrad = ausm ? round(lfm::dev::gradWords<T>(s->D) * nt * sizeof(T)) : 0;
+    const size_t q0 = fp32 ? std::max(bq, bFlux) : bq;
     a.q = reinterpret_cast<double*>(scratch);
-    a.prim = reinterpret_cast<T*>(scratch + bq);
+    a.prim = reinterpret_cast<T*>(scratch + q0);
     a.primW = a.prim;
-    a.V = reinterpret_cast<T*>(scratch + bq + bPrim);
-    a.grad = ausm ? reinterpret_cast<T*>(scratch + bq + bPrim + bV) : base.grad;
-    a.flux = reinterpret_cast<T*>(scratch + bq + bPrim + bV + bGrad);
+    a.V = reinterpret_cast<T*>(scratch + q0 + bPrim);
+    a.grad = ausm ? reinterpret_cast<T*>(scratch + q0 + bPrim + pV) : base.grad;
+    a.flux = reinterpret_cast<T*>(fp32 ? scratch : scratch + q0 + bPrim + pV + pGrad);
+    if (q0 + bPrim + pV + pGrad + (fp32 ? 0 : bFlux) > LFM_NOALLOC_SCRATCH_BYTES)
+        return lfm::setError(LFM_ERR_UNSUPPORTED, "lfm_solver_residual_noalloc: scratch layout exceeds its array");
     a.dq = nullptr;
     a.res = nullptr;
     // The array keeps the previous call's contents: the viscous terms and
     // gradients of the ghosts are read as zeros, so clear both blocks.
-    LFM_CUDA(cudaMemsetAsync(a.V, 0, bV, st));
-    if (ausm) LFM_CUDA(cudaMemsetAsync(a.grad, 0, bGrad, st));
+    LFM_CUDA(cudaMemsetAsync(a.V, 0, pV, st));
+    if (ausm) LFM_CUDA(cudaMemsetAsync(a.grad, 0, pGrad, st));
     if constexpr (sizeof(T) == sizeof(float)) {
         // the FP32-bulk kernels read the state as q - q_ref
         lfm::dev::launch_to_perturbation(a, q, qStride, st);
@@ -1548,10 +1575,16 @@ void partitionedStages(lfm_partitioned* P, double dt) {
         if (s0->needVis)
             for (size_t p = 0; p < np; ++p) {
                 const lfm_solver* s = P->parts[p];
-                const int rows = s->D * s->D + 2 * s->D + (args(p).smagC ? s->D * s->D : 0);
-                lfm::dev::launch_halo_gather<T>(args(p).V, s->nt, s->nc + s->ng, rows, s->nh, P->haloPart[p],
-                                                P->haloCell[p], reinterpret_cast<T* const*>(P->dV), P->dNt,
-                                                P->stream);
+                const bool les = args(p).smagC != nullptr;
+                if constexpr (sizeof(T) == sizeof(float))
+                    lfm::dev::launch_halo_gather_cells(args(p).V, s->nc + s->ng, lfm::dev::visStride32(s->D, les), s->nh,
+                                                       P->haloPart[p], P->haloCell[p],
+                                                       reinterpret_cast<float* const*>(P->dV), P->stream);
+                else
+                    lfm::dev::launch_halo_gather<T>(args(p).V, s->nt, s->nc + s->ng,
+                                                    (int)lfm::dev::visWords<T>(s->D, les), s->nh, P->haloPart[p],
+                                                    P->haloCell[p], reinterpret_cast<T* const*>(P->dV), P->dNt,
+                                                    P->stream);
             }
         for (int w = 3; w < 5; ++w)   // fluxes, update
             for (size_t p = 0; p < np; ++p) lfm::dev::launch_kernel<T>(args(p), c, w, P->stream);

@@ -19,8 +19,8 @@
 // and the indices of the one after are in flight. Every thread writes and
 // reads only its own columns of the buffers (threads are independent: no
 // block barrier, no wait on another thread), and cp.async.wait_group makes a
-// thread's own copies visible to it. The arithmetic is face_rhs32_cells on a
-// view of the buffers, so the rhs has the plain kernel's bits.
+// thread's own copies visible to it. The arithmetic is face_rhs32_core on
+// values of the buffers, so the rhs has the plain kernel's bits.
 //
 // Off by default: measured on GB300 (FP32-bulk, CUDA events, per step) the
 // staged kernels are slower than the plain one in every configuration tried.
@@ -57,6 +57,77 @@ __device__ __forceinline__ void cp_async_wait() {
     asm volatile("cp.async.wait_group %0;\n" ::"n"(N) : "memory");
 }
 
+// Row of a staged cell: rho', m'[D], u'[D], R psi'.
+template <int D>
+struct PRow {
+    static constexpr int r = 0, m = 1, u = 1 + D, Rpsi = 1 + 2 * D;
+};
+
+// Address of row r of cell t's primitives, and of value r of face f's staged
+// geometry (S[D], w, K[D], lapc), in the solver's arrays (solver_fp32.cuh).
+template <int D>
+__device__ __forceinline__ const float* prim_addr(const Args<float>& g, int r, int t) {
+    using P = PRow<D>;
+    const float* A = g.prim + 4 * (size_t)t;
+    const float* B = g.prim + prim_b((size_t)g.nt) + (size_t)(D == 2 ? 2 : 4) * t;
+    if (r == P::r) return D == 2 ? A + 3 : B + 3;
+    if (r < P::u) return B + (r - P::m);
+    if (r < P::Rpsi) return A + (r - P::u);
+    return A + D;
+}
+template <int D>
+__device__ __forceinline__ const float* geo_addr(const Args<float>& g, int r, int f) {
+    const float* g0 = reinterpret_cast<const float*>(g.fG0 + f);
+    const float* g1 = reinterpret_cast<const float*>(g.fG1 + f);
+    if (r <= D) return g0 + r;                 // S, w
+    if (r <= 2 * D) return g1 + (r - D - 1);   // K
+    return D == 2 ? g0 + 3 : g1 + 3;           // lapc
+}
+template <int D>
+__device__ __forceinline__ int face_P(const Args<float>& g, int f) {
+    return D == 2 ? __float_as_int(g.fG1[f].z) : g.fP[f];
+}
+template <int D>
+__device__ __forceinline__ int face_N(const Args<float>& g, int f) {   // with the boundary flag
+    return D == 2 ? __float_as_int(g.fG1[f].w) : g.fN[f];
+}
+
+// The rhs of a staged face: view v's rows of cells i and j, face column f.
+template <int D, int SCH, class View>
+__device__ __forceinline__ void staged_rhs(const View& v, int f, int i, int j, float* rhs) {
+    using P = PRow<D>;
+    Face32<D> geo;
+    Prim32<D> p[2];
+    const int at[2] = {i, j};
+#pragma unroll
+    for (int s = 0; s < 2; ++s) {
+        p[s].r = v.prim[P::r * v.nt + at[s]];
+        p[s].R = v.prim[P::Rpsi * v.nt + at[s]];
+#pragma unroll
+        for (int k = 0; k < D; ++k) {
+            p[s].m[k] = v.prim[(P::m + k) * v.nt + at[s]];
+            p[s].u[k] = v.prim[(P::u + k) * v.nt + at[s]];
+        }
+    }
+#pragma unroll
+    for (int k = 0; k < D; ++k) {
+        geo.S[k] = v.S[k * v.nf + f];
+        geo.K[k] = v.K[k * v.nf + f];
+    }
+    geo.w = v.w[f];
+    geo.lapc = v.lapc[f];
+    face_rhs32_core<D, SCH, true, false, false>(
+        v, f, i, j, v.fGhost[f] != 0, geo, p[0], p[1],
+        [&](float* Vi, float* Vj) {
+#pragma unroll
+            for (int r = 0; r < kVisRows<D>; ++r) {
+                Vi[r] = v.V[r * v.nt + i];
+                Vj[r] = v.V[r * v.nt + j];
+            }
+        },
+        rhs);
+}
+
 template <int D>
 struct StagedRows {
     static constexpr int PR = 2 * D + 2;        // the primitives the M1 / M2 flux reads (no c)
@@ -67,7 +138,7 @@ struct StagedRows {
     __host__ __device__ static constexpr int floats(int F) { return (2 * (PR + VR) + FR + GR) * F + F / 4; }
 };
 
-// The arrays face_rhs32_cells reads, pointing into one chunk's buffer.
+// The arrays staged_rhs reads, pointing into one chunk's buffer.
 struct StagedFace32 {
     const RefState32& ref;
     const float* prim;
@@ -95,22 +166,20 @@ __device__ __forceinline__ void stage_face(const Args<float>& g, float* b, int F
     float* fb = b + 2 * (R::PR + R::VR) * F;
 #pragma unroll
     for (int r = 0; r < R::PR; ++r) {
-        cp_async4(cb + r * 2 * F + t, g.prim + r * nt + i);
-        cp_async4(cb + r * 2 * F + F + t, g.prim + r * nt + j);
+        cp_async4(cb + r * 2 * F + t, prim_addr<D>(g, r, i));
+        cp_async4(cb + r * 2 * F + F + t, prim_addr<D>(g, r, j));
     }
 #pragma unroll
-    for (int k = 0; k < D; ++k) cp_async4(fb + k * F + t, g.S + k * nf + f);
-    cp_async4(fb + D * F + t, g.w + f);
+    for (int k = 0; k <= D; ++k) cp_async4(fb + k * F + t, geo_addr<D>(g, k, f));
     if (vis) {
 #pragma unroll
-        for (int k = 0; k < D; ++k) cp_async4(fb + (D + 1 + k) * F + t, g.K + k * nf + f);
-        cp_async4(fb + (2 * D + 1) * F + t, g.lapc + f);
+        for (int k = D + 1; k < 2 * D + 2; ++k) cp_async4(fb + k * F + t, geo_addr<D>(g, k, f));
         if (!ghost) {
             float* vb = cb + R::PR * 2 * F;
 #pragma unroll
             for (int r = 0; r < R::VR; ++r) {
-                cp_async4(vb + r * 2 * F + t, g.V + r * nt + i);
-                cp_async4(vb + r * 2 * F + F + t, g.V + r * nt + j);
+                cp_async4(vb + r * 2 * F + t, g.V + (size_t)i * kVisStride<D, false> + r);
+                cp_async4(vb + r * 2 * F + F + t, g.V + (size_t)j * kVisStride<D, false> + r);
             }
         } else {
             cp_async4(fb + R::FR * F + t, g.dinv + f);
@@ -139,9 +208,10 @@ __global__ void __launch_bounds__(256) k_flux32_staged(const __grid_constant__ A
     auto loadIdx = [&](int k) {
         const int f = faceOf(k);
         if (k < n && f < nf) {
-            ni = g.fP[f];
-            nj = g.fN[f];
-            ng = g.fGhost[f];
+            const int n = face_N<D>(g, f);
+            ni = face_P<D>(g, f);
+            nj = n & 0x7fffffff;
+            ng = n < 0 ? 1 : 0;
         }
     };
     auto issue = [&](int k) {
@@ -179,9 +249,8 @@ __global__ void __launch_bounds__(256) k_flux32_staged(const __grid_constant__ A
                                  2 * F,
                                  F};
             float rhs[D + 2];
-            face_rhs32_cells<D, SCH, true, false, false>(v, t, t, F + t, rhs);
-#pragma unroll
-            for (int q = 0; q < D + 2; ++q) g.flux[(size_t)q * (size_t)nf + f] = rhs[q];
+            staged_rhs<D, SCH>(v, t, t, F + t, rhs);
+            store_flux<D>(g, f, rhs);
         }
     }
     cp_async_wait<0>();   // no copy outlives the block
@@ -203,7 +272,7 @@ struct SlotRows {
     static constexpr int N = CELL + FACE;        // boundary faces keep 1/|d|, d/|d| in the V rows' place
 };
 
-// A face's values in registers, read by face_rhs32_cells with i = 0, j = 1, f = 0.
+// A face's values in registers, read by staged_rhs with i = 0, j = 1, f = 0.
 template <int D>
 struct RegFace32 {
     const RefState32& ref;
@@ -225,23 +294,21 @@ __device__ __forceinline__ void slot_issue(const Args<float>& g, float* slot, in
     constexpr int B = 256;   // threads of a block: the slot's row stride
 #pragma unroll
     for (int r = 0; r < R::PR; ++r) {
-        cp_async4(slot + (2 * r) * B, g.prim + r * nt + i);
-        cp_async4(slot + (2 * r + 1) * B, g.prim + r * nt + j);
+        cp_async4(slot + (2 * r) * B, prim_addr<D>(g, r, i));
+        cp_async4(slot + (2 * r + 1) * B, prim_addr<D>(g, r, j));
     }
     float* fb = slot + R::CELL * B;
 #pragma unroll
-    for (int k = 0; k < D; ++k) cp_async4(fb + k * B, g.S + k * nf + f);
-    cp_async4(fb + D * B, g.w + f);
+    for (int k = 0; k <= D; ++k) cp_async4(fb + k * B, geo_addr<D>(g, k, f));
     if (vis) {
 #pragma unroll
-        for (int k = 0; k < D; ++k) cp_async4(fb + (D + 1 + k) * B, g.K + k * nf + f);
-        cp_async4(fb + (2 * D + 1) * B, g.lapc + f);
+        for (int k = D + 1; k < 2 * D + 2; ++k) cp_async4(fb + k * B, geo_addr<D>(g, k, f));
         float* vb = slot + 2 * R::PR * B;
         if (!ghost) {
 #pragma unroll
             for (int r = 0; r < R::VR; ++r) {
-                cp_async4(vb + (2 * r) * B, g.V + r * nt + i);
-                cp_async4(vb + (2 * r + 1) * B, g.V + r * nt + j);
+                cp_async4(vb + (2 * r) * B, g.V + (size_t)i * kVisStride<D, false> + r);
+                cp_async4(vb + (2 * r + 1) * B, g.V + (size_t)j * kVisStride<D, false> + r);
             }
         } else {
             cp_async4(vb, g.dinv + f);
@@ -288,15 +355,17 @@ __global__ void __launch_bounds__(256, D == 2 ? 4 : 3) k_flux32_slot(const __gri
     const bool vis = g.ref.mu != 0.0f;
     int f = LFM_GLOBAL_ID();
     if (f >= nf) return;
-    bool gh = g.fGhost[f] != 0;
-    slot_issue<D>(g, slot, f, g.fP[f], g.fN[f], gh, vis);
+    const int n0 = face_N<D>(g, f);
+    bool gh = n0 < 0;
+    slot_issue<D>(g, slot, f, face_P<D>(g, f), n0 & 0x7fffffff, gh, vis);
     cp_async_commit();
     int fn = f + stride, ni = 0, nj = 0;
     bool ngh = false;
     if (fn < nf) {
-        ni = g.fP[fn];
-        nj = g.fN[fn];
-        ngh = g.fGhost[fn] != 0;
+        const int n = face_N<D>(g, fn);
+        ni = face_P<D>(g, fn);
+        nj = n & 0x7fffffff;
+        ngh = n < 0;
     }
     for (; f < nf; f += stride) {
         cp_async_wait<0>();   // face f is in the slot
@@ -314,14 +383,14 @@ __global__ void __launch_bounds__(256, D == 2 ? 4 : 3) k_flux32_slot(const __gri
         gh = ngh;
         const int fnn = fn + stride;
         if (fnn < nf) {
-            ni = g.fP[fnn];
-            nj = g.fN[fnn];
-            ngh = g.fGhost[fnn] != 0;
+            const int n = face_N<D>(g, fnn);
+            ni = face_P<D>(g, fnn);
+            nj = n & 0x7fffffff;
+            ngh = n < 0;
         }
         float rhs[D + 2];
-        face_rhs32_cells<D, SCH, true, false, false>(v, 0, 0, 1, rhs);
-#pragma unroll
-        for (int q = 0; q < D + 2; ++q) g.flux[(size_t)q * (size_t)nf + f] = rhs[q];
+        staged_rhs<D, SCH>(v, 0, 0, 1, rhs);
+        store_flux<D>(g, f, rhs);
         fn = fnn;
     }
     cp_async_wait<0>();

@@ -177,6 +177,10 @@ __device__ __forceinline__ T p5neg(T M, T alpha) {
     return T(0.5) * (M - fabs(M)) / M;
 }
 
+// x component of the area vector of face f.
+__device__ __forceinline__ double face_sx(const Args<double>& a, int f) { return a.S[f]; }
+__device__ __forceinline__ double face_sx(const Args<float>& a, int f) { return (double)a.fG0[f].x; }
+
 // Ghost state qv of ghost g from the conservative state qi of its interior
 // cell (FP64): the boundary condition of set_boundary_conditions
 // (src/cfd_v0.cpp:1009-1221).
@@ -191,7 +195,7 @@ __device__ __forceinline__ void ghost_bc(const Args<T>& a, int g, const double* 
         qv[D + 1] = qi[D + 1];
     } else if (kind >= 2 && kind <= 4) {
         bool inlet = (kind == 2);
-        if (kind == 4) inlet = (double)a.S[a.gFace[g]] <= 0.0;  // free stream along +x enters
+        if (kind == 4) inlet = face_sx(a, a.gFace[g]) <= 0.0;  // free stream along +x enters
         // The reference's expressions (TInt = pInt / (R rhoInt),
         // rhoExt = rhoInt TInt / TInf, rhoExt EExt with EExt = p / (rhoExt
         // (gamma - 1)) + |u|^2 / 2) with the divisions that cancel left out

@@ -37,13 +37,196 @@
 namespace lfm {
 namespace dev {
 
-// Row of the FP32 primitive array (rho', m'[D], u'[D], R psi', c).
+// ---------------------------------------------------------------------------
+// Layout. What a thread reads of one cell, ghost or face lies together, in
+// 16-byte parts, so that a gather is one to six vector loads where rows of
+// single values take 6 to 15 loads with their address arithmetic (a 2D viscous
+// face: 10 loads instead of 37):
+//   prim   [nt] float4 A, then [nt] B, then [nt] c (sound speed, M2AUSM only)
+//          2D: A = u'[2], R psi', rho'   B = m'[2]
+//          3D: A = u'[3], R psi'         B = m'[3], rho'
+//          (the viscous pass reads A alone)
+//   V      [nt] kVisStride floats: dudx, dTdx, sigmaU, then the LES stress
+//   grad   [nt] kGradStride floats: rho, p, u gradients
+//   flux   [nf] float4: the first four rhs, then (3D) [nf] the fifth
+//   fG0    [nf] float4  2D: S[2], w, |delta|/|d|   3D: S[3], w
+//   fG1    [nf] float4  2D: K[2], P, N (integers)  3D: K[3], |delta|/|d|
+//   fN, N  the N side, its top bit set on boundary faces
+//   cfEll, cfEllN  [nc][kEllWidth]: a cell's face entries and the cells across
+// Values and their order of evaluation do not depend on the layout. The kernels
+// wait for loads (ncu: long scoreboard), so what counts is the bytes a thread
+// has in flight and the round trips it makes. Measured on GB300 against rows
+// of single values, us a step: 768 x 512 M1 cylinder (in L2) 184 -> 164, of it
+// the flux 72 -> 54; 331 x 217 M2AUSM cylinder 118 -> 101; 192 x 128 x 48 wake
+// (HBM) 986 -> 920; 256 x 256 vortex 51 -> 45.
+// ---------------------------------------------------------------------------
 template <int D>
-struct PRow {
-    static constexpr int r = 0, m = 1, u = 1 + D, Rpsi = 1 + 2 * D, c = 2 + 2 * D;
+struct Prim32 {
+    float r, m[D], u[D], R;   // rho', m', u', R psi'
 };
 
-__device__ __forceinline__ float ld(const float* p, int row, size_t nt, int i) { return p[(size_t)row * nt + i]; }
+template <int D>
+struct Face32 {
+    float S[D], w, K[D], lapc;
+};
+
+template <int D, bool LES>
+constexpr int kVisStride = visStride32(D, LES);
+template <int D>
+constexpr int kGradStride = gradStride32(D);
+
+// Floats from the start of prim to its B part and to its sound speeds.
+__device__ __forceinline__ size_t prim_b(size_t nt) { return 4 * nt; }
+template <int D>
+__device__ __forceinline__ size_t prim_c(size_t nt) {
+    return (size_t)(2 * D + 2) * nt;
+}
+
+template <int D>
+__device__ __forceinline__ void load_prim(const Args<float>& a, int t, Prim32<D>& p) {
+    const float4 A = reinterpret_cast<const float4*>(a.prim)[t];
+    const float* b = a.prim + prim_b((size_t)a.nt);
+    p.u[0] = A.x;
+    p.u[1] = A.y;
+    if constexpr (D == 2) {
+        const float2 B = reinterpret_cast<const float2*>(b)[t];
+        p.R = A.z;
+        p.r = A.w;
+        p.m[0] = B.x;
+        p.m[1] = B.y;
+    } else {
+        const float4 B = reinterpret_cast<const float4*>(b)[t];
+        p.u[2] = A.z;
+        p.R = A.w;
+        p.m[0] = B.x;
+        p.m[1] = B.y;
+        p.m[2] = B.z;
+        p.r = B.w;
+    }
+}
+
+// u' and R psi' of cell t (and rho' in 2D).
+template <int D>
+__device__ __forceinline__ void load_uR(const Args<float>& a, int t, float* u, float& R) {
+    const float4 A = reinterpret_cast<const float4*>(a.prim)[t];
+    u[0] = A.x;
+    u[1] = A.y;
+    if constexpr (D == 2) {
+        R = A.z;
+    } else {
+        u[2] = A.z;
+        R = A.w;
+    }
+}
+
+template <int D>
+__device__ __forceinline__ void store_prim(const Args<float>& a, float* dst, int t, const Prim32<D>& p) {
+    float* b = dst + prim_b((size_t)a.nt);
+    if constexpr (D == 2) {
+        reinterpret_cast<float4*>(dst)[t] = make_float4(p.u[0], p.u[1], p.R, p.r);
+        reinterpret_cast<float2*>(b)[t] = make_float2(p.m[0], p.m[1]);
+    } else {
+        reinterpret_cast<float4*>(dst)[t] = make_float4(p.u[0], p.u[1], p.u[2], p.R);
+        reinterpret_cast<float4*>(b)[t] = make_float4(p.m[0], p.m[1], p.m[2], p.r);
+    }
+}
+
+template <int N>
+__device__ __forceinline__ void load_vec4(const float* p, float* out) {
+#pragma unroll
+    for (int k = 0; k < N / 4; ++k) {
+        const float4 x = reinterpret_cast<const float4*>(p)[k];
+        out[4 * k] = x.x;
+        out[4 * k + 1] = x.y;
+        out[4 * k + 2] = x.z;
+        out[4 * k + 3] = x.w;
+    }
+}
+template <int N>
+__device__ __forceinline__ void store_vec4(float* p, const float* v) {
+#pragma unroll
+    for (int k = 0; k < N / 4; ++k)
+        reinterpret_cast<float4*>(p)[k] = make_float4(v[4 * k], v[4 * k + 1], v[4 * k + 2], v[4 * k + 3]);
+}
+
+// Viscous rows of a cell: kVisRows values, padded to whole float4 (3D: 16).
+template <int D>
+constexpr int kVisVec = D == 2 ? 8 : 16;
+template <int D, bool LES>
+__device__ __forceinline__ void load_vis(const Args<float>& a, int t, float* v) {
+    load_vec4<kVisVec<D>>(a.V + (size_t)t * kVisStride<D, LES>, v);
+}
+
+// Face f: geometry, and its cells i (P) and j (N); ghost: a boundary face.
+template <int D>
+__device__ __forceinline__ void load_face(const Args<float>& a, int f, Face32<D>& g, int& i, int& j, bool& ghost) {
+    const float4 g0 = a.fG0[f], g1 = a.fG1[f];
+    int n;
+    g.S[0] = g0.x;
+    g.S[1] = g0.y;
+    g.K[0] = g1.x;
+    g.K[1] = g1.y;
+    if constexpr (D == 2) {
+        g.w = g0.z;
+        g.lapc = g0.w;
+        i = __float_as_int(g1.z);
+        n = __float_as_int(g1.w);
+    } else {
+        g.S[2] = g0.z;
+        g.w = g0.w;
+        g.K[2] = g1.z;
+        g.lapc = g1.w;
+        i = a.fP[f];
+        n = a.fN[f];
+    }
+    ghost = n < 0;
+    j = n & 0x7fffffff;
+}
+
+// S and w of face f.
+template <int D>
+__device__ __forceinline__ float load_Sw(const Args<float>& a, int f, float* S) {
+    const float4 g0 = a.fG0[f];
+    S[0] = g0.x;
+    S[1] = g0.y;
+    if constexpr (D == 2) {
+        return g0.z;
+    } else {
+        S[2] = g0.z;
+        return g0.w;
+    }
+}
+
+// The kEllWidth entries of cell c in a fixed-width table.
+template <int D>
+__device__ __forceinline__ void load_ell(const int* table, int c, int* out) {
+    if constexpr (D == 2) {
+        const int4 x = reinterpret_cast<const int4*>(table)[c];
+        out[0] = x.x;
+        out[1] = x.y;
+        out[2] = x.z;
+        out[3] = x.w;
+    } else {
+        const int2* p = reinterpret_cast<const int2*>(table) + 3 * (size_t)c;
+#pragma unroll
+        for (int k = 0; k < 3; ++k) {
+            const int2 x = p[k];
+            out[2 * k] = x.x;
+            out[2 * k + 1] = x.y;
+        }
+    }
+}
+
+template <int D>
+__device__ __forceinline__ void load_flux(const Args<float>& a, int f, float* v) {
+    load_vec4<4>(a.flux + 4 * (size_t)f, v);
+    if constexpr (D == 3) v[4] = a.flux[4 * (size_t)a.nf + f];
+}
+template <int D>
+__device__ __forceinline__ void store_flux(const Args<float>& a, int f, const float* v) {
+    store_vec4<4>(a.flux + 4 * (size_t)f, v);
+    if constexpr (D == 3) a.flux[4 * (size_t)a.nf + f] = v[4];
+}
 
 // p - p_ref of a state with perturbations r', R psi':
 // rho R psi - rho_inf R psi_inf = rho_inf R psi' + r' (R psi_inf + R psi').
@@ -58,7 +241,6 @@ __device__ __forceinline__ float pressure_dev(const RefState32& R, float r, floa
 // ---------------------------------------------------------------------------
 template <int D>
 __device__ __forceinline__ void prims32(const Args<float>& a, int t, const double* qp, float* dst) {
-    using P = PRow<D>;
     const RefState32& R = a.ref;
     const size_t nt = (size_t)a.nt;
     const float r = f64_to_f32(qp[0]);
@@ -80,14 +262,16 @@ __device__ __forceinline__ void prims32(const Args<float>& a, int t, const doubl
     const float K = __fmaf_rn(rho, __fmaf_rn(0.5f, uu, Uu), __fmul_rn(__fmul_rn(0.5f, r), U2));
     const float p = __fmul_rn(R.gm1, __fsub_rn(E, K));            // p - p_ref
     const float Rpsi = __fmul_rn(__fmaf_rn(-R.Rpsi, r, p), rinv);  // p/rho - p_ref/rho_inf
-    dst[(size_t)P::r * nt + t] = r;
+    Prim32<D> p32;
+    p32.r = r;
+    p32.R = Rpsi;
 #pragma unroll
     for (int k = 0; k < D; ++k) {
-        dst[(size_t)(P::m + k) * nt + t] = m[k];
-        dst[(size_t)(P::u + k) * nt + t] = u[k];
+        p32.m[k] = m[k];
+        p32.u[k] = u[k];
     }
-    dst[(size_t)P::Rpsi * nt + t] = Rpsi;
-    dst[(size_t)P::c * nt + t] = __fsqrt_rn(__fmul_rn(R.gamma, __fadd_rn(R.Rpsi, Rpsi)));
+    store_prim<D>(a, dst, t, p32);
+    if (a.primC) dst[prim_c<D>(nt) + t] = __fsqrt_rn(__fmul_rn(R.gamma, __fadd_rn(R.Rpsi, Rpsi)));
 }
 
 // ---------------------------------------------------------------------------
@@ -100,24 +284,23 @@ __device__ __forceinline__ void prims32(const Args<float>& a, int t, const doubl
 template <int D>
 __device__ __forceinline__ void ghost32(const Args<float>& a, int g, const double* qi, float* dst) {
     constexpr int NQ = D + 2;
-    using P = PRow<D>;
-    const size_t nt = (size_t)a.nt;
     const int t = a.nc + g;
     double qv[NQ];
     ghost_bc<float, D>(a, g, qi, qv);
     const double rinv = rcp64(qv[0]);
     double ke = 0.0;
-    dst[(size_t)P::r * nt + t] = (float)(qv[0] - a.qRef[0]);
+    Prim32<D> p32;
+    p32.r = (float)(qv[0] - a.qRef[0]);
 #pragma unroll
     for (int k = 0; k < D; ++k) {
-        dst[(size_t)(P::m + k) * nt + t] = (float)(qv[k + 1] - a.qRef[k + 1]);
-        dst[(size_t)(P::u + k) * nt + t] = (float)(qv[k + 1] * rinv - a.UInf[k]);
+        p32.m[k] = (float)(qv[k + 1] - a.qRef[k + 1]);
+        p32.u[k] = (float)(qv[k + 1] * rinv - a.UInf[k]);
         ke += qv[k + 1] * qv[k + 1];
     }
     const double p = a.gm1 * (qv[D + 1] - 0.5 * ke * rinv);
-    const float Rpsi = (float)(p * rinv - a.RpsiRef);
-    dst[(size_t)P::Rpsi * nt + t] = Rpsi;
-    dst[(size_t)P::c * nt + t] = sqrtf(a.ref.gamma * (a.ref.Rpsi + Rpsi));
+    p32.R = (float)(p * rinv - a.RpsiRef);
+    store_prim<D>(a, dst, t, p32);
+    if (a.primC) dst[prim_c<D>((size_t)a.nt) + t] = sqrtf(a.ref.gamma * (a.ref.Rpsi + p32.R));
 }
 
 // ---------------------------------------------------------------------------
@@ -127,7 +310,6 @@ __device__ __forceinline__ void ghost32(const Args<float>& a, int g, const doubl
 template <int D>
 __device__ __forceinline__ void prep32(const Args<float>& a, int t) {
     constexpr int NQ = D + 2;
-    using P = PRow<D>;
     const size_t nt = (size_t)a.nt;
     if (t < a.nc || t >= a.nc + a.ng) {
         double qp[NQ];
@@ -168,57 +350,59 @@ __device__ __forceinline__ void ghosts_of32(const Args<float>& a, int c, const d
     double qa[NQ];
 #pragma unroll
     for (int v = 0; v < NQ; ++v) qa[v] = qp[v] + a.qRef[v];
-    for_ghosts<float, D>(a, c, [&](int j) { ghost32<D>(a, j - a.nc, qa, dst); });
+    if (a.cfEllN) {
+        constexpr int W = kEllWidth<D>;
+        int nb[W];
+        load_ell<D>(a.cfEllN, c, nb);
+#pragma unroll 1
+        for (int k = 0; k < W; ++k) {
+            int j = nb[0];
+#pragma unroll
+            for (int m = 1; m < W; ++m) j = k == m ? nb[m] : j;
+            if (j >= a.nc && j < a.nc + a.ng) ghost32<D>(a, j - a.nc, qa, dst);
+        }
+    } else {
+        for_ghosts<float, D>(a, c, [&](int j) { ghost32<D>(a, j - a.nc, qa, dst); });
+    }
 }
 
-// gather32: the face rhs sum of cell c (ascending face order).
+// gather32: the face rhs sum of cell c (ascending face order). The face's sign
+// (+ where c is P, - where N) is a sign-bit flip of the loaded value, so an
+// entry costs one add (a - b is a + (-b) in IEEE arithmetic: the same bits).
 template <int D>
 __device__ __forceinline__ void gather32(const Args<float>& a, int c, float* sum) {
     constexpr int NQ = D + 2;
-    const size_t nf = (size_t)a.nf;
 #pragma unroll
     for (int v = 0; v < NQ; ++v) sum[v] = 0.0f;
     for (int e = a.cfOff[c]; e < a.cfOff[c + 1]; ++e) {
         const int code = a.cfList[e];
-        if (code >= 0) {
+        float x[NQ];
+        load_flux<D>(a, code >= 0 ? code : ~code, x);
 #pragma unroll
-            for (int v = 0; v < NQ; ++v) sum[v] += a.flux[v * nf + code];
-        } else {
-            const int f = ~code;
-#pragma unroll
-            for (int v = 0; v < NQ; ++v) sum[v] -= a.flux[v * nf + f];
-        }
+        for (int v = 0; v < NQ; ++v) sum[v] += code >= 0 ? x[v] : neg_bits(x[v]);
     }
 }
 
 // gather32_ell: gather32 through the fixed-width table. Every face index of
-// the cell is loaded at once (coalesced rows), then every flux value, so the
-// gather costs two memory round trips instead of one per face; the sum runs
-// in the same (ascending face) order, so it has gather32's bits.
+// the cell is loaded at once, then every face's rhs, so the gather costs two
+// memory round trips instead of one per face; the sum runs in the same
+// (ascending face) order, so it has gather32's bits.
 template <int D>
 __device__ __forceinline__ void gather32_ell(const Args<float>& a, int c, float* sum) {
     constexpr int NQ = D + 2, W = kEllWidth<D>;
-    const size_t nf = (size_t)a.nf, nc = (size_t)a.nc;
     int code[W];
+    load_ell<D>(a.cfEll, c, code);
+    float x[W][NQ];
 #pragma unroll
-    for (int k = 0; k < W; ++k) code[k] = a.cfEll[k * nc + c];
-    float fl[W][NQ];
-#pragma unroll
-    for (int k = 0; k < W; ++k) {
-        const int f = code[k] >= 0 ? code[k] : ~code[k];
-#pragma unroll
-        for (int v = 0; v < NQ; ++v) {   // the face's sign as a sign-bit flip: one add per entry
-            const float x = code[k] != kEllPad ? a.flux[v * nf + f] : 0.0f;
-            fl[k][v] = code[k] >= 0 ? x : neg_bits(x);
-        }
-    }
+    for (int k = 0; k < W; ++k)
+        if (code[k] != kEllPad) load_flux<D>(a, code[k] >= 0 ? code[k] : ~code[k], x[k]);
 #pragma unroll
     for (int v = 0; v < NQ; ++v) sum[v] = 0.0f;
 #pragma unroll
     for (int k = 0; k < W; ++k) {
         if (code[k] == kEllPad) continue;
 #pragma unroll
-        for (int v = 0; v < NQ; ++v) sum[v] += fl[k][v];
+        for (int v = 0; v < NQ; ++v) sum[v] += code[k] >= 0 ? x[k][v] : neg_bits(x[k][v]);
     }
 }
 
@@ -308,78 +492,74 @@ __device__ __forceinline__ void to_perturbation(const Args<float>& a, const doub
     for (int v = 0; v < D + 2; ++v) a.q[(size_t)v * a.nt + c] = q[(size_t)v * stride + c] - a.qRef[v];
 }
 
+// Calls f(code, o) for every face entry of cell c in ascending face order
+// (code: the face, one's complement where c is N; o: the cell across): through
+// the fixed-width tables (ELL), unrolled so that the entries' loads overlap, or
+// the face list.
+template <int D, bool ELL, class F>
+__device__ __forceinline__ void for_entries32(const Args<float>& a, int c, F f) {
+    if constexpr (ELL) {
+        constexpr int W = kEllWidth<D>;
+        int code[W], nb[W];
+        load_ell<D>(a.cfEll, c, code);
+        load_ell<D>(a.cfEllN, c, nb);
+#pragma unroll
+        for (int k = 0; k < W; ++k)
+            if (code[k] != kEllPad) f(code[k], nb[k]);
+    } else {
+        for (int e = a.cfOff[c]; e < a.cfOff[c + 1]; ++e) f(a.cfList[e], a.cfNbr[e]);
+    }
+}
+
 // ---------------------------------------------------------------------------
 // grad32: Gauss gradients of rho', p' and u' (those of rho, p and u up to
 // the reference state's closed-cell sum) for M2AUSM's minmod reconstruction.
 // ---------------------------------------------------------------------------
-template <int D>
+template <int D, bool ELL>
 __device__ __forceinline__ void grad32(const Args<float>& a, int c) {
-    using P = PRow<D>;
     const RefState32& R = a.ref;
-    const size_t nt = (size_t)a.nt, nf = (size_t)a.nf;
-    float gr[D], gp[D], gu[D][D];
+    float G[kGradStride<D>];   // rho, p, u gradients
 #pragma unroll
-    for (int k = 0; k < D; ++k) {
-        gr[k] = gp[k] = 0.0f;
-#pragma unroll
-        for (int l = 0; l < D; ++l) gu[k][l] = 0.0f;
-    }
+    for (int k = 0; k < kGradStride<D>; ++k) G[k] = 0.0f;
     const float vi = a.volInv32[c];
-    // the cell's own primitives once; the cell across each face from the
-    // face list's neighbour column (P and N sides kept for the interpolation)
-    float cu[D];
-#pragma unroll
-    for (int k = 0; k < D; ++k) cu[k] = ld(a.prim, P::u + k, nt, c);
-    const float cr = ld(a.prim, P::r, nt, c);
-    const float cpr = pressure_dev(R, cr, ld(a.prim, P::Rpsi, nt, c));
-    for (int e = a.cfOff[c]; e < a.cfOff[c + 1]; ++e) {
-        const int code = a.cfList[e];
-        const int o = a.cfNbr[e];
+    Prim32<D> self;
+    load_prim<D>(a, c, self);
+    const float cpr = pressure_dev(R, self.r, self.R);
+    for_entries32<D, ELL>(a, c, [&](int code, int o) {
         const bool own = code >= 0;   // c is the face's P side
-        const int f = own ? code : ~code;
-        const float w = a.w[f];
-        float ou[D];
-#pragma unroll
-        for (int k = 0; k < D; ++k) ou[k] = ld(a.prim, P::u + k, nt, o);
-        const float orr = ld(a.prim, P::r, nt, o);
-        const float opr = pressure_dev(R, orr, ld(a.prim, P::Rpsi, nt, o));
-        float so[D], uu[D];
+        float S[D], uu[D];
+        const float w = load_Sw<D>(a, own ? code : ~code, S);
+        Prim32<D> oth;
+        load_prim<D>(a, o, oth);
+        const float opr = pressure_dev(R, oth.r, oth.R);
+        float so[D];
 #pragma unroll
         for (int k = 0; k < D; ++k) {
-            const float Sk = a.S[(size_t)k * nf + f];
-            so[k] = own ? Sk * vi : -Sk * vi;
-            uu[k] = own ? interp(w, cu[k], ou[k]) : interp(w, ou[k], cu[k]);
+            so[k] = own ? S[k] * vi : -S[k] * vi;
+            uu[k] = own ? interp(w, self.u[k], oth.u[k]) : interp(w, oth.u[k], self.u[k]);
         }
-        const float ri = own ? cr : orr, rj = own ? orr : cr;
+        const float ri = own ? self.r : oth.r, rj = own ? oth.r : self.r;
         const float pi = own ? cpr : opr;
         const float pj = own ? opr : cpr;
         const float rho = interp(w, ri, rj);
         const float p = interp(w, pi, pj);
 #pragma unroll
         for (int x = 0; x < D; ++x) {
-            gp[x] += p * so[x];
-            gr[x] += rho * so[x];
+            G[D + x] += p * so[x];
+            G[x] += rho * so[x];
 #pragma unroll
-            for (int b = 0; b < D; ++b) gu[b][x] += uu[b] * so[x];
+            for (int b = 0; b < D; ++b) G[2 * D + b * D + x] += uu[b] * so[x];
         }
-    }
-#pragma unroll
-    for (int k = 0; k < D; ++k) {
-        a.grad[(size_t)k * nt + c] = gr[k];
-        a.grad[(size_t)(D + k) * nt + c] = gp[k];
-#pragma unroll
-        for (int l = 0; l < D; ++l) a.grad[(size_t)(2 * D + k * D + l) * nt + c] = gu[k][l];
-    }
+    });
+    store_vec4<kGradStride<D>>(a.grad + (size_t)c * kGradStride<D>, G);
 }
 
 // ---------------------------------------------------------------------------
 // vis32: dudx and dTdx from u' and T', sigmaU = (U_inf + u') . tau.
 // ---------------------------------------------------------------------------
 // LES compiles in the Smagorinsky SGS stress (cases with a.smagC).
-template <int D, bool LES = false>
+template <int D, bool LES, bool ELL>
 __device__ __forceinline__ void vis32(const Args<float>& a, int c) {
-    using P = PRow<D>;
-    const size_t nt = (size_t)a.nt, nf = (size_t)a.nf;
     float g[D][D], gT[D];
 #pragma unroll
     for (int k = 0; k < D; ++k) {
@@ -389,27 +569,18 @@ __device__ __forceinline__ void vis32(const Args<float>& a, int c) {
     }
     const float vi = a.volInv32[c];
     const float Rinv = a.ref.Rinv;
-    // the cell's own primitives once; the cell across each face from the
-    // face list's neighbour column (P and N sides kept for the interpolation)
-    float cu[D];
-#pragma unroll
-    for (int k = 0; k < D; ++k) cu[k] = ld(a.prim, P::u + k, nt, c);
-    const float cR = ld(a.prim, P::Rpsi, nt, c);
-    for (int e = a.cfOff[c]; e < a.cfOff[c + 1]; ++e) {
-        const int code = a.cfList[e];
-        const int o = a.cfNbr[e];
+    float cu[D], cR;
+    load_uR<D>(a, c, cu, cR);
+    for_entries32<D, ELL>(a, c, [&](int code, int o) {
         const bool own = code >= 0;   // c is the face's P side
-        const int f = own ? code : ~code;
-        const float w = a.w[f];
-        float so[D], fU[D];
+        float S[D], ou[D], oR, so[D], fU[D];
+        const float w = load_Sw<D>(a, own ? code : ~code, S);
+        load_uR<D>(a, o, ou, oR);
 #pragma unroll
         for (int k = 0; k < D; ++k) {
-            const float Sk = a.S[(size_t)k * nf + f];
-            const float ouk = ld(a.prim, P::u + k, nt, o);
-            so[k] = own ? Sk * vi : -Sk * vi;
-            fU[k] = own ? interp(w, cu[k], ouk) : interp(w, ouk, cu[k]);
+            so[k] = own ? S[k] * vi : -S[k] * vi;
+            fU[k] = own ? interp(w, cu[k], ou[k]) : interp(w, ou[k], cu[k]);
         }
-        const float oR = ld(a.prim, P::Rpsi, nt, o);
         const float fT = (own ? interp(w, cR, oR) : interp(w, oR, cR)) * Rinv;
 #pragma unroll
         for (int x = 0; x < D; ++x) {
@@ -417,28 +588,36 @@ __device__ __forceinline__ void vis32(const Args<float>& a, int c) {
             for (int y = 0; y < D; ++y) g[x][y] += fU[x] * so[y];
             gT[x] += fT * so[x];
         }
-    }
+    });
     const float mu = a.ref.mu;
     float tau[D][D];
     stress<float, D>(g, mu, tau);
-    float U[D];
+    float U[D], out[kVisVec<D>];
 #pragma unroll
     for (int k = 0; k < D; ++k) U[k] = a.ref.U[k] + cu[k];
 #pragma unroll
     for (int x = 0; x < D; ++x) {
 #pragma unroll
-        for (int y = 0; y < D; ++y) a.V[(size_t)(x * D + y) * nt + c] = g[x][y];
-        a.V[(size_t)(D * D + x) * nt + c] = gT[x];
-        a.V[(size_t)(D * D + D + x) * nt + c] = dotv<float, D>(U, tau[x]);
+        for (int y = 0; y < D; ++y) out[x * D + y] = g[x][y];
+        out[D * D + x] = gT[x];
+        out[D * D + D + x] = dotv<float, D>(U, tau[x]);
     }
+#pragma unroll
+    for (int k = kVisRows<D>; k < kVisVec<D>; ++k) out[k] = 0.0f;
+    float* row = a.V + (size_t)c * kVisStride<D, LES>;
     if (LES && a.smagC) {   // Smagorinsky LES: the cell's SGS stress
         float sg[D][D];
         sgs_stress<float, D>(g, a.smagC[c], sg);
 #pragma unroll
         for (int x = 0; x < D; ++x)
 #pragma unroll
-            for (int y = 0; y < D; ++y) a.V[(size_t)(kVisRows<D> + x * D + y) * nt + c] = sg[x][y];
+            for (int y = 0; y < D; ++y) {
+                const int k = kVisRows<D> + x * D + y;
+                if (k < kVisVec<D>) out[k < kVisVec<D> ? k : 0] = sg[x][y];
+                else row[k] = sg[x][y];
+            }
     }
+    store_vec4<kVisVec<D>>(row, out);
 }
 
 // d(M) = p5pos(M) - p5neg(M) is, for |M| < 1, the odd polynomial
@@ -456,51 +635,29 @@ __device__ __forceinline__ float p5diff_dd(float a, float b, float alpha) {
 // viscous terms (linear in the gradients, so unchanged in form).
 // ---------------------------------------------------------------------------
 // VIS = false compiles the viscous terms out (for callers that know mu = 0).
-// EARLYV loads the viscous rows of both cells and the face's viscous geometry
-// together with the primitives, so the gathers overlap instead of following
-// one another (2 x 8 more live values in 2D, 2 x 15 in 3D): the stand-alone
-// flux kernel (3D flux 4.05 -> 3.43 ms per step on the 9.4M-cell wake, whose
+// EARLYV loads the viscous rows of both cells together with the primitives, so
+// the gathers overlap instead of following one another: the stand-alone flux
+// kernel (3D flux 4.05 -> 3.43 ms per step on the 9.4M-cell wake, whose
 // gathers come from HBM; 2 % in 2D, whose gathers hit L2). The fused kernels,
 // whose registers other phases already fill, keep the late loads.
 //
-// face_rhs32_cells takes the face's cells i (P) and j (N) as arguments and
-// reads every array through `a`: the solver's Args, or a view of the same
-// rows staged in shared memory (the staged flux kernel, flux_staged_fp32.cu),
-// which gives the same bits because only the addresses differ.
-template <int D, int SCH, bool VIS, bool LES, bool EARLYV, class A>
-__device__ __forceinline__ void face_rhs32_cells(const A& a, int f, int i, int j, float* rhs) {
-    using P = PRow<D>;
+// face_rhs32_core takes the face's geometry and both cells' primitives as
+// values and loadV(Vi, Vj), which fills their viscous rows; `a` gives the
+// constants and what only some faces read. So a caller that holds a cell's
+// values in registers, or reads them from shared memory (the staged flux
+// kernel, flux_staged_fp32.cu), gets the same bits.
+template <int D, int SCH, bool VIS, bool LES, bool EARLYV, class A, class LV>
+__device__ __forceinline__ void face_rhs32_core(const A& a, int f, int i, int j, bool ghost, const Face32<D>& geo,
+                                                const Prim32<D>& pi_, const Prim32<D>& pj_, LV loadV, float* rhs) {
     const RefState32& R = a.ref;
-    const size_t nt = (size_t)a.nt, nf = (size_t)a.nf;
-    const float w = a.w[f];
-    float S[D];
-#pragma unroll
-    for (int k = 0; k < D; ++k) S[k] = a.S[(size_t)k * nf + f];
-    const float ri = ld(a.prim, P::r, nt, i), rj = ld(a.prim, P::r, nt, j);
-    float mi[D], mj[D], ui[D], uj[D];
-#pragma unroll
-    for (int k = 0; k < D; ++k) {
-        mi[k] = ld(a.prim, P::m + k, nt, i);
-        mj[k] = ld(a.prim, P::m + k, nt, j);
-        ui[k] = ld(a.prim, P::u + k, nt, i);
-        uj[k] = ld(a.prim, P::u + k, nt, j);
-    }
-    const float Ri = ld(a.prim, P::Rpsi, nt, i), Rj = ld(a.prim, P::Rpsi, nt, j);
-    constexpr bool early = VIS && EARLYV;
-    constexpr int VR = early ? kVisRows<D> : 1;
-    float Vi[VR], Vj[VR], eK[early ? D : 1], eLapc = 0.0f;
-    if (early && a.ref.mu != 0.0f) {
-#pragma unroll
-        for (int k = 0; k < (early ? D : 1); ++k) eK[k] = a.K[(size_t)k * nf + f];
-        eLapc = a.lapc[f];
-        if (!a.fGhost[f]) {
-#pragma unroll
-            for (int r = 0; r < VR; ++r) {
-                Vi[r] = a.V[(size_t)r * nt + i];
-                Vj[r] = a.V[(size_t)r * nt + j];
-            }
-        }
-    }
+    const float w = geo.w;
+    const float* S = geo.S;
+    const float ri = pi_.r, rj = pj_.r, Ri = pi_.R, Rj = pj_.R;
+    const float *mi = pi_.m, *mj = pj_.m, *ui = pi_.u, *uj = pj_.u;
+    constexpr bool needV = VIS || SCH == kSchemeAUSM;
+    float Vi[needV ? kVisVec<D> : 1], Vj[needV ? kVisVec<D> : 1];
+    const bool visc = VIS && a.ref.mu != 0.0f;
+    if (needV && (SCH == kSchemeAUSM || (EARLYV && visc && !ghost))) loadV(Vi, Vj);
     // Face state: linear interpolation for M1, the mid-point for M2 / M2AUSM.
     const float wf = (SCH == kSchemeM1) ? w : 0.5f;
     const float rf = interp(wf, ri, rj);
@@ -539,33 +696,31 @@ __device__ __forceinline__ void face_rhs32_cells(const A& a, int f, int i, int j
         }
         Hf = 0.5f * (Hi + Hj);
     }
-    if (SCH == kSchemeAUSM) {
+    if constexpr (SCH == kSchemeAUSM) {
         // shock sensor, minmod reconstructions and AUSM+ pressure dissipation
         // (src/cfd_v0.cpp:2288-2339) on the perturbation variables; minmod is
         // invariant under a common shift of both sides.
-        const float cavg = 0.5f * (ld(a.prim, P::c, nt, i) + ld(a.prim, P::c, nt, j));
-        float d[D];
+        const float* pc = a.prim + prim_c<D>((size_t)a.nt);
+        const float cavg = 0.5f * (pc[i] + pc[j]);
+        float d[D], Gi[kGradStride<D>], Gj[kGradStride<D>];
 #pragma unroll
-        for (int k = 0; k < D; ++k) d[k] = a.d[(size_t)k * nf + f];
+        for (int k = 0; k < D; ++k) d[k] = a.d[(size_t)k * a.nf + f];
+        load_vec4<kGradStride<D>>(a.grad + (size_t)i * kGradStride<D>, Gi);
+        load_vec4<kGradStride<D>>(a.grad + (size_t)j * kGradStride<D>, Gj);
         float cdiv = 0.0f, ndiv = 0.0f, ccurl = 0.0f, ncurl = 0.0f, unPos = 0.0f, unNeg = 0.0f, dUn = 0.0f,
               norm = 0.0f;
 #pragma unroll
         for (int x = 0; x < D; ++x) {
-            cdiv += a.V[(size_t)(x * D + x) * nt + i];
-            ndiv += a.V[(size_t)(x * D + x) * nt + j];
+            cdiv += Vi[x * D + x];
+            ndiv += Vj[x * D + x];
 #pragma unroll
             for (int y = x + 1; y < D; ++y) {
-                const float cc = a.V[(size_t)(x * D + y) * nt + i] - a.V[(size_t)(y * D + x) * nt + i];
-                const float nn = a.V[(size_t)(x * D + y) * nt + j] - a.V[(size_t)(y * D + x) * nt + j];
+                const float cc = Vi[x * D + y] - Vi[y * D + x];
+                const float nn = Vj[x * D + y] - Vj[y * D + x];
                 ccurl += cc * cc;
                 ncurl += nn * nn;
             }
-            float gi[D], gj[D];
-#pragma unroll
-            for (int y = 0; y < D; ++y) {
-                gi[y] = a.grad[(size_t)(2 * D + x * D + y) * nt + i];
-                gj[y] = a.grad[(size_t)(2 * D + x * D + y) * nt + j];
-            }
+            const float *gi = Gi + 2 * D + x * D, *gj = Gj + 2 * D + x * D;
             const float uP = minmod_interp<float, D>(ui[x], uj[x], gi, d, w, 1.0f);
             const float uN = minmod_interp<float, D>(ui[x], uj[x], gj, d, w, -1.0f);
             unPos += (R.U[x] + uP) * S[x];
@@ -579,14 +734,7 @@ __device__ __forceinline__ void face_rhs32_cells(const A& a, int f, int i, int j
         nt_ = (nt_ < 0.0f) ? 0.0f : nt_;
         const float theta = 0.5f * (ct + nt_);
         const float pi = pressure_dev(R, ri, Ri), pj = pressure_dev(R, rj, Rj);
-        float gri[D], grj[D], gpi[D], gpj[D];
-#pragma unroll
-        for (int y = 0; y < D; ++y) {
-            gri[y] = a.grad[(size_t)y * nt + i];
-            grj[y] = a.grad[(size_t)y * nt + j];
-            gpi[y] = a.grad[(size_t)(D + y) * nt + i];
-            gpj[y] = a.grad[(size_t)(D + y) * nt + j];
-        }
+        const float *gri = Gi, *grj = Gj, *gpi = Gi + D, *gpj = Gj + D;
         const float rhoPos = R.rho + minmod_interp<float, D>(ri, rj, gri, d, w, 1.0f);
         const float rhoNeg = R.rho + minmod_interp<float, D>(ri, rj, grj, d, w, -1.0f);
         const float pPos = minmod_interp<float, D>(pi, pj, gpi, d, w, 1.0f);    // p - p_ref
@@ -618,37 +766,26 @@ __device__ __forceinline__ void face_rhs32_cells(const A& a, int f, int i, int j
 
     // Viscous face terms (src/cfd_v0.cpp:2682-2796), as in the FP64 kernel.
     const float mu = a.ref.mu;
-    if (VIS && mu != 0.0f) {
+    if (visc) {
         const float Rinv = a.ref.Rinv;
         const float Ti = Ri * Rinv, Tj = Rj * Rinv;   // T - T_ref
-        const float lapc = early ? eLapc : a.lapc[f];
-        float Kf[D], g[D][D], gT[D], sU[D];
-#pragma unroll
-        for (int k = 0; k < D; ++k) {
-            if constexpr (early) Kf[k] = eK[k];
-            else Kf[k] = a.K[(size_t)k * nf + f];
-        }
-        if (!a.fGhost[f]) {
-            auto vI = [&](int r) -> float {
-                if constexpr (early) return Vi[r];
-                else return a.V[(size_t)r * nt + i];
-            };
-            auto vJ = [&](int r) -> float {
-                if constexpr (early) return Vj[r];
-                else return a.V[(size_t)r * nt + j];
-            };
+        const float lapc = geo.lapc;
+        const float* Kf = geo.K;
+        float g[D][D], gT[D], sU[D];
+        if (!ghost) {
+            if (!EARLYV && SCH != kSchemeAUSM) loadV(Vi, Vj);
 #pragma unroll
             for (int x = 0; x < D; ++x) {
 #pragma unroll
-                for (int y = 0; y < D; ++y) g[x][y] = interp(w, vI(x * D + y), vJ(x * D + y));
-                gT[x] = interp(w, vI(D * D + x), vJ(D * D + x));
-                sU[x] = interp(w, vI(D * D + D + x), vJ(D * D + D + x));
+                for (int y = 0; y < D; ++y) g[x][y] = interp(w, Vi[x * D + y], Vj[x * D + y]);
+                gT[x] = interp(w, Vi[D * D + x], Vj[D * D + x]);
+                sU[x] = interp(w, Vi[D * D + D + x], Vj[D * D + D + x]);
             }
         } else {
             const float dinv = a.dinv[f];
             float dn[D], tau[D][D], Uf[D];
 #pragma unroll
-            for (int k = 0; k < D; ++k) dn[k] = a.dnorm[(size_t)k * nf + f];
+            for (int k = 0; k < D; ++k) dn[k] = a.dnorm[(size_t)k * a.nf + f];
 #pragma unroll
             for (int x = 0; x < D; ++x) {
 #pragma unroll
@@ -673,33 +810,40 @@ __device__ __forceinline__ void face_rhs32_cells(const A& a, int f, int i, int j
             rhs[x + 1] += mu * gtS + dsum * S[x] + mu * (lapc * (uj[x] - ui[x]) + dotv<float, D>(Kf, g[x]));
         }
         rhs[D + 1] += dotv<float, D>(sU, S) + kc * (lapc * (Tj - Ti) + dotv<float, D>(Kf, gT));
-        if (LES && a.smagC && !a.fGhost[f]) {   // Smagorinsky LES, as in the FP64 kernel
+        if constexpr (LES) {
+            if (a.smagC && !ghost) {   // Smagorinsky LES, as in the FP64 kernel
+                const float* si = a.V + (size_t)i * kVisStride<D, true> + kVisRows<D>;
+                const float* sj = a.V + (size_t)j * kVisStride<D, true> + kVisRows<D>;
 #pragma unroll
-            for (int x = 0; x < D; ++x) {
-                float s = 0.0f;
+                for (int x = 0; x < D; ++x) {
+                    float s = 0.0f;
 #pragma unroll
-                for (int y = 0; y < D; ++y)
-                    s += interp(w, a.V[(size_t)(kVisRows<D> + x * D + y) * nt + i],
-                                a.V[(size_t)(kVisRows<D> + x * D + y) * nt + j]) *
-                         S[y];
-                rhs[x + 1] += s;
+                    for (int y = 0; y < D; ++y) s += interp(w, si[x * D + y], sj[x * D + y]) * S[y];
+                    rhs[x + 1] += s;
+                }
             }
         }
     }
 }
 
 template <int D, int SCH, bool VIS = true, bool LES = false, bool EARLYV = false>
-__device__ __forceinline__ void face_rhs32(const Args<float>& a, int f, float* rhs) {
-    face_rhs32_cells<D, SCH, VIS, LES, EARLYV>(a, f, a.fP[f], a.fN[f], rhs);
-}
-
-template <int D, int SCH, bool VIS = true, bool LES = false, bool EARLYV = false>
 __device__ __forceinline__ void flux32(const Args<float>& a, int f) {
+    Face32<D> geo;
+    Prim32<D> pi, pj;
+    int i, j;
+    bool ghost;
+    load_face<D>(a, f, geo, i, j, ghost);
+    load_prim<D>(a, i, pi);
+    load_prim<D>(a, j, pj);
     float rhs[D + 2];
-    face_rhs32<D, SCH, VIS, LES, EARLYV>(a, f, rhs);
-    const size_t nf = (size_t)a.nf;
-#pragma unroll
-    for (int v = 0; v < D + 2; ++v) a.flux[(size_t)v * nf + f] = rhs[v];
+    face_rhs32_core<D, SCH, VIS, LES, EARLYV>(
+        a, f, i, j, ghost, geo, pi, pj,
+        [&](float* Vi, float* Vj) {
+            load_vis<D, LES>(a, i, Vi);
+            load_vis<D, LES>(a, j, Vj);
+        },
+        rhs);
+    store_flux<D>(a, f, rhs);
 }
 
 // ---------------------------------------------------------------------------
@@ -707,61 +851,52 @@ __device__ __forceinline__ void flux32(const Args<float>& a, int f) {
 // after another in face order. The cell's own primitive and viscous rows are
 // read once, into registers, for all its faces (a face-per-thread kernel
 // reads them once per face); the cell across each face is read per face, its
-// index one face ahead. face_rhs32_cells sees the rows through a view of the
-// registers (side 0 = P, 1 = N), so the rhs keeps flux32's bits. M1 / M2
-// without the LES terms (whose extra rows the view does not carry).
+// index one face ahead. The rhs is face_rhs32_core's, so it keeps flux32's
+// bits. M1 / M2 without the LES terms.
 // ---------------------------------------------------------------------------
-template <int D>
-struct CellFaceView32 {
-    const RefState32& ref;
-    float prim[2 * (2 * D + 2)];   // [row][side]: rho', m'[D], u'[D], R psi'
-    float V[2 * kVisRows<D>];      // [row][side]: dudx, dTdx, sigmaU
-    const float *S, *d, *w, *K, *lapc, *dinv, *dnorm;
-    const uint8_t* fGhost;
-    const float *grad, *smagC;
-    int nt, nf;
-};
-
 template <int D, int SCH>
 __device__ __forceinline__ void flux32_cell(const Args<float>& a, int c) {
-    static_assert(SCH != kSchemeAUSM, "the cell-centred flux carries no sound speed or gradients");
+    static_assert(SCH != kSchemeAUSM, "the cell-centred flux holds no sound speed or gradients");
     const int f0 = a.fOwn[c], f1 = a.fOwn[c + 1];
     if (f0 >= f1) return;
-    const size_t nt = (size_t)a.nt, nf = (size_t)a.nf;
-    CellFaceView32<D> v{a.ref};
-    v.S = a.S;
-    v.d = a.d;
-    v.w = a.w;
-    v.K = a.K;
-    v.lapc = a.lapc;
-    v.dinv = a.dinv;
-    v.dnorm = a.dnorm;
-    v.fGhost = a.fGhost;
-    v.grad = nullptr;
-    v.smagC = nullptr;
-    v.nt = 2;
-    v.nf = a.nf;
     const bool vis = a.ref.mu != 0.0f;
-#pragma unroll
-    for (int r = 0; r < 2 * D + 2; ++r) v.prim[2 * r] = a.prim[(size_t)r * nt + c];
-    if (vis) {
-#pragma unroll
-        for (int r = 0; r < kVisRows<D>; ++r) v.V[2 * r] = a.V[(size_t)r * nt + c];
-    }
-    int jn = a.fN[f0];
+    Prim32<D> self;
+    load_prim<D>(a, c, self);
+    float Vc[kVisVec<D>];
+    if (vis) load_vis<D, false>(a, c, Vc);
+    int nn = a.fN[f0];
     for (int f = f0; f < f1; ++f) {
-        const int j = jn;
-        if (f + 1 < f1) jn = a.fN[f + 1];
-#pragma unroll
-        for (int r = 0; r < 2 * D + 2; ++r) v.prim[2 * r + 1] = a.prim[(size_t)r * nt + j];
-        if (vis && !a.fGhost[f]) {
-#pragma unroll
-            for (int r = 0; r < kVisRows<D>; ++r) v.V[2 * r + 1] = a.V[(size_t)r * nt + j];
+        const int n = nn;
+        if (f + 1 < f1) nn = a.fN[f + 1];
+        const int j = n & 0x7fffffff;
+        const bool ghost = n < 0;
+        Face32<D> geo;
+        const float4 g0 = a.fG0[f], g1 = a.fG1[f];
+        geo.S[0] = g0.x;
+        geo.S[1] = g0.y;
+        geo.K[0] = g1.x;
+        geo.K[1] = g1.y;
+        if constexpr (D == 2) {
+            geo.w = g0.z;
+            geo.lapc = g0.w;
+        } else {
+            geo.S[2] = g0.z;
+            geo.w = g0.w;
+            geo.K[2] = g1.z;
+            geo.lapc = g1.w;
         }
+        Prim32<D> oth;
+        load_prim<D>(a, j, oth);
         float rhs[D + 2];
-        face_rhs32_cells<D, SCH, true, false, false>(v, f, 0, 1, rhs);
+        face_rhs32_core<D, SCH, true, false, true>(
+            a, f, c, j, ghost, geo, self, oth,
+            [&](float* Vi, float* Vj) {
+                load_vis<D, false>(a, j, Vj);
 #pragma unroll
-        for (int q = 0; q < D + 2; ++q) a.flux[(size_t)q * nf + f] = rhs[q];
+                for (int k = 0; k < kVisVec<D>; ++k) Vi[k] = Vc[k];
+            },
+            rhs);
+        store_flux<D>(a, f, rhs);
     }
 }
 
@@ -772,24 +907,58 @@ __device__ __forceinline__ void flux32_cell(const Args<float>& a, int c) {
 // update's gather sums the stored values, then the update of apply32. The
 // face rhs never reaches memory and a stage needs one kernel less; the next
 // stage's primitives go to a.primW, the other of two buffers (the cells of
-// this launch still read a.prim).
+// this launch still read a.prim). The cell's own values are read once.
 // ---------------------------------------------------------------------------
-template <int D, int SCH, bool LES, bool RES, bool GH>
+template <int D, int SCH, bool VIS, bool RES, bool GH, bool ELL>
 __device__ __forceinline__ void fluxupdate32(const Args<float>& a, int c, double Ak, double Bk, double dt,
                                              float dt32, int first) {
     constexpr int NQ = D + 2;
     CellIn32<D> in;
     load_cell32<D>(a, c, first, in);
+    Prim32<D> self;
+    load_prim<D>(a, c, self);
+    constexpr bool needV = VIS || SCH == kSchemeAUSM;
+    float Vc[needV ? kVisVec<D> : 1];
+    if constexpr (needV) load_vis<D, false>(a, c, Vc);
     float sum[NQ];
 #pragma unroll
     for (int v = 0; v < NQ; ++v) sum[v] = 0.0f;
-    for (int e = a.cfOff[c]; e < a.cfOff[c + 1]; ++e) {
-        const int code = a.cfList[e];
-        float r[NQ];
-        face_rhs32<D, SCH, true, LES, false>(a, code >= 0 ? code : ~code, r);
+    for_entries32<D, ELL>(a, c, [&](int code, int o) {
+        const bool own = code >= 0;
+        const int f = own ? code : ~code;
+        Face32<D> geo;
+        int i, j;
+        bool ghost;
+        load_face<D>(a, f, geo, i, j, ghost);
+        Prim32<D> oth, pi, pj;
+        load_prim<D>(a, o, oth);
 #pragma unroll
-        for (int v = 0; v < NQ; ++v) sum[v] += code >= 0 ? r[v] : neg_bits(r[v]);
-    }
+        for (int k = 0; k < D; ++k) {
+            pi.m[k] = own ? self.m[k] : oth.m[k];
+            pj.m[k] = own ? oth.m[k] : self.m[k];
+            pi.u[k] = own ? self.u[k] : oth.u[k];
+            pj.u[k] = own ? oth.u[k] : self.u[k];
+        }
+        pi.r = own ? self.r : oth.r;
+        pj.r = own ? oth.r : self.r;
+        pi.R = own ? self.R : oth.R;
+        pj.R = own ? oth.R : self.R;
+        float r[NQ];
+        face_rhs32_core<D, SCH, VIS, false, true>(
+            a, f, own ? c : o, own ? o : c, ghost, geo, pi, pj,
+            [&](float* Vi, float* Vj) {
+                float Vo[kVisVec<D>];
+                load_vis<D, false>(a, o, Vo);
+#pragma unroll
+                for (int k = 0; k < kVisRows<D>; ++k) {
+                    Vi[k] = own ? Vc[needV ? k : 0] : Vo[k];
+                    Vj[k] = own ? Vo[k] : Vc[needV ? k : 0];
+                }
+            },
+            r);
+#pragma unroll
+        for (int v = 0; v < NQ; ++v) sum[v] += own ? r[v] : neg_bits(r[v]);
+    });
     apply32<D, RES, GH>(a, c, sum, in, Ak, Bk, dt, dt32, first);
 }
 

@@ -675,8 +675,26 @@ void launch_halo_gather(X* dst, int dstNt, int first, int rows, int nh, const in
 }
 template void launch_halo_gather<double>(double*, int, int, int, int, const int*, const int*, double* const*,
                                          const int*, cudaStream_t);
-template void launch_halo_gather<float>(float*, int, int, int, int, const int*, const int*, float* const*,
-                                        const int*, cudaStream_t);
+
+// Halo slots [first, first + nh) of an array of `words` floats per cell, one
+// thread per 16 bytes.
+__global__ void __launch_bounds__(256) k_halo_gather_cells(float4* dst, int first, int parts, int nh,
+                                                           const int* srcPart, const int* srcCell,
+                                                           float* const* srcBase) {
+    const int k = LFM_GLOBAL_ID();
+    if (k >= nh * parts) return;
+    const int h = k / parts, r = k - h * parts;
+    const float4* src = reinterpret_cast<const float4*>(srcBase[srcPart[h]]);
+    dst[(size_t)(first + h) * parts + r] = src[(size_t)srcCell[h] * parts + r];
+}
+
+void launch_halo_gather_cells(float* dst, int first, int words, int nh, const int* srcPart, const int* srcCell,
+                              float* const* srcBase, cudaStream_t st) {
+    const int parts = words / 4;
+    if (nh > 0)
+        k_halo_gather_cells<<<blocks(nh * parts, 256), 256, 0, st>>>(reinterpret_cast<float4*>(dst), first, parts, nh,
+                                                                    srcPart, srcCell, srcBase);
+}
 
 }  // namespace dev
 }  // namespace lfm

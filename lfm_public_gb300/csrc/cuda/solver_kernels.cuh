@@ -48,6 +48,11 @@ struct RefState32 {
     float gamma, gm1, Rinv, mu, kcond;   // gas constants (FP32 copies)
 };
 
+// Floats per cell of the FP32-bulk viscous rows (with the LES stress or
+// without) and of M2AUSM's gradients: whole 16-byte parts.
+constexpr int visStride32(int D, bool les) { return D == 2 ? (les ? 12 : 8) : (les ? 24 : 16); }
+constexpr int gradStride32(int D) { return D == 2 ? 8 : 16; }
+
 // Arguments shared by the kernels (all device pointers).
 // Fixed-width cell -> face table (Args::cfEll): four entries per 2D cell
 // (quads, triangles), six per 3D cell (hexahedra, prisms, tetrahedra).
@@ -66,7 +71,8 @@ struct Args {
                               // (it holds one step's increments and restarts every step)
     // per cell + ghost, computed every stage
     T* prim;                  // FP64: (D + 3) x nt: 1/rho, u[D], R psi, c
-                              // FP32: (2D + 3) x nt: rho', m'[D], u'[D], R psi', c
+                              // FP32: (2D + 3) x nt: rho', m'[D], u'[D], R psi', c in the
+                              // 16-byte parts of solver_fp32.cuh, as are V, grad and flux
     T* primW;                 // where an update writes the next stage's primitives: prim, or
                               // (fused flux-update stages) the other of two buffers, which no
                               // thread of that launch reads
@@ -115,11 +121,13 @@ struct Args {
     const int* fOwn;          // FP32-bulk cell-centred flux: nc + 1 offsets, the flux faces that
                               // cell c owns (is P of) are fOwn[c] .. fOwn[c + 1] - 1 (the faces
                               // are stored by owner); null where the face-per-thread kernel runs
-    const int* cfEll;         // FP32-bulk update gather (single cases beyond L2, batch cases):
-                              // the cfList entries of each cell at a fixed width
-                              // (kEllWidth<D>), entry k of cell c at k * nc + c, kEllPad
-                              // after the cell's faces; null where unused or a cell has more
-                              // faces (the update then gathers through cfOff / cfList)
+    const int* cfEll;         // FP32-bulk: the cfList entries of each cell at a fixed width
+                              // (kEllWidth<D>), entry k of cell c at c * kEllWidth<D> + k,
+                              // kEllPad after the cell's faces; null where a cell has more
+                              // faces (the gathers then go through cfOff / cfList / cfNbr)
+    const int* cfEllN;        // FP32-bulk, with cfEll: the cfNbr entries likewise, padded with -1
+    const float4* fG0;        // FP32-bulk: face geometry in 16-byte parts (solver_fp32.cuh); S, w, K,
+    const float4* fG1;        // lapc and fGhost are then null, fN carries the boundary flag
     // ghosts
     const int* gCell;
     const int* gKind;
@@ -136,7 +144,7 @@ struct Args {
     double pRef;              // (gamma - 1)(rho_inf E_inf - rho_inf |U_inf|^2 / 2)
     double RpsiRef;           // p_ref / rho_inf
     RefState32 ref;
-    // FP64 path: the primitives include the sound speed (read by M2AUSM only)
+    // the primitives include the sound speed (read by M2AUSM only)
     int primC;
     // error flag (non-finite state)
     int* flag;

@@ -16,17 +16,16 @@ __global__ void __launch_bounds__(256) k_prep32(const __grid_constant__ Args<flo
     if (t < a.nt) prep32<D>(a, t);
 }
 
-template <int D>
+template <int D, bool ELL>
 __global__ void __launch_bounds__(256) k_grad32(const __grid_constant__ Args<float> a) {
     const int c = LFM_GLOBAL_ID();
-    if (c < a.nc) grad32<D>(a, c);
+    if (c < a.nc) grad32<D, ELL>(a, c);
 }
 
-// Six blocks per SM (40 registers, no spills): full-occupancy gathers.
-template <int D, bool LES>
-__global__ void __launch_bounds__(256, 6) k_vis32(const __grid_constant__ Args<float> a) {
+template <int D, bool LES, bool ELL>
+__global__ void __launch_bounds__(256) k_vis32(const __grid_constant__ Args<float> a) {
     const int c = LFM_GLOBAL_ID();
-    if (c < a.nc) vis32<D, LES>(a, c);
+    if (c < a.nc) vis32<D, LES, ELL>(a, c);
 }
 
 template <int D, int SCH, bool LES>
@@ -68,47 +67,38 @@ __global__ void __launch_bounds__(256) k_update32(const __grid_constant__ Args<f
     update_thread<D, RES, GH, ELL>(a, Ak, Bk, dt, dt32, first);
 }
 
-// 2D list-gather updates at six blocks per SM (40 registers; the ghost branch
-// spills 40 bytes on the few cells that take it): 0.092 -> 0.087 ms per step
-// on the 768x512 cylinder, whose 393k cells then fill 1.7 waves instead of
-// 2.02. The table gathers keep their registers (all loads in flight).
-template <bool RES, bool GH>
-__global__ void __launch_bounds__(256, 6) k_update32_2d(const __grid_constant__ Args<float> a, double Ak, double Bk,
-                                                       double dt, float dt32, int first) {
-    update_thread<2, RES, GH, false>(a, Ak, Bk, dt, dt32, first);
-}
-
 // Fused flux + update (fluxupdate32): one thread per cell, cells mapped as
 // in the update kernel that writes ghosts (warp-interleaved chunks).
-template <int D, int SCH, bool RES>
+template <int D, int SCH, bool VIS, bool RES, bool ELL>
 __global__ void __launch_bounds__(256) k_fluxupdate32(const __grid_constant__ Args<float> a, double Ak, double Bk,
                                                       double dt, float dt32, int first) {
     const int c = (int)(((threadIdx.x >> 5) * gridDim.x + blockIdx.x) << 5) + (int)(threadIdx.x & 31u);
-    if (c < a.nc) fluxupdate32<D, SCH, false, RES, true>(a, c, Ak, Bk, dt, dt32, first);
+    if (c < a.nc) fluxupdate32<D, SCH, VIS, RES, true, ELL>(a, c, Ak, Bk, dt, dt32, first);
+}
+
+template <int D, int SCH, bool VIS, bool ELL>
+void launch_fluxupdate32_kernel(const Args<float>& a, const StageConfig& s, cudaStream_t st) {
+    const unsigned nb = (unsigned)((a.nc + 255) / 256);
+    const float dt32 = (float)s.dt;
+    if (s.withRes) k_fluxupdate32<D, SCH, VIS, true, ELL><<<nb, 256, 0, st>>>(a, s.A, s.B, s.dt, dt32, s.first);
+    else k_fluxupdate32<D, SCH, VIS, false, ELL><<<nb, 256, 0, st>>>(a, s.A, s.B, s.dt, dt32, s.first);
 }
 
 template <int D, int SCH>
 void launch_fluxupdate32_scheme(const Args<float>& a, const StageConfig& s, cudaStream_t st) {
-    const unsigned nb = (unsigned)((a.nc + 255) / 256);
-    const float dt32 = (float)s.dt;
-    if (s.withRes) k_fluxupdate32<D, SCH, true><<<nb, 256, 0, st>>>(a, s.A, s.B, s.dt, dt32, s.first);
-    else k_fluxupdate32<D, SCH, false><<<nb, 256, 0, st>>>(a, s.A, s.B, s.dt, dt32, s.first);
+    if (SCH != kSchemeAUSM && !s.needVis) {   // no viscous terms, no viscous rows
+        if (a.cfEll) launch_fluxupdate32_kernel<D, SCH, false, true>(a, s, st);
+        else launch_fluxupdate32_kernel<D, SCH, false, false>(a, s, st);
+    } else {
+        if (a.cfEll) launch_fluxupdate32_kernel<D, SCH, true, true>(a, s, st);
+        else launch_fluxupdate32_kernel<D, SCH, true, false>(a, s, st);
+    }
 }
 
 template <int D, bool ELL>
 void launch_update32(const Args<float>& a, const StageConfig& s, cudaStream_t st) {
     const unsigned nb = (unsigned)((a.nc + 255) / 256);   // eight 32-cell chunks per block
     const float dt32 = (float)s.dt;
-    if (D == 2 && !ELL) {
-        if (a.cellGhosts) {
-            if (s.withRes) k_update32_2d<true, true><<<nb, 256, 0, st>>>(a, s.A, s.B, s.dt, dt32, s.first);
-            else k_update32_2d<false, true><<<nb, 256, 0, st>>>(a, s.A, s.B, s.dt, dt32, s.first);
-        } else {
-            if (s.withRes) k_update32_2d<true, false><<<nb, 256, 0, st>>>(a, s.A, s.B, s.dt, dt32, s.first);
-            else k_update32_2d<false, false><<<nb, 256, 0, st>>>(a, s.A, s.B, s.dt, dt32, s.first);
-        }
-        return;
-    }
     if (a.cellGhosts) {
         if (s.withRes) k_update32<D, true, true, ELL><<<nb, 256, 0, st>>>(a, s.A, s.B, s.dt, dt32, s.first);
         else k_update32<D, false, true, ELL><<<nb, 256, 0, st>>>(a, s.A, s.B, s.dt, dt32, s.first);
@@ -146,11 +136,15 @@ void launch_fp32(const Args<float>& a, const StageConfig& s, int which, cudaStre
             break;
         }
         case 1:
-            if (s.needGrad) k_grad32<D><<<nblocks(a.nc, 256), 256, 0, st>>>(a);
+            if (s.needGrad && a.cfEll) k_grad32<D, true><<<nblocks(a.nc, 256), 256, 0, st>>>(a);
+            else if (s.needGrad) k_grad32<D, false><<<nblocks(a.nc, 256), 256, 0, st>>>(a);
             break;
         case 2:
-            if (s.needVis && a.smagC) k_vis32<D, true><<<nblocks(a.nc, 256), 256, 0, st>>>(a);
-            else if (s.needVis) k_vis32<D, false><<<nblocks(a.nc, 256), 256, 0, st>>>(a);
+            if (!s.needVis) break;
+            if (a.smagC && a.cfEll) k_vis32<D, true, true><<<nblocks(a.nc, 256), 256, 0, st>>>(a);
+            else if (a.smagC) k_vis32<D, true, false><<<nblocks(a.nc, 256), 256, 0, st>>>(a);
+            else if (a.cfEll) k_vis32<D, false, true><<<nblocks(a.nc, 256), 256, 0, st>>>(a);
+            else k_vis32<D, false, false><<<nblocks(a.nc, 256), 256, 0, st>>>(a);
             break;
         case 3:
             if (s.fluxStaging.stages > 0) {   // staged kernel (configured for this scheme, laminar)

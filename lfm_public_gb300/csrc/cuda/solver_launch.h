@@ -69,6 +69,16 @@ template <typename T>
 constexpr int primRows(int D) {
     return sizeof(T) == sizeof(double) ? D + 3 : 2 * D + 3;
 }
+// Values per cell of the viscous array and of M2AUSM's gradients (FP64: rows of
+// nt; FP32-bulk: whole 16-byte parts per cell).
+template <typename T>
+constexpr size_t visWords(int D, bool les) {
+    return sizeof(T) == sizeof(double) ? (size_t)(D * D + 2 * D + (les ? D * D : 0)) : (size_t)visStride32(D, les);
+}
+template <typename T>
+constexpr size_t gradWords(int D) {
+    return sizeof(T) == sizeof(double) ? (size_t)(2 * D + D * D) : (size_t)gradStride32(D);
+}
 // Offset added to the stored state before use (the FP32-bulk form stores
 // q - q_ref; zero for the FP64 path).
 struct QOffset {
@@ -90,6 +100,9 @@ void launch_offset_rows(double* dst, int64_t dstStride, const double* src, int64
 template <typename X>
 void launch_halo_gather(X* dst, int dstNt, int first, int rows, int nh, const int* srcPart, const int* srcCell,
                         X* const* srcBase, const int* srcNt, cudaStream_t st);
+// The same for an array of `words` floats per cell (a multiple of 4).
+void launch_halo_gather_cells(float* dst, int first, int words, int nh, const int* srcPart, const int* srcCell,
+                              float* const* srcBase, cudaStream_t st);
 
 // Post-processing (post_kernels.cu).
 void launch_stats(int D, const double* q, int64_t nt, QOffset qo, int nc, double gm1, int n, double* avg,
@@ -107,7 +120,6 @@ struct TileArgs {
     const TileDesc* tiles;
     const int* ints;
     const float* floats;
-    const uint8_t* bytes;
     const float* primIn;   // primitives at the stage start (the update writes the other buffer)
     int nTiles;
     int block;             // threads of a block

@@ -22,8 +22,8 @@ namespace {
 template <int D>
 struct TileRows {
     static constexpr int P = 2 * D + 3;        // primitives
-    static constexpr int V = D * D + 2 * D;    // dudx, dTdx, sigmaU
-    static constexpr int G = 2 * D + D * D;    // rho, p, U gradients
+    static constexpr int V = kVisStride<D, false>;   // dudx, dTdx, sigmaU
+    static constexpr int G = kGradStride<D>;         // rho, p, U gradients
     static constexpr int Q = D + 2;            // face rhs
 };
 
@@ -39,7 +39,7 @@ __global__ void __launch_bounds__(256) k_tile_stage(const __grid_constant__ Args
     // gradients and viscous terms only where the case reads them
     const int vRows = t.haveV ? R::V : 0, gRows = t.haveGrad ? R::G : 0;
     float* sPrim = sm;
-    float* sV = sPrim + (size_t)R::P * nL;
+    float* sV = sPrim + (((size_t)R::P * nL + 3) & ~(size_t)3);
     float* sGrad = sV + (size_t)vRows * nL;
     float* sFlux = sGrad + (size_t)gRows * nL;
     const int* L = t.ints + td.iOff;
@@ -61,29 +61,34 @@ __global__ void __launch_bounds__(256) k_tile_stage(const __grid_constant__ Args
         la.cfList = cfOff + td.nV + 1;
         la.cfNbr = la.cfList + td.nE;
         la.cfEll = nullptr;
-        la.S = F;
-        la.d = F + (size_t)D * nLF;
-        la.w = F + (size_t)2 * D * nLF;
-        la.K = F + (size_t)(2 * D + 1) * nLF;
-        la.lapc = F + (size_t)(3 * D + 1) * nLF;
-        la.dinv = F + (size_t)(3 * D + 2) * nLF;
-        la.dnorm = F + (size_t)(3 * D + 3) * nLF;
-        la.volInv32 = F + (size_t)(4 * D + 3) * nLF;
-        la.fGhost = t.bytes + td.bOff;
+        la.cfEllN = nullptr;
+        la.fG0 = reinterpret_cast<const float4*>(F);
+        la.fG1 = la.fG0 + nLF;
+        la.d = F + (size_t)8 * nLF;
+        la.dinv = la.d + (size_t)D * nLF;
+        la.dnorm = la.dinv + nLF;
+        la.volInv32 = la.dnorm + (size_t)D * nLF;
     }
     // primitives of every local cell (stage start), zero gradients and
     // viscous terms (ghosts keep zero, as the separate kernels' arrays do)
-    for (int k = threadIdx.x; k < R::P * nL; k += blockDim.x) {
-        const int row = k / nL, lc = k - row * nL;
-        sPrim[k] = t.primIn[(size_t)row * (size_t)g.nt + (size_t)L[lc]];
+    for (int lc = threadIdx.x; lc < nL; lc += blockDim.x) {
+        const size_t t0 = (size_t)L[lc], nt = (size_t)g.nt;
+        reinterpret_cast<float4*>(sPrim)[lc] = reinterpret_cast<const float4*>(t.primIn)[t0];
+        const float* b = t.primIn + prim_b(nt);
+        float* sb = sPrim + prim_b((size_t)nL);
+        if constexpr (D == 2)
+            reinterpret_cast<float2*>(sb)[lc] = reinterpret_cast<const float2*>(b)[t0];
+        else
+            reinterpret_cast<float4*>(sb)[lc] = reinterpret_cast<const float4*>(b)[t0];
+        if (SCH == kSchemeAUSM) sPrim[prim_c<D>((size_t)nL) + lc] = t.primIn[prim_c<D>(nt) + t0];
     }
     for (int k = threadIdx.x; k < (vRows + gRows) * nL; k += blockDim.x) sV[k] = 0.0f;
     __syncthreads();
     const Args<float>& a = la;
     if (t.needGrad || t.needVis)
         for (int lc = threadIdx.x; lc < td.nV; lc += blockDim.x) {
-            if (t.needGrad) grad32<D>(a, lc);
-            if (t.needVis) vis32<D>(a, lc);
+            if (t.needGrad) grad32<D, false>(a, lc);
+            if (t.needVis) vis32<D, false, false>(a, lc);
         }
     __syncthreads();
     for (int lf = threadIdx.x; lf < td.nFA; lf += blockDim.x) flux32<D, SCH>(a, lf);
@@ -115,9 +120,9 @@ cudaError_t launchTiles(const Args<float>& g, const TileArgs& t, const StageConf
 }  // namespace
 
 size_t tile_smem_bytes(int D, int maxL, int maxLF, bool haveV, bool haveGrad) {
-    const int P = 2 * D + 3, V = D * D + 2 * D, G = 2 * D + D * D;
-    const int rows = P + (haveV ? V : 0) + (haveGrad ? G : 0);
-    return sizeof(float) * ((size_t)rows * (size_t)maxL + (size_t)(D + 2) * (size_t)maxLF);
+    const int P = 2 * D + 3;
+    const int rows = P + (haveV ? visStride32(D, false) : 0) + (haveGrad ? gradStride32(D) : 0);
+    return sizeof(float) * ((size_t)rows * (size_t)maxL + 4 + (size_t)(D + 2) * (size_t)maxLF);
 }
 
 cudaError_t launch_tile_stage(const Args<float>& g, const TileArgs& t, const StageConfig& s, cudaStream_t st) {

@@ -4,6 +4,8 @@
 #include <algorithm>
 #include <stdexcept>
 
+#include "../cuda/face_pack.h"
+
 namespace lfm {
 
 namespace {
@@ -110,7 +112,7 @@ TileSet buildTiles(const lfm_solver_desc* d, int tileCells, int maxLocal) {
         for (int f : LF) {
             const int ln = localOf[(size_t)d->face_n[f]];
             if (ln < 0 || ln >= td.nL) throw std::runtime_error("tiles: face neighbour outside its tile");
-            ts.ints.push_back(ln);
+            ts.ints.push_back(setup::flaggedN(d, (size_t)f, ln));
         }
         std::vector<int> cfList, cfNbr;
         ts.ints.push_back(0);
@@ -132,23 +134,24 @@ TileSet buildTiles(const lfm_solver_desc* d, int tileCells, int maxLocal) {
         ts.ints.insert(ts.ints.end(), cfList.begin(), cfList.end());
         ts.ints.insert(ts.ints.end(), cfNbr.begin(), cfNbr.end());
 
-        // floats (converted as the solver's device copies are: (float) of the FP64 value)
+        // floats (the solver's device values: (float) of the FP64 value)
+        while (ts.floats.size() % 4) ts.floats.push_back(0.0f);
         td.fOff = (int64_t)ts.floats.size();
+        ts.floats.resize(ts.floats.size() + 8 * LF.size());
+        for (size_t k = 0; k < LF.size(); ++k) {
+            float* g0 = ts.floats.data() + td.fOff + 4 * k;
+            const int f = LF[k];
+            setup::packFace32(d, (size_t)f, localOf[(size_t)d->face_p[f]], setup::flaggedN(d, (size_t)f, localOf[(size_t)d->face_n[f]]), g0,
+                              g0 + 4 * LF.size());
+        }
         auto pushRows = [&](const double* src, int rows) {
             for (int k = 0; k < rows; ++k)
                 for (int f : LF) ts.floats.push_back((float)src[(size_t)k * (size_t)nf + (size_t)f]);
         };
-        pushRows(d->S, D);
         pushRows(d->d, D);
-        pushRows(d->w, 1);
-        pushRows(d->K, D);
-        for (int f : LF) ts.floats.push_back((float)(d->delta_mag[f] * d->dmag_inv[f]));
         pushRows(d->dmag_inv, 1);
         pushRows(d->dnorm, D);
         for (int v = 0; v < td.nV; ++v) ts.floats.push_back((float)d->vol_inv[L[(size_t)v]]);
-
-        td.bOff = (int64_t)ts.bytes.size();
-        for (int f : LF) ts.bytes.push_back(d->face_ghost[f]);
 
         ts.maxL = std::max(ts.maxL, td.nL);
         ts.maxLF = std::max(ts.maxLF, td.nLF);

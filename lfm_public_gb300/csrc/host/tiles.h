@@ -17,7 +17,6 @@ struct TileSet {
     std::vector<TileDesc> tiles;
     std::vector<int> ints;
     std::vector<float> floats;
-    std::vector<uint8_t> bytes;
     int maxL = 0, maxLF = 0;   // largest local cell and face counts
     int64_t localCells = 0;    // sum of nL (loads per stage, halos included)
     int64_t fluxFaces = 0;     // sum of nFA (faces whose rhs is computed)
