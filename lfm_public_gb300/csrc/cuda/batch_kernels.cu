@@ -80,15 +80,9 @@ __device__ __forceinline__ void item(const BatchCase& bc, int stage, int i) {
             flux32<D, kSchemeM2, FULL>(a, i);
         else
             flux32<D, kSchemeAUSM, FULL>(a, i);
-    } else {   // through the fixed-width face table where the case has one
+    } else {
         const int first = stage == 0;
-        if (bc.residuals && first) {
-            if (a.cfEll) update32<D, true, true, true>(a, i, bc.rkA[stage], bc.rkB[stage], bc.dt, bc.dt32, first);
-            else update32<D, true, true, false>(a, i, bc.rkA[stage], bc.rkB[stage], bc.dt, bc.dt32, first);
-        } else {
-            if (a.cfEll) update32<D, false, true, true>(a, i, bc.rkA[stage], bc.rkB[stage], bc.dt, bc.dt32, first);
-            else update32<D, false, true, false>(a, i, bc.rkA[stage], bc.rkB[stage], bc.dt, bc.dt32, first);
-        }
+        update32<D, true, kEntriesEither>(a, i, bc.rkA[stage], bc.rkB[stage], bc.dt32, first, bc.residuals && first);
     }
 }
 
@@ -127,6 +121,15 @@ __device__ __forceinline__ void phase_tiles(const BatchArgs& b, int stage, Batch
     }
 }
 
+// Resident blocks per SM the stage kernel is compiled for: its registers are
+// those of its largest phase, and every phase waits for loads, so threads
+// count: 1024 per SM for the 2D inviscid variant (64 registers), 768 with the
+// viscous terms and M2AUSM in 2D (80), 512 with 3D cases (128).
+constexpr int stage_blocks(int block, int dims, bool full) {
+    const int threads = dims == 2 ? (full ? 768 : 1024) : 512;
+    return threads >= block ? threads / block : 1;
+}
+
 // Stage `stage` of every case: [prep] | [grad + vis] | flux | update, with a
 // grid barrier between phases (none after the last; the bracketed phases and
 // their barriers only when they have tiles). Within the launch every array
@@ -134,7 +137,7 @@ __device__ __forceinline__ void phase_tiles(const BatchArgs& b, int stage, Batch
 // line it cached before another block rewrote it.
 // DIMS = 2: every case is 2D; DIMS = 0: 2D and 3D cases. FULL: see item().
 template <int BLOCK, int DIMS, bool FULL>
-__global__ void __launch_bounds__(BLOCK) k_batch_stage(const __grid_constant__ BatchArgs b, int stage) {
+__global__ void __launch_bounds__(BLOCK, stage_blocks(BLOCK, DIMS, FULL)) k_batch_stage(const __grid_constant__ BatchArgs b, int stage) {
     __shared__ BatchCase sc;
     __shared__ int sSlot;
     if (threadIdx.x == 0) sSlot = -1;

@@ -16,6 +16,7 @@
 #include "lfm_gpu.h"
 #include "../host/tiles.h"
 #include "args_setup.h"
+#include "solver_device.cuh"
 #include "solver_launch.h"
 
 using lfm::dev::Args;
@@ -188,6 +189,7 @@ int buildArgs(lfm_solver* s, const lfm_solver_desc* d, Args<T>& a, const int* fP
     a.cfSoN = nullptr;
     a.cellSoW = nullptr;
     constexpr bool fp64 = sizeof(T) == sizeof(double);
+    a.pdl = lfm::dev::pdl_pays(fp64, s->D, s->nc) ? 1 : 0;
     const size_t nt = (size_t)s->nt, nf = (size_t)s->nf, D = (size_t)s->D;
     int rc;
     if ((rc = devAlloc(s, &a.dq, (size_t)s->nq * s->nc))) return rc;
@@ -297,7 +299,11 @@ StageConfig stageConfig(const lfm_solver* s, int k, double dt) {
 
 template <typename T>
 void stageAll(lfm_solver* s, const Args<T>& a, double dt) {
-    for (int k = 0; k < s->rkOrder; ++k) lfm::dev::launch_stage<T>(a, stageConfig(s, k, dt), s->stream);
+    for (int k = 0; k < s->rkOrder; ++k) {
+        StageConfig c = stageConfig(s, k, dt);
+        c.pdl = true;
+        lfm::dev::launch_stage<T>(a, c, s->stream);
+    }
 }
 
 // Fused tile stage k of a step that starts from primitive buffer `parity`:
@@ -327,7 +333,8 @@ void fluxUpdateStage(lfm_solver* s, int k, double dt, int parity) {
     Args<float> g = s->a32;
     g.prim = buf[in];
     g.primW = buf[in ^ 1];
-    const StageConfig c = stageConfig(s, k, dt);
+    StageConfig c = stageConfig(s, k, dt);
+    c.pdl = true;
     for (int w = 0; w < 3; ++w) lfm::dev::launch_kernel<float>(g, c, w, s->stream);   // prep, grad, vis
     lfm::dev::launch_fluxupdate32(g, c, s->stream);
 }
@@ -1067,14 +1074,16 @@ int noallocScratch(int device, unsigned char** out) {
 // flux is [nq][nf]; FP32-bulk: [nf][4], then in 3D the fifth value's row).
 template <typename T, int D>
 __global__ void __launch_bounds__(256) k_gather_residual(const T* flux, int nf, int nc, const int* cfOff,
-                                                         const int* cfList, double* res) {
+                                                         const int* cfList, double* res, int pdl) {
     const int c = (int)(blockIdx.x * blockDim.x + threadIdx.x);
     if (c >= nc) return;
     constexpr int NQ = D + 2;
     T sum[NQ];
 #pragma unroll
     for (int v = 0; v < NQ; ++v) sum[v] = T(0);
-    for (int e = cfOff[c]; e < cfOff[c + 1]; ++e) {
+    const int e0 = cfOff[c], e1 = cfOff[c + 1];
+    lfm::dev::PdlWait{pdl}();
+    for (int e = e0; e < e1; ++e) {
         const int code = cfList[e];
         const size_t f = (size_t)(code >= 0 ? code : ~code);
         T x[NQ];
@@ -1155,12 +1164,13 @@ int residualNoalloc(const lfm_solver* s, const Args<T>& base, const double* q, i
     c.scheme = s->scheme;
     c.needGrad = s->needGrad;
     c.needVis = s->needVis;
-    for (int k = 0; k < 4; ++k) lfm::dev::launch_kernel<T>(a, c, k, st);   // prep, grad, vis, flux
+    for (int k = 0; k < 4; ++k) {   // prep (every cell: always launched), grad, vis, flux
+        lfm::dev::launch_kernel<T>(a, c, k, st);
+        c.pdl = true;
+    }
     const unsigned nb = (unsigned)((s->nc + 255) / 256);
-    if (s->D == 2)
-        k_gather_residual<T, 2><<<nb, 256, 0, st>>>(a.flux, s->nf, s->nc, a.cfOff, a.cfList, res);
-    else
-        k_gather_residual<T, 3><<<nb, 256, 0, st>>>(a.flux, s->nf, s->nc, a.cfOff, a.cfList, res);
+    lfm::dev::launch_kernel_pdl(a.pdl, s->D == 2 ? k_gather_residual<T, 2> : k_gather_residual<T, 3>, nb, 256, st, a.flux,
+                                s->nf, s->nc, a.cfOff, a.cfList, res, a.pdl);
     LFM_CUDA(cudaGetLastError());
     return LFM_OK;
 }
@@ -1432,7 +1442,8 @@ cudaError_t medianTime(lfm_solver* s, int reps, cudaEvent_t e0, cudaEvent_t e1, 
 }
 
 void launchOne(lfm_solver* s, const Launch& l, double dt) {
-    const StageConfig c = stageConfig(s, l.stage, dt);
+    StageConfig c = stageConfig(s, l.stage, dt);
+    c.pdl = true;   // as in the step
     if (s->fluxUpdate) {   // buffers of a step that starts from buffer 0
         float* buf[2] = {s->a32.prim, s->prim1};
         Args<float> g = s->a32;

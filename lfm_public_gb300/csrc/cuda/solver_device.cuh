@@ -8,6 +8,30 @@ namespace dev {
 
 #define LFM_GLOBAL_ID() ((int)(blockIdx.x * blockDim.x + threadIdx.x))
 
+// Programmatic dependent launch. The kernels of a time step are launched so
+// that a kernel's blocks may become resident once every block of its
+// predecessor has passed its own wait, instead of after the predecessor has
+// drained; each first loads what no kernel of the step writes (face lists,
+// geometry, cell constants) and then waits here for the predecessor's results.
+// Since a kernel releases its successor only after its wait, at most two
+// kernels of the chain overlap, and everything before the predecessor is
+// complete. Without it each kernel of a 2D case spends 2 to 4 of its 8 to 15 us
+// launching, loading indices and draining. Args::pdl says which cases launch
+// their kernels that way (pdl_pays, solver_launch.h); one launched plainly all
+// the same passes at once.
+struct PdlWait {
+    int pdl;
+    __device__ __forceinline__ void operator()() const {
+        if (!pdl) return;
+        asm volatile("griddepcontrol.wait;" ::: "memory");
+        asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+    }
+};
+// For device functions called inside one kernel (the batch, the tiles).
+struct NoWait {
+    __device__ __forceinline__ void operator()() const {}
+};
+
 template <typename T>
 __device__ __forceinline__ T interp(T w, T a, T b) {
     return w * a + (T(1) - w) * b;
@@ -321,24 +345,31 @@ __device__ __forceinline__ void ghosts_of64(const Args<double>& a, int c, const 
 // primitives from the registers it holds, and (a.cellGhosts) the next stage's
 // states and primitives of its boundary ghosts -- a ghost depends on its
 // interior cell only -- so that no preparation pass runs between the stages.
-template <typename T, int D, bool RES, bool PRIM = false>
-__device__ __forceinline__ void update_cell(const Args<T>& a, int c, double Ak, double Bk, double dt, int first) {
+template <typename T, int D, bool RES, bool PRIM = false, class Sync = NoWait>
+__device__ __forceinline__ void update_cell(const Args<T>& a, int c, double Ak, double Bk, double dt, int first,
+                                            Sync sync = Sync()) {
     constexpr int NQ = D + 2;
     const size_t nt = (size_t)a.nt, nf = (size_t)a.nf, nc = (size_t)a.nc;
-    double qv[NQ];
+    constexpr int W = kEllWidth<D>;
+    const int e0 = a.cfOff[c], e1 = a.cfOff[c + 1];
+    int code[W];
 #pragma unroll
-    for (int v = 0; v < NQ; ++v) qv[v] = a.q[v * nt + c];
+    for (int k = 0; k < W; ++k) code[k] = e0 + k < e1 ? a.cfList[e0 + k] : kEllPad;
+    const double vi = a.volInv[c], sg = a.sponge[c];
+    const bool ghosts = PRIM && a.cellGhosts && a.cellGhosts[c];
+    sync();
+    double qv[NQ], dq[NQ];
+#pragma unroll
+    for (int v = 0; v < NQ; ++v) {
+        qv[v] = a.q[v * nt + c];
+        dq[v] = first ? 0.0 : a.dq[v * nc + c];
+    }
     T sum[NQ];
 #pragma unroll
     for (int v = 0; v < NQ; ++v) sum[v] = T(0);
-    const int e0 = a.cfOff[c], e1 = a.cfOff[c + 1];
-    constexpr int W = kEllWidth<D>;
     if (e1 - e0 <= W) {
         // every face index of the cell, then every rhs value, in flight at
         // once; summed in the same (ascending face) order as the loop below
-        int code[W];
-#pragma unroll
-        for (int k = 0; k < W; ++k) code[k] = e0 + k < e1 ? a.cfList[e0 + k] : kEllPad;
         // The face's sign (+ where c is P, - where N) goes on the value as a
         // sign-bit flip on the integer pipe, so each entry costs one FP64 add
         // (a - b is a + (-b) in IEEE arithmetic: the same bits)
@@ -374,10 +405,9 @@ __device__ __forceinline__ void update_cell(const Args<T>& a, int c, double Ak, 
     }
     double acc[NQ];
     bool finite = true;
-    const double dtvi = dt * a.volInv[c];
+    const double dtvi = dt * vi;
 #pragma unroll
-    for (int v = 0; v < NQ; ++v) acc[v] = (first ? 0.0 : Ak * a.dq[v * nc + c]) + dtvi * (double)sum[v];
-    const double sg = a.sponge[c];
+    for (int v = 0; v < NQ; ++v) acc[v] = Ak * dq[v] + dtvi * (double)sum[v];
     if (sg != 0.0) {
         acc[0] += dt * sg * (a.rhoInf - qv[0]);
 #pragma unroll
@@ -396,7 +426,7 @@ __device__ __forceinline__ void update_cell(const Args<T>& a, int c, double Ak, 
     if (!finite) atomicOr(a.flag, 1);
     if constexpr (PRIM) {
         prims64<D>(a, c, qn);
-        if (a.cellGhosts && a.cellGhosts[c]) ghosts_of64<D>(a, c, qn);
+        if (ghosts) ghosts_of64<D>(a, c, qn);
     }
 }
 

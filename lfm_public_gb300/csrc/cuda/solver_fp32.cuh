@@ -388,10 +388,8 @@ __device__ __forceinline__ void gather32(const Args<float>& a, int c, float* sum
 // memory round trips instead of one per face; the sum runs in the same
 // (ascending face) order, so it has gather32's bits.
 template <int D>
-__device__ __forceinline__ void gather32_ell(const Args<float>& a, int c, float* sum) {
+__device__ __forceinline__ void gather32_ell(const Args<float>& a, const int* code, float* sum) {
     constexpr int NQ = D + 2, W = kEllWidth<D>;
-    int code[W];
-    load_ell<D>(a.cfEll, c, code);
     float x[W][NQ];
 #pragma unroll
     for (int k = 0; k < W; ++k)
@@ -413,25 +411,29 @@ struct CellIn32 {
     double qp[D + 2];   // q'
     float dq[D + 2];
     float vi, sg;       // 1/V, sponge sigma
+    int ghosts;         // it has boundary faces (GH)
 };
 
-template <int D>
-__device__ __forceinline__ void load_cell32(const Args<float>& a, int c, int first, CellIn32<D>& in) {
+template <int D, bool GH, class Sync = NoWait>
+__device__ __forceinline__ void load_cell32(const Args<float>& a, int c, int first, CellIn32<D>& in,
+                                            Sync sync = Sync()) {
     const size_t nt = (size_t)a.nt, nc = (size_t)a.nc;
+    in.vi = a.volInv32[c];
+    in.sg = a.sponge[c];
+    in.ghosts = GH ? a.cellGhosts[c] : 0;
+    sync();
 #pragma unroll
     for (int v = 0; v < D + 2; ++v) {
         in.qp[v] = a.q[v * nt + c];
         in.dq[v] = first ? 0.0f : a.dq[v * nc + c];
     }
-    in.vi = a.volInv32[c];
-    in.sg = a.sponge[c];
 }
 
 // apply32: the update of cell c from its rhs sum and its loaded values
 // (see update32).
-template <int D, bool RES, bool GH>
+template <int D, bool GH>
 __device__ __forceinline__ void apply32(const Args<float>& a, int c, const float* sum, const CellIn32<D>& in,
-                                        double Ak, double Bk, double dt, float dt32, int first) {
+                                        double Ak, double Bk, float dt32, int first, bool res) {
     constexpr int NQ = D + 2;
     const size_t nt = (size_t)a.nt, nc = (size_t)a.nc;
     const float dtvi = __fmul_rn(dt32, in.vi);
@@ -450,22 +452,28 @@ __device__ __forceinline__ void apply32(const Args<float>& a, int c, const float
         qn[v] = fma(Bk, f32_to_f64(acc), qp);
         a.q[v * nt + c] = qn[v];
         finite = finite && isfinite(sum[v]);
-        if (RES) a.res[v * nc + c] = f32_to_f64(sum[v]);
+        if (res) a.res[v * nc + c] = f32_to_f64(sum[v]);
     }
     if (!finite) atomicOr(a.flag, 1);
     prims32<D>(a, c, qn, a.primW);
-    if (GH && a.cellGhosts[c]) ghosts_of32<D>(a, c, qn, a.primW);
+    if (GH && in.ghosts) ghosts_of32<D>(a, c, qn, a.primW);
 }
 
-template <int D, bool RES, bool GH = false, bool ELL = false>
-__device__ __forceinline__ void update32(const Args<float>& a, int c, double Ak, double Bk, double dt,
-                                         float dt32, int first) {
+// ELL: the fixed-width table, the face list, or (the batch, one copy of whose
+// code serves every case) whichever the case has.
+enum Entries32 { kEntriesList, kEntriesEll, kEntriesEither };
+template <int D, bool GH, Entries32 ELL, class Sync = NoWait>
+__device__ __forceinline__ void update32(const Args<float>& a, int c, double Ak, double Bk, float dt32, int first,
+                                         bool res, Sync sync = Sync()) {
+    constexpr int W = kEllWidth<D>;
+    int code[ELL != kEntriesList ? W : 1];
+    if (ELL == kEntriesEll || (ELL == kEntriesEither && a.cfEll)) load_ell<D>(a.cfEll, c, code);
     CellIn32<D> in;
-    load_cell32<D>(a, c, first, in);
+    load_cell32<D, GH>(a, c, first, in, sync);
     float sum[D + 2];
-    if (ELL) gather32_ell<D>(a, c, sum);
+    if (ELL == kEntriesEll || (ELL == kEntriesEither && a.cfEll)) gather32_ell<D>(a, code, sum);
     else gather32<D>(a, c, sum);
-    apply32<D, RES, GH>(a, c, sum, in, Ak, Bk, dt, dt32, first);
+    apply32<D, GH>(a, c, sum, in, Ak, Bk, dt32, first, res);
 }
 
 // A new state: q' = q - q_ref of cell c from a caller's absolute state q
@@ -492,22 +500,40 @@ __device__ __forceinline__ void to_perturbation(const Args<float>& a, const doub
     for (int v = 0; v < D + 2; ++v) a.q[(size_t)v * a.nt + c] = q[(size_t)v * stride + c] - a.qRef[v];
 }
 
-// Calls f(code, o) for every face entry of cell c in ascending face order
-// (code: the face, one's complement where c is N; o: the cell across): through
-// the fixed-width tables (ELL), unrolled so that the entries' loads overlap, or
-// the face list.
-template <int D, bool ELL, class F>
-__device__ __forceinline__ void for_entries32(const Args<float>& a, int c, F f) {
+// Calls f(code, o, S, w) for every face entry of cell c in ascending face
+// order (code: the face, one's complement where c is N; o: the cell across; the
+// face's S and w): through the fixed-width tables (ELL), unrolled so that the
+// entries' loads overlap, or the face list. sync() comes after the loads of
+// constants (in 2D the geometry too; in 3D it would take 24 registers more)
+// and before the first f.
+template <int D, bool ELL, class Sync, class F>
+__device__ __forceinline__ void for_entries32(const Args<float>& a, int c, Sync sync, F f) {
     if constexpr (ELL) {
         constexpr int W = kEllWidth<D>;
         int code[W], nb[W];
         load_ell<D>(a.cfEll, c, code);
         load_ell<D>(a.cfEllN, c, nb);
+        float S[W][D], w[W];
+        if constexpr (D == 2) {
 #pragma unroll
-        for (int k = 0; k < W; ++k)
-            if (code[k] != kEllPad) f(code[k], nb[k]);
+            for (int k = 0; k < W; ++k)
+                if (code[k] != kEllPad) w[k] = load_Sw<D>(a, code[k] >= 0 ? code[k] : ~code[k], S[k]);
+        }
+        sync();
+#pragma unroll
+        for (int k = 0; k < W; ++k) {
+            if (code[k] == kEllPad) continue;
+            if constexpr (D == 3) w[k] = load_Sw<D>(a, code[k] >= 0 ? code[k] : ~code[k], S[k]);
+            f(code[k], nb[k], S[k], w[k]);
+        }
     } else {
-        for (int e = a.cfOff[c]; e < a.cfOff[c + 1]; ++e) f(a.cfList[e], a.cfNbr[e]);
+        sync();
+        for (int e = a.cfOff[c]; e < a.cfOff[c + 1]; ++e) {
+            const int code = a.cfList[e];
+            float S[D];
+            const float w = load_Sw<D>(a, code >= 0 ? code : ~code, S);
+            f(code, a.cfNbr[e], S, w);
+        }
     }
 }
 
@@ -515,20 +541,23 @@ __device__ __forceinline__ void for_entries32(const Args<float>& a, int c, F f) 
 // grad32: Gauss gradients of rho', p' and u' (those of rho, p and u up to
 // the reference state's closed-cell sum) for M2AUSM's minmod reconstruction.
 // ---------------------------------------------------------------------------
-template <int D, bool ELL>
-__device__ __forceinline__ void grad32(const Args<float>& a, int c) {
+template <int D, bool ELL, class Sync = NoWait>
+__device__ __forceinline__ void grad32(const Args<float>& a, int c, Sync sync = Sync()) {
     const RefState32& R = a.ref;
     float G[kGradStride<D>];   // rho, p, u gradients
 #pragma unroll
     for (int k = 0; k < kGradStride<D>; ++k) G[k] = 0.0f;
     const float vi = a.volInv32[c];
     Prim32<D> self;
-    load_prim<D>(a, c, self);
-    const float cpr = pressure_dev(R, self.r, self.R);
-    for_entries32<D, ELL>(a, c, [&](int code, int o) {
+    float cpr;
+    auto own_values = [&] {
+        sync();
+        load_prim<D>(a, c, self);
+        cpr = pressure_dev(R, self.r, self.R);
+    };
+    for_entries32<D, ELL>(a, c, own_values, [&](int code, int o, const float* S, float w) {
         const bool own = code >= 0;   // c is the face's P side
-        float S[D], uu[D];
-        const float w = load_Sw<D>(a, own ? code : ~code, S);
+        float uu[D];
         Prim32<D> oth;
         load_prim<D>(a, o, oth);
         const float opr = pressure_dev(R, oth.r, oth.R);
@@ -558,8 +587,8 @@ __device__ __forceinline__ void grad32(const Args<float>& a, int c) {
 // vis32: dudx and dTdx from u' and T', sigmaU = (U_inf + u') . tau.
 // ---------------------------------------------------------------------------
 // LES compiles in the Smagorinsky SGS stress (cases with a.smagC).
-template <int D, bool LES, bool ELL>
-__device__ __forceinline__ void vis32(const Args<float>& a, int c) {
+template <int D, bool LES, bool ELL, class Sync = NoWait>
+__device__ __forceinline__ void vis32(const Args<float>& a, int c, Sync sync = Sync()) {
     float g[D][D], gT[D];
 #pragma unroll
     for (int k = 0; k < D; ++k) {
@@ -570,11 +599,13 @@ __device__ __forceinline__ void vis32(const Args<float>& a, int c) {
     const float vi = a.volInv32[c];
     const float Rinv = a.ref.Rinv;
     float cu[D], cR;
-    load_uR<D>(a, c, cu, cR);
-    for_entries32<D, ELL>(a, c, [&](int code, int o) {
+    auto own_values = [&] {
+        sync();
+        load_uR<D>(a, c, cu, cR);
+    };
+    for_entries32<D, ELL>(a, c, own_values, [&](int code, int o, const float* S, float w) {
         const bool own = code >= 0;   // c is the face's P side
-        float S[D], ou[D], oR, so[D], fU[D];
-        const float w = load_Sw<D>(a, own ? code : ~code, S);
+        float ou[D], oR, so[D], fU[D];
         load_uR<D>(a, o, ou, oR);
 #pragma unroll
         for (int k = 0; k < D; ++k) {
@@ -826,13 +857,14 @@ __device__ __forceinline__ void face_rhs32_core(const A& a, int f, int i, int j,
     }
 }
 
-template <int D, int SCH, bool VIS = true, bool LES = false, bool EARLYV = false>
-__device__ __forceinline__ void flux32(const Args<float>& a, int f) {
+template <int D, int SCH, bool VIS = true, bool LES = false, bool EARLYV = false, class Sync = NoWait>
+__device__ __forceinline__ void flux32(const Args<float>& a, int f, Sync sync = Sync()) {
     Face32<D> geo;
     Prim32<D> pi, pj;
     int i, j;
     bool ghost;
     load_face<D>(a, f, geo, i, j, ghost);
+    sync();
     load_prim<D>(a, i, pi);
     load_prim<D>(a, j, pj);
     float rhs[D + 2];
@@ -854,17 +886,18 @@ __device__ __forceinline__ void flux32(const Args<float>& a, int f) {
 // index one face ahead. The rhs is face_rhs32_core's, so it keeps flux32's
 // bits. M1 / M2 without the LES terms.
 // ---------------------------------------------------------------------------
-template <int D, int SCH>
-__device__ __forceinline__ void flux32_cell(const Args<float>& a, int c) {
+template <int D, int SCH, class Sync = NoWait>
+__device__ __forceinline__ void flux32_cell(const Args<float>& a, int c, Sync sync = Sync()) {
     static_assert(SCH != kSchemeAUSM, "the cell-centred flux holds no sound speed or gradients");
     const int f0 = a.fOwn[c], f1 = a.fOwn[c + 1];
     if (f0 >= f1) return;
     const bool vis = a.ref.mu != 0.0f;
+    int nn = a.fN[f0];
+    sync();
     Prim32<D> self;
     load_prim<D>(a, c, self);
     float Vc[kVisVec<D>];
     if (vis) load_vis<D, false>(a, c, Vc);
-    int nn = a.fN[f0];
     for (int f = f0; f < f1; ++f) {
         const int n = nn;
         if (f + 1 < f1) nn = a.fN[f + 1];
@@ -909,27 +942,35 @@ __device__ __forceinline__ void flux32_cell(const Args<float>& a, int c) {
 // stage's primitives go to a.primW, the other of two buffers (the cells of
 // this launch still read a.prim). The cell's own values are read once.
 // ---------------------------------------------------------------------------
-template <int D, int SCH, bool VIS, bool RES, bool GH, bool ELL>
-__device__ __forceinline__ void fluxupdate32(const Args<float>& a, int c, double Ak, double Bk, double dt,
-                                             float dt32, int first) {
+template <int D, int SCH, bool VIS, bool GH, bool ELL, class Sync = NoWait>
+__device__ __forceinline__ void fluxupdate32(const Args<float>& a, int c, double Ak, double Bk, float dt32, int first,
+                                             bool res, Sync sync = Sync()) {
     constexpr int NQ = D + 2;
     CellIn32<D> in;
-    load_cell32<D>(a, c, first, in);
     Prim32<D> self;
-    load_prim<D>(a, c, self);
     constexpr bool needV = VIS || SCH == kSchemeAUSM;
     float Vc[needV ? kVisVec<D> : 1];
-    if constexpr (needV) load_vis<D, false>(a, c, Vc);
+    auto own_values = [&] {
+        load_cell32<D, GH>(a, c, first, in, sync);
+        load_prim<D>(a, c, self);
+        if constexpr (needV) load_vis<D, false>(a, c, Vc);
+    };
     float sum[NQ];
 #pragma unroll
     for (int v = 0; v < NQ; ++v) sum[v] = 0.0f;
-    for_entries32<D, ELL>(a, c, [&](int code, int o) {
+    for_entries32<D, ELL>(a, c, own_values, [&](int code, int o, const float* S, float w) {
         const bool own = code >= 0;
         const int f = own ? code : ~code;
         Face32<D> geo;
-        int i, j;
-        bool ghost;
-        load_face<D>(a, f, geo, i, j, ghost);
+        bool ghost = false;
+        if constexpr (VIS) {
+            int i, j;
+            load_face<D>(a, f, geo, i, j, ghost);
+        } else {   // S and w suffice without the viscous terms
+#pragma unroll
+            for (int k = 0; k < D; ++k) geo.S[k] = S[k];
+            geo.w = w;
+        }
         Prim32<D> oth, pi, pj;
         load_prim<D>(a, o, oth);
 #pragma unroll
@@ -959,7 +1000,7 @@ __device__ __forceinline__ void fluxupdate32(const Args<float>& a, int c, double
 #pragma unroll
         for (int v = 0; v < NQ; ++v) sum[v] += own ? r[v] : neg_bits(r[v]);
     });
-    apply32<D, RES, GH>(a, c, sum, in, Ak, Bk, dt, dt32, first);
+    apply32<D, GH>(a, c, sum, in, Ak, Bk, dt32, first, res);
 }
 
 }  // namespace dev

@@ -13,6 +13,7 @@ namespace dev {
 template <typename T, int D>
 __global__ void __launch_bounds__(256) k_prep(Args<T> a, int first) {
     const int t = first + LFM_GLOBAL_ID();
+    PdlWait{a.pdl}();
     if (t >= a.nt) return;
     constexpr int NQ = D + 2;
     double qv[NQ];
@@ -34,6 +35,39 @@ __device__ __forceinline__ void load_vec(const double* p, size_t i, double* out)
     }
 }
 
+// Calls f(j, so) for every face entry of cell c (the cell j across it and its
+// constant cfSoN). The entries of an ordinary cell are loaded together, in 2D
+// with their constants, before sync(), so that after it the gathers from the
+// cells across start at once.
+template <int D, class Sync, class F>
+__device__ __forceinline__ void for_entries64(const Args<double>& a, int c, Sync sync, F f) {
+    constexpr int W = kEllWidth<D>;
+    const int e0 = a.cfOff[c], n = a.cfOff[c + 1] - e0;
+    if (n <= W) {
+        int nb[W];
+        double so[W][D];
+#pragma unroll
+        for (int k = 0; k < W; ++k) {
+            nb[k] = k < n ? a.cfNbr[e0 + k] : 0;
+            if (D == 2 && k < n) load_vec<D>(a.cfSoN, (size_t)(e0 + k), so[k]);
+        }
+        sync();
+#pragma unroll
+        for (int k = 0; k < W; ++k) {
+            if (k >= n) continue;
+            if (D == 3) load_vec<D>(a.cfSoN, (size_t)(e0 + k), so[k]);
+            f(nb[k], so[k]);
+        }
+    } else {
+        sync();
+        for (int e = e0; e < e0 + n; ++e) {
+            double so[D];
+            load_vec<D>(a.cfSoN, (size_t)e, so);
+            f(a.cfNbr[e], so);
+        }
+    }
+}
+
 // ---------------------------------------------------------------------------
 // k_grad: gradients read by M2AUSM's minmod reconstruction.
 // ---------------------------------------------------------------------------
@@ -52,9 +86,10 @@ __global__ void __launch_bounds__(256) k_grad(Args<T> a) {
     // constant cellSoW, each neighbour's through the entry constant cfSoN
     // (the face values w v_P + (1 - w) v_N expanded)
     const size_t nt = (size_t)a.nt;
-    {
+    auto own = [&] {
         T sw[D], Uc[D];
         load_vec<D>(a.cellSoW, (size_t)c, sw);
+        PdlWait{a.pdl}();
 #pragma unroll
         for (int k = 0; k < D; ++k) Uc[k] = a.prim[(size_t)(1 + k) * nt + c];
         const T rhoc = a.q[c];
@@ -66,11 +101,8 @@ __global__ void __launch_bounds__(256) k_grad(Args<T> a) {
 #pragma unroll
             for (int b = 0; b < D; ++b) gu[b][x] = Uc[b] * sw[x];
         }
-    }
-    for (int e = a.cfOff[c]; e < a.cfOff[c + 1]; ++e) {
-        const int j = a.cfNbr[e];
-        T so[D];
-        load_vec<D>(a.cfSoN, (size_t)e, so);
+    };
+    for_entries64<D>(a, c, own, [&](int j, const T* so) {
         const T rhoj = a.q[j];
         const T pj = rhoj * a.prim[(size_t)(D + 1) * nt + j];
 #pragma unroll
@@ -80,7 +112,7 @@ __global__ void __launch_bounds__(256) k_grad(Args<T> a) {
 #pragma unroll
             for (int b = 0; b < D; ++b) gu[b][x] += a.prim[(size_t)(1 + b) * nt + j] * so[x];
         }
-    }
+    });
 #pragma unroll
     for (int k = 0; k < D; ++k) {
         a.grad[(size_t)k * a.nt + c] = gr[k];
@@ -110,22 +142,22 @@ __global__ void __launch_bounds__(256) k_vis(Args<T> a) {
     // and so = S/V seen from c, sum_f v_f so = v_c cellSoW_c + sum_e v_j
     // cfSoN_e: the cell's own share through one cell constant, each
     // neighbour's through an entry constant (the other cell j = cfNbr[e]).
-    {
+    T U[D];
+    auto own = [&] {
         T sw[D];
         load_vec<D>(a.cellSoW, (size_t)c, sw);
+        PdlWait{a.pdl}();
         const T Rc = a.prim[(size_t)(D + 1) * a.nt + c];
 #pragma unroll
         for (int x = 0; x < D; ++x) {
-            const T Ux = a.prim[(size_t)(1 + x) * a.nt + c];
+            U[x] = a.prim[(size_t)(1 + x) * a.nt + c];
 #pragma unroll
-            for (int y = 0; y < D; ++y) g[x][y] = Ux * sw[y];
+            for (int y = 0; y < D; ++y) g[x][y] = U[x] * sw[y];
             gT[x] = Rc * sw[x];
         }
-    }
-    for (int e = a.cfOff[c]; e < a.cfOff[c + 1]; ++e) {
-        const int j = a.cfNbr[e];
-        T so[D], fU[D];
-        load_vec<D>(a.cfSoN, (size_t)e, so);
+    };
+    for_entries64<D>(a, c, own, [&](int j, const T* so) {
+        T fU[D];
 #pragma unroll
         for (int k = 0; k < D; ++k) fU[k] = a.prim[(size_t)(1 + k) * a.nt + j];
         const T fR = a.prim[(size_t)(D + 1) * a.nt + j];
@@ -135,13 +167,10 @@ __global__ void __launch_bounds__(256) k_vis(Args<T> a) {
             for (int y = 0; y < D; ++y) g[x][y] += fU[x] * so[y];
             gT[x] += fR * so[x];
         }
-    }
+    });
     const T mu = (T)a.mu;
     T tau[D][D];
     stress<T, D>(g, mu, tau);
-    T U[D];
-#pragma unroll
-    for (int k = 0; k < D; ++k) U[k] = a.prim[(size_t)(1 + k) * a.nt + c];
     const size_t nt = (size_t)a.nt;
 #pragma unroll
     for (int x = 0; x < D; ++x) {
@@ -175,6 +204,7 @@ __global__ void __launch_bounds__(128) k_flux(Args<T> a) {
     T S[D];
 #pragma unroll
     for (int k = 0; k < D; ++k) S[k] = a.S[k * nf + f];
+    PdlWait{a.pdl}();
     T qi[NQ], qj[NQ];
 #pragma unroll
     for (int v = 0; v < NQ; ++v) {
@@ -404,7 +434,7 @@ template <typename T, int D, bool RES>
 __global__ void __launch_bounds__(256) k_update(const __grid_constant__ Args<T> a, double Ak, double Bk, double dt, int first) {
     const int c = LFM_GLOBAL_ID();
     if (c >= a.nc) return;
-    update_cell<T, D, RES, true>(a, c, Ak, Bk, dt, first);
+    update_cell<T, D, RES, true>(a, c, Ak, Bk, dt, first, PdlWait{a.pdl});
 }
 
 // ---------------------------------------------------------------------------
@@ -495,8 +525,8 @@ __global__ void k_set_flag(int* flag, int v) { *flag = v; }
 static inline unsigned blocks(int n, int b) { return (unsigned)((n + b - 1) / b); }
 
 template <typename T, int D, int SCH, bool LES>
-void launch_flux(const Args<T>& a, cudaStream_t st) {
-    k_flux<T, D, SCH, LES><<<blocks(a.nf, 128), 128, 0, st>>>(a);
+void launch_flux(const Args<T>& a, const StageConfig& s, cudaStream_t st) {
+    launch_kernel_pdl(s.pdl && a.pdl, k_flux<T, D, SCH, LES>, blocks(a.nf, 128), 128, st, a);
 }
 
 template <typename T, int D, bool LES>
@@ -506,23 +536,23 @@ void launch_fp64(const Args<T>& a, const StageConfig& s, int which, cudaStream_t
             // the update keeps the cells' and (a.cellGhosts) the ghosts'
             // primitives current: only halos remain, unless the state is new
             const int first = s.fullPrep ? 0 : (a.cellGhosts ? a.nc + a.ng : a.nc);
-            if (a.nt > first) k_prep<T, D><<<blocks(a.nt - first, 256), 256, 0, st>>>(a, first);
+            if (a.nt > first) launch_kernel_pdl(s.pdl && a.pdl, k_prep<T, D>, blocks(a.nt - first, 256), 256, st, a, first);
             break;
         }
         case 1:
-            if (s.needGrad) k_grad<T, D><<<blocks(a.nc, 256), 256, 0, st>>>(a);
+            if (s.needGrad) launch_kernel_pdl(s.pdl && a.pdl, k_grad<T, D>, blocks(a.nc, 256), 256, st, a);
             break;
         case 2:
-            if (s.needVis) k_vis<T, D, LES><<<blocks(a.nc, 256), 256, 0, st>>>(a);
+            if (s.needVis) launch_kernel_pdl(s.pdl && a.pdl, k_vis<T, D, LES>, blocks(a.nc, 256), 256, st, a);
             break;
         case 3:
-            if (s.scheme == kSchemeM1) launch_flux<T, D, kSchemeM1, LES>(a, st);
-            else if (s.scheme == kSchemeM2) launch_flux<T, D, kSchemeM2, LES>(a, st);
-            else launch_flux<T, D, kSchemeAUSM, LES>(a, st);
+            if (s.scheme == kSchemeM1) launch_flux<T, D, kSchemeM1, LES>(a, s, st);
+            else if (s.scheme == kSchemeM2) launch_flux<T, D, kSchemeM2, LES>(a, s, st);
+            else launch_flux<T, D, kSchemeAUSM, LES>(a, s, st);
             break;
         case 4:
-            if (s.withRes) k_update<T, D, true><<<blocks(a.nc, 256), 256, 0, st>>>(a, s.A, s.B, s.dt, s.first);
-            else k_update<T, D, false><<<blocks(a.nc, 256), 256, 0, st>>>(a, s.A, s.B, s.dt, s.first);
+            if (s.withRes) launch_kernel_pdl(s.pdl && a.pdl, k_update<T, D, true>, blocks(a.nc, 256), 256, st, a, s.A, s.B, s.dt, s.first);
+            else launch_kernel_pdl(s.pdl && a.pdl, k_update<T, D, false>, blocks(a.nc, 256), 256, st, a, s.A, s.B, s.dt, s.first);
             break;
         default: break;
     }

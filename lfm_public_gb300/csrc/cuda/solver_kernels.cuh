@@ -148,6 +148,8 @@ struct Args {
     int primC;
     // error flag (non-finite state)
     int* flag;
+    // the step's kernels are launched as programmatic dependents (pdl_pays)
+    int pdl;
 };
 
 }  // namespace dev

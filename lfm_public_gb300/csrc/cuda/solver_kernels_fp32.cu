@@ -13,25 +13,26 @@ namespace dev {
 template <int D>
 __global__ void __launch_bounds__(256) k_prep32(const __grid_constant__ Args<float> a, int first) {
     const int t = first + LFM_GLOBAL_ID();
+    PdlWait{a.pdl}();
     if (t < a.nt) prep32<D>(a, t);
 }
 
 template <int D, bool ELL>
 __global__ void __launch_bounds__(256) k_grad32(const __grid_constant__ Args<float> a) {
     const int c = LFM_GLOBAL_ID();
-    if (c < a.nc) grad32<D, ELL>(a, c);
+    if (c < a.nc) grad32<D, ELL>(a, c, PdlWait{a.pdl});
 }
 
 template <int D, bool LES, bool ELL>
 __global__ void __launch_bounds__(256) k_vis32(const __grid_constant__ Args<float> a) {
     const int c = LFM_GLOBAL_ID();
-    if (c < a.nc) vis32<D, LES, ELL>(a, c);
+    if (c < a.nc) vis32<D, LES, ELL>(a, c, PdlWait{a.pdl});
 }
 
 template <int D, int SCH, bool LES>
 __global__ void __launch_bounds__(256) k_flux32(const __grid_constant__ Args<float> a) {
     const int f = LFM_GLOBAL_ID();
-    if (f < a.nf) flux32<D, SCH, true, LES, true>(a, f);
+    if (f < a.nf) flux32<D, SCH, true, LES, true>(a, f, PdlWait{a.pdl});
 }
 
 // Cell-centred form (flux32_cell): one thread per cell over the faces it
@@ -41,7 +42,7 @@ __global__ void __launch_bounds__(256) k_flux32(const __grid_constant__ Args<flo
 template <int D, int SCH>
 __global__ void __launch_bounds__(256, 3) k_flux32_cell(const __grid_constant__ Args<float> a) {
     const int c = LFM_GLOBAL_ID();
-    if (c < a.nc) flux32_cell<D, SCH>(a, c);
+    if (c < a.nc) flux32_cell<D, SCH>(a, c, PdlWait{a.pdl});
 }
 
 // Warp-interleaved cells: warp j of block b updates the 32 cells of chunk
@@ -54,34 +55,33 @@ __global__ void __launch_bounds__(256, 3) k_flux32_cell(const __grid_constant__ 
 // finish last. Without the ghost work (GH false) a block keeps 256
 // consecutive cells, which the large cases' gathers from HBM prefer.
 template <int D, bool RES, bool GH, bool ELL>
-__device__ __forceinline__ void update_thread(const Args<float>& a, double Ak, double Bk, double dt, float dt32,
-                                              int first) {
+__device__ __forceinline__ void update_thread(const Args<float>& a, double Ak, double Bk, float dt32, int first) {
     const int c = GH ? (int)(((threadIdx.x >> 5) * gridDim.x + blockIdx.x) << 5) + (int)(threadIdx.x & 31u)
                      : (int)LFM_GLOBAL_ID();
-    if (c < a.nc) update32<D, RES, GH, ELL>(a, c, Ak, Bk, dt, dt32, first);
+    if (c < a.nc) update32<D, GH, ELL ? kEntriesEll : kEntriesList>(a, c, Ak, Bk, dt32, first, RES, PdlWait{a.pdl});
 }
 
 template <int D, bool RES, bool GH, bool ELL>
 __global__ void __launch_bounds__(256) k_update32(const __grid_constant__ Args<float> a, double Ak, double Bk,
-                                                  double dt, float dt32, int first) {
-    update_thread<D, RES, GH, ELL>(a, Ak, Bk, dt, dt32, first);
+                                                  float dt32, int first) {
+    update_thread<D, RES, GH, ELL>(a, Ak, Bk, dt32, first);
 }
 
 // Fused flux + update (fluxupdate32): one thread per cell, cells mapped as
 // in the update kernel that writes ghosts (warp-interleaved chunks).
 template <int D, int SCH, bool VIS, bool RES, bool ELL>
 __global__ void __launch_bounds__(256) k_fluxupdate32(const __grid_constant__ Args<float> a, double Ak, double Bk,
-                                                      double dt, float dt32, int first) {
+                                                      float dt32, int first) {
     const int c = (int)(((threadIdx.x >> 5) * gridDim.x + blockIdx.x) << 5) + (int)(threadIdx.x & 31u);
-    if (c < a.nc) fluxupdate32<D, SCH, VIS, RES, true, ELL>(a, c, Ak, Bk, dt, dt32, first);
+    if (c < a.nc) fluxupdate32<D, SCH, VIS, true, ELL>(a, c, Ak, Bk, dt32, first, RES, PdlWait{a.pdl});
 }
 
 template <int D, int SCH, bool VIS, bool ELL>
 void launch_fluxupdate32_kernel(const Args<float>& a, const StageConfig& s, cudaStream_t st) {
     const unsigned nb = (unsigned)((a.nc + 255) / 256);
     const float dt32 = (float)s.dt;
-    if (s.withRes) k_fluxupdate32<D, SCH, VIS, true, ELL><<<nb, 256, 0, st>>>(a, s.A, s.B, s.dt, dt32, s.first);
-    else k_fluxupdate32<D, SCH, VIS, false, ELL><<<nb, 256, 0, st>>>(a, s.A, s.B, s.dt, dt32, s.first);
+    if (s.withRes) launch_kernel_pdl(s.pdl && a.pdl, k_fluxupdate32<D, SCH, VIS, true, ELL>, nb, 256, st, a, s.A, s.B, dt32, s.first);
+    else launch_kernel_pdl(s.pdl && a.pdl, k_fluxupdate32<D, SCH, VIS, false, ELL>, nb, 256, st, a, s.A, s.B, dt32, s.first);
 }
 
 template <int D, int SCH>
@@ -100,11 +100,11 @@ void launch_update32(const Args<float>& a, const StageConfig& s, cudaStream_t st
     const unsigned nb = (unsigned)((a.nc + 255) / 256);   // eight 32-cell chunks per block
     const float dt32 = (float)s.dt;
     if (a.cellGhosts) {
-        if (s.withRes) k_update32<D, true, true, ELL><<<nb, 256, 0, st>>>(a, s.A, s.B, s.dt, dt32, s.first);
-        else k_update32<D, false, true, ELL><<<nb, 256, 0, st>>>(a, s.A, s.B, s.dt, dt32, s.first);
+        if (s.withRes) launch_kernel_pdl(s.pdl && a.pdl, k_update32<D, true, true, ELL>, nb, 256, st, a, s.A, s.B, dt32, s.first);
+        else launch_kernel_pdl(s.pdl && a.pdl, k_update32<D, false, true, ELL>, nb, 256, st, a, s.A, s.B, dt32, s.first);
     } else {
-        if (s.withRes) k_update32<D, true, false, ELL><<<nb, 256, 0, st>>>(a, s.A, s.B, s.dt, dt32, s.first);
-        else k_update32<D, false, false, ELL><<<nb, 256, 0, st>>>(a, s.A, s.B, s.dt, dt32, s.first);
+        if (s.withRes) launch_kernel_pdl(s.pdl && a.pdl, k_update32<D, true, false, ELL>, nb, 256, st, a, s.A, s.B, dt32, s.first);
+        else launch_kernel_pdl(s.pdl && a.pdl, k_update32<D, false, false, ELL>, nb, 256, st, a, s.A, s.B, dt32, s.first);
     }
 }
 
@@ -132,35 +132,36 @@ void launch_fp32(const Args<float>& a, const StageConfig& s, int which, cudaStre
     switch (which) {
         case 0: {
             const int first = s.fullPrep ? 0 : (a.cellGhosts ? a.nc + a.ng : a.nc);
-            if (a.nt > first) k_prep32<D><<<nblocks(a.nt - first, 256), 256, 0, st>>>(a, first);
+            // not as a dependent: few blocks of FP64 work, crowded when released early
+            if (a.nt > first) launch_kernel_pdl(false, k_prep32<D>, nblocks(a.nt - first, 256), 256, st, a, first);
             break;
         }
         case 1:
-            if (s.needGrad && a.cfEll) k_grad32<D, true><<<nblocks(a.nc, 256), 256, 0, st>>>(a);
-            else if (s.needGrad) k_grad32<D, false><<<nblocks(a.nc, 256), 256, 0, st>>>(a);
+            if (s.needGrad && a.cfEll) launch_kernel_pdl(s.pdl && a.pdl, k_grad32<D, true>, nblocks(a.nc, 256), 256, st, a);
+            else if (s.needGrad) launch_kernel_pdl(s.pdl && a.pdl, k_grad32<D, false>, nblocks(a.nc, 256), 256, st, a);
             break;
         case 2:
             if (!s.needVis) break;
-            if (a.smagC && a.cfEll) k_vis32<D, true, true><<<nblocks(a.nc, 256), 256, 0, st>>>(a);
-            else if (a.smagC) k_vis32<D, true, false><<<nblocks(a.nc, 256), 256, 0, st>>>(a);
-            else if (a.cfEll) k_vis32<D, false, true><<<nblocks(a.nc, 256), 256, 0, st>>>(a);
-            else k_vis32<D, false, false><<<nblocks(a.nc, 256), 256, 0, st>>>(a);
+            if (a.smagC && a.cfEll) launch_kernel_pdl(s.pdl && a.pdl, k_vis32<D, true, true>, nblocks(a.nc, 256), 256, st, a);
+            else if (a.smagC) launch_kernel_pdl(s.pdl && a.pdl, k_vis32<D, true, false>, nblocks(a.nc, 256), 256, st, a);
+            else if (a.cfEll) launch_kernel_pdl(s.pdl && a.pdl, k_vis32<D, false, true>, nblocks(a.nc, 256), 256, st, a);
+            else launch_kernel_pdl(s.pdl && a.pdl, k_vis32<D, false, false>, nblocks(a.nc, 256), 256, st, a);
             break;
         case 3:
             if (s.fluxStaging.stages > 0) {   // staged kernel (configured for this scheme, laminar)
                 launch_flux32_staged(a, s, st);
             } else if (a.nf == 0) {
             } else if (a.fOwn && !a.smagC && s.scheme != kSchemeAUSM) {   // cell-centred
-                if (s.scheme == kSchemeM1) k_flux32_cell<D, kSchemeM1><<<nblocks(a.nc, 256), 256, 0, st>>>(a);
-                else k_flux32_cell<D, kSchemeM2><<<nblocks(a.nc, 256), 256, 0, st>>>(a);
+                if (s.scheme == kSchemeM1) launch_kernel_pdl(s.pdl && a.pdl, k_flux32_cell<D, kSchemeM1>, nblocks(a.nc, 256), 256, st, a);
+                else launch_kernel_pdl(s.pdl && a.pdl, k_flux32_cell<D, kSchemeM2>, nblocks(a.nc, 256), 256, st, a);
             } else if (a.smagC) {   // Smagorinsky LES variants
-                if (s.scheme == kSchemeM1) k_flux32<D, kSchemeM1, true><<<nblocks(a.nf, 256), 256, 0, st>>>(a);
-                else if (s.scheme == kSchemeM2) k_flux32<D, kSchemeM2, true><<<nblocks(a.nf, 256), 256, 0, st>>>(a);
-                else k_flux32<D, kSchemeAUSM, true><<<nblocks(a.nf, 256), 256, 0, st>>>(a);
+                if (s.scheme == kSchemeM1) launch_kernel_pdl(s.pdl && a.pdl, k_flux32<D, kSchemeM1, true>, nblocks(a.nf, 256), 256, st, a);
+                else if (s.scheme == kSchemeM2) launch_kernel_pdl(s.pdl && a.pdl, k_flux32<D, kSchemeM2, true>, nblocks(a.nf, 256), 256, st, a);
+                else launch_kernel_pdl(s.pdl && a.pdl, k_flux32<D, kSchemeAUSM, true>, nblocks(a.nf, 256), 256, st, a);
             } else {
-                if (s.scheme == kSchemeM1) k_flux32<D, kSchemeM1, false><<<nblocks(a.nf, 256), 256, 0, st>>>(a);
-                else if (s.scheme == kSchemeM2) k_flux32<D, kSchemeM2, false><<<nblocks(a.nf, 256), 256, 0, st>>>(a);
-                else k_flux32<D, kSchemeAUSM, false><<<nblocks(a.nf, 256), 256, 0, st>>>(a);
+                if (s.scheme == kSchemeM1) launch_kernel_pdl(s.pdl && a.pdl, k_flux32<D, kSchemeM1, false>, nblocks(a.nf, 256), 256, st, a);
+                else if (s.scheme == kSchemeM2) launch_kernel_pdl(s.pdl && a.pdl, k_flux32<D, kSchemeM2, false>, nblocks(a.nf, 256), 256, st, a);
+                else launch_kernel_pdl(s.pdl && a.pdl, k_flux32<D, kSchemeAUSM, false>, nblocks(a.nf, 256), 256, st, a);
             }
             break;
         case 4:

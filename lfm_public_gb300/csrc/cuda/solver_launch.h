@@ -20,8 +20,46 @@ struct FluxStaging {
     size_t smem = 0;
 };
 
+// Whether a case's step launches its kernels as programmatic dependents
+// (PdlWait, solver_device.cuh). A dependent's blocks go where room appears
+// first; one with fewer blocks than the chip holds at once is crowded onto part
+// of the SMs, and FP64 work then waits for their FP64 pipes, while a larger one
+// fills every SM anyway and a very small one finds idle SMs. Measured on GB300,
+// us a step without and with:
+//   FP64 2D   4k cells  65.5  57.3 |  16k  67.6  64.1 |  33k 129.0 131.0 | 66k 190.4 231.4
+//           101k cells 255.9 272.4 | 135k 330.7 311.3 | 393k 798.7 772.1
+//   FP64 3D   5k cells 157.7 147.4 |  18k 184.3 194.5 |  43k 305.2 343.5 | 83k 460.7 475.0
+//           117k cells 608.2 587.7 | 229k 1047.5 1029.1
+//   FP32 2D   4k cells  45.1  43.0 |  16k  47.1  43.0 | 101k  73.7  65.5 | 393k 157.6 143.3
+//   FP32 3D   5k cells  94.2  86.0 |  43k 104.4  98.4 |  61k 114.7 118.8 | 83k 124.9 126.9
+//           117k cells 133.1 131.0 | 229k 209.9 200.7
+inline bool pdl_pays(bool fp64, int D, int nc) {
+    if (nc >= 114688) return true;
+    if (fp64) return nc <= (D == 2 ? 16384 : 8192);
+    return D == 2 || nc <= 49152;
+}
+
+// Launches k, with `pdl` as a programmatic dependent of the stream's previous
+// kernel (PdlWait, solver_device.cuh).
+template <class... P, class... V>
+inline void launch_kernel_pdl(bool pdl, void (*k)(P...), unsigned grid, unsigned block, cudaStream_t st, V... args) {
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3(grid);
+    cfg.blockDim = dim3(block);
+    cfg.stream = st;
+    cudaLaunchAttribute attr[1];
+    attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr[0].val.programmaticStreamSerializationAllowed = 1;
+    cfg.attrs = attr;
+    cfg.numAttrs = pdl ? 1 : 0;
+    cudaLaunchKernelEx(&cfg, k, P(args)...);
+}
+
 // What one RK stage runs (src/mesh_solver.cpp:500-672).
 struct StageConfig {
+    // the kernel follows another of the same chain (or nothing) on its stream:
+    // with Args::pdl it is launched as its programmatic dependent
+    bool pdl = false;
     int scheme = 0;       // kSchemeM1 / M2 / AUSM
     bool needGrad = false;
     bool needVis = true;

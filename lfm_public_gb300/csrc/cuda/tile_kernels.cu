@@ -30,7 +30,7 @@ struct TileRows {
 template <int D, int SCH, bool RES>
 __global__ void __launch_bounds__(256) k_tile_stage(const __grid_constant__ Args<float> g,
                                                     const __grid_constant__ TileArgs t, double Ak, double Bk,
-                                                    double dt, float dt32, int first) {
+                                                    float dt32, int first) {
     using R = TileRows<D>;
     extern __shared__ float sm[];
     __shared__ Args<float> la;
@@ -95,10 +95,10 @@ __global__ void __launch_bounds__(256) k_tile_stage(const __grid_constant__ Args
     __syncthreads();
     for (int lc = threadIdx.x; lc < td.nA; lc += blockDim.x) {
         CellIn32<D> in;
-        load_cell32<D>(g, td.c0 + lc, first, in);
+        load_cell32<D, true>(g, td.c0 + lc, first, in);
         float sum[R::Q];
         gather32<D>(a, lc, sum);
-        apply32<D, RES, true>(g, td.c0 + lc, sum, in, Ak, Bk, dt, dt32, first);
+        apply32<D, true>(g, td.c0 + lc, sum, in, Ak, Bk, dt32, first, RES);
     }
 }
 
@@ -113,7 +113,7 @@ cudaError_t launchTiles(const Args<float>& g, const TileArgs& t, const StageConf
         if (e != cudaSuccess) return e;
         smemSet[s.withRes ? 1 : 0] = smem;
     }
-    k<<<t.nTiles, t.block, smem, st>>>(g, t, s.A, s.B, s.dt, (float)s.dt, s.first);
+    k<<<t.nTiles, t.block, smem, st>>>(g, t, s.A, s.B, (float)s.dt, s.first);
     return cudaGetLastError();
 }
 
