@@ -827,21 +827,24 @@ namespace {
 
 // The state upload of lfm_solver_set_state, enqueued on the solver stream.
 int enqueueSetState(lfm_solver* s, const double* q) {
-    // a new state starts with a clear non-finite flag
-    LFM_CUDA(cudaMemsetAsync(s->flag, 0, sizeof(int), s->stream));
+    // one pass writes the stored state, the primitives of the cells and those
+    // of the ghosts that the update keeps, and clears the non-finite flag: the
+    // per-stage preparation covers the other ghosts and halos
     const size_t nc = (size_t)s->nc;
+    const double* direct = lfm::dev::kernel_address(q);
     if (s->precision == LFM_FP32_BULK) {   // stored as q - q_ref
-        LFM_CUDA(cudaMemcpyAsync(s->stage, q, (size_t)s->nq * nc * sizeof(double), cudaMemcpyHostToDevice,
-                                 s->stream));
-        // q' with the cells' primitives (and the ghosts' the update keeps) in
-        // one pass: the per-stage preparation covers the other ghosts and halos
-        lfm::dev::launch_set_state32(s->a32, s->stage, s->nc, s->stream);
-        LFM_CUDA(cudaGetLastError());
-    } else {   // rows of nc values into rows of nt
-        LFM_CUDA(cudaMemcpy2DAsync(s->q, (size_t)s->nt * sizeof(double), q, nc * sizeof(double),
-                                   nc * sizeof(double), (size_t)s->nq, cudaMemcpyHostToDevice, s->stream));
+        if (!direct)
+            LFM_CUDA(cudaMemcpyAsync(s->stage, q, (size_t)s->nq * nc * sizeof(double), cudaMemcpyHostToDevice,
+                                     s->stream));
+        lfm::dev::launch_set_state32(s->a32, direct ? direct : s->stage, s->nc, s->stream);
+    } else {
+        if (!direct)   // rows of nc values into rows of nt
+            LFM_CUDA(cudaMemcpy2DAsync(s->q, (size_t)s->nt * sizeof(double), q, nc * sizeof(double),
+                                       nc * sizeof(double), (size_t)s->nq, cudaMemcpyHostToDevice, s->stream));
+        lfm::dev::launch_set_state64(s->a64, direct ? direct : s->q, direct ? s->nc : s->nt, s->stream);
     }
-    s->primsValid = s->precision == LFM_FP32_BULK;   // FP64: rebuilt by ensurePrims
+    LFM_CUDA(cudaGetLastError());
+    s->primsValid = true;
     s->primParity = 0;
     s->ghostRowsValid = false;
     return LFM_OK;
@@ -852,8 +855,10 @@ int enqueueGetState(lfm_solver* s, double* q) {
     if (s->precision == LFM_FP32_BULK) {   // stored as q - q_ref
         lfm::dev::QOffset qo;
         for (int v = 0; v < 5; ++v) qo.v[v] = s->qRef[v];
-        lfm::dev::launch_offset_rows(s->stage, s->nc, s->q, s->nt, s->nc, s->nq, qo, 1.0, s->stream);
+        double* direct = lfm::dev::kernel_address(q);
+        lfm::dev::launch_offset_rows(direct ? direct : s->stage, s->nc, s->q, s->nt, s->nc, s->nq, qo, 1.0, s->stream);
         LFM_CUDA(cudaGetLastError());
+        if (direct) return LFM_OK;
         LFM_CUDA(cudaMemcpyAsync(q, s->stage, (size_t)s->nq * s->nc * sizeof(double), cudaMemcpyDeviceToHost,
                                  s->stream));
     } else {
@@ -885,15 +890,6 @@ extern "C" int lfm_solver_get_state(lfm_solver* s, double* q) {
 }
 
 namespace {
-
-bool pageLocked(const void* p) {
-    cudaPointerAttributes at{};
-    if (cudaPointerGetAttributes(&at, p) != cudaSuccess) {
-        cudaGetLastError();
-        return false;
-    }
-    return at.type == cudaMemoryTypeHost;
-}
 
 // The whole advance between page-locked host states as one graph launch
 // (device work only; the host-side state flags are set as the enqueued path
@@ -947,7 +943,7 @@ extern "C" int lfm_solver_advance(lfm_solver* s, const double* q_in, int nsteps,
     if (!s || nsteps < 0) return lfm::setError(LFM_ERR_INVALID, "bad argument");
     LFM_CUDA(cudaSetDevice(s->device));
     int rc = LFM_OK;
-    if (q_in && q_out && nsteps > 0 && s->rkOrder > 0 && pageLocked(q_in) && pageLocked(q_out))
+    if (q_in && q_out && nsteps > 0 && s->rkOrder > 0 && lfm::dev::kernel_address(q_in) && lfm::dev::kernel_address(q_out))
         return advanceGraph(s, q_in, nsteps, dt, q_out);
     if (q_in && (rc = enqueueSetState(s, q_in))) return rc;
     if (nsteps > 0 && (rc = lfm_solver_step(s, nsteps, dt))) return rc;

@@ -21,6 +21,32 @@ __global__ void __launch_bounds__(256) k_prep(Args<T> a, int first) {
     prims64<D>(a, t, qv);
 }
 
+// A new state: the rows of the stored state from the caller's q ([nq][stride];
+// the stored rows themselves after a copy, stride nt), the cells' primitives
+// and (a.cellGhosts) their boundary ghosts' states and primitives, and a clear
+// non-finite flag.
+template <int D>
+__global__ void __launch_bounds__(256) k_set_state64(const __grid_constant__ Args<double> a, const double* q,
+                                                     int64_t stride) {
+    const int c = LFM_GLOBAL_ID();
+    if (c == 0) *a.flag = 0;
+    if (c >= a.nc) return;
+    double qv[D + 2];
+#pragma unroll
+    for (int v = 0; v < D + 2; ++v) {
+        qv[v] = q[(size_t)v * stride + c];
+        a.q[(size_t)v * a.nt + c] = qv[v];
+    }
+    prims64<D>(a, c, qv);
+    if (a.cellGhosts && a.cellGhosts[c]) ghosts_of64<D>(a, c, qv);
+}
+
+void launch_set_state64(const Args<double>& a, const double* q, int64_t stride, cudaStream_t st) {
+    const unsigned nb = (unsigned)((a.nc + 255) / 256);
+    if (a.D == 2) k_set_state64<2><<<nb, 256, 0, st>>>(a, q, stride);
+    else k_set_state64<3><<<nb, 256, 0, st>>>(a, q, stride);
+}
+
 // D consecutive FP64 values starting at an index that is a multiple of D:
 // one 16-byte load in 2D (the constants of an incidence entry or a cell).
 template <int D>
@@ -518,6 +544,15 @@ __global__ void __launch_bounds__(256) k_res_sq(const double* res, int nc, doubl
 }
 
 __global__ void k_set_flag(int* flag, int v) { *flag = v; }
+
+double* kernel_address(const double* p) {
+    cudaPointerAttributes at{};
+    if (cudaPointerGetAttributes(&at, p) != cudaSuccess) {
+        cudaGetLastError();
+        return nullptr;
+    }
+    return at.type == cudaMemoryTypeHost ? static_cast<double*>(at.devicePointer) : nullptr;
+}
 
 // ---------------------------------------------------------------------------
 // Launchers.

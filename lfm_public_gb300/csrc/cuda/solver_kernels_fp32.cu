@@ -112,6 +112,7 @@ template <int D>
 __global__ void __launch_bounds__(256) k_set_state32(const __grid_constant__ Args<float> a, const double* q,
                                                      int64_t stride) {
     const int c = LFM_GLOBAL_ID();
+    if (c == 0) *a.flag = 0;   // a new state starts with a clear non-finite flag
     if (c < a.nc) set_state32<D>(a, q, stride, c);
 }
 

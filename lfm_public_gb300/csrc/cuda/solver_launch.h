@@ -97,6 +97,14 @@ void launch_flux32_staged(const Args<float>& a, const StageConfig& s, cudaStream
 // q' = q - q_ref for the cells of an FP32-bulk solver from an absolute state
 // [nq][stride] on the device.
 void launch_to_perturbation(const Args<float>& a, const double* q, int64_t stride, cudaStream_t st);
+// The address at which kernels read and write page-locked host memory p, or null
+// for other memory. A state in page-locked memory is read and written by the
+// kernels that convert it: the C2C link moves it at the copy engines' rate, and
+// the stream does not change between engine and kernels, which costs a batch
+// of eight cases about 30 us a case.
+double* kernel_address(const double* p);
+// A new FP64 state from an absolute one (or from the stored rows, stride nt).
+void launch_set_state64(const Args<double>& a, const double* q, int64_t stride, cudaStream_t st);
 // A new FP32-bulk state from an absolute one: q', the cells' primitives and
 // (with a.cellGhosts) their boundary ghosts' states and primitives.
 void launch_set_state32(const Args<float>& a, const double* q, int64_t stride, cudaStream_t st);
