@@ -5,7 +5,10 @@
 // arrays of a single-case solver (Args<float>). A stage is four phases over
 // all cases -- ghost states and primitives (of every cell too, right after a
 // case's state was set); gradients and viscous terms; face fluxes; gather, RK
-// update and the cells' next primitives -- separated by grid-wide barriers. Work
+// update and the cells' next primitives -- separated by grid-wide barriers. While
+// every case of a batch is 2D, inviscid and M1 / M2 (fusable), a stage is one
+// phase without a barrier instead: each cell evaluates its own faces and updates,
+// between two primitive buffers that alternate. Work
 // is a flat list of tiles per phase (a tile is a run of consecutive cells or
 // faces of one case); each block takes an equal contiguous range of it, so
 // uneven cases load-balance at tile granularity. The tile lists and case table are read
@@ -52,6 +55,7 @@ struct BatchArgs {
     int* error;                 // set when a grid barrier gives up waiting
     int itemsPerThread;
     unsigned barrierExtra;      // arrivals every barrier waits for beyond the grid's (test aid; 0)
+    int parity;                 // which of a case's two primitive buffers is current
 };
 
 // Kernel variants, chosen from the cases in the batch: compiling out what no
@@ -64,12 +68,28 @@ constexpr int kBatchVariantGeneral = 2;      // 2D and 3D, any scheme, viscous
 // `cooperative`) kernel of `grid` blocks of `block` threads (128, 256 or 512).
 cudaError_t launch_batch_stage(const BatchArgs& b, int stage, int block, int variant, int grid, bool cooperative,
                                cudaStream_t st);
+// Up to kBatchStates cases and their absolute states ([nq][nc], page-locked host
+// or device memory).
+constexpr int kBatchStates = 32;
+struct BatchStates {
+    int slot[kBatchStates];
+    double* q[kBatchStates];
+};
+// The states of n cases in (`set`; parity: BatchArgs) or out.
+cudaError_t launch_batch_states(const BatchCase* cases, const BatchStates& m, int n, int maxCells, bool set, int parity,
+                                cudaStream_t st);
+// Stage `stage` of a batch of fusable cases with current primitives.
+cudaError_t launch_batch_fused(const BatchArgs& b, int stage, int block, int bps, int sms, cudaStream_t st);
 // Resident blocks per SM of the stage kernel at `block` threads.
 int batch_blocks_per_sm(int block, int variant);
-// Stage `stage` as one kernel per phase (grid-stride over each phase's
-// tiles, kernel boundaries in place of the grid barriers); each kernel's grid
-// is bps (0 = all that fit) resident blocks per SM x sms.
-cudaError_t launch_batch_phased(const BatchArgs& b, int stage, int block, int variant, int bps, int sms,
+// Stage `stage` as one kernel per phase with tiles (kernel boundaries in place of
+// the grid barriers); each kernel's grid is at most blocksPerSm (0 = all that
+// fit) resident blocks per SM x sms, and no more than its tiles.
+struct PhasedShape {
+    int tiles[kBatchPhases];
+    int blocksPerSm, sms;
+};
+cudaError_t launch_batch_phased(const BatchArgs& b, int stage, int block, int variant, const PhasedShape& p,
                                 cudaStream_t st);
 
 }  // namespace dev

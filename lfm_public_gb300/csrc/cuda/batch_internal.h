@@ -79,7 +79,8 @@ private:
 // Byte offsets of every array of one case inside its arena block.
 struct CaseLayout {
     size_t total = 0;
-    size_t q, dq, res, prim, V, grad, flux, fG0, fG1, d, dinv, dnorm, fP, fN, volInv32, sponge, cfOff, cfList,
+    bool fusable;   // flux and update at once (fluxupdate32)
+    size_t q, dq, res, prim, prim1, V, grad, flux, fG0, fG1, d, dinv, dnorm, fP, fN, volInv32, sponge, cfOff, cfList,
         cfNbr, cfEll, cfEllN, cellGhosts, gCell, gKind, gFace;
 
     explicit CaseLayout(const lfm_solver_desc* d) {
@@ -90,6 +91,12 @@ struct CaseLayout {
         dq = add(nq * nc * 4);
         res = d->residuals ? add(nq * nc * 8) : npos();
         prim = add((size_t)lfm::dev::primRows<float>(d->dim) * nt * 4);
+        // As in the single-case solver, evaluating each face twice pays where
+        // the flux is short (2D inviscid M1 / M2): a stage then is one phase
+        // without a grid barrier. The second primitive buffer takes the space
+        // the second copy of the face lists took.
+        fusable = D == 2 && !lfm::setup::needVis(d) && !ausm && lfm::setup::ellFits(d);
+        prim1 = fusable ? add((size_t)lfm::dev::primRows<float>(d->dim) * nt * 4) : npos();
         V = lfm::setup::needVis(d) ? add((size_t)lfm::dev::visStride32(d->dim, false) * nt * 4) : npos();
         grad = ausm ? add((size_t)lfm::dev::gradStride32(d->dim) * nt * 4) : npos();
         flux = add(nq * nf * 4);
@@ -130,7 +137,7 @@ struct Slot {
     bool used = false;
     size_t off = 0, bytes = 0;
     int D = 2, nq = 4, nc = 0, ng = 0, nf = 0, nt = 0;
-    bool needGradVis = false;
+    bool needGradVis = false, fusable = false;
     bool primsValid = false;   // cells' primitives current (kept so by the update phase)
     double qRef[5] = {0, 0, 0, 0, 0};   // the device state is q - qRef
     double* q = nullptr;   // device
@@ -174,11 +181,20 @@ struct lfm_batch {
     int* dNTiles = nullptr;
     std::vector<lfm::batch::Slot> slots;
     int sms = 0;
-    lfm_batch_tuning tune{256, 1, 0, 1, 0};
+    // One kernel per phase at 128 threads until a shape is asked for: small
+    // batches are latency-bound, and their phases then overlap as programmatic
+    // dependents where the persistent kernel waits at its grid barriers (three
+    // cases of 11k-29k cells, 2D and 3D: 139 -> 112 us a step, GB300).
+    lfm_batch_tuning tune{128, 1, 0, 1, 1};
     int variant = lfm::dev::kBatchVariantGeneral;   // stage-kernel variant of the current cases
+    bool untuned = true;        // no launch shape was asked for
+    int block = 0;              // threads per block of the current tiles
+    int nTiles[lfm::dev::kBatchPhases] = {};
     int grid = 0;
     bool tilesDirty = true;
-    cudaGraphExec_t graph = nullptr;
+    bool lean = false;          // every case is fusable and has current primitives
+    int parity = 0;             // the fusable cases' current primitive buffer
+    cudaGraphExec_t graph[2][2] = {};   // a step's graph, by [lean][parity]
     cudaEvent_t ev0 = nullptr, ev1 = nullptr;
     void* scrub = nullptr;
     size_t scrubBytes = 0;

@@ -3,6 +3,7 @@
 
 #include "batch.cuh"
 #include "solver_fp32.cuh"
+#include "solver_launch.h"
 
 namespace lfm {
 namespace dev {
@@ -23,25 +24,33 @@ __device__ __forceinline__ unsigned long long global_ns() {
 
 // Grid-wide barrier of the blocks of one launch (all resident: the launch is
 // cooperative, or its grid is sized to the resident capacity). Arrival is an
-// atomic increment after a release fence; waiting is bounded: after about a
-// second, or once another block has given up, the block sets the error flag
-// and the caller returns without touching further data.
-__device__ __forceinline__ bool grid_barrier(unsigned* counter, unsigned target, int* error) {
+// atomic increment after a release fence; between its arrival and its wait the
+// block runs `meanwhile` (loads of what no phase writes). Waiting is bounded:
+// after about a second, or once another block has given up, the block sets the
+// error flag and the caller returns without touching further data. The flag
+// and the timer are read every 64th poll only: with every poll they doubled
+// the time from the last arrival to the wake-up.
+template <class F>
+__device__ __forceinline__ bool grid_barrier(unsigned* counter, unsigned target, int* error, F meanwhile) {
     __shared__ int sOk;
     __syncthreads();
     if (threadIdx.x == 0) {
         __threadfence();
         atomicAdd(counter, 1u);
+    }
+    meanwhile();
+    if (threadIdx.x == 0) {
         int ok = 1;
         unsigned spins = 0;
         const unsigned long long t0 = global_ns();
         while (*(volatile unsigned*)counter < target) {
-            if (*(volatile int*)error != 0 || ++spins > kBarrierSpinLimit || global_ns() - t0 > kBarrierTimeoutNs) {
+            if ((++spins & 63u) == 0 && (*(volatile int*)error != 0 || spins > kBarrierSpinLimit ||
+                                         global_ns() - t0 > kBarrierTimeoutNs)) {
                 atomicOr(error, 1);
                 ok = 0;
                 break;
             }
-            __nanosleep(40);
+            __nanosleep(20);
         }
         __threadfence();
         sOk = ok;
@@ -82,32 +91,62 @@ __device__ __forceinline__ void item(const BatchCase& bc, int stage, int i) {
             flux32<D, kSchemeAUSM, FULL>(a, i);
     } else {
         const int first = stage == 0;
-        update32<D, true, kEntriesEither>(a, i, bc.rkA[stage], bc.rkB[stage], bc.dt32, first, bc.residuals && first);
+        const bool res = bc.residuals && first;
+        update32<D, true, kEntriesEither>(a, i, bc.rkA[stage], bc.rkB[stage], bc.dt32, first, res);
     }
+}
+
+// Makes case `slot` the block's current one (in shared memory), its primitive
+// buffers as the stage reads (in) and writes (out) them: 0 or 1 of its two (a
+// case that is never fused has the same one twice).
+template <int BLOCK>
+__device__ __forceinline__ void load_case(const BatchArgs& b, int slot, int in, int out, BatchCase& sc, int& sSlot) {
+    const bool reload = slot != sSlot;
+    __syncthreads();
+    if (!reload) return;
+    const int4* src = reinterpret_cast<const int4*>(b.cases + slot);
+    int4* dst = reinterpret_cast<int4*>(&sc);
+    constexpr int n16 = (int)(sizeof(BatchCase) / 16);
+    for (int k = threadIdx.x; k < n16; k += BLOCK) dst[k] = src[k];
+    if (threadIdx.x == 0) sSlot = slot;
+    __syncthreads();
+    if (threadIdx.x == 0) {
+        float* buf[2] = {sc.a.prim, sc.a.primW};
+        sc.a.prim = in ? buf[1] : buf[0];
+        sc.a.primW = out ? buf[1] : buf[0];
+    }
+    __syncthreads();
 }
 
 // The tiles of phase PH assigned to this block: a contiguous range of the
 // phase's tile list (neighbouring tiles of a case share cached neighbours).
-// The block keeps the current tile's case in shared memory and reloads it when
-// the case changes.
-template <int PH, int BLOCK, int DIMS, bool FULL>
-__device__ __forceinline__ void phase_tiles(const BatchArgs& b, int stage, BatchCase& sc, int& sSlot) {
+struct BlockTiles {
+    int t0, t1;
+    BatchTile first;
+};
+
+// The block's range of phase PH, its first tile and that tile's case: what the
+// host wrote before the step, so a block loads it while it still waits for the
+// phase before.
+template <int PH, int BLOCK>
+__device__ __forceinline__ BlockTiles block_tiles(const BatchArgs& b, int in, int out, BatchCase& sc, int& sSlot) {
     const int nT = b.nTiles[PH];
-    const long long t0 = (long long)nT * blockIdx.x / gridDim.x;
-    const long long t1 = (long long)nT * (blockIdx.x + 1) / gridDim.x;
-    const BatchTile* tiles = b.tiles[PH];
-    for (long long t = t0; t < t1; ++t) {
-        const BatchTile td = tiles[t];
-        const bool reload = td.slot != sSlot;
-        __syncthreads();
-        if (reload) {
-            const int4* src = reinterpret_cast<const int4*>(b.cases + td.slot);
-            int4* dst = reinterpret_cast<int4*>(&sc);
-            constexpr int n16 = (int)(sizeof(BatchCase) / 16);
-            for (int k = threadIdx.x; k < n16; k += BLOCK) dst[k] = src[k];
-            if (threadIdx.x == 0) sSlot = td.slot;
-            __syncthreads();
-        }
+    BlockTiles r;
+    r.t0 = (int)((long long)nT * blockIdx.x / gridDim.x);
+    r.t1 = (int)((long long)nT * (blockIdx.x + 1) / gridDim.x);
+    if (r.t0 < r.t1) {
+        r.first = b.tiles[PH][r.t0];
+        load_case<BLOCK>(b, r.first.slot, in, out, sc, sSlot);
+    }
+    return r;
+}
+
+template <int PH, int BLOCK, int DIMS, bool FULL>
+__device__ __forceinline__ void phase_tiles(const BatchArgs& b, int stage, const BlockTiles& r, BatchCase& sc,
+                                            int& sSlot) {
+    for (int t = r.t0; t < r.t1; ++t) {
+        const BatchTile td = t == r.t0 ? r.first : b.tiles[PH][t];
+        load_case<BLOCK>(b, td.slot, b.parity, b.parity, sc, sSlot);
         const int end = td.start + td.count;
         for (int k = 0; k < b.itemsPerThread; ++k) {
             const int i = td.start + (int)threadIdx.x + k * BLOCK;
@@ -137,27 +176,73 @@ constexpr int stage_blocks(int block, int dims, bool full) {
 // line it cached before another block rewrote it.
 // DIMS = 2: every case is 2D; DIMS = 0: 2D and 3D cases. FULL: see item().
 template <int BLOCK, int DIMS, bool FULL>
-__global__ void __launch_bounds__(BLOCK, stage_blocks(BLOCK, DIMS, FULL)) k_batch_stage(const __grid_constant__ BatchArgs b, int stage) {
+__global__ void __launch_bounds__(BLOCK, stage_blocks(BLOCK, DIMS, FULL)) k_batch_stage(const __grid_constant__ BatchArgs b,
+                                                                                       int stage) {
     __shared__ BatchCase sc;
     __shared__ int sSlot;
     if (threadIdx.x == 0) sSlot = -1;
     __syncthreads();
     unsigned* counter = &b.ctl->barrier[stage];
     unsigned target = b.barrierExtra;   // 0 except under lfm_batch_debug_barrier
+    BlockTiles r;
+    auto barrier = [&](auto next) {
+        target += gridDim.x;
+        return grid_barrier(counter, target, b.error, next);
+    };
+    auto next1 = [&] { r = block_tiles<1, BLOCK>(b, b.parity, b.parity, sc, sSlot); };
+    auto next2 = [&] { r = block_tiles<2, BLOCK>(b, b.parity, b.parity, sc, sSlot); };
+    auto next3 = [&] { r = block_tiles<3, BLOCK>(b, b.parity, b.parity, sc, sSlot); };
+    const bool grad = FULL && b.nTiles[1] > 0;
+    auto after_prep = [&] { grad ? next1() : next2(); };
     if (b.nTiles[0] > 0) {
-        phase_tiles<0, BLOCK, DIMS, FULL>(b, stage, sc, sSlot);
-        target += gridDim.x;
-        if (!grid_barrier(counter, target, b.error)) return;
+        r = block_tiles<0, BLOCK>(b, b.parity, b.parity, sc, sSlot);
+        phase_tiles<0, BLOCK, DIMS, FULL>(b, stage, r, sc, sSlot);
+        if (!barrier(after_prep)) return;
+    } else {
+        after_prep();
     }
-    if (FULL && b.nTiles[1] > 0) {
-        phase_tiles<1, BLOCK, DIMS, FULL>(b, stage, sc, sSlot);
-        target += gridDim.x;
-        if (!grid_barrier(counter, target, b.error)) return;
+    if (grad) {
+        phase_tiles<1, BLOCK, DIMS, FULL>(b, stage, r, sc, sSlot);
+        if (!barrier(next2)) return;
     }
-    phase_tiles<2, BLOCK, DIMS, FULL>(b, stage, sc, sSlot);
-    target += gridDim.x;
-    if (!grid_barrier(counter, target, b.error)) return;
-    phase_tiles<3, BLOCK, DIMS, FULL>(b, stage, sc, sSlot);
+    phase_tiles<2, BLOCK, DIMS, FULL>(b, stage, r, sc, sSlot);
+    if (!barrier(next3)) return;
+    phase_tiles<3, BLOCK, DIMS, FULL>(b, stage, r, sc, sSlot);
+}
+
+// Flux and update of cell i of a case that can do both at once (fluxupdate32).
+__device__ __forceinline__ void fused_item(const BatchCase& bc, int stage, int i) {
+    const int first = stage == 0;
+    const bool res = bc.residuals && first;
+    if (bc.scheme == kSchemeM1)
+        fluxupdate32<2, kSchemeM1, false, true, true>(bc.a, i, bc.rkA[stage], bc.rkB[stage], bc.dt32, first, res);
+    else
+        fluxupdate32<2, kSchemeM2, false, true, true>(bc.a, i, bc.rkA[stage], bc.rkB[stage], bc.dt32, first, res);
+}
+
+// A stage of a batch whose cases can all do flux and update at once
+// (CaseLayout::fusable) and have current primitives: one phase, no barrier, so stages follow one another as programmatic dependents (each loads
+// its first tile's case before it waits for the stage before).
+// 768 threads per SM (80 registers, 28 bytes spilled) beat 512 without spills
+// and 1024 (64, 120 bytes): 143, 150 and 149 us a step of eight cases.
+template <int BLOCK>
+__global__ void __launch_bounds__(BLOCK, BLOCK > 256 ? 1 : 768 / BLOCK) k_batch_fused(const __grid_constant__ BatchArgs b,
+                                                                                     int stage) {
+    __shared__ BatchCase sc;
+    __shared__ int sSlot;
+    if (threadIdx.x == 0) sSlot = -1;
+    __syncthreads();
+    const int in = (b.parity + stage) & 1;
+    const BlockTiles r = block_tiles<3, BLOCK>(b, in, in ^ 1, sc, sSlot);
+    PdlWait{1}();
+    for (int t = r.t0; t < r.t1; ++t) {
+        const BatchTile td = t == r.t0 ? r.first : b.tiles[3][t];
+        load_case<BLOCK>(b, td.slot, in, in ^ 1, sc, sSlot);
+        for (int k = 0; k < b.itemsPerThread; ++k) {
+            const int i = td.start + (int)threadIdx.x + k * BLOCK;
+            if (i < td.start + td.count) fused_item(sc, stage, i);
+        }
+    }
 }
 
 // One phase of a stage over every case, for the phased launch mode.
@@ -167,37 +252,75 @@ __global__ void __launch_bounds__(BLOCK) k_batch_phase(const __grid_constant__ B
     __shared__ int sSlot;
     if (threadIdx.x == 0) sSlot = -1;
     __syncthreads();
-    phase_tiles<PH, BLOCK, DIMS, FULL>(b, stage, sc, sSlot);
+    const BlockTiles r = block_tiles<PH, BLOCK>(b, b.parity, b.parity, sc, sSlot);
+    PdlWait{1}();
+    phase_tiles<PH, BLOCK, DIMS, FULL>(b, stage, r, sc, sSlot);
 }
 
+// New states of several cases, and their states out, in one launch each: one
+// row of blocks per case, so that the copies over the C2C link overlap.
+__global__ void __launch_bounds__(256) k_batch_set(const BatchCase* cases, const __grid_constant__ BatchStates m,
+                                                   int parity) {
+    __shared__ Args<float> a;
+    const BatchCase& bc = cases[m.slot[blockIdx.y]];
+    if ((int)(blockIdx.x * blockDim.x) >= bc.a.nc) return;
+    if (threadIdx.x == 0) {
+        a = bc.a;
+        if (parity) a.prim = a.primW;   // the buffer the next step reads
+    }
+    __syncthreads();
+    const int c = LFM_GLOBAL_ID();
+    const double* q = m.q[blockIdx.y];
+    if (c == 0) *a.flag = 0;   // a new state starts with a clear non-finite flag
+    if (c >= a.nc) return;
+    if (a.D == 2) set_state32<2>(a, q, a.nc, c);
+    else set_state32<3>(a, q, a.nc, c);
+}
+
+__global__ void __launch_bounds__(256) k_batch_get(const BatchCase* cases, const __grid_constant__ BatchStates m) {
+    const Args<float>& a = cases[m.slot[blockIdx.y]].a;
+    const int c = LFM_GLOBAL_ID(), nc = a.nc;
+    if (c >= nc) return;
+    double* out = m.q[blockIdx.y];
+    for (int v = 0; v < a.nq; ++v) out[(size_t)v * nc + c] = a.q[(size_t)v * a.nt + c] + a.qRef[v];
+}
+
+// The phases of a stage that have tiles, one kernel each, every one but the
+// step's first a programmatic dependent of the one before.
 template <int PH, int BLOCK, int DIMS, bool FULL>
-cudaError_t launch_phase(const BatchArgs& b, int stage, int bps, int sms, cudaStream_t st) {
+cudaError_t launch_phase(const BatchArgs& b, int stage, const PhasedShape& p, bool* chained, cudaStream_t st) {
+    if (p.tiles[PH] == 0) return cudaSuccess;
     static thread_local int fit = -1;   // resident blocks per SM of this kernel
     auto k = k_batch_phase<PH, BLOCK, DIMS, FULL>;
     if (fit < 0) {
         cudaError_t e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&fit, k, BLOCK, 0);
-        if (e != cudaSuccess || fit < 1) return e != cudaSuccess ? e : cudaErrorInvalidConfiguration;
+        if (e != cudaSuccess || fit < 1) {
+            fit = -1;
+            return e != cudaSuccess ? e : cudaErrorInvalidConfiguration;
+        }
     }
-    const int per = bps > 0 ? std::min(bps, fit) : fit;
-    k<<<per * sms, BLOCK, 0, st>>>(b, stage);
+    const int per = p.blocksPerSm > 0 ? std::min(p.blocksPerSm, fit) : fit;
+    launch_kernel_pdl(*chained, k, (unsigned)std::min(p.tiles[PH], per * p.sms), BLOCK, st, b, stage);
+    *chained = true;
     return cudaGetLastError();
 }
 
 template <int BLOCK, int DIMS, bool FULL>
-cudaError_t launch_phases(const BatchArgs& b, int stage, int bps, int sms, cudaStream_t st) {
-    cudaError_t e = launch_phase<0, BLOCK, DIMS, FULL>(b, stage, bps, sms, st);
-    if (e == cudaSuccess && FULL) e = launch_phase<1, BLOCK, DIMS, FULL>(b, stage, bps, sms, st);
-    if (e == cudaSuccess) e = launch_phase<2, BLOCK, DIMS, FULL>(b, stage, bps, sms, st);
-    if (e == cudaSuccess) e = launch_phase<3, BLOCK, DIMS, FULL>(b, stage, bps, sms, st);
+cudaError_t launch_phases(const BatchArgs& b, int stage, const PhasedShape& p, cudaStream_t st) {
+    bool chained = stage > 0;
+    cudaError_t e = launch_phase<0, BLOCK, DIMS, FULL>(b, stage, p, &chained, st);
+    if (e == cudaSuccess && FULL) e = launch_phase<1, BLOCK, DIMS, FULL>(b, stage, p, &chained, st);
+    if (e == cudaSuccess) e = launch_phase<2, BLOCK, DIMS, FULL>(b, stage, p, &chained, st);
+    if (e == cudaSuccess) e = launch_phase<3, BLOCK, DIMS, FULL>(b, stage, p, &chained, st);
     return e;
 }
 
 template <int BLOCK>
-cudaError_t launch_phases_variant(const BatchArgs& b, int stage, int variant, int bps, int sms, cudaStream_t st) {
+cudaError_t launch_phases_variant(const BatchArgs& b, int stage, int variant, const PhasedShape& p, cudaStream_t st) {
     switch (variant) {
-        case kBatchVariant2DInviscid: return launch_phases<BLOCK, 2, false>(b, stage, bps, sms, st);
-        case kBatchVariant2D: return launch_phases<BLOCK, 2, true>(b, stage, bps, sms, st);
-        default: return launch_phases<BLOCK, 0, true>(b, stage, bps, sms, st);
+        case kBatchVariant2DInviscid: return launch_phases<BLOCK, 2, false>(b, stage, p, st);
+        case kBatchVariant2D: return launch_phases<BLOCK, 2, true>(b, stage, p, st);
+        default: return launch_phases<BLOCK, 0, true>(b, stage, p, st);
     }
 }
 
@@ -237,12 +360,46 @@ cudaError_t launch_batch_stage(const BatchArgs& b, int stage, int block, int var
     }
 }
 
-cudaError_t launch_batch_phased(const BatchArgs& b, int stage, int block, int variant, int bps, int sms,
+template <int BLOCK>
+static cudaError_t launch_fused(const BatchArgs& b, int stage, int bps, int sms, cudaStream_t st) {
+    static thread_local int fit = -1;   // resident blocks per SM
+    if (fit < 0) {
+        cudaError_t e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&fit, k_batch_fused<BLOCK>, BLOCK, 0);
+        if (e != cudaSuccess || fit < 1) {
+            fit = -1;
+            return e != cudaSuccess ? e : cudaErrorInvalidConfiguration;
+        }
+    }
+    // Two grids' worth of blocks: a block that ends early makes room for one
+    // whose share was cut half as large. Eight cases of 14k-56k cells, us a step:
+    // one grid 123, two 90, four 94 (256 threads), 108, 84, 88 (128 threads).
+    const int per = bps > 0 ? std::min(bps, fit) : fit;
+    launch_kernel_pdl(stage > 0, k_batch_fused<BLOCK>, (unsigned)(2 * per * sms), BLOCK, st, b, stage);
+    return cudaGetLastError();
+}
+
+cudaError_t launch_batch_fused(const BatchArgs& b, int stage, int block, int bps, int sms, cudaStream_t st) {
+    switch (block) {
+        case 128: return launch_fused<128>(b, stage, bps, sms, st);
+        case 512: return launch_fused<512>(b, stage, bps, sms, st);
+        default: return launch_fused<256>(b, stage, bps, sms, st);
+    }
+}
+
+cudaError_t launch_batch_states(const BatchCase* cases, const BatchStates& m, int n, int maxCells, bool set, int parity,
+                                cudaStream_t st) {
+    const dim3 grid((unsigned)((maxCells + 255) / 256), (unsigned)n);
+    if (set) k_batch_set<<<grid, 256, 0, st>>>(cases, m, parity);
+    else k_batch_get<<<grid, 256, 0, st>>>(cases, m);
+    return cudaGetLastError();
+}
+
+cudaError_t launch_batch_phased(const BatchArgs& b, int stage, int block, int variant, const PhasedShape& p,
                                 cudaStream_t st) {
     switch (block) {
-        case 128: return launch_phases_variant<128>(b, stage, variant, bps, sms, st);
-        case 512: return launch_phases_variant<512>(b, stage, variant, bps, sms, st);
-        default: return launch_phases_variant<256>(b, stage, variant, bps, sms, st);
+        case 128: return launch_phases_variant<128>(b, stage, variant, p, st);
+        case 512: return launch_phases_variant<512>(b, stage, variant, p, st);
+        default: return launch_phases_variant<256>(b, stage, variant, p, st);
     }
 }
 

@@ -112,18 +112,38 @@ int currentVariant(const lfm_batch* b) {
     return full ? lfm::dev::kBatchVariant2D : lfm::dev::kBatchVariant2DInviscid;
 }
 
+void dropGraphs(lfm_batch* b) {
+    for (auto& byParity : b->graph)
+        for (cudaGraphExec_t& g : byParity) {
+            if (g) cudaGraphExecDestroy(g);
+            g = nullptr;
+        }
+}
+
 int rebuildTiles(lfm_batch* b) {
-    const int tileSize = b->tune.block * b->tune.items_per_thread;
+    // a step whose cases are all fusable and have current primitives is fused
+    bool lean = (b->untuned || !b->tune.phased) && b->barrierExtra == 0;
+    int64_t cells = 0;
+    for (const Slot& sl : b->slots)
+        if (sl.used) {
+            lean = lean && sl.fusable && sl.primsValid;
+            cells += sl.nc;
+        }
+    // untuned, 128 threads, but 256 for fused steps beyond L2's reach. Us a step,
+    // 128 / 256 threads, GB300: fused 0.22M cells 88 / 100, 0.84M 338 / 328,
+    // 2.5M 932 / 845, 9.1M 3097 / 2768; by phases, 0.75M cells 2D and 3D 1084 /
+    // 1242, 0.31M viscous 2D 335 / 384.
+    const int block = lean && b->untuned && cells > (1 << 21) ? 256 : b->tune.block;
+    const int tileSize = block * b->tune.items_per_thread;
     std::vector<BatchTile> tl[kBatchPhases];
     for (int s = 0; s < (int)b->slots.size(); ++s) {
         const Slot& sl = b->slots[(size_t)s];
         if (!sl.used) continue;
         // the update phase keeps the primitives of the cells and ghosts
         // current: preparation runs only in a case's first step after a new state
-        const int first[kBatchPhases] = {0, 0, 0, 0};
         const int end[kBatchPhases] = {sl.primsValid ? 0 : sl.nt, sl.needGradVis ? sl.nc : 0, sl.nf, sl.nc};
         for (int ph = 0; ph < kBatchPhases; ++ph)
-            for (int st = first[ph]; st < end[ph]; st += tileSize)
+            for (int st = 0; st < end[ph]; st += tileSize)
                 tl[ph].push_back(BatchTile{s, st, std::min(tileSize, end[ph] - st), 0});
     }
     int n[kBatchPhases];
@@ -147,11 +167,16 @@ int rebuildTiles(lfm_batch* b) {
     // the host vectors die here: wait for the copies out of them
     LFM_CUDA(cudaStreamSynchronize(b->stream));
     const int variant = currentVariant(b);
-    if ((realloc || variant != b->variant) && b->graph) {
-        cudaGraphExecDestroy(b->graph);
-        b->graph = nullptr;
+    // a phased step's grids follow the tiles
+    bool changed = realloc || variant != b->variant || block != b->block;
+    b->block = block;
+    for (int ph = 0; ph < kBatchPhases; ++ph) {
+        changed = changed || (b->tune.phased && n[ph] != b->nTiles[ph]);
+        b->nTiles[ph] = n[ph];
     }
+    if (changed) dropGraphs(b);
     b->variant = variant;
+    b->lean = lean;
     b->tilesDirty = false;
     return LFM_OK;
 }
@@ -165,19 +190,23 @@ BatchArgs makeArgs(lfm_batch* b) {
     a.error = b->dError;
     a.itemsPerThread = b->tune.items_per_thread;
     a.barrierExtra = b->barrierExtra;
+    a.parity = b->parity;
     return a;
 }
 
 int captureStep(lfm_batch* b, bool cooperative, cudaGraphExec_t* out) {
     const BatchArgs args = makeArgs(b);
+    lfm::dev::PhasedShape shape{{0, 0, 0, 0}, b->tune.blocks_per_sm, b->sms};
+    for (int ph = 0; ph < kBatchPhases; ++ph) shape.tiles[ph] = b->nTiles[ph];
     cudaGraph_t g = nullptr;
     LFM_CUDA(cudaStreamBeginCapture(b->stream, cudaStreamCaptureModeThreadLocal));
     cudaError_t le = cudaMemsetAsync(b->dCtl, 0, sizeof(BatchCtl), b->stream);
     for (int k = 0; k < b->rkOrder && le == cudaSuccess; ++k)
-        le = b->tune.phased ? lfm::dev::launch_batch_phased(args, k, b->tune.block, b->variant, b->tune.blocks_per_sm,
-                                                            b->sms, b->stream)
-                            : lfm::dev::launch_batch_stage(args, k, b->tune.block, b->variant, b->grid, cooperative,
-                                                           b->stream);
+        le = b->lean          ? lfm::dev::launch_batch_fused(args, k, b->block, b->tune.blocks_per_sm, b->sms,
+                                                             b->stream)
+             : b->tune.phased ? lfm::dev::launch_batch_phased(args, k, b->tune.block, b->variant, shape, b->stream)
+                         : lfm::dev::launch_batch_stage(args, k, b->tune.block, b->variant, b->grid, cooperative,
+                                                        b->stream);
     cudaError_t e = cudaStreamEndCapture(b->stream, &g);
     if (le != cudaSuccess || e != cudaSuccess) {
         if (g) cudaGraphDestroy(g);
@@ -201,8 +230,9 @@ int ensureGraph(lfm_batch* b) {
         int rc = rebuildTiles(b);
         if (rc) return rc;
     }
-    if (b->graph) return LFM_OK;
-    if (b->tune.phased) return captureStep(b, false, &b->graph);   // no co-residency needed
+    cudaGraphExec_t* graph = &b->graph[b->lean ? 1 : 0][b->parity];
+    if (*graph) return LFM_OK;
+    if (b->tune.phased || b->lean) return captureStep(b, false, graph);   // no co-residency needed
     const int fit = lfm::dev::batch_blocks_per_sm(b->tune.block, b->variant);
     if (fit <= 0) return lfm::setError(LFM_ERR_UNSUPPORTED, "batch kernel does not fit on an SM");
     const int bps = b->tune.blocks_per_sm > 0 ? std::min(b->tune.blocks_per_sm, fit) : fit;
@@ -210,12 +240,32 @@ int ensureGraph(lfm_batch* b) {
     // A cooperative launch guarantees co-residency; where capture of one is
     // refused, a grid within the resident capacity is launched plainly.
     int rc = LFM_ERR_CUDA;
-    if (b->tune.cooperative) rc = captureStep(b, true, &b->graph);
+    if (b->tune.cooperative) rc = captureStep(b, true, graph);
     if (rc != LFM_OK) {
         b->tune.cooperative = 0;
-        rc = captureStep(b, false, &b->graph);
+        rc = captureStep(b, false, graph);
     }
     return rc;
+}
+
+// One time step: the graph of the current tiles and primitive buffer. Fused
+// stages leave the primitives in the other buffer when their count is odd.
+int launchStep(lfm_batch* b) {
+    int rc = ensureGraph(b);
+    if (rc) return rc;
+    LFM_CUDA(cudaGraphLaunch(b->graph[b->lean ? 1 : 0][b->parity], b->stream));
+    if (b->lean) b->parity ^= b->rkOrder & 1;
+    return LFM_OK;
+}
+
+// After the first step with cases whose state was just set: they prepared all
+// their cells in it, the tile lists shrink.
+void markPrepared(lfm_batch* b) {
+    for (Slot& sl : b->slots)
+        if (sl.used && !sl.primsValid) {
+            sl.primsValid = true;
+            b->tilesDirty = true;
+        }
 }
 
 // Device buffer for a case's absolute state in transit to or from the host.
@@ -296,7 +346,7 @@ extern "C" void lfm_batch_destroy(lfm_batch* b) {
     if (!b) return;
     cudaSetDevice(b->device);
     if (b->stream) cudaStreamSynchronize(b->stream);
-    if (b->graph) cudaGraphExecDestroy(b->graph);
+    dropGraphs(b);
     for (int ph = 0; ph < kBatchPhases; ++ph)
         if (b->dTiles[ph]) cudaFree(b->dTiles[ph]);
     cudaFree(b->arenaBase);
@@ -377,7 +427,7 @@ int commitCase(lfm_batch* b, const PreparedCase& pc, int* slot) {
     a.dq = reinterpret_cast<float*>(P(L.dq));
     a.res = reinterpret_cast<double*>(P(L.res));
     a.prim = reinterpret_cast<float*>(P(L.prim));
-    a.primW = a.prim;
+    a.primW = L.fusable ? reinterpret_cast<float*>(P(L.prim1)) : a.prim;
     a.V = reinterpret_cast<float*>(P(L.V));
     a.grad = reinterpret_cast<float*>(P(L.grad));
     a.flux = reinterpret_cast<float*>(P(L.flux));
@@ -421,6 +471,7 @@ int commitCase(lfm_batch* b, const PreparedCase& pc, int* slot) {
     sl.nf = pc.nf;
     sl.nt = pc.nc + pc.ng;
     sl.needGradVis = pc.needGradVis;
+    sl.fusable = L.fusable;
     sl.primsValid = false;
     for (int v = 0; v < 5; ++v) sl.qRef[v] = pc.bc.a.qRef[v];
     sl.q = a.q;
@@ -463,15 +514,18 @@ namespace {
 // shared staging buffer (stream order keeps successive cases apart).
 int enqueueBatchSet(lfm_batch* b, int slot, const double* q) {
     Slot& sl = b->slots[(size_t)slot];
-    // a new state starts with a clear non-finite flag
-    LFM_CUDA(cudaMemsetAsync(b->dFlags + slot, 0, sizeof(int), b->stream));
     const size_t bytes = (size_t)sl.nq * sl.nc * sizeof(double);
-    int rc = ensureStage(b, bytes);
-    if (rc) return rc;
-    LFM_CUDA(cudaMemcpyAsync(b->dStage, q, bytes, cudaMemcpyHostToDevice, b->stream));
+    const double* direct = lfm::dev::kernel_address(q);
+    if (!direct) {
+        int rc = ensureStage(b, bytes);
+        if (rc) return rc;
+        LFM_CUDA(cudaMemcpyAsync(b->dStage, q, bytes, cudaMemcpyHostToDevice, b->stream));
+    }
     // stored as q - qRef, with the primitives of the cells and their ghosts
     // derived in the same pass: the tile lists need no preparation phase
-    lfm::dev::launch_set_state32(sl.a, b->dStage, sl.nc, b->stream);
+    Args<float> a = sl.a;
+    if (b->parity) std::swap(a.prim, a.primW);   // into the buffer the next step reads
+    lfm::dev::launch_set_state32(a, direct ? direct : b->dStage, sl.nc, b->stream);
     LFM_CUDA(cudaGetLastError());
     return LFM_OK;
 }
@@ -479,13 +533,58 @@ int enqueueBatchSet(lfm_batch* b, int slot, const double* q) {
 int enqueueBatchGet(lfm_batch* b, int slot, double* q) {
     const Slot& sl = b->slots[(size_t)slot];
     const size_t bytes = (size_t)sl.nq * sl.nc * sizeof(double);
-    int rc = ensureStage(b, bytes);
-    if (rc) return rc;
+    double* direct = lfm::dev::kernel_address(q);
+    if (!direct) {
+        int rc = ensureStage(b, bytes);
+        if (rc) return rc;
+    }
     lfm::dev::QOffset qo;   // stored as q - qRef
     for (int v = 0; v < 5; ++v) qo.v[v] = sl.qRef[v];
-    lfm::dev::launch_offset_rows(b->dStage, sl.nc, sl.q, sl.nt, sl.nc, sl.nq, qo, 1.0, b->stream);
+    lfm::dev::launch_offset_rows(direct ? direct : b->dStage, sl.nc, sl.q, sl.nt, sl.nc, sl.nq, qo, 1.0, b->stream);
     LFM_CUDA(cudaGetLastError());
-    LFM_CUDA(cudaMemcpyAsync(q, b->dStage, bytes, cudaMemcpyDeviceToHost, b->stream));
+    if (!direct) LFM_CUDA(cudaMemcpyAsync(q, b->dStage, bytes, cudaMemcpyDeviceToHost, b->stream));
+    return LFM_OK;
+}
+
+}  // namespace
+
+namespace {
+
+// The states of several cases in or out (null entries skipped): those in
+// page-locked memory by one kernel per kBatchStates cases, which copies all at
+// once; the others one after another through the staging buffer, sized before
+// anything is enqueued.
+int enqueueBatchStates(lfm_batch* b, int n, const int* slots, const double* const* q, bool set) {
+    size_t most = 0;
+    std::vector<int> staged;
+    lfm::dev::BatchStates m{};
+    int count = 0, maxCells = 0;
+    auto flush = [&]() -> int {
+        if (count > 0)
+            LFM_CUDA(lfm::dev::launch_batch_states(b->dCases, m, count, maxCells, set, b->parity, b->stream));
+        count = maxCells = 0;
+        return LFM_OK;
+    };
+    int rc;
+    for (int i = 0; i < n; ++i) {
+        if (!q[i]) continue;
+        const Slot& sl = b->slots[(size_t)slots[i]];
+        double* direct = lfm::dev::kernel_address(q[i]);
+        if (!direct) {
+            staged.push_back(i);
+            most = std::max(most, (size_t)sl.nq * sl.nc * sizeof(double));
+            continue;
+        }
+        m.slot[count] = slots[i];
+        m.q[count] = direct;
+        maxCells = std::max(maxCells, sl.nc);
+        if (++count == lfm::dev::kBatchStates && (rc = flush())) return rc;
+    }
+    if ((rc = flush())) return rc;
+    if (!staged.empty() && (rc = ensureStage(b, most))) return rc;
+    for (int i : staged)
+        if ((rc = set ? enqueueBatchSet(b, slots[i], q[i]) : enqueueBatchGet(b, slots[i], const_cast<double*>(q[i]))))
+            return rc;
     return LFM_OK;
 }
 
@@ -514,20 +613,15 @@ extern "C" int lfm_batch_get_state(lfm_batch* b, int slot, double* q) {
 extern "C" int lfm_batch_advance(lfm_batch* b, int n, const int* slots, const double* const* q_in, int nsteps,
                                  double* const* q_out) {
     if (!b || n < 0 || (n > 0 && !slots) || nsteps < 0) return lfm::setError(LFM_ERR_INVALID, "bad argument");
-    size_t most = 0;
     for (int i = 0; i < n; ++i) {
         int rc = checkSlot(b, slots[i]);
         if (rc) return rc;
-        const Slot& sl = b->slots[(size_t)slots[i]];
-        most = std::max(most, (size_t)sl.nq * sl.nc * sizeof(double));
     }
     LFM_CUDA(cudaSetDevice(b->device));
-    int rc = ensureStage(b, most);   // sized once, before anything is enqueued
-    for (int i = 0; i < n && !rc && q_in; ++i)
-        if (q_in[i]) rc = enqueueBatchSet(b, slots[i], q_in[i]);
+    int rc = LFM_OK;
+    if (q_in) rc = enqueueBatchStates(b, n, slots, q_in, true);
     if (!rc && nsteps > 0) rc = lfm_batch_step(b, nsteps);
-    for (int i = 0; i < n && !rc && q_out; ++i)
-        if (q_out[i]) rc = enqueueBatchGet(b, slots[i], q_out[i]);
+    if (!rc && q_out) rc = enqueueBatchStates(b, n, slots, q_out, false);
     if (rc) return rc;
     return lfm_batch_sync(b);
 }
@@ -537,24 +631,11 @@ extern "C" int lfm_batch_step(lfm_batch* b, int nsteps) {
     if (nsteps < 0) return lfm::setError(LFM_ERR_INVALID, "negative step count");
     LFM_CUDA(cudaSetDevice(b->device));
     int rc = ensureGraph(b);
-    if (rc) return rc;
-    if (nsteps == 0) return LFM_OK;
-    // Cases whose state was just set prepare all their cells in the first
-    // step; after it the update phase keeps their primitives current and the
-    // tile lists shrink to their ghosts.
-    bool stale = false;
-    for (Slot& sl : b->slots)
-        if (sl.used && !sl.primsValid) {
-            stale = true;
-            sl.primsValid = true;
-        }
-    LFM_CUDA(cudaGraphLaunch(b->graph, b->stream));
-    if (stale) {
-        b->tilesDirty = true;
-        if ((rc = ensureGraph(b))) return rc;
+    for (int k = 0; k < nsteps && !rc; ++k) {
+        rc = launchStep(b);
+        if (k == 0 && !rc) markPrepared(b);
     }
-    for (int k = 1; k < nsteps; ++k) LFM_CUDA(cudaGraphLaunch(b->graph, b->stream));
-    return LFM_OK;
+    return rc;
 }
 
 extern "C" int lfm_batch_sync(lfm_batch* b) {
@@ -622,10 +703,8 @@ extern "C" int lfm_batch_set_tuning(lfm_batch* b, const lfm_batch_tuning* t) {
     LFM_CUDA(cudaSetDevice(b->device));
     LFM_CUDA(cudaStreamSynchronize(b->stream));
     b->tune = *t;
-    if (b->graph) {
-        cudaGraphExecDestroy(b->graph);
-        b->graph = nullptr;
-    }
+    b->untuned = false;
+    dropGraphs(b);
     b->tilesDirty = true;
     return LFM_OK;
 }
@@ -635,10 +714,8 @@ extern "C" int lfm_batch_debug_barrier(lfm_batch* b, int extra_arrivals) {
     LFM_CUDA(cudaSetDevice(b->device));
     LFM_CUDA(cudaStreamSynchronize(b->stream));
     b->barrierExtra = (unsigned)extra_arrivals;
-    if (b->graph) {   // the step graph holds the kernels' arguments
-        cudaGraphExecDestroy(b->graph);
-        b->graph = nullptr;
-    }
+    dropGraphs(b);   // they hold the kernels' arguments
+    b->tilesDirty = true;
     return LFM_OK;
 }
 
@@ -666,21 +743,13 @@ extern "C" int lfm_batch_bench(lfm_batch* b, int nsteps, size_t flush_bytes, flo
     if (rc) return rc;
     std::vector<cudaEvent_t> ev(2 * (size_t)nsteps);
     for (auto& e : ev) LFM_CUDA(cudaEventCreate(&e));
-    bool stale = false;   // as in lfm_batch_step: stale cases prepare all cells in the first step
-    for (Slot& sl : b->slots)
-        if (sl.used && !sl.primsValid) {
-            stale = true;
-            sl.primsValid = true;
-        }
     for (int k = 0; k < nsteps; ++k) {
         if ((rc = flushL2(b, flush_bytes))) break;
+        if ((rc = ensureGraph(b))) break;   // outside the timing
         cudaEventRecord(ev[2 * (size_t)k], b->stream);
-        cudaGraphLaunch(b->graph, b->stream);
+        if ((rc = launchStep(b))) break;
         cudaEventRecord(ev[2 * (size_t)k + 1], b->stream);
-        if (k == 0 && stale) {
-            b->tilesDirty = true;
-            if ((rc = ensureGraph(b))) break;
-        }
+        if (k == 0) markPrepared(b);
     }
     cudaError_t e = cudaStreamSynchronize(b->stream);
     for (int k = 0; k < nsteps && e == cudaSuccess; ++k)
