@@ -5,6 +5,17 @@
 namespace lfm {
 namespace dev {
 
+// Threads per block: small ones share the FP64 pipes evenly to the end (a
+// 393k-cell update is 10 blocks of 256 per SM on some, 11 on others) and a
+// boundary cell's ghost work holds few threads. Measured on GB300, us a step at
+// 256, 128 and 64 threads: update, 48 x 48 vortex 39.9, 27.7, 29.3, 768 x 512
+// cylinder 168.2, 160.6, 159.1, 192 x 128 x 48 wake 836, 792, 756; flux of the
+// cylinder at 256, 128, 64 461, 451, 451, of the wake 2974, 3001, 3001.
+template <int D>
+constexpr int kCellThreads = D == 2 ? 128 : 64;
+template <int D>
+constexpr int kFaceThreads = D == 2 ? 128 : 256;
+
 // ---------------------------------------------------------------------------
 // k_prep: ghost states and per-cell primitives of entries [first, nt). The
 // update writes the cells' and ghosts' primitives for the next stage, so
@@ -98,7 +109,7 @@ __device__ __forceinline__ void for_entries64(const Args<double>& a, int c, Sync
 // k_grad: gradients read by M2AUSM's minmod reconstruction.
 // ---------------------------------------------------------------------------
 template <typename T, int D>
-__global__ void __launch_bounds__(256) k_grad(Args<T> a) {
+__global__ void __launch_bounds__(kCellThreads<D>) k_grad(Args<T> a) {
     const int c = LFM_GLOBAL_ID();
     if (c >= a.nc) return;
     T gr[D], gp[D], gu[D][D];
@@ -153,7 +164,7 @@ __global__ void __launch_bounds__(256) k_grad(Args<T> a) {
 // ---------------------------------------------------------------------------
 // LES compiles in the Smagorinsky SGS stress (cases with a.smagC).
 template <typename T, int D, bool LES>
-__global__ void __launch_bounds__(256) k_vis(Args<T> a) {
+__global__ void __launch_bounds__(kCellThreads<D>) k_vis(Args<T> a) {
     const int c = LFM_GLOBAL_ID();
     if (c >= a.nc) return;
     T g[D][D], gT[D];
@@ -219,7 +230,7 @@ __global__ void __launch_bounds__(256) k_vis(Args<T> a) {
 // k_flux: rhs of one face.
 // ---------------------------------------------------------------------------
 template <typename T, int D, int SCH, bool LES>
-__global__ void __launch_bounds__(128) k_flux(Args<T> a) {
+__global__ void __launch_bounds__(kFaceThreads<D>) k_flux(Args<T> a) {
     const int f = LFM_GLOBAL_ID();
     if (f >= a.nf) return;
     constexpr int NQ = D + 2;
@@ -457,7 +468,7 @@ __global__ void __launch_bounds__(128) k_flux(Args<T> a) {
 // and primitives of its boundary ghosts.
 // ---------------------------------------------------------------------------
 template <typename T, int D, bool RES>
-__global__ void __launch_bounds__(256) k_update(const __grid_constant__ Args<T> a, double Ak, double Bk, double dt, int first) {
+__global__ void __launch_bounds__(kCellThreads<D>) k_update(const __grid_constant__ Args<T> a, double Ak, double Bk, double dt, int first) {
     const int c = LFM_GLOBAL_ID();
     if (c >= a.nc) return;
     update_cell<T, D, RES, true>(a, c, Ak, Bk, dt, first, PdlWait{a.pdl});
@@ -561,7 +572,7 @@ static inline unsigned blocks(int n, int b) { return (unsigned)((n + b - 1) / b)
 
 template <typename T, int D, int SCH, bool LES>
 void launch_flux(const Args<T>& a, const StageConfig& s, cudaStream_t st) {
-    launch_kernel_pdl(s.pdl && a.pdl, k_flux<T, D, SCH, LES>, blocks(a.nf, 128), 128, st, a);
+    launch_kernel_pdl(s.pdl && a.pdl, k_flux<T, D, SCH, LES>, blocks(a.nf, kFaceThreads<D>), kFaceThreads<D>, st, a);
 }
 
 template <typename T, int D, bool LES>
@@ -575,10 +586,10 @@ void launch_fp64(const Args<T>& a, const StageConfig& s, int which, cudaStream_t
             break;
         }
         case 1:
-            if (s.needGrad) launch_kernel_pdl(s.pdl && a.pdl, k_grad<T, D>, blocks(a.nc, 256), 256, st, a);
+            if (s.needGrad) launch_kernel_pdl(s.pdl && a.pdl, k_grad<T, D>, blocks(a.nc, kCellThreads<D>), kCellThreads<D>, st, a);
             break;
         case 2:
-            if (s.needVis) launch_kernel_pdl(s.pdl && a.pdl, k_vis<T, D, LES>, blocks(a.nc, 256), 256, st, a);
+            if (s.needVis) launch_kernel_pdl(s.pdl && a.pdl, k_vis<T, D, LES>, blocks(a.nc, kCellThreads<D>), kCellThreads<D>, st, a);
             break;
         case 3:
             if (s.scheme == kSchemeM1) launch_flux<T, D, kSchemeM1, LES>(a, s, st);
@@ -586,8 +597,8 @@ void launch_fp64(const Args<T>& a, const StageConfig& s, int which, cudaStream_t
             else launch_flux<T, D, kSchemeAUSM, LES>(a, s, st);
             break;
         case 4:
-            if (s.withRes) launch_kernel_pdl(s.pdl && a.pdl, k_update<T, D, true>, blocks(a.nc, 256), 256, st, a, s.A, s.B, s.dt, s.first);
-            else launch_kernel_pdl(s.pdl && a.pdl, k_update<T, D, false>, blocks(a.nc, 256), 256, st, a, s.A, s.B, s.dt, s.first);
+            if (s.withRes) launch_kernel_pdl(s.pdl && a.pdl, k_update<T, D, true>, blocks(a.nc, kCellThreads<D>), kCellThreads<D>, st, a, s.A, s.B, s.dt, s.first);
+            else launch_kernel_pdl(s.pdl && a.pdl, k_update<T, D, false>, blocks(a.nc, kCellThreads<D>), kCellThreads<D>, st, a, s.A, s.B, s.dt, s.first);
             break;
         default: break;
     }

@@ -7,6 +7,16 @@
 namespace lfm {
 namespace dev {
 
+// Threads per block. These kernels wait for loads or (M2AUSM's flux) for
+// divisions and square roots; small blocks leave and enter an SM one by one, so
+// the last wave is short and a boundary cell's ghost work holds few threads.
+// Measured on GB300, us a step at 256, 128 and 64 threads: 768 x 512 cylinder,
+// update 58.5, 55.4, 53.8, M1 flux 45.4, 43.8, 67.2; 331 x 217 M2AUSM flux
+// 70.7, 54.4, 48.1; 192 x 128 x 48 wake, update 287, 269, 266.
+constexpr int kCellThreads = 128;
+template <int SCH>
+constexpr int kFaceThreads = SCH == kSchemeAUSM ? 64 : 128;
+
 // Primitives of cells, ghosts and halos [first, a.nt): first = 0 after a new
 // state; once the update kernels keep the cells' current, first = nc (ghosts
 // and halos), or nc + ng (halos only) when the update also writes the ghosts.
@@ -18,19 +28,19 @@ __global__ void __launch_bounds__(256) k_prep32(const __grid_constant__ Args<flo
 }
 
 template <int D, bool ELL>
-__global__ void __launch_bounds__(256) k_grad32(const __grid_constant__ Args<float> a) {
+__global__ void __launch_bounds__(kCellThreads) k_grad32(const __grid_constant__ Args<float> a) {
     const int c = LFM_GLOBAL_ID();
     if (c < a.nc) grad32<D, ELL>(a, c, PdlWait{a.pdl});
 }
 
 template <int D, bool LES, bool ELL>
-__global__ void __launch_bounds__(256) k_vis32(const __grid_constant__ Args<float> a) {
+__global__ void __launch_bounds__(kCellThreads) k_vis32(const __grid_constant__ Args<float> a) {
     const int c = LFM_GLOBAL_ID();
     if (c < a.nc) vis32<D, LES, ELL>(a, c, PdlWait{a.pdl});
 }
 
 template <int D, int SCH, bool LES>
-__global__ void __launch_bounds__(256) k_flux32(const __grid_constant__ Args<float> a) {
+__global__ void __launch_bounds__(kFaceThreads<SCH>) k_flux32(const __grid_constant__ Args<float> a) {
     const int f = LFM_GLOBAL_ID();
     if (f < a.nf) flux32<D, SCH, true, LES, true>(a, f, PdlWait{a.pdl});
 }
@@ -40,29 +50,33 @@ __global__ void __launch_bounds__(256) k_flux32(const __grid_constant__ Args<flo
 // rows across its faces): the 9.4M-cell wake's flux 3.42 -> 3.27 ms per step;
 // at four blocks per SM it spills (3.66 ms).
 template <int D, int SCH>
-__global__ void __launch_bounds__(256, 3) k_flux32_cell(const __grid_constant__ Args<float> a) {
+__global__ void __launch_bounds__(kCellThreads, 768 / kCellThreads) k_flux32_cell(const __grid_constant__ Args<float> a) {
     const int c = LFM_GLOBAL_ID();
     if (c < a.nc) flux32_cell<D, SCH>(a, c, PdlWait{a.pdl});
 }
 
 // Warp-interleaved cells: warp j of block b updates the 32 cells of chunk
-// j * gridDim.x + b (coalesced within the warp), so a block's eight warps lie
-// in chunks spread over the mesh. The cells with boundary faces come first in
-// the solver order and write their ghosts' next state in FP64 (boundary
-// conditions with divisions, on an FP64 pipe that issues about two
-// instructions per clock per SM); interleaved, their warps land on different
-// SMs instead of filling the first few blocks, whose SMs would otherwise
-// finish last. Without the ghost work (GH false) a block keeps 256
-// consecutive cells, which the large cases' gathers from HBM prefer.
+// j * gridDim.x + b (coalesced within the warp), so a block's warps lie in
+// chunks spread over the mesh. The cells with boundary faces come first in
+// the solver order and write their ghosts' next state in FP64 (on an FP64 pipe
+// that issues about two instructions per clock per SM); interleaved, their
+// warps land on different SMs instead of filling the first few blocks, whose
+// SMs would otherwise finish last. Beyond kSpreadCells a block keeps consecutive
+// cells, which gathers from HBM prefer; the first blocks start first there and
+// are done long before the last.
+template <int D>
+constexpr int kSpreadCells = D == 2 ? 1 << 20 : 1 << 18;
+
 template <int D, bool RES, bool GH, bool ELL>
 __device__ __forceinline__ void update_thread(const Args<float>& a, double Ak, double Bk, float dt32, int first) {
-    const int c = GH ? (int)(((threadIdx.x >> 5) * gridDim.x + blockIdx.x) << 5) + (int)(threadIdx.x & 31u)
-                     : (int)LFM_GLOBAL_ID();
+    const bool spread = GH && a.nc <= kSpreadCells<D>;
+    const int c = spread ? (int)(((threadIdx.x >> 5) * gridDim.x + blockIdx.x) << 5) + (int)(threadIdx.x & 31u)
+                         : (int)LFM_GLOBAL_ID();
     if (c < a.nc) update32<D, GH, ELL ? kEntriesEll : kEntriesList>(a, c, Ak, Bk, dt32, first, RES, PdlWait{a.pdl});
 }
 
 template <int D, bool RES, bool GH, bool ELL>
-__global__ void __launch_bounds__(256) k_update32(const __grid_constant__ Args<float> a, double Ak, double Bk,
+__global__ void __launch_bounds__(kCellThreads) k_update32(const __grid_constant__ Args<float> a, double Ak, double Bk,
                                                   float dt32, int first) {
     update_thread<D, RES, GH, ELL>(a, Ak, Bk, dt32, first);
 }
@@ -70,7 +84,7 @@ __global__ void __launch_bounds__(256) k_update32(const __grid_constant__ Args<f
 // Fused flux + update (fluxupdate32): one thread per cell, cells mapped as
 // in the update kernel that writes ghosts (warp-interleaved chunks).
 template <int D, int SCH, bool VIS, bool RES, bool ELL>
-__global__ void __launch_bounds__(256) k_fluxupdate32(const __grid_constant__ Args<float> a, double Ak, double Bk,
+__global__ void __launch_bounds__(kCellThreads) k_fluxupdate32(const __grid_constant__ Args<float> a, double Ak, double Bk,
                                                       float dt32, int first) {
     const int c = (int)(((threadIdx.x >> 5) * gridDim.x + blockIdx.x) << 5) + (int)(threadIdx.x & 31u);
     if (c < a.nc) fluxupdate32<D, SCH, VIS, true, ELL>(a, c, Ak, Bk, dt32, first, RES, PdlWait{a.pdl});
@@ -78,10 +92,10 @@ __global__ void __launch_bounds__(256) k_fluxupdate32(const __grid_constant__ Ar
 
 template <int D, int SCH, bool VIS, bool ELL>
 void launch_fluxupdate32_kernel(const Args<float>& a, const StageConfig& s, cudaStream_t st) {
-    const unsigned nb = (unsigned)((a.nc + 255) / 256);
+    const unsigned nb = (unsigned)((a.nc + kCellThreads - 1) / kCellThreads);
     const float dt32 = (float)s.dt;
-    if (s.withRes) launch_kernel_pdl(s.pdl && a.pdl, k_fluxupdate32<D, SCH, VIS, true, ELL>, nb, 256, st, a, s.A, s.B, dt32, s.first);
-    else launch_kernel_pdl(s.pdl && a.pdl, k_fluxupdate32<D, SCH, VIS, false, ELL>, nb, 256, st, a, s.A, s.B, dt32, s.first);
+    if (s.withRes) launch_kernel_pdl(s.pdl && a.pdl, k_fluxupdate32<D, SCH, VIS, true, ELL>, nb, kCellThreads, st, a, s.A, s.B, dt32, s.first);
+    else launch_kernel_pdl(s.pdl && a.pdl, k_fluxupdate32<D, SCH, VIS, false, ELL>, nb, kCellThreads, st, a, s.A, s.B, dt32, s.first);
 }
 
 template <int D, int SCH>
@@ -97,14 +111,14 @@ void launch_fluxupdate32_scheme(const Args<float>& a, const StageConfig& s, cuda
 
 template <int D, bool ELL>
 void launch_update32(const Args<float>& a, const StageConfig& s, cudaStream_t st) {
-    const unsigned nb = (unsigned)((a.nc + 255) / 256);   // eight 32-cell chunks per block
+    const unsigned nb = (unsigned)((a.nc + kCellThreads - 1) / kCellThreads);   // a 32-cell chunk per warp
     const float dt32 = (float)s.dt;
     if (a.cellGhosts) {
-        if (s.withRes) launch_kernel_pdl(s.pdl && a.pdl, k_update32<D, true, true, ELL>, nb, 256, st, a, s.A, s.B, dt32, s.first);
-        else launch_kernel_pdl(s.pdl && a.pdl, k_update32<D, false, true, ELL>, nb, 256, st, a, s.A, s.B, dt32, s.first);
+        if (s.withRes) launch_kernel_pdl(s.pdl && a.pdl, k_update32<D, true, true, ELL>, nb, kCellThreads, st, a, s.A, s.B, dt32, s.first);
+        else launch_kernel_pdl(s.pdl && a.pdl, k_update32<D, false, true, ELL>, nb, kCellThreads, st, a, s.A, s.B, dt32, s.first);
     } else {
-        if (s.withRes) launch_kernel_pdl(s.pdl && a.pdl, k_update32<D, true, false, ELL>, nb, 256, st, a, s.A, s.B, dt32, s.first);
-        else launch_kernel_pdl(s.pdl && a.pdl, k_update32<D, false, false, ELL>, nb, 256, st, a, s.A, s.B, dt32, s.first);
+        if (s.withRes) launch_kernel_pdl(s.pdl && a.pdl, k_update32<D, true, false, ELL>, nb, kCellThreads, st, a, s.A, s.B, dt32, s.first);
+        else launch_kernel_pdl(s.pdl && a.pdl, k_update32<D, false, false, ELL>, nb, kCellThreads, st, a, s.A, s.B, dt32, s.first);
     }
 }
 
@@ -138,31 +152,31 @@ void launch_fp32(const Args<float>& a, const StageConfig& s, int which, cudaStre
             break;
         }
         case 1:
-            if (s.needGrad && a.cfEll) launch_kernel_pdl(s.pdl && a.pdl, k_grad32<D, true>, nblocks(a.nc, 256), 256, st, a);
-            else if (s.needGrad) launch_kernel_pdl(s.pdl && a.pdl, k_grad32<D, false>, nblocks(a.nc, 256), 256, st, a);
+            if (s.needGrad && a.cfEll) launch_kernel_pdl(s.pdl && a.pdl, k_grad32<D, true>, nblocks(a.nc, kCellThreads), kCellThreads, st, a);
+            else if (s.needGrad) launch_kernel_pdl(s.pdl && a.pdl, k_grad32<D, false>, nblocks(a.nc, kCellThreads), kCellThreads, st, a);
             break;
         case 2:
             if (!s.needVis) break;
-            if (a.smagC && a.cfEll) launch_kernel_pdl(s.pdl && a.pdl, k_vis32<D, true, true>, nblocks(a.nc, 256), 256, st, a);
-            else if (a.smagC) launch_kernel_pdl(s.pdl && a.pdl, k_vis32<D, true, false>, nblocks(a.nc, 256), 256, st, a);
-            else if (a.cfEll) launch_kernel_pdl(s.pdl && a.pdl, k_vis32<D, false, true>, nblocks(a.nc, 256), 256, st, a);
-            else launch_kernel_pdl(s.pdl && a.pdl, k_vis32<D, false, false>, nblocks(a.nc, 256), 256, st, a);
+            if (a.smagC && a.cfEll) launch_kernel_pdl(s.pdl && a.pdl, k_vis32<D, true, true>, nblocks(a.nc, kCellThreads), kCellThreads, st, a);
+            else if (a.smagC) launch_kernel_pdl(s.pdl && a.pdl, k_vis32<D, true, false>, nblocks(a.nc, kCellThreads), kCellThreads, st, a);
+            else if (a.cfEll) launch_kernel_pdl(s.pdl && a.pdl, k_vis32<D, false, true>, nblocks(a.nc, kCellThreads), kCellThreads, st, a);
+            else launch_kernel_pdl(s.pdl && a.pdl, k_vis32<D, false, false>, nblocks(a.nc, kCellThreads), kCellThreads, st, a);
             break;
         case 3:
             if (s.fluxStaging.stages > 0) {   // staged kernel (configured for this scheme, laminar)
                 launch_flux32_staged(a, s, st);
             } else if (a.nf == 0) {
             } else if (a.fOwn && !a.smagC && s.scheme != kSchemeAUSM) {   // cell-centred
-                if (s.scheme == kSchemeM1) launch_kernel_pdl(s.pdl && a.pdl, k_flux32_cell<D, kSchemeM1>, nblocks(a.nc, 256), 256, st, a);
-                else launch_kernel_pdl(s.pdl && a.pdl, k_flux32_cell<D, kSchemeM2>, nblocks(a.nc, 256), 256, st, a);
+                if (s.scheme == kSchemeM1) launch_kernel_pdl(s.pdl && a.pdl, k_flux32_cell<D, kSchemeM1>, nblocks(a.nc, kCellThreads), kCellThreads, st, a);
+                else launch_kernel_pdl(s.pdl && a.pdl, k_flux32_cell<D, kSchemeM2>, nblocks(a.nc, kCellThreads), kCellThreads, st, a);
             } else if (a.smagC) {   // Smagorinsky LES variants
-                if (s.scheme == kSchemeM1) launch_kernel_pdl(s.pdl && a.pdl, k_flux32<D, kSchemeM1, true>, nblocks(a.nf, 256), 256, st, a);
-                else if (s.scheme == kSchemeM2) launch_kernel_pdl(s.pdl && a.pdl, k_flux32<D, kSchemeM2, true>, nblocks(a.nf, 256), 256, st, a);
-                else launch_kernel_pdl(s.pdl && a.pdl, k_flux32<D, kSchemeAUSM, true>, nblocks(a.nf, 256), 256, st, a);
+                if (s.scheme == kSchemeM1) launch_kernel_pdl(s.pdl && a.pdl, k_flux32<D, kSchemeM1, true>, nblocks(a.nf, kFaceThreads<kSchemeM1>), kFaceThreads<kSchemeM1>, st, a);
+                else if (s.scheme == kSchemeM2) launch_kernel_pdl(s.pdl && a.pdl, k_flux32<D, kSchemeM2, true>, nblocks(a.nf, kFaceThreads<kSchemeM2>), kFaceThreads<kSchemeM2>, st, a);
+                else launch_kernel_pdl(s.pdl && a.pdl, k_flux32<D, kSchemeAUSM, true>, nblocks(a.nf, kFaceThreads<kSchemeAUSM>), kFaceThreads<kSchemeAUSM>, st, a);
             } else {
-                if (s.scheme == kSchemeM1) launch_kernel_pdl(s.pdl && a.pdl, k_flux32<D, kSchemeM1, false>, nblocks(a.nf, 256), 256, st, a);
-                else if (s.scheme == kSchemeM2) launch_kernel_pdl(s.pdl && a.pdl, k_flux32<D, kSchemeM2, false>, nblocks(a.nf, 256), 256, st, a);
-                else launch_kernel_pdl(s.pdl && a.pdl, k_flux32<D, kSchemeAUSM, false>, nblocks(a.nf, 256), 256, st, a);
+                if (s.scheme == kSchemeM1) launch_kernel_pdl(s.pdl && a.pdl, k_flux32<D, kSchemeM1, false>, nblocks(a.nf, kFaceThreads<kSchemeM1>), kFaceThreads<kSchemeM1>, st, a);
+                else if (s.scheme == kSchemeM2) launch_kernel_pdl(s.pdl && a.pdl, k_flux32<D, kSchemeM2, false>, nblocks(a.nf, kFaceThreads<kSchemeM2>), kFaceThreads<kSchemeM2>, st, a);
+                else launch_kernel_pdl(s.pdl && a.pdl, k_flux32<D, kSchemeAUSM, false>, nblocks(a.nf, kFaceThreads<kSchemeAUSM>), kFaceThreads<kSchemeAUSM>, st, a);
             }
             break;
         case 4:

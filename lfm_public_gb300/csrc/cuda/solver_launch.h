@@ -26,17 +26,17 @@ struct FluxStaging {
 // of the SMs, and FP64 work then waits for their FP64 pipes, while a larger one
 // fills every SM anyway and a very small one finds idle SMs. Measured on GB300,
 // us a step without and with:
-//   FP64 2D   4k cells  65.5  57.3 |  16k  67.6  64.1 |  33k 129.0 131.0 | 66k 190.4 231.4
-//           101k cells 255.9 272.4 | 135k 330.7 311.3 | 393k 798.7 772.1
-//   FP64 3D   5k cells 157.7 147.4 |  18k 184.3 194.5 |  43k 305.2 343.5 | 83k 460.7 475.0
-//           117k cells 608.2 587.7 | 229k 1047.5 1029.1
-//   FP32 2D   4k cells  45.1  43.0 |  16k  47.1  43.0 | 101k  73.7  65.5 | 393k 157.6 143.3
-//   FP32 3D   5k cells  94.2  86.0 |  43k 104.4  98.4 |  61k 114.7 118.8 | 83k 124.9 126.9
-//           117k cells 133.1 131.0 | 229k 209.9 200.7
+//   FP64 2D   2k cells  83.9  71.6 |  16k  57.3  51.1 | 33k 122.8 137.2 | 66k 184.2 233.4
+//           101k cells 247.7 256.5 | 135k 305.1 307.1 | 194k 425.9 405.1 | 262k 272.3 266.2
+//   FP64 3D   5k cells 141.3 133.1 |  10k 145.3 159.7 | 43k 284.6 298.9 | 83k 430.0 454.6
+//           117k cells 585.6 582.6 | 229k 1037.2 1015.7
+//   FP32 2D   2k cells  57.6  51.1 |  16k  45.0  42.9 | 101k 73.6  65.4 | 194k 90.0  79.8
+//   FP32 3D   5k cells  90.0  81.8 |  43k  98.2  90.0 | 61k 110.6 112.5 | 83k 114.6 128.9
+//           117k cells 130.1 135.1 | 229k 196.5 185.3
+// (between 90k and 160k cells, inviscid FP64 2D gains 4 %, viscous loses 1-4 %).
 inline bool pdl_pays(bool fp64, int D, int nc) {
-    if (nc >= 114688) return true;
-    if (fp64) return nc <= (D == 2 ? 16384 : 8192);
-    return D == 2 || nc <= 49152;
+    if (D == 2) return !fp64 || nc <= 16384 || nc >= 163840;
+    return fp64 ? nc <= 8192 || nc >= 131072 : nc <= 49152 || nc >= 163840;
 }
 
 // Launches k, with `pdl` as a programmatic dependent of the stream's previous
