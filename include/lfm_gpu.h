@@ -323,9 +323,9 @@ const char* lfm_solver_kernel_name(int i);
 /* Flux kernel of an FP32-bulk solver (no reference counterpart: the
  * reference evaluates its faces in one loop). Every variant gives the same
  * bits; they differ in how a face's values reach the SM:
- *   LFM_FLUX_FACE    one thread per face;
+ *   LFM_FLUX_FACE    one thread per face (the default);
  *   LFM_FLUX_CELL    one thread per cell over the faces it owns, the cell's
- *                    own rows read once (the default for 3D cases);
+ *                    own rows read once;
  *   LFM_FLUX_STAGED  the values each face reads copied into shared memory
  *                    ahead of use with cp.async: staging_depth buffers per
  *                    thread (1: one slot beside the registers; 2..4: chunks

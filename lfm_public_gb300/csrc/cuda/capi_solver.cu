@@ -416,15 +416,6 @@ cudaError_t launchStepGraph(lfm_solver* s) {
 
 namespace {
 
-// FP32-bulk: the update kernel writes the boundary ghosts' next state (no
-// preparation launch per stage) up to these cell counts. The ghost branch
-// raises the update kernel's registers (2D 32 -> 48, 3D 32 -> 58); measured on
-// GB300 the saved launch wins for a 393k-cell 2D case (0.224 against 0.239 ms
-// per step) and the lower occupancy loses for a 1.57M-cell 2D case (0.838
-// against 0.826) and for a 9.4M-cell 3D case (8.65 against 7.75 ms).
-constexpr int kFuseGhostCells2D = 1 << 20;
-constexpr int kFuseGhostCells3D = 1 << 18;
-
 // Fused tile stages (tile_kernels.cu): cells per tile, 0 = off. Off by
 // default: measured on GB300 (768x512 cylinder, Hilbert order, FP32-bulk M1)
 // a step took 0.352 ms in 256-cell tiles against 0.226 ms with the separate
@@ -455,28 +446,27 @@ int tileCellsOption() {
 constexpr bool kFaceOrderBySlot3D = false;
 
 // Fused flux + update stages (LFM_FLUX_UPDATE=0/1 in the environment
-// overrides for a solver created afterwards). Measured on GB300, FP32-bulk,
-// per step: the 256 x 256 inviscid M1 vortex 0.075 -> 0.070 ms; the 768 x 512
-// viscous cylinder 0.192 -> 0.259 ms (M1), 0.198 -> 0.255 (M2), 0.45 -> 0.89
-// (M2AUSM); a 96 x 64 x 24 viscous 3D wake 0.201 -> 0.263. Each face is
-// evaluated twice, and with the viscous rows of both cells the fused kernel
-// needs 64 (2D) to 123 (3D M2AUSM) registers: it gains only where the flux is
-// short, the inviscid M1/M2 cases.
+// overrides for a solver created afterwards). Each face is evaluated twice, so
+// they pay where the flux is short, the inviscid M1 / M2 cases in 2D. Measured
+// on GB300, FP32-bulk, us a step without and with: M2 vortex of 512 x 512 cells
+// 67.5, 59.3, 1000 x 1000 241.6, 237.4, 1800 x 1800 755.6, 681.4; the viscous
+// 768 x 512 cylinder 162, 233, the 331 x 217 M2AUSM one 135, 182.
 bool fluxUpdateOption(const lfm_solver* s) {
     const char* e = getenv("LFM_FLUX_UPDATE");
     if (e) return atoi(e) != 0;
     return s->D == 2 && !s->needVis && s->scheme != LFM_SOLVER_M2AUSM;
 }
 
-// Cell-centred flux kernel (flux32_cell), on for 3D cases. Measured on
-// GB300, FP32-bulk M2, per step: the 9.4M-cell wake's flux 3.42 -> 3.27 ms
-// (the step 6.97 -> 6.82), the 1.18M-cell wake's 0.445 -> 0.416; the 768 x 512
-// M1 cylinder's 0.068 -> 0.085 (a 2D cell owns two faces, too few to repay
-// the registers it keeps). LFM_FLUX_CELL=0/1 in the environment overrides
-// for a solver created afterwards.
-bool fluxCellOption(const lfm_solver* s) {
+// Cell-centred flux kernel (flux32_cell), off. With the cells' values in
+// 16-byte parts a thread per face reads a cell's rows in six loads, and holding
+// them across a cell's faces costs more in registers (80 against 64) than it
+// saves: FP32-bulk M2 flux, us a step, by cell and by face, 192 x 128 x 48
+// cells 353, 334, 256 x 184 x 64 858, 828, 1536 x 1024 231, 204 (GB300).
+// LFM_FLUX_CELL=0/1 in the environment overrides for a solver created
+// afterwards.
+bool fluxCellOption() {
     const char* e = getenv("LFM_FLUX_CELL");
-    return e ? atoi(e) != 0 : s->D == 3;
+    return e && atoi(e) != 0;
 }
 
 // Staged flux kernel (flux_staged_fp32.cu): shared-memory buffers per
@@ -689,11 +679,11 @@ int createSolver(const lfm_solver_desc* d, const lfm_solver_opts* opts, cudaStre
             }
         }
     }
-    // the tile stages need the update to write the ghosts; the FP64 update
-    // always writes them (its kernel is bound by the FP64 pipe, not by the
-    // registers the ghost branch adds)
-    if (s->precision == LFM_FP64 ||
-        tiled || s->nc <= (s->D == 2 ? kFuseGhostCells2D : kFuseGhostCells3D)) {
+    // The update writes the boundary ghosts' next state, so that no preparation
+    // launch runs between the stages: us a step without and with (GB300,
+    // FP32-bulk) of 192 x 128 x 48 cells 867, 824, 256 x 184 x 64 2002, 1952,
+    // 1536 x 1024 603, 571.
+    {
         // cells with boundary faces: their update writes the ghosts' next state
         std::vector<uint8_t> cg(nc, 0);
         for (size_t f = 0; f < nf; ++f)
@@ -770,7 +760,7 @@ int createSolver(const lfm_solver_desc* d, const lfm_solver_opts* opts, cudaStre
             for (size_t f = 0; f < nf; ++f) ++own[(size_t)fP[f] + 1];
             for (size_t c = 0; c < nc; ++c) own[c + 1] += own[c];
             if ((rc = upload(s, &s->fOwnDev, own.data(), nc + 1))) return fail(rc);
-            if (fluxCellOption(s)) s->a32.fOwn = s->fOwnDev;
+            if (fluxCellOption()) s->a32.fOwn = s->fOwnDev;
         }
     }
     if (s->fluxVariants) {
