@@ -1,8 +1,8 @@
 // C ABI, device half: the solver handle (include/lfm_gpu.h).
 //
 // A solver owns its device arrays and one CUDA stream. A full time step
-// (rk_order stages of 3-5 kernels) is captured once into a CUDA graph and
-// replayed; the graph is captured again only when dt changes.
+// (rk_order stages of 1-5 kernels) is captured once into a CUDA graph and
+// replayed; the kernels read dt from device memory.
 #include <algorithm>
 #include <cmath>
 #include <cstdio>
@@ -51,7 +51,12 @@ struct lfm_solver {
     double* cellS = nullptr;
     double* volInv = nullptr;
     cudaGraphExec_t graph = nullptr;
-    double graphDt = 0;
+    // the time step in device memory (a graph serves every dt), its host copy
+    lfm::dev::StepDt* step = nullptr;
+    double stepDt = 0;
+    bool stepSet = false;
+    unsigned* arrived = nullptr;     // k_cfl's arrival counter
+    double* scalarHost = nullptr;    // page-locked: k_cfl's result
     // FP32-bulk: q holds q - q_ref, and the update kernel keeps the cells'
     // primitives current; they are stale after a new state is set.
     bool primsValid = false;
@@ -98,12 +103,11 @@ struct lfm_solver {
     int* flagHost = nullptr;
     // lfm_solver_advance between page-locked host states as one graph (copy
     // in, conversion, primitives, steps, conversion, copy out, flag), kept
-    // for the pointers, step count and dt it was captured with
+    // for the pointers and step count it was captured with
     cudaGraphExec_t advGraph = nullptr;
     const double* advIn = nullptr;
     double* advOut = nullptr;
     int advSteps = 0;
-    double advDt = 0;
 };
 
 namespace {
@@ -177,6 +181,7 @@ int buildArgs(lfm_solver* s, const lfm_solver_desc* d, Args<T>& a, const int* fP
     a.gKind = gKind;
     a.gFace = gFace;
     a.flag = s->flag;
+    a.step = s->step;
     a.cellGhosts = nullptr;
     a.cfEll = nullptr;
     a.cfEllN = nullptr;
@@ -282,14 +287,13 @@ int buildArgs(lfm_solver* s, const lfm_solver_desc* d, Args<T>& a, const int* fP
     return LFM_OK;
 }
 
-StageConfig stageConfig(const lfm_solver* s, int k, double dt) {
+StageConfig stageConfig(const lfm_solver* s, int k) {
     StageConfig c;
     c.scheme = s->scheme;
     c.needGrad = s->needGrad;
     c.needVis = s->needVis;
     c.A = s->rkA[(size_t)k];
     c.B = s->rkB[(size_t)k];
-    c.dt = dt;
     c.first = (k == 0);
     c.withRes = (s->residuals && k == 0) ? 1 : 0;
     c.fullPrep = false;   // FP32-bulk: cells' primitives come from the previous update
@@ -298,9 +302,9 @@ StageConfig stageConfig(const lfm_solver* s, int k, double dt) {
 }
 
 template <typename T>
-void stageAll(lfm_solver* s, const Args<T>& a, double dt) {
+void stageAll(lfm_solver* s, const Args<T>& a) {
     for (int k = 0; k < s->rkOrder; ++k) {
-        StageConfig c = stageConfig(s, k, dt);
+        StageConfig c = stageConfig(s, k);
         c.pdl = true;
         lfm::dev::launch_stage<T>(a, c, s->stream);
     }
@@ -308,7 +312,7 @@ void stageAll(lfm_solver* s, const Args<T>& a, double dt) {
 
 // Fused tile stage k of a step that starts from primitive buffer `parity`:
 // reads buffer (parity + k) % 2, writes the other.
-void tileStage(lfm_solver* s, int k, double dt, int parity) {
+void tileStage(lfm_solver* s, int k, int parity) {
     float* buf[2] = {s->a32.prim, s->prim1};
     const int in = (parity + k) & 1;
     Args<float> g = s->a32;
@@ -316,7 +320,7 @@ void tileStage(lfm_solver* s, int k, double dt, int parity) {
     g.primW = g.prim;
     lfm::dev::TileArgs t = s->tile;
     t.primIn = buf[in];
-    lfm::dev::launch_tile_stage(g, t, stageConfig(s, k, dt), s->stream);
+    lfm::dev::launch_tile_stage(g, t, stageConfig(s, k), s->stream);
 }
 
 // Stage kernels that alternate two primitive buffers (tile stages, fused
@@ -327,13 +331,13 @@ bool alternating(const lfm_solver* s) { return s->tiled || s->fluxUpdate; }
 // `parity`: the preparation (halos and ghosts it still has), gradient and
 // viscous kernels read buffer (parity + k) % 2, the fused kernel writes the
 // other.
-void fluxUpdateStage(lfm_solver* s, int k, double dt, int parity) {
+void fluxUpdateStage(lfm_solver* s, int k, int parity) {
     float* buf[2] = {s->a32.prim, s->prim1};
     const int in = (parity + k) & 1;
     Args<float> g = s->a32;
     g.prim = buf[in];
     g.primW = buf[in ^ 1];
-    StageConfig c = stageConfig(s, k, dt);
+    StageConfig c = stageConfig(s, k);
     c.pdl = true;
     for (int w = 0; w < 3; ++w) lfm::dev::launch_kernel<float>(g, c, w, s->stream);   // prep, grad, vis
     lfm::dev::launch_fluxupdate32(g, c, s->stream);
@@ -368,21 +372,21 @@ int ensurePrims(lfm_solver* s) {
     return LFM_OK;
 }
 
-void launchStep(lfm_solver* s, double dt, int parity) {
+void launchStep(lfm_solver* s, int parity) {
     if (s->tiled)
-        for (int k = 0; k < s->rkOrder; ++k) tileStage(s, k, dt, parity);
+        for (int k = 0; k < s->rkOrder; ++k) tileStage(s, k, parity);
     else if (s->fluxUpdate)
-        for (int k = 0; k < s->rkOrder; ++k) fluxUpdateStage(s, k, dt, parity);
+        for (int k = 0; k < s->rkOrder; ++k) fluxUpdateStage(s, k, parity);
     else if (s->precision == LFM_FP32_BULK)
-        stageAll<float>(s, s->a32, dt);
+        stageAll<float>(s, s->a32);
     else
-        stageAll<double>(s, s->a64, dt);
+        stageAll<double>(s, s->a64);
 }
 
-int captureStep(lfm_solver* s, double dt, int parity, cudaGraphExec_t* out) {
+int captureStep(lfm_solver* s, int parity, cudaGraphExec_t* out) {
     cudaGraph_t g = nullptr;
     LFM_CUDA(cudaStreamBeginCapture(s->stream, cudaStreamCaptureModeThreadLocal));
-    launchStep(s, dt, parity);
+    launchStep(s, parity);
     cudaError_t e = cudaStreamEndCapture(s->stream, &g);
     if (e != cudaSuccess) return cudaFail(e, "cudaStreamEndCapture");
     e = cudaGraphInstantiate(out, g, 0);
@@ -391,18 +395,25 @@ int captureStep(lfm_solver* s, double dt, int parity, cudaGraphExec_t* out) {
     return LFM_OK;
 }
 
-// One graph per time step; with tile stages a second one for steps that
+// The time step of what is launched next. A run that adapts its dt changes it
+// every step: one store on the stream, where capturing and instantiating the
+// step's graph again for each dt took about as long as a small case's step.
+int setStep(lfm_solver* s, double dt) {
+    if (s->stepSet && s->stepDt == dt) return LFM_OK;
+    lfm::dev::launch_set_step(s->step, dt, s->stream);
+    LFM_CUDA(cudaGetLastError());
+    s->stepDt = dt;
+    s->stepSet = true;
+    return LFM_OK;
+}
+
+// One graph per time step; with alternating buffers a second one for steps that
 // start from prim1 (an odd stage count swaps the buffers every step).
 int ensureGraph(lfm_solver* s, double dt) {
-    if (s->graph && s->graphDt == dt) return LFM_OK;
-    if (s->graph) cudaGraphExecDestroy(s->graph);
-    if (s->graphOdd) cudaGraphExecDestroy(s->graphOdd);
-    s->graph = s->graphOdd = nullptr;
-    int rc = captureStep(s, dt, 0, &s->graph);
-    if (!rc && alternating(s)) rc = captureStep(s, dt, 1, &s->graphOdd);
-    if (rc) return rc;
-    s->graphDt = dt;
-    return LFM_OK;
+    int rc = LFM_OK;
+    if (!s->graph) rc = captureStep(s, 0, &s->graph);
+    if (!rc && alternating(s) && !s->graphOdd) rc = captureStep(s, 1, &s->graphOdd);
+    return rc ? rc : setStep(s, dt);
 }
 
 // Launches the step graph matching the current primitive buffer.
@@ -623,6 +634,8 @@ int createSolver(const lfm_solver_desc* d, const lfm_solver_opts* opts, cudaStre
     if ((rc = devAlloc(s, &s->partial, nPartial))) return fail(rc);
     if ((rc = devAlloc(s, &s->scalar, 16))) return fail(rc);
     if ((rc = devAlloc(s, &s->flag, 1))) return fail(rc);
+    if ((rc = devAlloc(s, &s->step, 1))) return fail(rc);
+    if ((rc = devAlloc(s, &s->arrived, 1))) return fail(rc);
     if ((rc = upload(s, &s->volInv, d->vol_inv, nc))) return fail(rc);
 
     // connectivity as 32-bit indices
@@ -778,6 +791,9 @@ int createSolver(const lfm_solver_desc* d, const lfm_solver_opts* opts, cudaStre
     if ((e = cudaHostAlloc(reinterpret_cast<void**>(&s->flagHost), sizeof(int), cudaHostAllocDefault)) != cudaSuccess)
         return fail(cudaFail(e, "cudaHostAlloc"));
     *s->flagHost = 0;
+    if ((e = cudaHostAlloc(reinterpret_cast<void**>(&s->scalarHost), sizeof(double), cudaHostAllocDefault)) !=
+        cudaSuccess)
+        return fail(cudaFail(e, "cudaHostAlloc"));
     if (d->q0) {
         if ((e = cudaStreamSynchronize(s->stream)) != cudaSuccess) return fail(cudaFail(e, "create"));
         if ((rc = lfm_solver_set_state(s, d->q0))) return fail(rc);
@@ -801,6 +817,7 @@ extern "C" void lfm_solver_destroy(lfm_solver* s) {
     if (s->graphOdd) cudaGraphExecDestroy(s->graphOdd);
     if (s->advGraph) cudaGraphExecDestroy(s->advGraph);
     if (s->flagHost) cudaFreeHost(s->flagHost);
+    if (s->scalarHost) cudaFreeHost(s->scalarHost);
     for (void* p : s->allocations) cudaFree(p);
     if (s->scrub) cudaFree(s->scrub);
     if (s->dPatches) cudaFree(s->dPatches);
@@ -883,9 +900,9 @@ namespace {
 
 // The whole advance between page-locked host states as one graph launch
 // (device work only; the host-side state flags are set as the enqueued path
-// leaves them). Captured once per (q_in, q_out, nsteps, dt).
+// leaves them). Captured once per (q_in, q_out, nsteps).
 int advanceGraph(lfm_solver* s, const double* qIn, int nsteps, double dt, double* qOut) {
-    if (!(s->advGraph && s->advIn == qIn && s->advOut == qOut && s->advSteps == nsteps && s->advDt == dt)) {
+    if (!(s->advGraph && s->advIn == qIn && s->advOut == qOut && s->advSteps == nsteps)) {
         if (s->advGraph) cudaGraphExecDestroy(s->advGraph);
         s->advGraph = nullptr;
         cudaGraph_t g = nullptr;
@@ -896,7 +913,7 @@ int advanceGraph(lfm_solver* s, const double* qIn, int nsteps, double dt, double
         // the current primitives to the other buffer after an odd stage count
         int parity = 0;
         for (int k = 0; k < nsteps && !rc; ++k) {
-            launchStep(s, dt, parity);
+            launchStep(s, parity);
             if (alternating(s)) parity ^= (s->rkOrder & 1);
         }
         if (!rc) rc = enqueueGetState(s, qOut);
@@ -913,8 +930,9 @@ int advanceGraph(lfm_solver* s, const double* qIn, int nsteps, double dt, double
         s->advIn = qIn;
         s->advOut = qOut;
         s->advSteps = nsteps;
-        s->advDt = dt;
     }
+    const int rc = setStep(s, dt);
+    if (rc) return rc;
     LFM_CUDA(cudaGraphLaunch(s->advGraph, s->stream));
     // the flags the enqueued path leaves: a new state, its primitives, stages run
     s->primParity = alternating(s) ? ((nsteps * s->rkOrder) & 1) : 0;
@@ -947,9 +965,10 @@ extern "C" int lfm_solver_stage(lfm_solver* s, int rk, double dt) {
     LFM_CUDA(cudaSetDevice(s->device));
     untile(s);
     int rc = ensurePrims(s);
+    if (!rc) rc = setStep(s, dt);
     if (rc) return rc;
     s->lastStageB = s->rkB[(size_t)rk];
-    const StageConfig c = stageConfig(s, rk, dt);
+    const StageConfig c = stageConfig(s, rk);
     if (s->precision == LFM_FP32_BULK)
         lfm::dev::launch_stage<float>(s->a32, c, s->stream);
     else
@@ -992,10 +1011,10 @@ static int reduceScalar(lfm_solver* s, double dt, int mode, double maxCo, double
     lfm::dev::QOffset qo;
     for (int v = 0; v < 5; ++v) qo.v[v] = s->qRef[v];
     lfm::dev::launch_cfl(s->D, s->q, qo, s->nt, s->nc, s->volInv, s->sOff, s->cellS, dt, mode, maxCo, s->partial,
-                         s->scalar, s->stream);
+                         s->arrived, s->scalarHost, s->stream);
     LFM_CUDA(cudaGetLastError());
-    LFM_CUDA(cudaMemcpyAsync(out, s->scalar, sizeof(double), cudaMemcpyDeviceToHost, s->stream));
     LFM_CUDA(cudaStreamSynchronize(s->stream));
+    *out = *s->scalarHost;
     return LFM_OK;
 }
 
@@ -1427,8 +1446,8 @@ cudaError_t medianTime(lfm_solver* s, int reps, cudaEvent_t e0, cudaEvent_t e1, 
     return cudaSuccess;
 }
 
-void launchOne(lfm_solver* s, const Launch& l, double dt) {
-    StageConfig c = stageConfig(s, l.stage, dt);
+void launchOne(lfm_solver* s, const Launch& l) {
+    StageConfig c = stageConfig(s, l.stage);
     c.pdl = true;   // as in the step
     if (s->fluxUpdate) {   // buffers of a step that starts from buffer 0
         float* buf[2] = {s->a32.prim, s->prim1};
@@ -1446,13 +1465,13 @@ void launchOne(lfm_solver* s, const Launch& l, double dt) {
 }
 
 // Graph of the launches [0, m) of `seq` (nullptr when m == 0).
-cudaError_t prefixGraph(lfm_solver* s, const std::vector<Launch>& seq, size_t m, double dt, cudaGraphExec_t* out) {
+cudaError_t prefixGraph(lfm_solver* s, const std::vector<Launch>& seq, size_t m, cudaGraphExec_t* out) {
     *out = nullptr;
     if (m == 0) return cudaSuccess;
     cudaGraph_t g = nullptr;
     cudaError_t e = cudaStreamBeginCapture(s->stream, cudaStreamCaptureModeThreadLocal);
     if (e != cudaSuccess) return e;
-    for (size_t k = 0; k < m; ++k) launchOne(s, seq[k], dt);
+    for (size_t k = 0; k < m; ++k) launchOne(s, seq[k]);
     e = cudaStreamEndCapture(s->stream, &g);
     if (e == cudaSuccess) e = cudaGraphInstantiate(out, g, 0);
     if (g) cudaGraphDestroy(g);
@@ -1467,6 +1486,7 @@ extern "C" int lfm_solver_profile_step(lfm_solver* s, double dt, int n, float* m
     for (int k = 0; k < n; ++k) ms[k] = 0.f;
     if (s->rkOrder == 0) return LFM_OK;   // no stage, no kernel
     int rc = ensurePrims(s);
+    if (!rc) rc = setStep(s, dt);
     if (rc) return rc;
     constexpr int kReps = 7;
     cudaEvent_t e0 = nullptr, e1 = nullptr;
@@ -1496,7 +1516,7 @@ extern "C" int lfm_solver_profile_step(lfm_solver* s, double dt, int n, float* m
                 cudaGraph_t g = nullptr;
                 e = cudaStreamBeginCapture(s->stream, cudaStreamCaptureModeThreadLocal);
                 if (e != cudaSuccess) break;
-                launchOne(s, Launch{k, w}, dt);
+                launchOne(s, Launch{k, w});
                 e = cudaStreamEndCapture(s->stream, &g);
                 size_t nodes = 0;
                 if (e == cudaSuccess) e = cudaGraphGetNodes(g, nullptr, &nodes);
@@ -1506,7 +1526,7 @@ extern "C" int lfm_solver_profile_step(lfm_solver* s, double dt, int n, float* m
         float prev = t0;
         for (size_t m = 1; m <= seq.size() && e == cudaSuccess; ++m) {
             cudaGraphExec_t ge = nullptr;
-            e = prefixGraph(s, seq, m, dt, &ge);
+            e = prefixGraph(s, seq, m, &ge);
             float t = 0.f;
             if (e == cudaSuccess) e = medianTime(s, kReps, e0, e1, [s, ge] { return cudaGraphLaunch(ge, s->stream); }, &t);
             if (ge) cudaGraphExecDestroy(ge);
@@ -1547,13 +1567,12 @@ struct lfm_partitioned {
     void** dV = nullptr;                    // per-partition viscous-term base pointers
     int* dNt = nullptr;                     // per-partition row strides
     cudaGraphExec_t graph = nullptr;
-    double graphDt = 0;
 };
 
 namespace {
 
 template <typename T>
-void partitionedStages(lfm_partitioned* P, double dt) {
+void partitionedStages(lfm_partitioned* P) {
     const size_t np = P->parts.size();
     auto args = [&](size_t p) -> const Args<T>& {
         if constexpr (sizeof(T) == sizeof(float)) return P->parts[p]->a32;
@@ -1561,7 +1580,7 @@ void partitionedStages(lfm_partitioned* P, double dt) {
     };
     lfm_solver* s0 = P->parts[0];
     for (int k = 0; k < s0->rkOrder; ++k) {
-        const StageConfig c = stageConfig(s0, k, dt);
+        const StageConfig c = stageConfig(s0, k);
         for (size_t p = 0; p < np; ++p) {
             const lfm_solver* s = P->parts[p];
             lfm::dev::launch_halo_gather<double>(s->q, s->nt, s->nc + s->ng, s->nq, s->nh, P->haloPart[p],
@@ -1588,24 +1607,19 @@ void partitionedStages(lfm_partitioned* P, double dt) {
     }
 }
 
-int partitionedGraph(lfm_partitioned* P, double dt) {
-    if (P->graph && P->graphDt == dt) return LFM_OK;
-    if (P->graph) {
-        cudaGraphExecDestroy(P->graph);
-        P->graph = nullptr;
-    }
+int partitionedGraph(lfm_partitioned* P) {
+    if (P->graph) return LFM_OK;
     cudaGraph_t g = nullptr;
     LFM_CUDA(cudaStreamBeginCapture(P->stream, cudaStreamCaptureModeThreadLocal));
     if (P->precision == LFM_FP32_BULK)
-        partitionedStages<float>(P, dt);
+        partitionedStages<float>(P);
     else
-        partitionedStages<double>(P, dt);
+        partitionedStages<double>(P);
     cudaError_t e = cudaStreamEndCapture(P->stream, &g);
     if (e != cudaSuccess) return cudaFail(e, "cudaStreamEndCapture");
     e = cudaGraphInstantiate(&P->graph, g, 0);
     cudaGraphDestroy(g);
     if (e != cudaSuccess) return cudaFail(e, "cudaGraphInstantiate");
-    P->graphDt = dt;
     return LFM_OK;
 }
 
@@ -1717,10 +1731,10 @@ extern "C" int lfm_partitioned_step(lfm_partitioned* P, int nsteps, double dt) {
     if (!P || nsteps < 0) return lfm::setError(LFM_ERR_INVALID, "bad argument");
     if (nsteps == 0) return LFM_OK;
     LFM_CUDA(cudaSetDevice(P->device));
-    int rc = partitionedGraph(P, dt);
+    int rc = partitionedGraph(P);
     if (rc) return rc;
     for (lfm_solver* s : P->parts)
-        if ((rc = ensurePrims(s))) return rc;
+        if ((rc = ensurePrims(s)) || (rc = setStep(s, dt))) return rc;
     for (int k = 0; k < nsteps; ++k) LFM_CUDA(cudaGraphLaunch(P->graph, P->stream));
     return LFM_OK;
 }
@@ -1755,7 +1769,6 @@ void dropGraphs(lfm_solver* s) {
     if (s->graphOdd) cudaGraphExecDestroy(s->graphOdd);
     if (s->advGraph) cudaGraphExecDestroy(s->advGraph);
     s->graph = s->graphOdd = s->advGraph = nullptr;
-    s->graphDt = 0;
     s->advIn = nullptr;
     s->advOut = nullptr;
 }

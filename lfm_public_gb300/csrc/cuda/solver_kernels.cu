@@ -468,10 +468,10 @@ __global__ void __launch_bounds__(kFaceThreads<D>) k_flux(Args<T> a) {
 // and primitives of its boundary ghosts.
 // ---------------------------------------------------------------------------
 template <typename T, int D, bool RES>
-__global__ void __launch_bounds__(kCellThreads<D>) k_update(const __grid_constant__ Args<T> a, double Ak, double Bk, double dt, int first) {
+__global__ void __launch_bounds__(kCellThreads<D>) k_update(const __grid_constant__ Args<T> a, double Ak, double Bk, int first) {
     const int c = LFM_GLOBAL_ID();
     if (c >= a.nc) return;
-    update_cell<T, D, RES, true>(a, c, Ak, Bk, dt, first, PdlWait{a.pdl});
+    update_cell<T, D, RES, true>(a, c, Ak, Bk, a.step->dt, first, PdlWait{a.pdl});
 }
 
 // ---------------------------------------------------------------------------
@@ -479,47 +479,70 @@ __global__ void __launch_bounds__(kCellThreads<D>) k_update(const __grid_constan
 // squared cell residuals. Block results go to partials, a single block
 // finishes; both levels use a fixed tree, so results are reproducible.
 // ---------------------------------------------------------------------------
+//
+// k_cfl does both levels in one launch: the last block to finish (an arrival
+// counter that it resets) reduces the block results and writes the value to
+// page-locked host memory, so a caller waits for one launch and no copy. A run
+// with adjustTimeStep asks for one of these per step.
 template <int D>
 __global__ void __launch_bounds__(256) k_cfl(const double* q, QOffset qo, int nt, int nc, const double* volInv,
                                              const int* sOff, const double* cellS, double dt, int mode, double maxCo,
-                                             double* partial) {
+                                             double* partial, unsigned* arrived, double* out) {
     __shared__ double sh[256];
+    __shared__ bool last;
     const int c = LFM_GLOBAL_ID();
-    double v = (mode == 0) ? 0.0 : 100.0;
+    const double none = (mode == 0) ? 0.0 : 100.0;
+    double v = none;
     if (c < nc) {
         const double rho = q[c] + qo.v[0];
-        if (mode == 0) {
-            double cfl = 0;
-            for (int e = sOff[c]; e < sOff[c + 1]; ++e) {
-                double flux = 0.;
-                for (int k = 0; k < D; ++k) flux += (q[(size_t)(k + 1) * nt + c] + qo.v[k + 1]) * cellS[(size_t)e * D + k];
-                cfl += fabs(flux);
+        double m[D];
+#pragma unroll
+        for (int k = 0; k < D; ++k) m[k] = q[(size_t)(k + 1) * nt + c] + qo.v[k + 1];
+        double sum = 0.0;
+        for (int e = sOff[c]; e < sOff[c + 1]; ++e) {
+            double flux = 0.0, s2 = 0.0;
+#pragma unroll
+            for (int k = 0; k < D; ++k) {
+                const double S = cellS[(size_t)e * D + k];
+                flux += m[k] * S;
+                s2 += S * S;
             }
-            v = cfl * ((1.0 / rho) * volInv[c] * dt);
-        } else {
-            double sumFlux = 0;
-            for (int e = sOff[c]; e < sOff[c + 1]; ++e) {
-                const double* S = &cellS[(size_t)e * D];
-                double sMag = 0.;
-                for (int k = 0; k < D; ++k) sMag += S[k] * S[k];
-                sMag = sqrt(sMag);
-                double flux = 0.;
-                for (int k = 0; k < D; ++k) flux += (q[(size_t)(k + 1) * nt + c] + qo.v[k + 1]) * S[k] / sMag;
-                sumFlux += fabs(flux);
-            }
-            v = maxCo * rho * 2.0 * (1.0 / volInv[c]) / sumFlux;
+            // min dt: the flux through the unit area vector
+            sum += (mode == 0) ? fabs(flux) : fabs(flux * rsqrt(s2));
         }
+        v = (mode == 0) ? sum * ((1.0 / rho) * volInv[c] * dt) : maxCo * rho * 2.0 * (1.0 / volInv[c]) / sum;
     }
-    sh[threadIdx.x] = v;
-    __syncthreads();
-    for (int s = blockDim.x / 2; s > 0; s >>= 1) {
-        if (threadIdx.x < s) {
-            const double o = sh[threadIdx.x + s];
-            sh[threadIdx.x] = (mode == 0) ? fmax(sh[threadIdx.x], o) : fmin(sh[threadIdx.x], o);
-        }
+    auto reduce = [&](double x) {
+        sh[threadIdx.x] = x;
         __syncthreads();
+        for (int s = blockDim.x / 2; s > 0; s >>= 1) {
+            if (threadIdx.x < s) {
+                const double o = sh[threadIdx.x + s];
+                sh[threadIdx.x] = (mode == 0) ? fmax(sh[threadIdx.x], o) : fmin(sh[threadIdx.x], o);
+            }
+            __syncthreads();
+        }
+    };
+    reduce(v);
+    if (threadIdx.x == 0) {
+        partial[blockIdx.x] = sh[0];
+        __threadfence();
+        last = atomicAdd(arrived, 1u) == gridDim.x - 1;
     }
-    if (threadIdx.x == 0) partial[blockIdx.x] = sh[0];
+    __syncthreads();
+    if (!last) return;
+    __threadfence();
+    v = none;
+    for (int k = threadIdx.x; k < (int)gridDim.x; k += blockDim.x) {
+        const double o = *(volatile double*)(partial + k);
+        v = (mode == 0) ? fmax(v, o) : fmin(v, o);
+    }
+    __syncthreads();
+    reduce(v);
+    if (threadIdx.x == 0) {
+        *out = sh[0];
+        *arrived = 0;
+    }
 }
 
 __global__ void __launch_bounds__(256) k_reduce_final(const double* partial, int n, int mode, double* out) {
@@ -597,8 +620,8 @@ void launch_fp64(const Args<T>& a, const StageConfig& s, int which, cudaStream_t
             else launch_flux<T, D, kSchemeAUSM, LES>(a, s, st);
             break;
         case 4:
-            if (s.withRes) launch_kernel_pdl(s.pdl && a.pdl, k_update<T, D, true>, blocks(a.nc, kCellThreads<D>), kCellThreads<D>, st, a, s.A, s.B, s.dt, s.first);
-            else launch_kernel_pdl(s.pdl && a.pdl, k_update<T, D, false>, blocks(a.nc, kCellThreads<D>), kCellThreads<D>, st, a, s.A, s.B, s.dt, s.first);
+            if (s.withRes) launch_kernel_pdl(s.pdl && a.pdl, k_update<T, D, true>, blocks(a.nc, kCellThreads<D>), kCellThreads<D>, st, a, s.A, s.B, s.first);
+            else launch_kernel_pdl(s.pdl && a.pdl, k_update<T, D, false>, blocks(a.nc, kCellThreads<D>), kCellThreads<D>, st, a, s.A, s.B, s.first);
             break;
         default: break;
     }
@@ -631,14 +654,20 @@ void launch_kernel<float>(const Args<float>& a, const StageConfig& s, int which,
 }
 
 void launch_cfl(int D, const double* q, QOffset qo, int nt, int nc, const double* volInv, const int* sOff, const double* cellS,
-                double dt, int mode, double maxCo, double* partial, double* out, cudaStream_t st) {
+                double dt, int mode, double maxCo, double* partial, unsigned* arrived, double* out, cudaStream_t st) {
     const unsigned nb = blocks(nc, 256);
     if (D == 2)
-        k_cfl<2><<<nb, 256, 0, st>>>(q, qo, nt, nc, volInv, sOff, cellS, dt, mode, maxCo, partial);
+        k_cfl<2><<<nb, 256, 0, st>>>(q, qo, nt, nc, volInv, sOff, cellS, dt, mode, maxCo, partial, arrived, out);
     else
-        k_cfl<3><<<nb, 256, 0, st>>>(q, qo, nt, nc, volInv, sOff, cellS, dt, mode, maxCo, partial);
-    k_reduce_final<<<1, 256, 0, st>>>(partial, (int)nb, mode, out);
+        k_cfl<3><<<nb, 256, 0, st>>>(q, qo, nt, nc, volInv, sOff, cellS, dt, mode, maxCo, partial, arrived, out);
 }
+
+__global__ void k_set_step(StepDt* step, double dt, float dt32) {
+    step->dt = dt;
+    step->dt32 = dt32;
+}
+
+void launch_set_step(StepDt* step, double dt, cudaStream_t st) { k_set_step<<<1, 1, 0, st>>>(step, dt, (float)dt); }
 
 void launch_res_sum(const double* res, int nc, double* partial, double* out, cudaStream_t st) {
     const unsigned nb = blocks(nc, 256);

@@ -53,6 +53,13 @@ struct RefState32 {
 constexpr int visStride32(int D, bool les) { return D == 2 ? (les ? 12 : 8) : (les ? 24 : 16); }
 constexpr int gradStride32(int D) { return D == 2 ? 8 : 16; }
 
+// The time step of the single-case kernels, in device memory: a step's graph
+// serves every dt.
+struct StepDt {
+    double dt;
+    float dt32;   // dt rounded to FP32
+};
+
 // Arguments shared by the kernels (all device pointers).
 // Fixed-width cell -> face table (Args::cfEll): four entries per 2D cell
 // (quads, triangles), six per 3D cell (hexahedra, prisms, tetrahedra).
@@ -146,6 +153,7 @@ struct Args {
     RefState32 ref;
     // the primitives include the sound speed (read by M2AUSM only)
     int primC;
+    const StepDt* step;       // single cases: the time step, set before the step's kernels
     // error flag (non-finite state)
     int* flag;
     // the step's kernels are launched as programmatic dependents (pdl_pays)

@@ -68,34 +68,33 @@ template <int D>
 constexpr int kSpreadCells = D == 2 ? 1 << 20 : 1 << 18;
 
 template <int D, bool RES, bool GH, bool ELL>
-__device__ __forceinline__ void update_thread(const Args<float>& a, double Ak, double Bk, float dt32, int first) {
+__device__ __forceinline__ void update_thread(const Args<float>& a, double Ak, double Bk, int first) {
     const bool spread = GH && a.nc <= kSpreadCells<D>;
     const int c = spread ? (int)(((threadIdx.x >> 5) * gridDim.x + blockIdx.x) << 5) + (int)(threadIdx.x & 31u)
                          : (int)LFM_GLOBAL_ID();
-    if (c < a.nc) update32<D, GH, ELL ? kEntriesEll : kEntriesList>(a, c, Ak, Bk, dt32, first, RES, PdlWait{a.pdl});
+    if (c < a.nc) update32<D, GH, ELL ? kEntriesEll : kEntriesList>(a, c, Ak, Bk, a.step->dt32, first, RES, PdlWait{a.pdl});
 }
 
 template <int D, bool RES, bool GH, bool ELL>
 __global__ void __launch_bounds__(kCellThreads) k_update32(const __grid_constant__ Args<float> a, double Ak, double Bk,
-                                                  float dt32, int first) {
-    update_thread<D, RES, GH, ELL>(a, Ak, Bk, dt32, first);
+                                                            int first) {
+    update_thread<D, RES, GH, ELL>(a, Ak, Bk, first);
 }
 
 // Fused flux + update (fluxupdate32): one thread per cell, cells mapped as
 // in the update kernel that writes ghosts (warp-interleaved chunks).
 template <int D, int SCH, bool VIS, bool RES, bool ELL>
 __global__ void __launch_bounds__(kCellThreads) k_fluxupdate32(const __grid_constant__ Args<float> a, double Ak, double Bk,
-                                                      float dt32, int first) {
+                                                                int first) {
     const int c = (int)(((threadIdx.x >> 5) * gridDim.x + blockIdx.x) << 5) + (int)(threadIdx.x & 31u);
-    if (c < a.nc) fluxupdate32<D, SCH, VIS, true, ELL>(a, c, Ak, Bk, dt32, first, RES, PdlWait{a.pdl});
+    if (c < a.nc) fluxupdate32<D, SCH, VIS, true, ELL>(a, c, Ak, Bk, a.step->dt32, first, RES, PdlWait{a.pdl});
 }
 
 template <int D, int SCH, bool VIS, bool ELL>
 void launch_fluxupdate32_kernel(const Args<float>& a, const StageConfig& s, cudaStream_t st) {
     const unsigned nb = (unsigned)((a.nc + kCellThreads - 1) / kCellThreads);
-    const float dt32 = (float)s.dt;
-    if (s.withRes) launch_kernel_pdl(s.pdl && a.pdl, k_fluxupdate32<D, SCH, VIS, true, ELL>, nb, kCellThreads, st, a, s.A, s.B, dt32, s.first);
-    else launch_kernel_pdl(s.pdl && a.pdl, k_fluxupdate32<D, SCH, VIS, false, ELL>, nb, kCellThreads, st, a, s.A, s.B, dt32, s.first);
+    if (s.withRes) launch_kernel_pdl(s.pdl && a.pdl, k_fluxupdate32<D, SCH, VIS, true, ELL>, nb, kCellThreads, st, a, s.A, s.B, s.first);
+    else launch_kernel_pdl(s.pdl && a.pdl, k_fluxupdate32<D, SCH, VIS, false, ELL>, nb, kCellThreads, st, a, s.A, s.B, s.first);
 }
 
 template <int D, int SCH>
@@ -112,13 +111,12 @@ void launch_fluxupdate32_scheme(const Args<float>& a, const StageConfig& s, cuda
 template <int D, bool ELL>
 void launch_update32(const Args<float>& a, const StageConfig& s, cudaStream_t st) {
     const unsigned nb = (unsigned)((a.nc + kCellThreads - 1) / kCellThreads);   // a 32-cell chunk per warp
-    const float dt32 = (float)s.dt;
     if (a.cellGhosts) {
-        if (s.withRes) launch_kernel_pdl(s.pdl && a.pdl, k_update32<D, true, true, ELL>, nb, kCellThreads, st, a, s.A, s.B, dt32, s.first);
-        else launch_kernel_pdl(s.pdl && a.pdl, k_update32<D, false, true, ELL>, nb, kCellThreads, st, a, s.A, s.B, dt32, s.first);
+        if (s.withRes) launch_kernel_pdl(s.pdl && a.pdl, k_update32<D, true, true, ELL>, nb, kCellThreads, st, a, s.A, s.B, s.first);
+        else launch_kernel_pdl(s.pdl && a.pdl, k_update32<D, false, true, ELL>, nb, kCellThreads, st, a, s.A, s.B, s.first);
     } else {
-        if (s.withRes) launch_kernel_pdl(s.pdl && a.pdl, k_update32<D, true, false, ELL>, nb, kCellThreads, st, a, s.A, s.B, dt32, s.first);
-        else launch_kernel_pdl(s.pdl && a.pdl, k_update32<D, false, false, ELL>, nb, kCellThreads, st, a, s.A, s.B, dt32, s.first);
+        if (s.withRes) launch_kernel_pdl(s.pdl && a.pdl, k_update32<D, true, false, ELL>, nb, kCellThreads, st, a, s.A, s.B, s.first);
+        else launch_kernel_pdl(s.pdl && a.pdl, k_update32<D, false, false, ELL>, nb, kCellThreads, st, a, s.A, s.B, s.first);
     }
 }
 

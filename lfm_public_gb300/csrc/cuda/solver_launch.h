@@ -64,7 +64,6 @@ struct StageConfig {
     bool needGrad = false;
     bool needVis = true;
     double A = 0, B = 1;  // low-storage RK coefficients of this stage
-    double dt = 0;
     int first = 0;        // stage 0: dq starts from zero (prepare_for_timestep)
     int withRes = 0;      // record the stage-0 residual
     // FP32-bulk: the update writes the next stage's cell primitives, so the
@@ -133,9 +132,12 @@ struct QOffset {
 // FP64 path, at set-up: the face, entry and cell constants of a (wN, cfSoN,
 // cellSoW and, where allocated, mS .. kl) from its geometry.
 void launch_fp64_constants(const Args<double>& a, cudaStream_t st);
-// mode 0: max CFL, mode 1: min dt
+// mode 0: max CFL, mode 1: min dt; *arrived 0 before and after, out may be
+// page-locked host memory
 void launch_cfl(int D, const double* q, QOffset qo, int nt, int nc, const double* volInv, const int* sOff, const double* cellS,
-                double dt, int mode, double maxCo, double* partial, double* out, cudaStream_t st);
+                double dt, int mode, double maxCo, double* partial, unsigned* arrived, double* out, cudaStream_t st);
+// Sets the time step the single-case kernels read.
+void launch_set_step(StepDt* step, double dt, cudaStream_t st);
 void launch_res_sum(const double* res, int nc, double* partial, double* out, cudaStream_t st);
 void launch_set_flag(int* flag, int v, cudaStream_t st);
 // dst[v][c] = src[v][c] + sign * off.v[v], v < nq, c < n (row strides in elements).

@@ -30,7 +30,7 @@ struct TileRows {
 template <int D, int SCH, bool RES>
 __global__ void __launch_bounds__(256) k_tile_stage(const __grid_constant__ Args<float> g,
                                                     const __grid_constant__ TileArgs t, double Ak, double Bk,
-                                                    float dt32, int first) {
+                                                    int first) {
     using R = TileRows<D>;
     extern __shared__ float sm[];
     __shared__ Args<float> la;
@@ -98,7 +98,7 @@ __global__ void __launch_bounds__(256) k_tile_stage(const __grid_constant__ Args
         load_cell32<D, true>(g, td.c0 + lc, first, in);
         float sum[R::Q];
         gather32<D>(a, lc, sum);
-        apply32<D, true>(g, td.c0 + lc, sum, in, Ak, Bk, dt32, first, RES);
+        apply32<D, true>(g, td.c0 + lc, sum, in, Ak, Bk, g.step->dt32, first, RES);
     }
 }
 
@@ -113,7 +113,7 @@ cudaError_t launchTiles(const Args<float>& g, const TileArgs& t, const StageConf
         if (e != cudaSuccess) return e;
         smemSet[s.withRes ? 1 : 0] = smem;
     }
-    k<<<t.nTiles, t.block, smem, st>>>(g, t, s.A, s.B, (float)s.dt, s.first);
+    k<<<t.nTiles, t.block, smem, st>>>(g, t, s.A, s.B, s.first);
     return cudaGetLastError();
 }
 
