@@ -1137,8 +1137,8 @@ int residualNoalloc(const lfm_solver* s, const Args<T>& base, const double* q, i
     if (rc) return rc;
     Args<T> a = base;
     // FP32-bulk: the padded viscous and gradient rows take 4 bytes a cell each
-    // more in 3D, the space of q' (at least 32 bytes a cell) holds the face rhs:
-    // the fluxes read the primitives alone, so q' is dead by then.
+    // more in 3D; q' is not kept, and the face rhs take its space (at least 32
+    // bytes a cell).
     constexpr bool fp32 = sizeof(T) == sizeof(float);
     const size_t pV = round(lfm::dev::visWords<T>(s->D, base.smagC != nullptr) * nt * sizeof(T));
     const size_t pGrad = ausm ? round(lfm::dev::gradWords<T>(s->D) * nt * sizeof(T)) : 0;
@@ -1154,25 +1154,18 @@ int residualNoalloc(const lfm_solver* s, const Args<T>& base, const double* q, i
     a.dq = nullptr;
     a.res = nullptr;
     // The array keeps the previous call's contents: the viscous terms and
-    // gradients of the ghosts are read as zeros, so clear both blocks.
-    LFM_CUDA(cudaMemsetAsync(a.V, 0, pV, st));
-    if (ausm) LFM_CUDA(cudaMemsetAsync(a.grad, 0, pGrad, st));
-    if constexpr (sizeof(T) == sizeof(float)) {
-        // the FP32-bulk kernels read the state as q - q_ref
-        lfm::dev::launch_to_perturbation(a, q, qStride, st);
-    } else {
-        // rows of nc values (stride q_stride) into rows of nt, one strided copy
-        LFM_CUDA(cudaMemcpy2DAsync(a.q, nt * sizeof(double), q, (size_t)qStride * sizeof(double),
-                                   (size_t)s->nc * sizeof(double), nq, cudaMemcpyDeviceToDevice, st));
-    }
+    // gradients of the ghosts are read as zeros, so the preparation clears them.
+    const int vWords = (int)lfm::dev::visWords<T>(s->D, base.smagC != nullptr);
+    const int gradWords = ausm ? (int)lfm::dev::gradWords<T>(s->D) : 0;
+    const int cellGrad = ausm && !s->needGrad ? 1 : 0;   // M2AUSM without minmod reads zeros everywhere
+    if constexpr (fp32) lfm::dev::launch_prep_residual32(a, q, qStride, vWords, gradWords, cellGrad, st);
+    else lfm::dev::launch_prep_residual64(a, q, qStride, vWords, gradWords, cellGrad, st);
     StageConfig c;
     c.scheme = s->scheme;
     c.needGrad = s->needGrad;
     c.needVis = s->needVis;
-    for (int k = 0; k < 4; ++k) {   // prep (every cell: always launched), grad, vis, flux
-        lfm::dev::launch_kernel<T>(a, c, k, st);
-        c.pdl = true;
-    }
+    c.pdl = true;
+    for (int k = 1; k < 4; ++k) lfm::dev::launch_kernel<T>(a, c, k, st);   // grad, vis, flux
     const unsigned nb = (unsigned)((s->nc + 255) / 256);
     lfm::dev::launch_kernel_pdl(a.pdl, s->D == 2 ? k_gather_residual<T, 2> : k_gather_residual<T, 3>, nb, 256, st, a.flux,
                                 s->nf, s->nc, a.cfOff, a.cfList, res, a.pdl);

@@ -27,6 +27,13 @@ struct PdlWait {
         asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
     }
 };
+// The first kernel of a chain has nothing to wait for.
+struct PdlRelease {
+    int pdl;
+    __device__ __forceinline__ void operator()() const {
+        if (pdl) asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+    }
+};
 // For device functions called inside one kernel (the batch, the tiles).
 struct NoWait {
     __device__ __forceinline__ void operator()() const {}

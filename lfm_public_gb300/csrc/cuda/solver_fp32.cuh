@@ -492,14 +492,6 @@ __device__ __forceinline__ void set_state32(const Args<float>& a, const double* 
     if (a.cellGhosts && a.cellGhosts[c]) ghosts_of32<D>(a, c, qp, a.prim);
 }
 
-// Perturbation state q' = q - q_ref of cells [0, n) from a caller's absolute
-// state q ([nq][stride] doubles).
-template <int D>
-__device__ __forceinline__ void to_perturbation(const Args<float>& a, const double* q, int64_t stride, int c) {
-#pragma unroll
-    for (int v = 0; v < D + 2; ++v) a.q[(size_t)v * a.nt + c] = q[(size_t)v * stride + c] - a.qRef[v];
-}
-
 // Calls f(code, o, S, w) for every face entry of cell c in ascending face
 // order (code: the face, one's complement where c is N; o: the cell across; the
 // face's S and w): through the fixed-width tables (ELL), unrolled so that the

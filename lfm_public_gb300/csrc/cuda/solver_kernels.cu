@@ -579,6 +579,45 @@ __global__ void __launch_bounds__(256) k_res_sq(const double* res, int nc, doubl
 
 __global__ void k_set_flag(int* flag, int v) { *flag = v; }
 
+// Preparation for one residual of a caller's state q ([nq][stride], read only):
+// the stored rows, the primitives of every cell and the states and primitives of
+// the ghosts, whose viscous rows and gradients (read as zeros; cellGrad: the
+// cells' too, which no pass computes then) are cleared --
+// what a memset, a copy and a preparation pass did in three launches, each about
+// as long as the residual's own kernels on a small mesh.
+template <int D>
+__global__ void __launch_bounds__(128) k_prep_residual64(const __grid_constant__ Args<double> a, const double* q,
+                                                         int64_t stride, int vRows, int gradRows, int cellGrad) {
+    const int t = LFM_GLOBAL_ID();
+    PdlRelease{a.pdl}();
+    if (t >= a.nt) return;
+    constexpr int NQ = D + 2;
+    const size_t nt = (size_t)a.nt;
+    const int c = t < a.nc ? t : a.gCell[t - a.nc];
+    double qi[NQ], qv[NQ];
+#pragma unroll
+    for (int v = 0; v < NQ; ++v) qi[v] = q[(size_t)v * stride + c];
+    if (t < a.nc) {
+#pragma unroll
+        for (int v = 0; v < NQ; ++v) qv[v] = qi[v];
+    } else {
+        ghost_bc<double, D>(a, t - a.nc, qi, qv);
+        for (int r = 0; r < vRows; ++r) a.V[r * nt + t] = 0.0;
+    }
+    if (t >= a.nc || cellGrad)
+        for (int r = 0; r < gradRows; ++r) a.grad[r * nt + t] = 0.0;
+#pragma unroll
+    for (int v = 0; v < NQ; ++v) a.q[(size_t)v * nt + t] = qv[v];
+    prims64<D>(a, t, qv);
+}
+
+void launch_prep_residual64(const Args<double>& a, const double* q, int64_t stride, int vRows, int gradRows, int cellGrad,
+                            cudaStream_t st) {
+    const unsigned nb = (unsigned)((a.nt + 127) / 128);
+    if (a.D == 2) k_prep_residual64<2><<<nb, 128, 0, st>>>(a, q, stride, vRows, gradRows, cellGrad);
+    else k_prep_residual64<3><<<nb, 128, 0, st>>>(a, q, stride, vRows, gradRows, cellGrad);
+}
+
 double* kernel_address(const double* p) {
     cudaPointerAttributes at{};
     if (cudaPointerGetAttributes(&at, p) != cudaSuccess) {

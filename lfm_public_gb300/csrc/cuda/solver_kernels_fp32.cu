@@ -128,11 +128,30 @@ __global__ void __launch_bounds__(256) k_set_state32(const __grid_constant__ Arg
     if (c < a.nc) set_state32<D>(a, q, stride, c);
 }
 
+// Preparation for one residual of a caller's state (k_prep_residual64): the
+// primitives of every cell and ghost; q' itself is not kept, the fluxes read the
+// primitives alone.
 template <int D>
-__global__ void __launch_bounds__(256) k_to_perturbation(const __grid_constant__ Args<float> a, const double* q,
-                                                         int64_t stride) {
-    const int c = LFM_GLOBAL_ID();
-    if (c < a.nc) to_perturbation<D>(a, q, stride, c);
+__global__ void __launch_bounds__(128) k_prep_residual32(const __grid_constant__ Args<float> a, const double* q,
+                                                         int64_t stride, int vWords, int gradWords, int cellGrad) {
+    const int t = LFM_GLOBAL_ID();
+    PdlRelease{a.pdl}();
+    if (t >= a.nt) return;
+    constexpr int NQ = D + 2;
+    const int c = t < a.nc ? t : a.gCell[t - a.nc];
+    double qp[NQ];
+#pragma unroll
+    for (int v = 0; v < NQ; ++v) qp[v] = q[(size_t)v * stride + c] - a.qRef[v];
+    if (t >= a.nc || cellGrad)
+        for (int k = 0; k < gradWords; ++k) a.grad[(size_t)t * gradWords + k] = 0.0f;
+    if (t < a.nc) {
+        prims32<D>(a, t, qp, a.prim);
+        return;
+    }
+#pragma unroll
+    for (int v = 0; v < NQ; ++v) qp[v] += a.qRef[v];
+    ghost32<D>(a, t - a.nc, qp, a.prim);
+    for (int k = 0; k < vWords; ++k) a.V[(size_t)t * vWords + k] = 0.0f;
 }
 
 // ---------------------------------------------------------------------------
@@ -211,11 +230,12 @@ void launch_set_state32(const Args<float>& a, const double* q, int64_t stride, c
         k_set_state32<3><<<nblocks(a.nc, 256), 256, 0, st>>>(a, q, stride);
 }
 
-void launch_to_perturbation(const Args<float>& a, const double* q, int64_t stride, cudaStream_t st) {
+void launch_prep_residual32(const Args<float>& a, const double* q, int64_t stride, int vWords, int gradWords, int cellGrad,
+                            cudaStream_t st) {
     if (a.D == 2)
-        k_to_perturbation<2><<<nblocks(a.nc, 256), 256, 0, st>>>(a, q, stride);
+        k_prep_residual32<2><<<nblocks(a.nt, 128), 128, 0, st>>>(a, q, stride, vWords, gradWords, cellGrad);
     else
-        k_to_perturbation<3><<<nblocks(a.nc, 256), 256, 0, st>>>(a, q, stride);
+        k_prep_residual32<3><<<nblocks(a.nt, 128), 128, 0, st>>>(a, q, stride, vWords, gradWords, cellGrad);
 }
 
 }  // namespace dev

@@ -93,9 +93,13 @@ void launch_fluxupdate32(const Args<float>& a, const StageConfig& s, cudaStream_
 bool flux_staging_supported(int scheme, bool les);
 cudaError_t configure_flux_staging(int D, int scheme, int nf, FluxStaging& fs);
 void launch_flux32_staged(const Args<float>& a, const StageConfig& s, cudaStream_t st);
-// q' = q - q_ref for the cells of an FP32-bulk solver from an absolute state
-// [nq][stride] on the device.
-void launch_to_perturbation(const Args<float>& a, const double* q, int64_t stride, cudaStream_t st);
+// Preparation for one residual of the state q ([nq][stride] on the device):
+// primitives (FP64: the stored rows too) of the cells and ghosts, the ghosts' V
+// rows (vRows / vWords per cell) and gradients (cellGrad: the cells' too) cleared.
+void launch_prep_residual64(const Args<double>& a, const double* q, int64_t stride, int vRows, int gradRows, int cellGrad,
+                            cudaStream_t st);
+void launch_prep_residual32(const Args<float>& a, const double* q, int64_t stride, int vWords, int gradWords, int cellGrad,
+                            cudaStream_t st);
 // The address at which kernels read and write page-locked host memory p, or null
 // for other memory. A state in page-locked memory is read and written by the
 // kernels that convert it: the C2C link moves it at the copy engines' rate, and

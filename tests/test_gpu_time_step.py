@@ -1,4 +1,7 @@
-"""The time step in device memory and the one-launch reductions."""
+"""The time step in device memory, the one-launch reductions, and the residual's
+one-launch preparation."""
+import ctypes as C
+
 import numpy as np
 import pytest
 
@@ -54,3 +57,40 @@ def test_reductions_match_the_oracle(shape):
         assert abs(s.min_dt(0.5) / P.min_dt(ch, q, 0.5) - 1) <= 1e-13
         assert abs(s.cfl(1e-6) / P.cfl(ch, q, 1e-6) - 1) <= 1e-13
     s.close()
+
+
+@pytest.mark.parametrize("precision", [N.LFM_FP64, N.LFM_FP32_BULK])
+@pytest.mark.parametrize("shape", [(24, 11, 1), (16, 8, 5)])
+def test_residual_after_other_contents_of_the_scratch(shape, precision):
+    """M2AUSM without minmod reads zero gradients in every cell and ghost: the
+    scratch array still holds the previous call's. Also replayed from a graph."""
+    torch = pytest.importorskip("torch")
+    lib = N.load_library()
+    got = {}
+    stream = torch.cuda.Stream()
+    for minmod in (True, False, True, False):
+        case = _case(*shape, solver=2, minmod=minmod)
+        case.residuals = True   # the oracle records them then
+        ch = N.CaseHandle.from_case(case)
+        s = N.Solver(ch, precision=precision)
+        q = torch.from_numpy(ch.q0()).to("cuda")
+        res = torch.full_like(q, float("nan"))
+        torch.cuda.synchronize()
+        call = lambda: N.check(lib.lfm_solver_residual_noalloc(  # noqa: E731
+            s._h, C.c_void_p(q.data_ptr()), q.shape[1], C.c_void_p(res.data_ptr()), C.c_void_p(stream.cuda_stream)))
+        call()
+        stream.synchronize()
+        first = res.cpu().numpy()
+        _, expected = P.cell_residual(ch, ch.q0(), 1, case.delta_t)
+        scale = np.abs(expected).max(axis=1, keepdims=True)
+        assert np.max(np.abs(first - expected) / scale) <= (1e-11 if precision == N.LFM_FP64 else 1e-4)
+        assert np.array_equal(got.setdefault(minmod, first), first)
+        g = torch.cuda.CUDAGraph()
+        with torch.cuda.graph(g, stream=stream):
+            call()
+        res.fill_(float("nan"))
+        torch.cuda.synchronize()
+        g.replay()
+        torch.cuda.synchronize()
+        assert np.array_equal(res.cpu().numpy(), first)
+        s.close()
