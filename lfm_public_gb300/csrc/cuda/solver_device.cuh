@@ -216,9 +216,8 @@ __device__ __forceinline__ double face_sx(const Args<float>& a, int f) { return 
 // cell (FP64): the boundary condition of set_boundary_conditions
 // (src/cfd_v0.cpp:1009-1221).
 template <typename T, int D>
-__device__ __forceinline__ void ghost_bc(const Args<T>& a, int g, const double* qi, double* qv) {
+__device__ __forceinline__ void ghost_bc(const Args<T>& a, int g, int kind, const double* qi, double* qv) {
     constexpr int NQ = D + 2;
-    const int kind = a.gKind[g];
     if (kind == 1) {  // wall: mirror the momentum
         qv[0] = qi[0];
 #pragma unroll
@@ -266,6 +265,11 @@ __device__ __forceinline__ void ghost_bc(const Args<T>& a, int g, const double* 
     }
 }
 
+template <typename T, int D>
+__device__ __forceinline__ void ghost_bc(const Args<T>& a, int g, const double* qi, double* qv) {
+    ghost_bc<T, D>(a, g, a.gKind[g], qi, qv);
+}
+
 // Conservative state of cell, ghost or halo t in FP64 (FP64 path: q holds the
 // state itself). A ghost's state is computed from its interior cell and
 // stored into q; a halo's was copied in from its partition.
@@ -308,37 +312,71 @@ __device__ __forceinline__ void prims64(const Args<double>& a, int t, const doub
     if (a.primC) a.prim[(size_t)(D + 2) * nt + t] = sqrt(a.gamma * Rpsi);   // read by M2AUSM only
 }
 
-// Calls f(j) for every boundary ghost j of cell c (cells with boundary faces
-// only). A ghost is only ever across a face of its own cell, so the list's
-// neighbour column alone names it; the entries of an ordinary cell are loaded
-// together, where following the face list to the face's N side costs two
-// dependent loads per face.
-template <typename T, int D, class F>
-__device__ __forceinline__ void for_ghosts(const Args<T>& a, int c, F f) {
+// The boundary ghosts of a cell with boundary faces. A ghost is only ever across
+// a face of its own cell, so the neighbour column alone names it; the entries of
+// an ordinary cell are loaded together, where following the face list to the
+// face's N side costs two dependent loads per face. The first ghost (most have
+// one) and its boundary condition are loaded ahead of the cell's new state, so
+// that the update's last serial part is arithmetic alone.
+struct CellGhosts {
+    int j = -1, kind = 0, count = 0;   // the first ghost, its kind, their number
+};
+
+template <typename T, int D>
+__device__ __forceinline__ int entry_cell(const Args<T>& a, int c, int k) {   // the cell across entry k, -1 past the last
+    if constexpr (sizeof(T) == sizeof(float)) {
+        if (a.cfEllN) return k < kEllWidth<D> ? a.cfEllN[(size_t)c * kEllWidth<D> + k] : -1;
+    }
+    return a.cfOff[c] + k < a.cfOff[c + 1] ? a.cfNbr[a.cfOff[c] + k] : -1;
+}
+
+template <typename T, int D>
+__device__ __forceinline__ CellGhosts cell_ghosts(const Args<T>& a, int c) {
     constexpr int W = kEllWidth<D>;
-    const int e0 = a.cfOff[c], n = a.cfOff[c + 1] - e0;
+    CellGhosts g;
     int nb[W];
 #pragma unroll
-    for (int k = 0; k < W; ++k) nb[k] = k < n ? a.cfNbr[e0 + k] : -1;
-#pragma unroll 1
-    for (int k = 0; k < n; ++k) {
-        int j = nb[0];
+    for (int k = 0; k < W; ++k) nb[k] = entry_cell<T, D>(a, c, k);
 #pragma unroll
-        for (int m = 1; m < W; ++m) j = k == m ? nb[m] : j;
-        if (k >= W) j = a.cfNbr[e0 + k];
-        if (j >= a.nc && j < a.nc + a.ng) f(j);
+    for (int k = W - 1; k >= 0; --k)
+        if (nb[k] >= a.nc && nb[k] < a.nc + a.ng) {
+            g.j = nb[k];
+            ++g.count;
+        }
+    if (nb[W - 1] >= 0)   // a cell of more faces
+        for (int k = W, j; (j = entry_cell<T, D>(a, c, k)) >= 0; ++k)
+            if (j >= a.nc && j < a.nc + a.ng) {
+                if (g.count++ == 0) g.j = j;
+            }
+    if (g.count) g.kind = a.gKind[g.j - a.nc];
+    return g;
+}
+
+// f(j, kind) for each of them.
+template <typename T, int D, class F>
+__device__ __forceinline__ void for_ghosts(const Args<T>& a, int c, const CellGhosts& g, F f) {
+    int j = g.j, kind = g.kind, left = g.count;
+#pragma unroll 1
+    for (int k = 0; left > 0; ++k) {   // the first, then the others in entry order
+        if (k > 0) {
+            j = entry_cell<T, D>(a, c, k - 1);
+            if (j < a.nc || j >= a.nc + a.ng || j == g.j) continue;
+            kind = a.gKind[j - a.nc];
+        }
+        f(j, kind);
+        --left;
     }
 }
 
 // FP64 path: the states and primitives of the boundary ghosts of cell c from
 // its conservative state qc (those k_prep computes for the next stage).
 template <int D>
-__device__ __forceinline__ void ghosts_of64(const Args<double>& a, int c, const double* qc) {
+__device__ __forceinline__ void ghosts_of64(const Args<double>& a, int c, const CellGhosts& g, const double* qc) {
     constexpr int NQ = D + 2;
     const size_t nt = (size_t)a.nt;
-    for_ghosts<double, D>(a, c, [&](int j) {
+    for_ghosts<double, D>(a, c, g, [&](int j, int kind) {
         double qv[NQ];
-        ghost_bc<double, D>(a, j - a.nc, qc, qv);
+        ghost_bc<double, D>(a, j - a.nc, kind, qc, qv);
 #pragma unroll
         for (int v = 0; v < NQ; ++v) a.q[(size_t)v * nt + j] = qv[v];
         prims64<D>(a, j, qv);
@@ -364,6 +402,7 @@ __device__ __forceinline__ void update_cell(const Args<T>& a, int c, double Ak, 
     for (int k = 0; k < W; ++k) code[k] = e0 + k < e1 ? a.cfList[e0 + k] : kEllPad;
     const double vi = a.volInv[c], sg = a.sponge[c];
     const bool ghosts = PRIM && a.cellGhosts && a.cellGhosts[c];
+    CellGhosts gh;
     sync();
     double qv[NQ], dq[NQ];
 #pragma unroll
@@ -390,6 +429,7 @@ __device__ __forceinline__ void update_cell(const Args<T>& a, int c, double Ak, 
                 fl[k][v] = code[k] >= 0 ? x : neg_bits(x);
             }
         }
+        if (ghosts) gh = cell_ghosts<T, D>(a, c);   // while the rhs are in flight
         // the first face starts the sum (a cell has at least one face)
 #pragma unroll
         for (int k = 0; k < W; ++k) {
@@ -398,6 +438,7 @@ __device__ __forceinline__ void update_cell(const Args<T>& a, int c, double Ak, 
             for (int v = 0; v < NQ; ++v) sum[v] = k ? sum[v] + fl[k][v] : fl[0][v];
         }
     } else {
+        if (ghosts) gh = cell_ghosts<T, D>(a, c);
         for (int e = e0; e < e1; ++e) {
             const int code = a.cfList[e];
             if (code >= 0) {
@@ -433,7 +474,7 @@ __device__ __forceinline__ void update_cell(const Args<T>& a, int c, double Ak, 
     if (!finite) atomicOr(a.flag, 1);
     if constexpr (PRIM) {
         prims64<D>(a, c, qn);
-        if (ghosts) ghosts_of64<D>(a, c, qn);
+        if (ghosts) ghosts_of64<D>(a, c, gh, qn);
     }
 }
 

@@ -282,11 +282,11 @@ __device__ __forceinline__ void prims32(const Args<float>& a, int t, const doubl
 // theirs is FP64.
 // ---------------------------------------------------------------------------
 template <int D>
-__device__ __forceinline__ void ghost32(const Args<float>& a, int g, const double* qi, float* dst) {
+__device__ __forceinline__ void ghost32(const Args<float>& a, int g, int kind, const double* qi, float* dst) {
     constexpr int NQ = D + 2;
     const int t = a.nc + g;
     double qv[NQ];
-    ghost_bc<float, D>(a, g, qi, qv);
+    ghost_bc<float, D>(a, g, kind, qi, qv);
     const double rinv = rcp64(qv[0]);
     double ke = 0.0;
     Prim32<D> p32;
@@ -323,7 +323,7 @@ __device__ __forceinline__ void prep32(const Args<float>& a, int t) {
     double qi[NQ];
 #pragma unroll
     for (int v = 0; v < NQ; ++v) qi[v] = a.q[(size_t)v * nt + in] + a.qRef[v];
-    ghost32<D>(a, g, qi, a.prim);
+    ghost32<D>(a, g, a.gKind[g], qi, a.prim);
 }
 
 // ---------------------------------------------------------------------------
@@ -345,25 +345,13 @@ __device__ __forceinline__ void prep32(const Args<float>& a, int t) {
 // ghosts_of32: the FP64 states and FP32 primitives of the boundary ghosts of
 // cell c from its perturbation state qp (those prep32 computes).
 template <int D>
-__device__ __forceinline__ void ghosts_of32(const Args<float>& a, int c, const double* qp, float* dst) {
+__device__ __forceinline__ void ghosts_of32(const Args<float>& a, int c, const CellGhosts& g, const double* qp,
+                                            float* dst) {
     constexpr int NQ = D + 2;
     double qa[NQ];
 #pragma unroll
     for (int v = 0; v < NQ; ++v) qa[v] = qp[v] + a.qRef[v];
-    if (a.cfEllN) {
-        constexpr int W = kEllWidth<D>;
-        int nb[W];
-        load_ell<D>(a.cfEllN, c, nb);
-#pragma unroll 1
-        for (int k = 0; k < W; ++k) {
-            int j = nb[0];
-#pragma unroll
-            for (int m = 1; m < W; ++m) j = k == m ? nb[m] : j;
-            if (j >= a.nc && j < a.nc + a.ng) ghost32<D>(a, j - a.nc, qa, dst);
-        }
-    } else {
-        for_ghosts<float, D>(a, c, [&](int j) { ghost32<D>(a, j - a.nc, qa, dst); });
-    }
+    for_ghosts<float, D>(a, c, g, [&](int j, int kind) { ghost32<D>(a, j - a.nc, kind, qa, dst); });
 }
 
 // gather32: the face rhs sum of cell c (ascending face order). The face's sign
@@ -387,13 +375,14 @@ __device__ __forceinline__ void gather32(const Args<float>& a, int c, float* sum
 // the cell is loaded at once, then every face's rhs, so the gather costs two
 // memory round trips instead of one per face; the sum runs in the same
 // (ascending face) order, so it has gather32's bits.
-template <int D>
-__device__ __forceinline__ void gather32_ell(const Args<float>& a, const int* code, float* sum) {
+template <int D, class F>
+__device__ __forceinline__ void gather32_ell(const Args<float>& a, const int* code, float* sum, F meanwhile) {
     constexpr int NQ = D + 2, W = kEllWidth<D>;
     float x[W][NQ];
 #pragma unroll
     for (int k = 0; k < W; ++k)
         if (code[k] != kEllPad) load_flux<D>(a, code[k] >= 0 ? code[k] : ~code[k], x[k]);
+    meanwhile();   // while they are in flight
 #pragma unroll
     for (int v = 0; v < NQ; ++v) sum[v] = 0.0f;
 #pragma unroll
@@ -412,6 +401,7 @@ struct CellIn32 {
     float dq[D + 2];
     float vi, sg;       // 1/V, sponge sigma
     int ghosts;         // it has boundary faces (GH)
+    CellGhosts gh;
 };
 
 template <int D, bool GH, class Sync = NoWait>
@@ -456,7 +446,7 @@ __device__ __forceinline__ void apply32(const Args<float>& a, int c, const float
     }
     if (!finite) atomicOr(a.flag, 1);
     prims32<D>(a, c, qn, a.primW);
-    if (GH && in.ghosts) ghosts_of32<D>(a, c, qn, a.primW);
+    if (GH && in.ghosts) ghosts_of32<D>(a, c, in.gh, qn, a.primW);
 }
 
 // ELL: the fixed-width table, the face list, or (the batch, one copy of whose
@@ -471,8 +461,15 @@ __device__ __forceinline__ void update32(const Args<float>& a, int c, double Ak,
     CellIn32<D> in;
     load_cell32<D, GH>(a, c, first, in, sync);
     float sum[D + 2];
-    if (ELL == kEntriesEll || (ELL == kEntriesEither && a.cfEll)) gather32_ell<D>(a, code, sum);
-    else gather32<D>(a, c, sum);
+    auto ghosts = [&] {
+        if (GH && in.ghosts) in.gh = cell_ghosts<float, D>(a, c);
+    };
+    if (ELL == kEntriesEll || (ELL == kEntriesEither && a.cfEll)) {
+        gather32_ell<D>(a, code, sum, ghosts);
+    } else {
+        ghosts();
+        gather32<D>(a, c, sum);
+    }
     apply32<D, GH>(a, c, sum, in, Ak, Bk, dt32, first, res);
 }
 
@@ -489,7 +486,7 @@ __device__ __forceinline__ void set_state32(const Args<float>& a, const double* 
         a.q[(size_t)v * a.nt + c] = qp[v];
     }
     prims32<D>(a, c, qp, a.prim);
-    if (a.cellGhosts && a.cellGhosts[c]) ghosts_of32<D>(a, c, qp, a.prim);
+    if (a.cellGhosts && a.cellGhosts[c]) ghosts_of32<D>(a, c, cell_ghosts<float, D>(a, c), qp, a.prim);
 }
 
 // Calls f(code, o, S, w) for every face entry of cell c in ascending face
@@ -946,6 +943,7 @@ __device__ __forceinline__ void fluxupdate32(const Args<float>& a, int c, double
         load_cell32<D, GH>(a, c, first, in, sync);
         load_prim<D>(a, c, self);
         if constexpr (needV) load_vis<D, false>(a, c, Vc);
+        if (GH && in.ghosts) in.gh = cell_ghosts<float, D>(a, c);
     };
     float sum[NQ];
 #pragma unroll

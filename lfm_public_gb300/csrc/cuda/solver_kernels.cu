@@ -49,7 +49,7 @@ __global__ void __launch_bounds__(256) k_set_state64(const __grid_constant__ Arg
         a.q[(size_t)v * a.nt + c] = qv[v];
     }
     prims64<D>(a, c, qv);
-    if (a.cellGhosts && a.cellGhosts[c]) ghosts_of64<D>(a, c, qv);
+    if (a.cellGhosts && a.cellGhosts[c]) ghosts_of64<D>(a, c, cell_ghosts<double, D>(a, c), qv);
 }
 
 void launch_set_state64(const Args<double>& a, const double* q, int64_t stride, cudaStream_t st) {
@@ -284,11 +284,13 @@ __global__ void __launch_bounds__(kFaceThreads<D>) k_flux(Args<T> a) {
             u2 += m[k] * m[k];
         }
         const T phi = mS * rinv;                          // u_f . S
+        const T gh2 = T(2) * (T)a.gh;
         const T p = rho * Rpsi;
         rhs[0] = -mS;
 #pragma unroll
         for (int k = 0; k < D; ++k) rhs[k + 1] = -(m[k] * phi + p * S[k]);
-        rhs[D + 1] = -mS * ((T)a.gh * Rpsi + T(0.5) * u2 * (rinv * rinv));
+        // mS (gh Rpsi + |u|^2 / 2) with mS Rpsi = phi p and mS |u|^2 = phi |m|^2 / rho
+        rhs[D + 1] = -(T(0.5) * phi) * (gh2 * p + u2 * rinv);
     } else {
         // Pirozzoli kinetic-energy-preserving mid-point flux (src/cfd_v0.cpp:1966-2023)
         // on the sums of the two sides: rho u.S = (m_P + m_N).S / 2 and
@@ -389,7 +391,7 @@ __global__ void __launch_bounds__(kFaceThreads<D>) k_flux(Args<T> a) {
     // 459 us a step, of the 97 x 61 x 23 M2 wake from 484 to 390 (GB300).
     const T mu = (T)a.mu;
     if (mu != T(0)) {
-        T g[D][D], eV;
+        T g[D][D];
         if (!ghost) {
             T ei = T(0), ej = T(0);
 #pragma unroll
@@ -403,12 +405,12 @@ __global__ void __launch_bounds__(kFaceThreads<D>) k_flux(Args<T> a) {
                 ei += a.V[(D * D + D + x) * nt + i] * S[x];
                 ej += a.V[(D * D + D + x) * nt + j] * S[x];
             }
-            eV = interp2(w, wN, ei, ej);
+            rhs[D + 1] += wN * ej;
+            rhs[D + 1] += w * ei;
         } else {
             // explicit two-point gradients on physical boundaries
             const T dinv = a.dinv[f];
-            T dn[D], tau[D][D], Uf[D];
-            eV = T(0);
+            T dn[D], tau[D][D], Uf[D], eV = T(0);
 #pragma unroll
             for (int k = 0; k < D; ++k) {
                 dn[k] = a.dnorm[k * nf + f] * dinv;
@@ -423,6 +425,7 @@ __global__ void __launch_bounds__(kFaceThreads<D>) k_flux(Args<T> a) {
             stress<T, D>(g, mu, tau);
 #pragma unroll
             for (int x = 0; x < D; ++x) eV += dotv<T, D>(Uf, tau[x]) * S[x];
+            rhs[D + 1] += eV;
         }
         const T ml = a.ml[f];
 #pragma unroll
@@ -441,7 +444,6 @@ __global__ void __launch_bounds__(kFaceThreads<D>) k_flux(Args<T> a) {
             r += off * a.mT[x * nf + f];
             rhs[x + 1] = r + ml * (aU[x] - cU[x]);
         }
-        rhs[D + 1] += eV;
         rhs[D + 1] += a.kl[f] * dR;
         // Smagorinsky LES: the face tauMC also interpolates the cells' SGS
         // stress (boundary faces keep the laminar two-point one, as in the
