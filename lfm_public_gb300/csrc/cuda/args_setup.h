@@ -164,7 +164,9 @@ void setConstants(dev::Args<T>& a, const lfm_solver_desc* d) {
     a.RpsiRef = RpsiRef;
     a.gh = gh;
     a.gm1Inv = 1.0 / a.gm1;
+    a.RT = d->Rgas * d->TInf;
     a.RTInv = a.Rinv / d->TInf;
+    a.pInfInv = 1.0 / d->pInf;
     a.keInf = 0.5 * u2;
     a.mu23 = d->mu * 2.0 / 3.0;
     a.ref.rho = (float)d->rhoInf;

@@ -212,83 +212,95 @@ __device__ __forceinline__ T p5neg(T M, T alpha) {
 __device__ __forceinline__ double face_sx(const Args<double>& a, int f) { return a.S[f]; }
 __device__ __forceinline__ double face_sx(const Args<float>& a, int f) { return (double)a.fG0[f].x; }
 
-// Ghost state qv of ghost g from the conservative state qi of its interior
-// cell (FP64): the boundary condition of set_boundary_conditions
-// (src/cfd_v0.cpp:1009-1221).
+// Boundary ghosts (set_boundary_conditions, src/cfd_v0.cpp:1009-1221), state
+// and primitives from those of the interior cell (FP64). The reference's
+// expressions (TInt = pInt / (R rhoInt), rhoExt = rhoInt TInt / TInf, rhoExt EExt
+// with EExt = p / (rhoExt (gamma - 1)) + |u|^2 / 2, then 1/rhoExt, uExt and
+// p/rhoExt) with the divisions that cancel left out and those by constants
+// turned into host-side factors.
+//
+// What counts is the depth of the chain: it is the last serial part of a
+// boundary cell's update, FP64 results take about a hundred cycles each to come
+// back, and the update kernel of a small case waits for the cell at a corner,
+// which has two ghosts. What depends on the interior cell is therefore formed
+// once for all its ghosts (ghost_in), and a ghost takes at most three operations
+// more: its primitives follow from the interior's, not from its own state.
+// Measured on GB300 against a state and primitives per ghost, us a step: 48 x 48
+// FP64 vortex 45.0 -> 40.9, 256 x 256 vortex FP64 106.4 -> 100.3 and FP32-bulk
+// 43.0 -> 36.8 (16 of which the ghosts took, in a copy without them).
+template <int D>
+struct GhostIn {
+    double rho, rinv, m[D], u[D], E;
+    double p, pinv, R, ke;   // pressure, its reciprocal, R psi, |u|^2 / 2
+};
+template <int D>
+struct GhostState {
+    double q[D + 2], rinv, u[D], R;
+};
+
 template <typename T, int D>
-__device__ __forceinline__ void ghost_bc(const Args<T>& a, int g, int kind, const double* qi, double* qv) {
-    constexpr int NQ = D + 2;
-    if (kind == 1) {  // wall: mirror the momentum
-        qv[0] = qi[0];
+__device__ __forceinline__ GhostIn<D> ghost_in(const Args<T>& a, const double* qi) {
+    GhostIn<D> g;
+    g.rho = qi[0];
+    g.E = qi[D + 1];
+    g.rinv = rcp64(qi[0]);
+    double s = 0.0;   // rho |u|^2
 #pragma unroll
-        for (int k = 0; k < D; ++k) qv[k + 1] = -qi[k + 1];
-        qv[D + 1] = qi[D + 1];
-    } else if (kind >= 2 && kind <= 4) {
-        bool inlet = (kind == 2);
-        if (kind == 4) inlet = face_sx(a, a.gFace[g]) <= 0.0;  // free stream along +x enters
-        // The reference's expressions (TInt = pInt / (R rhoInt),
-        // rhoExt = rhoInt TInt / TInf, rhoExt EExt with EExt = p / (rhoExt
-        // (gamma - 1)) + |u|^2 / 2) with the divisions that cancel left out
-        // and those by constants turned into host-side factors: this serial
-        // chain ends a boundary cell's update, and the update kernel of a small
-        // case waits for it. With the ghosts named by for_ghosts, measured on
-        // GB300: a 48 x 48 FP64 vortex 73.4 -> 62.6 us a step, the 256 x 256
-        // FP32-bulk vortex 60.8 -> 52.4, a batch of eight 2D cases of 14k-56k
-        // cells 202 -> 163.
-        const double rhoInt = qi[0];
-        const double rinv = rcp64(rhoInt);
-        double Uint[D], um2 = 0.0;
-#pragma unroll
-        for (int k = 0; k < D; ++k) {
-            Uint[k] = qi[k + 1] * rinv;
-            um2 += Uint[k] * Uint[k];
-        }
-        const double pInt = (qi[D + 1] - 0.5 * um2 * rhoInt) * a.gm1;
-        if (inlet) {
-            const double rhoExt = pInt * a.RTInv;
-            qv[0] = rhoExt;
-#pragma unroll
-            for (int k = 0; k < D; ++k) qv[k + 1] = rhoExt * a.UInf[k];
-            qv[D + 1] = pInt * a.gm1Inv + rhoExt * a.keInf;
-        } else {
-            const double rhoExt = rhoInt * a.pInf * rcp64(pInt);
-            qv[0] = rhoExt;
-#pragma unroll
-            for (int k = 0; k < D; ++k) qv[k + 1] = rhoExt * Uint[k];
-            qv[D + 1] = a.pInf * a.gm1Inv + 0.5 * um2 * rhoExt;
-        }
-    } else {
-        // Patches without a boundary condition keep a zero ghost state, as
-        // in the reference (src/cfd_v0.cpp:406-416).
-#pragma unroll
-        for (int v = 0; v < NQ; ++v) qv[v] = 0.0;
+    for (int k = 0; k < D; ++k) {
+        g.m[k] = qi[k + 1];
+        g.u[k] = qi[k + 1] * g.rinv;
+        s = k ? fma(g.m[k], g.u[k], s) : g.m[0] * g.u[0];
     }
+    const double e = fma(-0.5, s, g.E);
+    g.p = e * a.gm1;
+    g.pinv = rcp64(g.p);
+    g.R = e * (a.gm1 * g.rinv);
+    g.ke = s * (0.5 * g.rinv);
+    return g;
 }
 
+// One sequence for the three kinds, operands selected by kind (on the integer
+// pipe): the boundary cells of a warp alternate between inlet and outlet on a
+// row-ordered mesh, and branches would run one after another. A wall mirrors the
+// momentum, an inlet takes pInt, TInf, UInf, an outlet pInf, TInt, uInt.
 template <typename T, int D>
-__device__ __forceinline__ void ghost_bc(const Args<T>& a, int g, const double* qi, double* qv) {
-    ghost_bc<T, D>(a, g, a.gKind[g], qi, qv);
-}
-
-// Conservative state of cell, ghost or halo t in FP64 (FP64 path: q holds the
-// state itself). A ghost's state is computed from its interior cell and
-// stored into q; a halo's was copied in from its partition.
-template <typename T, int D>
-__device__ __forceinline__ void stage_state(const Args<T>& a, int t, double* qv) {
-    constexpr int NQ = D + 2;
-    if (t < a.nc || t >= a.nc + a.ng) {
+__device__ __forceinline__ void ghost_state(const Args<T>& a, int g, int kind, const GhostIn<D>& in, GhostState<D>& o) {
+    if (kind < 1 || kind > 4) {
+        // Patches without a boundary condition keep a zero ghost state, as
+        // in the reference (src/cfd_v0.cpp:406-416): its primitives are not finite.
 #pragma unroll
-        for (int v = 0; v < NQ; ++v) qv[v] = a.q[(size_t)v * a.nt + t];
+        for (int v = 0; v < D + 2; ++v) o.q[v] = 0.0;
+        o.rinv = rcp64(o.q[0]);
+#pragma unroll
+        for (int k = 0; k < D; ++k) o.u[k] = o.q[k + 1] * o.rinv;
+        o.R = o.q[D + 1] * o.rinv;
         return;
     }
-    const int g = t - a.nc;
-    const int in = a.gCell[g];
-    double qi[NQ];
+    const bool wall = kind == 1;
+    bool inlet = kind == 2;
+    if (kind == 4) inlet = face_sx(a, a.gFace[g]) <= 0.0;  // free stream along +x enters
+    // rho: p / (R TInf) | rho pInf / p | rho;  1/rho: R TInf / p | p / (rho pInf) | 1/rho
+    o.q[0] = (wall ? in.rho : inlet ? in.p : in.rho * a.pInf) * (wall ? 1.0 : inlet ? a.RTInv : in.pinv);
+    o.rinv = (wall ? in.rinv : inlet ? a.RT : in.rinv * a.pInfInv) * (wall ? 1.0 : inlet ? in.pinv : in.p);
+    const double Rout = a.pInf * o.rinv;
+    o.R = wall ? in.R : inlet ? a.RT : Rout;
+    const double e = fma(inlet ? a.keInf : in.ke, o.q[0], (inlet ? in.p : a.pInf) * a.gm1Inv);
+    o.q[D + 1] = wall ? in.E : e;
 #pragma unroll
-    for (int v = 0; v < NQ; ++v) qi[v] = a.q[(size_t)v * a.nt + in];
-    ghost_bc<T, D>(a, g, qi, qv);
+    for (int k = 0; k < D; ++k) {
+        o.u[k] = wall ? neg_bits(in.u[k]) : inlet ? a.UInf[k] : in.u[k];
+        const double m = o.q[0] * o.u[k];
+        o.q[k + 1] = wall ? neg_bits(in.m[k]) : m;
+    }
+}
+
+// The state alone, of ghost g from its interior cell's state qi.
+template <typename T, int D>
+__device__ __forceinline__ void ghost_bc(const Args<T>& a, int g, const double* qi, double* qv) {
+    GhostState<D> o;
+    ghost_state<T, D>(a, g, a.gKind[g], ghost_in<T, D>(a, qi), o);
 #pragma unroll
-    for (int v = 0; v < NQ; ++v) a.q[(size_t)v * a.nt + t] = qv[v];
+    for (int v = 0; v < D + 2; ++v) qv[v] = o.q[v];
 }
 
 // FP64 path: the primitives every face reads (1/rho, u, R psi = p/rho, c) of
@@ -315,11 +327,12 @@ __device__ __forceinline__ void prims64(const Args<double>& a, int t, const doub
 // The boundary ghosts of a cell with boundary faces. A ghost is only ever across
 // a face of its own cell, so the neighbour column alone names it; the entries of
 // an ordinary cell are loaded together, where following the face list to the
-// face's N side costs two dependent loads per face. The first ghost (most have
-// one) and its boundary condition are loaded ahead of the cell's new state, so
+// face's N side costs two dependent loads per face. The first two ghosts (a corner
+// has two) and their kinds are loaded ahead of the cell's new state, so
 // that the update's last serial part is arithmetic alone.
 struct CellGhosts {
-    int j = -1, kind = 0, count = 0;   // the first ghost, its kind, their number
+    int j[2] = {-1, -1}, kind[2] = {0, 0};   // the first two ghosts and their kinds
+    int count = 0;
 };
 
 template <typename T, int D>
@@ -337,30 +350,33 @@ __device__ __forceinline__ CellGhosts cell_ghosts(const Args<T>& a, int c) {
     int nb[W];
 #pragma unroll
     for (int k = 0; k < W; ++k) nb[k] = entry_cell<T, D>(a, c, k);
+    auto found = [&](int j) {
+        if (j < a.nc || j >= a.nc + a.ng) return;
+        if (g.count == 0) g.j[0] = j;
+        if (g.count == 1) g.j[1] = j;
+        ++g.count;
+    };
 #pragma unroll
-    for (int k = W - 1; k >= 0; --k)
-        if (nb[k] >= a.nc && nb[k] < a.nc + a.ng) {
-            g.j = nb[k];
-            ++g.count;
-        }
+    for (int k = 0; k < W; ++k) found(nb[k]);
     if (nb[W - 1] >= 0)   // a cell of more faces
-        for (int k = W, j; (j = entry_cell<T, D>(a, c, k)) >= 0; ++k)
-            if (j >= a.nc && j < a.nc + a.ng) {
-                if (g.count++ == 0) g.j = j;
-            }
-    if (g.count) g.kind = a.gKind[g.j - a.nc];
+        for (int k = W, j; (j = entry_cell<T, D>(a, c, k)) >= 0; ++k) found(j);
+#pragma unroll
+    for (int k = 0; k < 2; ++k)
+        if (g.count > k) g.kind[k] = a.gKind[g.j[k] - a.nc];
     return g;
 }
 
-// f(j, kind) for each of them.
+// f(j, kind) for each of them: the first two, then (a cell with more boundary
+// faces) the others in entry order.
 template <typename T, int D, class F>
 __device__ __forceinline__ void for_ghosts(const Args<T>& a, int c, const CellGhosts& g, F f) {
-    int j = g.j, kind = g.kind, left = g.count;
+    int left = g.count;
 #pragma unroll 1
-    for (int k = 0; left > 0; ++k) {   // the first, then the others in entry order
-        if (k > 0) {
-            j = entry_cell<T, D>(a, c, k - 1);
-            if (j < a.nc || j >= a.nc + a.ng || j == g.j) continue;
+    for (int k = 0; left > 0; ++k) {
+        int j = k == 0 ? g.j[0] : g.j[1], kind = k == 0 ? g.kind[0] : g.kind[1];
+        if (k >= 2) {
+            j = entry_cell<T, D>(a, c, k - 2);
+            if (j < a.nc || j >= a.nc + a.ng || j == g.j[0] || j == g.j[1]) continue;
             kind = a.gKind[j - a.nc];
         }
         f(j, kind);
@@ -370,17 +386,25 @@ __device__ __forceinline__ void for_ghosts(const Args<T>& a, int c, const CellGh
 
 // FP64 path: the states and primitives of the boundary ghosts of cell c from
 // its conservative state qc (those k_prep computes for the next stage).
+// FP64 path: state and primitives of ghost g into the stored arrays.
+template <int D>
+__device__ __forceinline__ void ghost64(const Args<double>& a, int g, int kind, const GhostIn<D>& in) {
+    const size_t nt = (size_t)a.nt, t = (size_t)(a.nc + g);
+    GhostState<D> o;
+    ghost_state<double, D>(a, g, kind, in, o);
+#pragma unroll
+    for (int v = 0; v < D + 2; ++v) a.q[v * nt + t] = o.q[v];
+    a.prim[t] = o.rinv;
+#pragma unroll
+    for (int k = 0; k < D; ++k) a.prim[(1 + k) * nt + t] = o.u[k];
+    a.prim[(D + 1) * nt + t] = o.R;
+    if (a.primC) a.prim[(D + 2) * nt + t] = sqrt(a.gamma * o.R);
+}
+
 template <int D>
 __device__ __forceinline__ void ghosts_of64(const Args<double>& a, int c, const CellGhosts& g, const double* qc) {
-    constexpr int NQ = D + 2;
-    const size_t nt = (size_t)a.nt;
-    for_ghosts<double, D>(a, c, g, [&](int j, int kind) {
-        double qv[NQ];
-        ghost_bc<double, D>(a, j - a.nc, kind, qc, qv);
-#pragma unroll
-        for (int v = 0; v < NQ; ++v) a.q[(size_t)v * nt + j] = qv[v];
-        prims64<D>(a, j, qv);
-    });
+    const GhostIn<D> in = ghost_in<double, D>(a, qc);
+    for_ghosts<double, D>(a, c, g, [&](int j, int kind) { ghost64<D>(a, j - a.nc, kind, in); });
 }
 
 // FP64 path: gather of the face rhs of cell c, sponge source and low-storage

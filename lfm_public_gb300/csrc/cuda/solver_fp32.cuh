@@ -282,23 +282,18 @@ __device__ __forceinline__ void prims32(const Args<float>& a, int t, const doubl
 // theirs is FP64.
 // ---------------------------------------------------------------------------
 template <int D>
-__device__ __forceinline__ void ghost32(const Args<float>& a, int g, int kind, const double* qi, float* dst) {
-    constexpr int NQ = D + 2;
+__device__ __forceinline__ void ghost32(const Args<float>& a, int g, int kind, const GhostIn<D>& in, float* dst) {
     const int t = a.nc + g;
-    double qv[NQ];
-    ghost_bc<float, D>(a, g, kind, qi, qv);
-    const double rinv = rcp64(qv[0]);
-    double ke = 0.0;
+    GhostState<D> o;
+    ghost_state<float, D>(a, g, kind, in, o);
     Prim32<D> p32;
-    p32.r = (float)(qv[0] - a.qRef[0]);
+    p32.r = (float)(o.q[0] - a.qRef[0]);
 #pragma unroll
     for (int k = 0; k < D; ++k) {
-        p32.m[k] = (float)(qv[k + 1] - a.qRef[k + 1]);
-        p32.u[k] = (float)(qv[k + 1] * rinv - a.UInf[k]);
-        ke += qv[k + 1] * qv[k + 1];
+        p32.m[k] = (float)(o.q[k + 1] - a.qRef[k + 1]);
+        p32.u[k] = (float)(o.u[k] - a.UInf[k]);
     }
-    const double p = a.gm1 * (qv[D + 1] - 0.5 * ke * rinv);
-    p32.R = (float)(p * rinv - a.RpsiRef);
+    p32.R = (float)(o.R - a.RpsiRef);
     store_prim<D>(a, dst, t, p32);
     if (a.primC) dst[prim_c<D>((size_t)a.nt) + t] = sqrtf(a.ref.gamma * (a.ref.Rpsi + p32.R));
 }
@@ -323,7 +318,7 @@ __device__ __forceinline__ void prep32(const Args<float>& a, int t) {
     double qi[NQ];
 #pragma unroll
     for (int v = 0; v < NQ; ++v) qi[v] = a.q[(size_t)v * nt + in] + a.qRef[v];
-    ghost32<D>(a, g, a.gKind[g], qi, a.prim);
+    ghost32<D>(a, g, a.gKind[g], ghost_in<float, D>(a, qi), a.prim);
 }
 
 // ---------------------------------------------------------------------------
@@ -351,7 +346,8 @@ __device__ __forceinline__ void ghosts_of32(const Args<float>& a, int c, const C
     double qa[NQ];
 #pragma unroll
     for (int v = 0; v < NQ; ++v) qa[v] = qp[v] + a.qRef[v];
-    for_ghosts<float, D>(a, c, g, [&](int j, int kind) { ghost32<D>(a, j - a.nc, kind, qa, dst); });
+    const GhostIn<D> in = ghost_in<float, D>(a, qa);
+    for_ghosts<float, D>(a, c, g, [&](int j, int kind) { ghost32<D>(a, j - a.nc, kind, in, dst); });
 }
 
 // gather32: the face rhs sum of cell c (ascending face order). The face's sign

@@ -27,9 +27,13 @@ __global__ void __launch_bounds__(256) k_prep(Args<T> a, int first) {
     PdlWait{a.pdl}();
     if (t >= a.nt) return;
     constexpr int NQ = D + 2;
+    const bool ghost = t >= a.nc && t < a.nc + a.ng;
+    const int c = ghost ? a.gCell[t - a.nc] : t;   // a halo's state was copied in from its partition
     double qv[NQ];
-    stage_state<T, D>(a, t, qv);
-    prims64<D>(a, t, qv);
+#pragma unroll
+    for (int v = 0; v < NQ; ++v) qv[v] = a.q[(size_t)v * a.nt + c];
+    if (ghost) ghost64<D>(a, t - a.nc, a.gKind[t - a.nc], ghost_in<T, D>(a, qv));
+    else prims64<D>(a, t, qv);
 }
 
 // A new state: the rows of the stored state from the caller's q ([nq][stride];
@@ -596,18 +600,16 @@ __global__ void __launch_bounds__(128) k_prep_residual64(const __grid_constant__
     constexpr int NQ = D + 2;
     const size_t nt = (size_t)a.nt;
     const int c = t < a.nc ? t : a.gCell[t - a.nc];
-    double qi[NQ], qv[NQ];
+    double qv[NQ];
 #pragma unroll
-    for (int v = 0; v < NQ; ++v) qi[v] = q[(size_t)v * stride + c];
-    if (t < a.nc) {
-#pragma unroll
-        for (int v = 0; v < NQ; ++v) qv[v] = qi[v];
-    } else {
-        ghost_bc<double, D>(a, t - a.nc, qi, qv);
-        for (int r = 0; r < vRows; ++r) a.V[r * nt + t] = 0.0;
-    }
+    for (int v = 0; v < NQ; ++v) qv[v] = q[(size_t)v * stride + c];
     if (t >= a.nc || cellGrad)
         for (int r = 0; r < gradRows; ++r) a.grad[r * nt + t] = 0.0;
+    if (t >= a.nc) {
+        for (int r = 0; r < vRows; ++r) a.V[r * nt + t] = 0.0;
+        ghost64<D>(a, t - a.nc, a.gKind[t - a.nc], ghost_in<double, D>(a, qv));
+        return;
+    }
 #pragma unroll
     for (int v = 0; v < NQ; ++v) a.q[(size_t)v * nt + t] = qv[v];
     prims64<D>(a, t, qv);

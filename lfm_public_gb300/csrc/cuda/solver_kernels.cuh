@@ -142,8 +142,8 @@ struct Args {
     // constants
     double gamma, gm1, Rinv, rhoInf, EInf, pInf, TInf, UInf[3], mu, kcond;
     double gh;                // gamma / (gamma - 1): enthalpy per unit R psi
-    double gm1Inv;            // boundary states: 1 / (gamma - 1), 1 / (R T_inf), |U_inf|^2 / 2
-    double RTInv, keInf;
+    double gm1Inv;            // boundary states: 1 / (gamma - 1), R T_inf, 1 / (R T_inf), 1 / p_inf,
+    double RT, RTInv, pInfInv, keInf;   // |U_inf|^2 / 2
     double mu23;              // 2/3 mu (the trace term of the deviatoric stress)
     // FP32-bulk: conservative reference state q_ref = (rho_inf, rho_inf U_inf,
     // rho_inf E_inf) in FP64 (index = variable) and its derived FP32 constants

@@ -150,7 +150,7 @@ __global__ void __launch_bounds__(128) k_prep_residual32(const __grid_constant__
     }
 #pragma unroll
     for (int v = 0; v < NQ; ++v) qp[v] += a.qRef[v];
-    ghost32<D>(a, t - a.nc, a.gKind[t - a.nc], qp, a.prim);
+    ghost32<D>(a, t - a.nc, a.gKind[t - a.nc], ghost_in<float, D>(a, qp), a.prim);
     for (int k = 0; k < vWords; ++k) a.V[(size_t)t * vWords + k] = 0.0f;
 }
 
