@@ -78,6 +78,8 @@ struct BatchStates {
 // The states of n cases in (`set`; parity: BatchArgs) or out.
 cudaError_t launch_batch_states(const BatchCase* cases, const BatchStates& m, int n, int maxCells, bool set, int parity,
                                 cudaStream_t st);
+// The primitives of a case's nt cells and ghosts from its stored state.
+cudaError_t launch_batch_prims(const BatchCase* cases, int slot, int nt, int parity, cudaStream_t st);
 // Stage `stage` of a batch of fusable cases with current primitives.
 cudaError_t launch_batch_fused(const BatchArgs& b, int stage, int block, int bps, int sms, cudaStream_t st);
 // Resident blocks per SM of the stage kernel at `block` threads.

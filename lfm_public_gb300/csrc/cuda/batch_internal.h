@@ -195,6 +195,7 @@ struct lfm_batch {
     bool lean = false;          // every case is fusable and has current primitives
     int parity = 0;             // the fusable cases' current primitive buffer
     cudaGraphExec_t graph[2][2] = {};   // a step's graph, by [lean][parity]
+    bool graphStale[2][2] = {};         // its kernels, grids or arguments have changed
     cudaEvent_t ev0 = nullptr, ev1 = nullptr;
     void* scrub = nullptr;
     size_t scrubBytes = 0;

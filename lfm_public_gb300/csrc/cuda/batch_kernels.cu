@@ -277,6 +277,20 @@ __global__ void __launch_bounds__(256) k_batch_set(const BatchCase* cases, const
     else set_state32<3>(a, q, a.nc, c);
 }
 
+// Primitives of one case's cells and ghosts from its stored state.
+__global__ void __launch_bounds__(256) k_batch_prims(const BatchCase* cases, int slot, int parity) {
+    __shared__ Args<float> a;
+    if (threadIdx.x == 0) {
+        a = cases[slot].a;
+        if (parity) a.prim = a.primW;
+    }
+    __syncthreads();
+    const int t = LFM_GLOBAL_ID();
+    if (t >= a.nt) return;
+    if (a.D == 2) prep32<2>(a, t);
+    else prep32<3>(a, t);
+}
+
 __global__ void __launch_bounds__(256) k_batch_get(const BatchCase* cases, const __grid_constant__ BatchStates m) {
     const Args<float>& a = cases[m.slot[blockIdx.y]].a;
     const int c = LFM_GLOBAL_ID(), nc = a.nc;
@@ -384,6 +398,11 @@ cudaError_t launch_batch_fused(const BatchArgs& b, int stage, int block, int bps
         case 512: return launch_fused<512>(b, stage, bps, sms, st);
         default: return launch_fused<256>(b, stage, bps, sms, st);
     }
+}
+
+cudaError_t launch_batch_prims(const BatchCase* cases, int slot, int nt, int parity, cudaStream_t st) {
+    k_batch_prims<<<(unsigned)((nt + 255) / 256), 256, 0, st>>>(cases, slot, parity);
+    return cudaGetLastError();
 }
 
 cudaError_t launch_batch_states(const BatchCase* cases, const BatchStates& m, int n, int maxCells, bool set, int parity,

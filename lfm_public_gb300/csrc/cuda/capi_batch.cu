@@ -174,7 +174,9 @@ int rebuildTiles(lfm_batch* b) {
         changed = changed || (b->tune.phased && n[ph] != b->nTiles[ph]);
         b->nTiles[ph] = n[ph];
     }
-    if (changed) dropGraphs(b);
+    if (changed)
+        for (auto& byParity : b->graphStale)
+            for (bool& stale : byParity) stale = true;
     b->variant = variant;
     b->lean = lean;
     b->tilesDirty = false;
@@ -213,6 +215,18 @@ int captureStep(lfm_batch* b, bool cooperative, cudaGraphExec_t* out) {
         cudaGetLastError();
         return cudaFail(le != cudaSuccess ? le : e, "batch step capture");
     }
+    // a graph of the same kernels takes the new grids and arguments in place, for
+    // a fraction of the time of another instantiation
+    if (*out) {
+        cudaGraphExecUpdateResultInfo info;
+        if (cudaGraphExecUpdate(*out, g, &info) == cudaSuccess) {
+            cudaGraphDestroy(g);
+            return LFM_OK;
+        }
+        cudaGetLastError();
+        cudaGraphExecDestroy(*out);
+        *out = nullptr;
+    }
     e = cudaGraphInstantiate(out, g, 0);
     cudaGraphDestroy(g);
     if (e != cudaSuccess) {
@@ -231,8 +245,14 @@ int ensureGraph(lfm_batch* b) {
         if (rc) return rc;
     }
     cudaGraphExec_t* graph = &b->graph[b->lean ? 1 : 0][b->parity];
-    if (*graph) return LFM_OK;
-    if (b->tune.phased || b->lean) return captureStep(b, false, graph);   // no co-residency needed
+    bool& stale = b->graphStale[b->lean ? 1 : 0][b->parity];
+    if (*graph && !stale) return LFM_OK;
+    stale = true;   // until its capture has succeeded
+    if (b->tune.phased || b->lean) {   // no co-residency needed
+        const int rc = captureStep(b, false, graph);
+        if (rc == LFM_OK) stale = false;
+        return rc;
+    }
     const int fit = lfm::dev::batch_blocks_per_sm(b->tune.block, b->variant);
     if (fit <= 0) return lfm::setError(LFM_ERR_UNSUPPORTED, "batch kernel does not fit on an SM");
     const int bps = b->tune.blocks_per_sm > 0 ? std::min(b->tune.blocks_per_sm, fit) : fit;
@@ -245,6 +265,7 @@ int ensureGraph(lfm_batch* b) {
         b->tune.cooperative = 0;
         rc = captureStep(b, false, graph);
     }
+    if (rc == LFM_OK) stale = false;
     return rc;
 }
 
@@ -454,6 +475,10 @@ int commitCase(lfm_batch* b, const PreparedCase& pc, int* slot) {
     if (e == cudaSuccess)
         e = cudaMemcpyAsync(b->dCases + s, &bc, sizeof(bc), cudaMemcpyHostToDevice, b->stream);
     if (e == cudaSuccess) e = cudaMemsetAsync(b->dFlags + s, 0, sizeof(int), b->stream);
+    // its primitives now: a preparation phase in its first step would have every
+    // case's step captured twice more
+    if (e == cudaSuccess)
+        e = lfm::dev::launch_batch_prims(b->dCases, s, pc.nc + pc.ng, b->parity, b->stream);
     // bc is a host temporary: the copies must finish before it goes
     if (e == cudaSuccess) e = cudaStreamSynchronize(b->stream);
     if (e != cudaSuccess) {
@@ -472,7 +497,7 @@ int commitCase(lfm_batch* b, const PreparedCase& pc, int* slot) {
     sl.nt = pc.nc + pc.ng;
     sl.needGradVis = pc.needGradVis;
     sl.fusable = L.fusable;
-    sl.primsValid = false;
+    sl.primsValid = true;
     for (int v = 0; v < 5; ++v) sl.qRef[v] = pc.bc.a.qRef[v];
     sl.q = a.q;
     sl.a = a;
