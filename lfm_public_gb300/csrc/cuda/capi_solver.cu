@@ -194,7 +194,7 @@ int buildArgs(lfm_solver* s, const lfm_solver_desc* d, Args<T>& a, const int* fP
     a.cfSoN = nullptr;
     a.cellSoW = nullptr;
     constexpr bool fp64 = sizeof(T) == sizeof(double);
-    a.pdl = lfm::dev::pdl_pays(fp64, s->D, s->nc) ? 1 : 0;
+    a.pdl = lfm::dev::pdl_pays(fp64, s->D, s->scheme, s->nc) ? 1 : 0;
     const size_t nt = (size_t)s->nt, nf = (size_t)s->nf, D = (size_t)s->D;
     int rc;
     if ((rc = devAlloc(s, &a.dq, (size_t)s->nq * s->nc))) return rc;

@@ -24,19 +24,21 @@ struct FluxStaging {
 // (PdlWait, solver_device.cuh). A dependent's blocks go where room appears
 // first; one with fewer blocks than the chip holds at once is crowded onto part
 // of the SMs, and FP64 work then waits for their FP64 pipes, while a larger one
-// fills every SM anyway and a very small one finds idle SMs. Measured on GB300,
-// us a step without and with:
-//   FP64 2D   2k cells  83.9  71.6 |  16k  57.3  51.1 | 33k 122.8 137.2 | 66k 184.2 233.4
-//           101k cells 247.7 256.5 | 135k 305.1 307.1 | 194k 425.9 405.1 | 262k 272.3 266.2
-//   FP64 3D   5k cells 141.3 133.1 |  10k 145.3 159.7 | 43k 284.6 298.9 | 83k 430.0 454.6
-//           117k cells 585.6 582.6 | 229k 1037.2 1015.7
-//   FP32 2D   2k cells  57.6  51.1 |  16k  45.0  42.9 | 101k 73.6  65.4 | 194k 90.0  79.8
-//   FP32 3D   5k cells  90.0  81.8 |  43k  98.2  90.0 | 61k 110.6 112.5 | 83k 114.6 128.9
-//           117k cells 130.1 135.1 | 229k 196.5 185.3
-// (between 90k and 160k cells, inviscid FP64 2D gains 4 %, viscous loses 1-4 %).
-inline bool pdl_pays(bool fp64, int D, int nc) {
-    if (D == 2) return !fp64 || nc <= 16384 || nc >= 163840;
-    return fp64 ? nc <= 8192 || nc >= 131072 : nc <= 49152 || nc >= 163840;
+// fills every SM anyway and a smaller one finds idle SMs. FP32 kernels wait for
+// loads, which crowded SMs serve as well. Measured on GB300, us a step without
+// and with (one unit of the timer is 2 us):
+//   FP64 2D M1   2k cells  45.0  38.8 |  36k  69.6  61.4 | 51k  88.0  79.8 | 58k  86.0 112.6
+//               81k cells 116.7 124.7 | 101k 239.6 253.9 | 135k 296.9 293.3 | 144k 325.6 311.2
+//   FP64 2D M2AUSM 15k cells 9 % less | 22k 255.9 243.7 | 33k 305.1 341.9 | 135k 932.8 932.3
+//   FP64 3D      5k cells 135.1 124.9 |  10k 137.2 151.5 | 61k 330.1 391.1 | 117k 579.0 581.1
+//              134k cells 641.0 632.8 | 171k 794.5 772.0
+//   FP32 2D      2k cells  36.8  34.7 |  46k  57.2  49.9 | 135k 73.7 67.5
+//   FP32 3D      5k cells  61.4  53.2 |  51k  81.9  83.9 | 83k 98.2 99.9 | 134k 118.7 116.7 | 171k 147.4 137.1
+// (viscous but for the FP64 2D M1 sizes below 100k).
+inline bool pdl_pays(bool fp64, int D, int scheme, int nc) {
+    if (!fp64 || nc >= 131072) return true;
+    if (D == 3) return nc <= 8192;
+    return nc <= (scheme == kSchemeAUSM ? 24576 : 53248);
 }
 
 // Launches k, with `pdl` as a programmatic dependent of the stream's previous

@@ -4,8 +4,8 @@ The step graph overlaps each kernel's first blocks with its predecessor's last
 ones; the single-stage calls launch the same kernels one after another. Both
 must give the same bits, on either side of the sizes at which the rule
 (pdl_pays, csrc/cuda/solver_launch.h) turns the overlap on and off: FP64 2D up
-to 16,384 cells and from 163,840, FP64 3D up to 8,192 and from 131,072,
-FP32-bulk 3D up to 49,152 and from 163,840."""
+to 53,248 cells (M2AUSM 24,576), 3D up to 8,192, both from 131,072; FP32-bulk at
+every size."""
 import numpy as np
 import pytest
 
@@ -21,7 +21,8 @@ def _cylinder(nt, nr, ns, solver):
 
 SHAPES = [(8, 4, 1, 0), (128, 128, 1, 0), (129, 128, 1, 1), (128, 128, 1, 2), (512, 320, 1, 1), (512, 319, 1, 0),
           (32, 16, 16, 1), (33, 16, 16, 1), (32, 16, 16, 2), (64, 32, 24, 0), (64, 33, 24, 1), (64, 48, 38, 1), (64, 64, 32, 1),
-          (80, 64, 32, 0)]
+          (80, 64, 32, 0), (256, 208, 1, 0), (257, 208, 1, 1), (192, 128, 1, 2), (193, 128, 1, 2), (512, 256, 1, 2),
+          (511, 256, 1, 1)]
 
 
 @pytest.mark.parametrize("precision", [N.LFM_FP64, N.LFM_FP32_BULK])
