@@ -338,10 +338,8 @@ __global__ void __launch_bounds__(kFaceThreads<D>) k_flux(Args<T> a) {
                 unPos += uP * S[x];
                 unNeg += uN * S[x];
             }
-            T ct = -cdiv * rsqrt(cdiv * cdiv + ccurl + T(4e-2));
-            ct = (ct < T(0)) ? T(0) : ct;
-            T nt_ = -ndiv * rsqrt(ndiv * ndiv + ncurl + T(4e-2));
-            nt_ = (nt_ < T(0)) ? T(0) : nt_;
+            const T ct = pos_part(-cdiv * rsqrt64(cdiv * cdiv + ccurl + T(4e-2)));
+            const T nt_ = pos_part(-ndiv * rsqrt64(ndiv * ndiv + ncurl + T(4e-2)));
             const T theta = T(0.5) * (ct + nt_);
             const T cp = qi[0] * cRpsi, np = qj[0] * aRpsi;   // p = rho R psi
             T gri[D], grj[D], gpi[D], gpj[D];
@@ -364,11 +362,10 @@ __global__ void __launch_bounds__(kFaceThreads<D>) k_flux(Args<T> a) {
             const T M0 = sqrt(m);
             const T fa = M0 * (T(2) - M0);
             const T alpha = T(3.0 / 16.0) * (T(5) * fa * fa - T(4));
-            const T ppP = p5pos(MPos, alpha), pnP = p5neg(MPos, alpha);
-            const T ppN = p5pos(MNeg, alpha), pnN = p5neg(MNeg, alpha);
-            const T phalf = pNeg * (ppN - pnN) - pPos * (ppP - pnP);
-            const T pu = T(-0.75) * ppP * pnN * (rhoPos + rhoNeg) * cavg * fa * (unNeg - unPos);
-            pavg += theta * (pu - T(0.5) * phalf);
+            const T hP = p5half(MPos, alpha), hN = p5half(MNeg, alpha);
+            const T phalf = pNeg * hN - pPos * hP;   // half of p (p5pos - p5neg), N less P
+            const T pu = T(-0.75) * (T(0.5) + hP) * (T(0.5) - hN) * (rhoPos + rhoNeg) * cavg * fa * (unNeg - unPos);
+            pavg += theta * (pu - phalf);
         }
         const T hphi = T(0.5) * mS2 * rcp64(rho2);   // u_f . S / 2
         const T mS = T(0.5) * mS2;
