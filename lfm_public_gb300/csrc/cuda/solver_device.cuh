@@ -142,23 +142,30 @@ template <int D>
 constexpr int kVisRows = D * D + 2 * D;
 
 // Minmod-limited face reconstruction from the upwind side (calc_r and
-// interp_minmod, api/cfdv0_solver.h:310-370): flux = +1 reconstructs from P,
-// -1 from N.
-template <typename T, int D>
-__device__ __forceinline__ T minmod_interp(T cp, T ap, const T* grad, const T* d, T w, T flux) {
-    const T gradf = ap - cp + T(1.0e-30);
-    T gradcf = T(0);
+// interp_minmod, api/cfdv0_solver.h:310-370), FP32: FROMP from P with its
+// gradient, else from N. The limiter 2 (gradcf / gradf) - 1, held to [0, 1], is
+// 1 or 0 unless the quotient is between 1/2 and 1, which the comparisons tell
+// exactly (the reference's largest quotient, 1000, lies beyond): only then it is
+// divided. (|gradf| is 0 or at least 2^-123, so its half is exact.) The flux of
+// a 331 x 217 M2AUSM cylinder executed 1200 instructions a face, many of them
+// the long form of a division, of the very small differences of a uniform flow:
+// 53 -> 36 us a step from uniform flow, 1 % of the step in a disturbed one; with
+// branches in place of the selects that one was 4 % slower (GB300). Values that
+// are no numbers come to the quotient.
+template <int D, bool FROMP>
+__device__ __forceinline__ float minmod_interp(float cp, float ap, const float* grad, const float* d, float w) {
+    const float gradf = ap - cp + 1.0e-30f;
+    float gradcf = d[0] * grad[0];
 #pragma unroll
-    for (int k = 0; k < D; ++k) gradcf += d[k] * grad[k];
-    T r;
-    if (fabs(gradcf) >= T(1000) * fabs(gradf))
-        r = T(2000) * (gradcf < T(0) ? T(-1) : T(1)) * (gradf < T(0) ? T(-1) : T(1)) - T(1);
-    else
-        r = T(2) * (gradcf / gradf) - T(1);
-    T lim = (T(1) < r) ? T(1) : r;
-    lim = (lim < T(0)) ? T(0) : lim;
-    const T weight = lim * w + (T(1) - lim) * (T(1) + flux) * T(0.5);
-    return weight * cp + (T(1) - weight) * ap;
+    for (int k = 1; k < D; ++k) gradcf += d[k] * grad[k];
+    // the quotient's sign moved to its upper part
+    const float af = fabsf(gradf);
+    const float gc = __uint_as_float(__float_as_uint(gradcf) ^ (__float_as_uint(gradf) & 0x80000000u));
+    const bool zero = gc < 0.5f * af, fixed = zero || gc >= af;   // 1 / 1 in a fixed one's place
+    float lim = 2.0f * ((fixed ? 1.0f : gc) / (fixed ? 1.0f : af)) - 1.0f;
+    if (zero) lim = 0.0f;
+    const float weight = FROMP ? lim * w + (1.0f - lim) : lim * w;
+    return weight * cp + (1.0f - weight) * ap;
 }
 
 // Comparisons of a double on the integer pipe, from its upper word (an FP64

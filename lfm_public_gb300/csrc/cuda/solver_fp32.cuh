@@ -737,8 +737,8 @@ __device__ __forceinline__ void face_rhs32_core(const A& a, int f, int i, int j,
                 ncurl += nn * nn;
             }
             const float *gi = Gi + 2 * D + x * D, *gj = Gj + 2 * D + x * D;
-            const float uP = minmod_interp<float, D>(ui[x], uj[x], gi, d, w, 1.0f);
-            const float uN = minmod_interp<float, D>(ui[x], uj[x], gj, d, w, -1.0f);
+            const float uP = minmod_interp<D, true>(ui[x], uj[x], gi, d, w);
+            const float uN = minmod_interp<D, false>(ui[x], uj[x], gj, d, w);
             unPos += (R.U[x] + uP) * S[x];
             unNeg += (R.U[x] + uN) * S[x];
             dUn += (uN - uP) * S[x];
@@ -751,10 +751,10 @@ __device__ __forceinline__ void face_rhs32_core(const A& a, int f, int i, int j,
         const float theta = 0.5f * (ct + nt_);
         const float pi = pressure_dev(R, ri, Ri), pj = pressure_dev(R, rj, Rj);
         const float *gri = Gi, *grj = Gj, *gpi = Gi + D, *gpj = Gj + D;
-        const float rhoPos = R.rho + minmod_interp<float, D>(ri, rj, gri, d, w, 1.0f);
-        const float rhoNeg = R.rho + minmod_interp<float, D>(ri, rj, grj, d, w, -1.0f);
-        const float pPos = minmod_interp<float, D>(pi, pj, gpi, d, w, 1.0f);    // p - p_ref
-        const float pNeg = minmod_interp<float, D>(pi, pj, gpj, d, w, -1.0f);
+        const float rhoPos = R.rho + minmod_interp<D, true>(ri, rj, gri, d, w);
+        const float rhoNeg = R.rho + minmod_interp<D, false>(ri, rj, grj, d, w);
+        const float pPos = minmod_interp<D, true>(pi, pj, gpi, d, w);    // p - p_ref
+        const float pNeg = minmod_interp<D, false>(pi, pj, gpj, d, w);
         const float Msq = (unPos * unPos + unNeg * unNeg) / (2.0f * cavg * cavg * norm);
         const float sc = 1.0f / (sqrtf(norm) * cavg);
         const float MPos = unPos * sc, MNeg = unNeg * sc;
