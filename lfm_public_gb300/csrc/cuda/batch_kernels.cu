@@ -66,33 +66,34 @@ __device__ __forceinline__ bool grid_barrier(unsigned* counter, unsigned target,
 // for batches of M1/M2 cases without viscosity: no gradient or viscous code
 // is compiled in, which keeps the kernel's register count (and so its
 // occupancy) down.
-template <int PH, int D, bool FULL>
-__device__ __forceinline__ void item(const BatchCase& bc, int stage, int i) {
+template <int PH, int D, bool FULL, class Sync>
+__device__ __forceinline__ void item(const BatchCase& bc, int stage, int i, Sync sync) {
     const Args<float>& a = bc.a;
     if (PH == 0) {
+        sync();
         prep32<D>(a, i);
     } else if (PH == 1) {
         if (FULL) {
             if (bc.needGrad) {
-                if (a.cfEll) grad32<D, true>(a, i);
-                else grad32<D, false>(a, i);
+                if (a.cfEll) grad32<D, true>(a, i, sync);
+                else grad32<D, false>(a, i, sync);
             }
             if (bc.needVis) {
-                if (a.cfEll) vis32<D, false, true>(a, i);
-                else vis32<D, false, false>(a, i);
+                if (a.cfEll) vis32<D, false, true>(a, i, sync);
+                else vis32<D, false, false>(a, i, sync);
             }
         }
     } else if (PH == 2) {
         if (bc.scheme == kSchemeM1)
-            flux32<D, kSchemeM1, FULL>(a, i);
+            flux32<D, kSchemeM1, FULL, false, false>(a, i, sync);
         else if (!FULL || bc.scheme == kSchemeM2)
-            flux32<D, kSchemeM2, FULL>(a, i);
+            flux32<D, kSchemeM2, FULL, false, false>(a, i, sync);
         else
-            flux32<D, kSchemeAUSM, FULL>(a, i);
+            flux32<D, kSchemeAUSM, FULL, false, false>(a, i, sync);
     } else {
         const int first = stage == 0;
         const bool res = bc.residuals && first;
-        update32<D, true, kEntriesEither>(a, i, bc.rkA[stage], bc.rkB[stage], bc.dt32, first, res);
+        update32<D, true, kEntriesEither>(a, i, bc.rkA[stage], bc.rkB[stage], bc.dt32, first, res, sync);
     }
 }
 
@@ -141,9 +142,9 @@ __device__ __forceinline__ BlockTiles block_tiles(const BatchArgs& b, int in, in
     return r;
 }
 
-template <int PH, int BLOCK, int DIMS, bool FULL>
+template <int PH, int BLOCK, int DIMS, bool FULL, class Sync = NoWait>
 __device__ __forceinline__ void phase_tiles(const BatchArgs& b, int stage, const BlockTiles& r, BatchCase& sc,
-                                            int& sSlot) {
+                                            int& sSlot, Sync sync = Sync()) {
     for (int t = r.t0; t < r.t1; ++t) {
         const BatchTile td = t == r.t0 ? r.first : b.tiles[PH][t];
         load_case<BLOCK>(b, td.slot, b.parity, b.parity, sc, sSlot);
@@ -152,9 +153,9 @@ __device__ __forceinline__ void phase_tiles(const BatchArgs& b, int stage, const
             const int i = td.start + (int)threadIdx.x + k * BLOCK;
             if (i < end) {
                 if (DIMS == 2 || sc.a.D == 2)
-                    item<PH, 2, FULL>(sc, stage, i);
+                    item<PH, 2, FULL>(sc, stage, i, sync);
                 else
-                    item<PH, 3, FULL>(sc, stage, i);
+                    item<PH, 3, FULL>(sc, stage, i, sync);
             }
         }
     }
@@ -253,8 +254,8 @@ __global__ void __launch_bounds__(BLOCK) k_batch_phase(const __grid_constant__ B
     if (threadIdx.x == 0) sSlot = -1;
     __syncthreads();
     const BlockTiles r = block_tiles<PH, BLOCK>(b, b.parity, b.parity, sc, sSlot);
-    PdlWait{1}();
-    phase_tiles<PH, BLOCK, DIMS, FULL>(b, stage, r, sc, sSlot);
+    phase_tiles<PH, BLOCK, DIMS, FULL>(b, stage, r, sc, sSlot, PdlWait{1});
+    PdlWait{1}();   // also where a block had no item: the next phase waits for this one alone
 }
 
 // New states of several cases, and their states out, in one launch each: one
