@@ -90,6 +90,7 @@ int batch_blocks_per_sm(int block, int variant);
 struct PhasedShape {
     int tiles[kBatchPhases];
     int blocksPerSm, sms;
+    bool plain;   // no case is M2AUSM, and all have fixed-width tables
 };
 cudaError_t launch_batch_phased(const BatchArgs& b, int stage, int block, int variant, const PhasedShape& p,
                                 cudaStream_t st);

@@ -137,7 +137,7 @@ struct Slot {
     bool used = false;
     size_t off = 0, bytes = 0;
     int D = 2, nq = 4, nc = 0, ng = 0, nf = 0, nt = 0;
-    bool needGradVis = false, fusable = false;
+    bool needGradVis = false, fusable = false, plain = false;
     bool primsValid = false;   // cells' primitives current (kept so by the update phase)
     double qRef[5] = {0, 0, 0, 0, 0};   // the device state is q - qRef
     double* q = nullptr;   // device
@@ -187,6 +187,7 @@ struct lfm_batch {
     // cases of 11k-29k cells, 2D and 3D: 139 -> 112 us a step, GB300).
     lfm_batch_tuning tune{128, 1, 0, 1, 1};
     int variant = lfm::dev::kBatchVariantGeneral;   // stage-kernel variant of the current cases
+    bool plain = false;                 // its phases' (PhasedShape::plain)
     bool untuned = true;        // no launch shape was asked for
     int block = 0;              // threads per block of the current tiles
     int nTiles[lfm::dev::kBatchPhases] = {};

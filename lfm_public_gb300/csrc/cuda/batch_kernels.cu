@@ -66,7 +66,7 @@ __device__ __forceinline__ bool grid_barrier(unsigned* counter, unsigned target,
 // for batches of M1/M2 cases without viscosity: no gradient or viscous code
 // is compiled in, which keeps the kernel's register count (and so its
 // occupancy) down.
-template <int PH, int D, bool FULL, class Sync>
+template <int PH, int D, bool FULL, bool PLAIN, class Sync>
 __device__ __forceinline__ void item(const BatchCase& bc, int stage, int i, Sync sync) {
     const Args<float>& a = bc.a;
     if (PH == 0) {
@@ -74,26 +74,26 @@ __device__ __forceinline__ void item(const BatchCase& bc, int stage, int i, Sync
         prep32<D>(a, i);
     } else if (PH == 1) {
         if (FULL) {
-            if (bc.needGrad) {
+            if (!PLAIN && bc.needGrad) {
                 if (a.cfEll) grad32<D, true>(a, i, sync);
                 else grad32<D, false>(a, i, sync);
             }
             if (bc.needVis) {
-                if (a.cfEll) vis32<D, false, true>(a, i, sync);
+                if (PLAIN || a.cfEll) vis32<D, false, true>(a, i, sync);
                 else vis32<D, false, false>(a, i, sync);
             }
         }
     } else if (PH == 2) {
         if (bc.scheme == kSchemeM1)
             flux32<D, kSchemeM1, FULL, false, false>(a, i, sync);
-        else if (!FULL || bc.scheme == kSchemeM2)
+        else if (!FULL || PLAIN || bc.scheme == kSchemeM2)
             flux32<D, kSchemeM2, FULL, false, false>(a, i, sync);
         else
             flux32<D, kSchemeAUSM, FULL, false, false>(a, i, sync);
     } else {
         const int first = stage == 0;
         const bool res = bc.residuals && first;
-        update32<D, true, kEntriesEither>(a, i, bc.rkA[stage], bc.rkB[stage], bc.dt32, first, res, sync);
+        update32<D, true, PLAIN ? kEntriesEll : kEntriesEither>(a, i, bc.rkA[stage], bc.rkB[stage], bc.dt32, first, res, sync);
     }
 }
 
@@ -142,7 +142,7 @@ __device__ __forceinline__ BlockTiles block_tiles(const BatchArgs& b, int in, in
     return r;
 }
 
-template <int PH, int BLOCK, int DIMS, bool FULL, class Sync = NoWait>
+template <int PH, int BLOCK, int DIMS, bool FULL, bool PLAIN, class Sync = NoWait>
 __device__ __forceinline__ void phase_tiles(const BatchArgs& b, int stage, const BlockTiles& r, BatchCase& sc,
                                             int& sSlot, Sync sync = Sync()) {
     for (int t = r.t0; t < r.t1; ++t) {
@@ -153,9 +153,9 @@ __device__ __forceinline__ void phase_tiles(const BatchArgs& b, int stage, const
             const int i = td.start + (int)threadIdx.x + k * BLOCK;
             if (i < end) {
                 if (DIMS == 2 || sc.a.D == 2)
-                    item<PH, 2, FULL>(sc, stage, i, sync);
+                    item<PH, 2, FULL, PLAIN>(sc, stage, i, sync);
                 else
-                    item<PH, 3, FULL>(sc, stage, i, sync);
+                    item<PH, 3, FULL, PLAIN>(sc, stage, i, sync);
             }
         }
     }
@@ -197,18 +197,18 @@ __global__ void __launch_bounds__(BLOCK, stage_blocks(BLOCK, DIMS, FULL)) k_batc
     auto after_prep = [&] { grad ? next1() : next2(); };
     if (b.nTiles[0] > 0) {
         r = block_tiles<0, BLOCK>(b, b.parity, b.parity, sc, sSlot);
-        phase_tiles<0, BLOCK, DIMS, FULL>(b, stage, r, sc, sSlot);
+        phase_tiles<0, BLOCK, DIMS, FULL, false>(b, stage, r, sc, sSlot);
         if (!barrier(after_prep)) return;
     } else {
         after_prep();
     }
     if (grad) {
-        phase_tiles<1, BLOCK, DIMS, FULL>(b, stage, r, sc, sSlot);
+        phase_tiles<1, BLOCK, DIMS, FULL, false>(b, stage, r, sc, sSlot);
         if (!barrier(next2)) return;
     }
-    phase_tiles<2, BLOCK, DIMS, FULL>(b, stage, r, sc, sSlot);
+    phase_tiles<2, BLOCK, DIMS, FULL, false>(b, stage, r, sc, sSlot);
     if (!barrier(next3)) return;
-    phase_tiles<3, BLOCK, DIMS, FULL>(b, stage, r, sc, sSlot);
+    phase_tiles<3, BLOCK, DIMS, FULL, false>(b, stage, r, sc, sSlot);
 }
 
 // Flux and update of cell i of a case that can do both at once (fluxupdate32).
@@ -246,15 +246,28 @@ __global__ void __launch_bounds__(BLOCK, BLOCK > 256 ? 1 : 768 / BLOCK) k_batch_
     }
 }
 
-// One phase of a stage over every case, for the phased launch mode.
-template <int PH, int BLOCK, int DIMS, bool FULL>
-__global__ void __launch_bounds__(BLOCK) k_batch_phase(const __grid_constant__ BatchArgs b, int stage) {
+// One phase of a stage over every case, for the phased launch mode. PLAIN: no
+// case is M2AUSM and all have fixed-width tables (PhasedShape::plain). A phase
+// waits for loads, and without M2AUSM's reconstruction and the face lists it
+// fits 1024 threads on an SM (64 registers; the 3D update then spills 212
+// bytes, and is faster all the same); with them 512 (128). Us a step, GB300, of
+// the general phases, of plain ones at 768 threads and at 1024: 2D and 3D of
+// 14k cells each 88, 72, 74; viscous 2D of 289k 172, 156, 149; 3D of 365k 552,
+// 414, 434; 2D and 3D of 308k 478, 399, 385.
+template <bool PLAIN>
+constexpr int phase_blocks(int block) {
+    constexpr int threads = PLAIN ? 1024 : 512;
+    return threads >= block ? threads / block : 1;
+}
+
+template <int PH, int BLOCK, int DIMS, bool FULL, bool PLAIN>
+__global__ void __launch_bounds__(BLOCK, phase_blocks<PLAIN>(BLOCK)) k_batch_phase(const __grid_constant__ BatchArgs b, int stage) {
     __shared__ BatchCase sc;
     __shared__ int sSlot;
     if (threadIdx.x == 0) sSlot = -1;
     __syncthreads();
     const BlockTiles r = block_tiles<PH, BLOCK>(b, b.parity, b.parity, sc, sSlot);
-    phase_tiles<PH, BLOCK, DIMS, FULL>(b, stage, r, sc, sSlot, PdlWait{1});
+    phase_tiles<PH, BLOCK, DIMS, FULL, PLAIN>(b, stage, r, sc, sSlot, PdlWait{1});
     PdlWait{1}();   // also where a block had no item: the next phase waits for this one alone
 }
 
@@ -302,11 +315,11 @@ __global__ void __launch_bounds__(256) k_batch_get(const BatchCase* cases, const
 
 // The phases of a stage that have tiles, one kernel each, every one but the
 // step's first a programmatic dependent of the one before.
-template <int PH, int BLOCK, int DIMS, bool FULL>
+template <int PH, int BLOCK, int DIMS, bool FULL, bool PLAIN>
 cudaError_t launch_phase(const BatchArgs& b, int stage, const PhasedShape& p, bool* chained, cudaStream_t st) {
     if (p.tiles[PH] == 0) return cudaSuccess;
     static thread_local int fit = -1;   // resident blocks per SM of this kernel
-    auto k = k_batch_phase<PH, BLOCK, DIMS, FULL>;
+    auto k = k_batch_phase<PH, BLOCK, DIMS, FULL, PLAIN>;
     if (fit < 0) {
         cudaError_t e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&fit, k, BLOCK, 0);
         if (e != cudaSuccess || fit < 1) {
@@ -315,27 +328,34 @@ cudaError_t launch_phase(const BatchArgs& b, int stage, const PhasedShape& p, bo
         }
     }
     const int per = p.blocksPerSm > 0 ? std::min(p.blocksPerSm, fit) : fit;
-    launch_kernel_pdl(*chained, k, (unsigned)std::min(p.tiles[PH], per * p.sms), BLOCK, st, b, stage);
+    // up to four grids' worth of blocks: their tiles differ in work, and a block
+    // that ends early makes room for another (2D and 3D of 368k cells, one, two
+    // and four grids: 438, 385, 377 us a step; M2AUSM and M1 of 150k 363, 266, 260)
+    launch_kernel_pdl(*chained, k, (unsigned)std::min(p.tiles[PH], 4 * per * p.sms), BLOCK, st, b, stage);
     *chained = true;
     return cudaGetLastError();
 }
 
-template <int BLOCK, int DIMS, bool FULL>
+template <int BLOCK, int DIMS, bool FULL, bool PLAIN>
 cudaError_t launch_phases(const BatchArgs& b, int stage, const PhasedShape& p, cudaStream_t st) {
     bool chained = stage > 0;
-    cudaError_t e = launch_phase<0, BLOCK, DIMS, FULL>(b, stage, p, &chained, st);
-    if (e == cudaSuccess && FULL) e = launch_phase<1, BLOCK, DIMS, FULL>(b, stage, p, &chained, st);
-    if (e == cudaSuccess) e = launch_phase<2, BLOCK, DIMS, FULL>(b, stage, p, &chained, st);
-    if (e == cudaSuccess) e = launch_phase<3, BLOCK, DIMS, FULL>(b, stage, p, &chained, st);
+    cudaError_t e = launch_phase<0, BLOCK, DIMS, FULL, PLAIN>(b, stage, p, &chained, st);
+    if (e == cudaSuccess && FULL) e = launch_phase<1, BLOCK, DIMS, FULL, PLAIN>(b, stage, p, &chained, st);
+    if (e == cudaSuccess) e = launch_phase<2, BLOCK, DIMS, FULL, PLAIN>(b, stage, p, &chained, st);
+    if (e == cudaSuccess) e = launch_phase<3, BLOCK, DIMS, FULL, PLAIN>(b, stage, p, &chained, st);
     return e;
 }
 
 template <int BLOCK>
 cudaError_t launch_phases_variant(const BatchArgs& b, int stage, int variant, const PhasedShape& p, cudaStream_t st) {
     switch (variant) {
-        case kBatchVariant2DInviscid: return launch_phases<BLOCK, 2, false>(b, stage, p, st);
-        case kBatchVariant2D: return launch_phases<BLOCK, 2, true>(b, stage, p, st);
-        default: return launch_phases<BLOCK, 0, true>(b, stage, p, st);
+        case kBatchVariant2DInviscid: return launch_phases<BLOCK, 2, false, false>(b, stage, p, st);
+        case kBatchVariant2D:
+            return p.plain ? launch_phases<BLOCK, 2, true, true>(b, stage, p, st)
+                           : launch_phases<BLOCK, 2, true, false>(b, stage, p, st);
+        default:
+            return p.plain ? launch_phases<BLOCK, 0, true, true>(b, stage, p, st)
+                           : launch_phases<BLOCK, 0, true, false>(b, stage, p, st);
     }
 }
 

@@ -122,11 +122,12 @@ void dropGraphs(lfm_batch* b) {
 
 int rebuildTiles(lfm_batch* b) {
     // a step whose cases are all fusable and have current primitives is fused
-    bool lean = (b->untuned || !b->tune.phased) && b->barrierExtra == 0;
+    bool lean = (b->untuned || !b->tune.phased) && b->barrierExtra == 0, plain = true;
     int64_t cells = 0;
     for (const Slot& sl : b->slots)
         if (sl.used) {
             lean = lean && sl.fusable && sl.primsValid;
+            plain = plain && sl.plain;
             cells += sl.nc;
         }
     // untuned, 128 threads, but 256 for fused steps beyond L2's reach. Us a step,
@@ -168,7 +169,7 @@ int rebuildTiles(lfm_batch* b) {
     LFM_CUDA(cudaStreamSynchronize(b->stream));
     const int variant = currentVariant(b);
     // a phased step's grids follow the tiles
-    bool changed = realloc || variant != b->variant || block != b->block;
+    bool changed = realloc || variant != b->variant || block != b->block || plain != b->plain;
     b->block = block;
     for (int ph = 0; ph < kBatchPhases; ++ph) {
         changed = changed || (b->tune.phased && n[ph] != b->nTiles[ph]);
@@ -178,6 +179,7 @@ int rebuildTiles(lfm_batch* b) {
         for (auto& byParity : b->graphStale)
             for (bool& stale : byParity) stale = true;
     b->variant = variant;
+    b->plain = plain;
     b->lean = lean;
     b->tilesDirty = false;
     return LFM_OK;
@@ -198,7 +200,7 @@ BatchArgs makeArgs(lfm_batch* b) {
 
 int captureStep(lfm_batch* b, bool cooperative, cudaGraphExec_t* out) {
     const BatchArgs args = makeArgs(b);
-    lfm::dev::PhasedShape shape{{0, 0, 0, 0}, b->tune.blocks_per_sm, b->sms};
+    lfm::dev::PhasedShape shape{{0, 0, 0, 0}, b->tune.blocks_per_sm, b->sms, b->plain};
     for (int ph = 0; ph < kBatchPhases; ++ph) shape.tiles[ph] = b->nTiles[ph];
     cudaGraph_t g = nullptr;
     LFM_CUDA(cudaStreamBeginCapture(b->stream, cudaStreamCaptureModeThreadLocal));
@@ -497,6 +499,7 @@ int commitCase(lfm_batch* b, const PreparedCase& pc, int* slot) {
     sl.nt = pc.nc + pc.ng;
     sl.needGradVis = pc.needGradVis;
     sl.fusable = L.fusable;
+    sl.plain = pc.bc.scheme != dev::kSchemeAUSM && a.cfEll;
     sl.primsValid = true;
     for (int v = 0; v < 5; ++v) sl.qRef[v] = pc.bc.a.qRef[v];
     sl.q = a.q;
