@@ -414,15 +414,17 @@ int lfm_tiles_stats(const lfm_solver_desc* d, int tile_cells, int max_local, int
 int lfm_selftest_fp_convert(int64_t n, const uint32_t* f32_bits, const uint64_t* f64_bits, uint64_t* f64_of_f32,
                             uint32_t* f32_of_f64);
 
-/* ---- batch engine: many cases, one persistent kernel per RK stage ---------
+/* ---- batch engine: many cases, a few kernels per RK stage -----------------
  *
  * No single reference call corresponds: the reference advances one case per
  * MPI job (Mesh::solve, src/mesh_solver.cpp:474-853). A batch advances any
  * number of independent cases -- uneven sizes, 2D and 3D, M1/M2/M2AUSM --
  * with the FP32-bulk arithmetic (LFM_FP32_BULK), each case at its own constant
- * dt. A time step of all cases is one CUDA graph: one persistent kernel per RK
- * stage whose blocks work through per-phase tile lists of every case, with
- * grid-wide barriers between the phases. Case data lives in one device arena
+ * dt. A time step of all cases is one CUDA graph whose kernels' blocks work
+ * through per-phase tile lists of every case: one kernel per phase of an RK
+ * stage (the default), one per stage while all cases are 2D, inviscid and
+ * M1/M2, or one persistent kernel per stage with grid-wide barriers between
+ * the phases (lfm_batch_tuning). Case data lives in one device arena
  * reserved at creation; a case is admitted when a free block of its footprint
  * exists (lfm_batch_case_bytes) and its block is returned on removal. Cases may
  * be added and removed between steps. Calls on one batch are not re-entrant;
@@ -436,7 +438,8 @@ typedef struct lfm_batch_opts {
     int max_cases;        /* case slots; 0 = 256 */
 } lfm_batch_opts;
 
-/* Launch shape of the stage kernel, chosen by lfm_batch_autotune. */
+/* Launch shape of the stage kernels: 128 threads, one item a thread, phased,
+ * until lfm_batch_set_tuning or lfm_batch_autotune. */
 typedef struct lfm_batch_tuning {
     int block;            /* threads per block: 128, 256 or 512 */
     int items_per_thread; /* cells or faces per thread and tile (tile = block x items) */

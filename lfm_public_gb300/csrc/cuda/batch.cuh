@@ -1,12 +1,14 @@
 // Batched multi-case time step: many independent cases (uneven cell counts,
-// mixed schemes and dimensions) advanced by one persistent kernel per RK stage.
+// mixed schemes and dimensions) advanced together, by default with one kernel per
+// phase of an RK stage, optionally with one persistent kernel per stage.
 //
 // Every case lives in its own block of a device arena, with the FP32-bulk
 // arrays of a single-case solver (Args<float>). A stage is four phases over
 // all cases -- ghost states and primitives (of every cell too, right after a
 // case's state was set); gradients and viscous terms; face fluxes; gather, RK
-// update and the cells' next primitives -- separated by grid-wide barriers. While
-// every case of a batch is 2D, inviscid and M1 / M2 (fusable), a stage is one
+// update and the cells' next primitives -- separated by kernel boundaries, each
+// kernel a programmatic dependent of the one before, or by grid-wide barriers
+// inside the persistent kernel. While every case of a batch is 2D, inviscid and M1 / M2 (fusable), a stage is one
 // phase without a barrier instead: each cell evaluates its own faces and updates,
 // between two primitive buffers that alternate. Work
 // is a flat list of tiles per phase (a tile is a run of consecutive cells or

@@ -5,7 +5,8 @@
 // (FP32-bulk layout of a single-case solver). Admission is by footprint: a
 // case is admitted when a free block of its size exists (first fit, blocks
 // coalesce when cases leave). A time step of all cases is one CUDA graph --
-// a memset of the barrier counters and one persistent kernel per RK stage --
+// a memset of the barrier counters, then per RK stage one kernel per phase (or
+// one fused or persistent kernel) --
 // whose kernels read the case table and tile lists from device memory, so
 // admissions and removals between steps only rewrite those tables.
 #include <algorithm>

@@ -8,7 +8,7 @@
 // (a request that does not fit is passed over, but only max_bypass times
 // before admission waits for it); advance every admitted request together
 // by a chunk of steps -- the smallest remaining step count, at most
-// chunk_steps -- in the batch's persistent stage kernels; retire the
+// chunk_steps -- in the batch's stage kernels; retire the
 // requests that have finished (or whose state became non-finite), copying
 // their state out and freeing their slot and block. Requests arriving while
 // others run join at the next chunk boundary, so their work overlaps on the

@@ -1,13 +1,14 @@
 // Device kernels of the explicit finite-volume time step (sm_103a).
 //
-// One RK stage of the reference (src/mesh_solver.cpp:500-672) becomes five
-// kernels over structure-of-arrays data, all deterministic (no atomics on
-// values, every sum in a fixed order):
+// One RK stage of the reference (src/mesh_solver.cpp:500-672) becomes at most
+// four kernels, all deterministic (no atomics on values, every sum in a fixed
+// order). Arrays are structures of arrays in FP64, 16-byte parts per cell and
+// face in FP32-bulk (solver_fp32.cuh):
 //
-//   k_prep     per cell and ghost: boundary-ghost state (set_boundary_conditions,
+//   k_prep     after a new state, and for processor halos in every stage:
+//              boundary-ghost state (set_boundary_conditions,
 //              src/cfd_v0.cpp:1009-1221) and the primitives every face reads
-//              (1/rho, u, R psi = p/rho, c), computed once per stage instead of
-//              once per face side.
+//              (1/rho, u, R psi = p/rho, c); between stages k_update writes both.
 //   k_grad     per cell, gather over incident faces: Gauss-linear gradients of
 //              rho, p and u that M2AUSM's minmod reconstruction reads
 //              (calc_gradients_M2AUSM, :1383-1495). Only with M2AUSM + minmod;
@@ -20,8 +21,9 @@
 //   k_flux     per flux face: the face rhs of one_rk_step_M1 / _M2 / _M2AUSM
 //              (:2529-2796, :1896-2133, :2185-2489) into a face buffer.
 //   k_update   per cell, gather of the face rhs in ascending face order (the
-//              reference's scatter order), sponge source and the low-storage RK
-//              update (:2800-2822).
+//              reference's scatter order), sponge source, the low-storage RK
+//              update (:2800-2822), then the next stage's primitives of the cell
+//              and its boundary ghosts.
 //
 // The gather replaces the reference's scatter: within a stage every face is
 // evaluated once from the stage-start state, because a cell's owned faces
@@ -123,7 +125,7 @@ struct Args {
                               // v_c cellSoW_c + sum over entries of v_across cfSoN)
     const T* smagC;           // Smagorinsky LES: the constant each cell's tauMC is built with
                               // (V then holds D x D more rows: its SGS stress), or null
-    const uint8_t* cellGhosts;  // FP32-bulk single case: boundary faces of each cell
+    const uint8_t* cellGhosts;  // boundary faces of each cell
                                 // (its update writes their ghosts' primitives), or null
     const int* fOwn;          // FP32-bulk cell-centred flux: nc + 1 offsets, the flux faces that
                               // cell c owns (is P of) are fOwn[c] .. fOwn[c + 1] - 1 (the faces
