@@ -82,13 +82,11 @@ cudaError_t launch_batch_states(const BatchCase* cases, const BatchStates& m, in
                                 cudaStream_t st);
 // The primitives of a case's nt cells and ghosts from its stored state.
 cudaError_t launch_batch_prims(const BatchCase* cases, int slot, int nt, int parity, cudaStream_t st);
-// Stage `stage` of a batch of fusable cases with current primitives.
-cudaError_t launch_batch_fused(const BatchArgs& b, int stage, int block, int bps, int sms, cudaStream_t st);
 // Resident blocks per SM of the stage kernel at `block` threads.
 int batch_blocks_per_sm(int block, int variant);
 // Stage `stage` as one kernel per phase with tiles (kernel boundaries in place of
-// the grid barriers); each kernel's grid is at most blocksPerSm (0 = all that
-// fit) resident blocks per SM x sms, and no more than its tiles.
+// the grid barriers); each kernel's grid is at most a few times blocksPerSm (0 =
+// all that fit) resident blocks per SM x sms, and no more than its tiles.
 struct PhasedShape {
     int tiles[kBatchPhases];
     int blocksPerSm, sms;
@@ -96,6 +94,8 @@ struct PhasedShape {
 };
 cudaError_t launch_batch_phased(const BatchArgs& b, int stage, int block, int variant, const PhasedShape& p,
                                 cudaStream_t st);
+// Stage `stage` of a batch of fusable cases with current primitives.
+cudaError_t launch_batch_fused(const BatchArgs& b, int stage, int block, const PhasedShape& p, cudaStream_t st);
 
 }  // namespace dev
 }  // namespace lfm

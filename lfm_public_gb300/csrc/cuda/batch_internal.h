@@ -189,7 +189,6 @@ struct lfm_batch {
     int variant = lfm::dev::kBatchVariantGeneral;   // stage-kernel variant of the current cases
     bool plain = false;                 // its phases' (PhasedShape::plain)
     bool untuned = true;        // no launch shape was asked for
-    int block = 0;              // threads per block of the current tiles
     int nTiles[lfm::dev::kBatchPhases] = {};
     int grid = 0;
     bool tilesDirty = true;

@@ -102,9 +102,11 @@ __device__ __forceinline__ void item(const BatchCase& bc, int stage, int i, Sync
 // case that is never fused has the same one twice).
 template <int BLOCK>
 __device__ __forceinline__ void load_case(const BatchArgs& b, int slot, int in, int out, BatchCase& sc, int& sSlot) {
-    const bool reload = slot != sSlot;
+    // every thread of the block comes here with the same slot, and sSlot is
+    // written between barriers, so the warps of a block need not wait for one
+    // another until the case changes
+    if (slot == sSlot) return;
     __syncthreads();
-    if (!reload) return;
     const int4* src = reinterpret_cast<const int4*>(b.cases + slot);
     int4* dst = reinterpret_cast<int4*>(&sc);
     constexpr int n16 = (int)(sizeof(BatchCase) / 16);
@@ -396,7 +398,7 @@ cudaError_t launch_batch_stage(const BatchArgs& b, int stage, int block, int var
 }
 
 template <int BLOCK>
-static cudaError_t launch_fused(const BatchArgs& b, int stage, int bps, int sms, cudaStream_t st) {
+static cudaError_t launch_fused(const BatchArgs& b, int stage, const PhasedShape& p, cudaStream_t st) {
     static thread_local int fit = -1;   // resident blocks per SM
     if (fit < 0) {
         cudaError_t e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&fit, k_batch_fused<BLOCK>, BLOCK, 0);
@@ -405,19 +407,21 @@ static cudaError_t launch_fused(const BatchArgs& b, int stage, int bps, int sms,
             return e != cudaSuccess ? e : cudaErrorInvalidConfiguration;
         }
     }
-    // Two grids' worth of blocks: a block that ends early makes room for one
-    // whose share was cut half as large. Eight cases of 14k-56k cells, us a step:
-    // one grid 123, two 90, four 94 (256 threads), 108, 84, 88 (128 threads).
-    const int per = bps > 0 ? std::min(bps, fit) : fit;
-    launch_kernel_pdl(stage > 0, k_batch_fused<BLOCK>, (unsigned)(2 * per * sms), BLOCK, st, b, stage);
+    // Up to 32 grids' worth of blocks: one that ends early makes room for
+    // another, and few tiles a block leave its warps out of step. At 128 threads,
+    // us a step with two, eight and 32 grids: 2.5M cells 850, 698, 706; 9.7M cells
+    // with eight and 32: 2806, 2536. Below 230k cells there is a tile a block.
+    const int per = p.blocksPerSm > 0 ? std::min(p.blocksPerSm, fit) : fit;
+    launch_kernel_pdl(stage > 0, k_batch_fused<BLOCK>, (unsigned)std::min(p.tiles[3], 32 * per * p.sms), BLOCK, st, b,
+                      stage);
     return cudaGetLastError();
 }
 
-cudaError_t launch_batch_fused(const BatchArgs& b, int stage, int block, int bps, int sms, cudaStream_t st) {
+cudaError_t launch_batch_fused(const BatchArgs& b, int stage, int block, const PhasedShape& p, cudaStream_t st) {
     switch (block) {
-        case 128: return launch_fused<128>(b, stage, bps, sms, st);
-        case 512: return launch_fused<512>(b, stage, bps, sms, st);
-        default: return launch_fused<256>(b, stage, bps, sms, st);
+        case 128: return launch_fused<128>(b, stage, p, st);
+        case 512: return launch_fused<512>(b, stage, p, st);
+        default: return launch_fused<256>(b, stage, p, st);
     }
 }
 

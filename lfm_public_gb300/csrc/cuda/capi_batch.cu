@@ -124,19 +124,12 @@ void dropGraphs(lfm_batch* b) {
 int rebuildTiles(lfm_batch* b) {
     // a step whose cases are all fusable and have current primitives is fused
     bool lean = (b->untuned || !b->tune.phased) && b->barrierExtra == 0, plain = true;
-    int64_t cells = 0;
     for (const Slot& sl : b->slots)
         if (sl.used) {
             lean = lean && sl.fusable && sl.primsValid;
             plain = plain && sl.plain;
-            cells += sl.nc;
         }
-    // untuned, 128 threads, but 256 for fused steps beyond L2's reach. Us a step,
-    // 128 / 256 threads, GB300: fused 0.22M cells 88 / 100, 0.84M 338 / 328,
-    // 2.5M 932 / 845, 9.1M 3097 / 2768; by phases, 0.75M cells 2D and 3D 1084 /
-    // 1242, 0.31M viscous 2D 335 / 384.
-    const int block = lean && b->untuned && cells > (1 << 21) ? 256 : b->tune.block;
-    const int tileSize = block * b->tune.items_per_thread;
+    const int tileSize = b->tune.block * b->tune.items_per_thread;
     std::vector<BatchTile> tl[kBatchPhases];
     for (int s = 0; s < (int)b->slots.size(); ++s) {
         const Slot& sl = b->slots[(size_t)s];
@@ -169,11 +162,10 @@ int rebuildTiles(lfm_batch* b) {
     // the host vectors die here: wait for the copies out of them
     LFM_CUDA(cudaStreamSynchronize(b->stream));
     const int variant = currentVariant(b);
-    // a phased step's grids follow the tiles
-    bool changed = realloc || variant != b->variant || block != b->block || plain != b->plain;
-    b->block = block;
+    // a phased or fused step's grids follow the tiles
+    bool changed = realloc || variant != b->variant || plain != b->plain;
     for (int ph = 0; ph < kBatchPhases; ++ph) {
-        changed = changed || (b->tune.phased && n[ph] != b->nTiles[ph]);
+        changed = changed || ((b->tune.phased || lean) && n[ph] != b->nTiles[ph]);
         b->nTiles[ph] = n[ph];
     }
     if (changed)
@@ -207,8 +199,7 @@ int captureStep(lfm_batch* b, bool cooperative, cudaGraphExec_t* out) {
     LFM_CUDA(cudaStreamBeginCapture(b->stream, cudaStreamCaptureModeThreadLocal));
     cudaError_t le = cudaMemsetAsync(b->dCtl, 0, sizeof(BatchCtl), b->stream);
     for (int k = 0; k < b->rkOrder && le == cudaSuccess; ++k)
-        le = b->lean          ? lfm::dev::launch_batch_fused(args, k, b->block, b->tune.blocks_per_sm, b->sms,
-                                                             b->stream)
+        le = b->lean          ? lfm::dev::launch_batch_fused(args, k, b->tune.block, shape, b->stream)
              : b->tune.phased ? lfm::dev::launch_batch_phased(args, k, b->tune.block, b->variant, shape, b->stream)
                          : lfm::dev::launch_batch_stage(args, k, b->tune.block, b->variant, b->grid, cooperative,
                                                         b->stream);
