@@ -104,18 +104,18 @@ WORKLOAD_DESC = {
 
 
 # DRAM bytes (read + write) of one launch of the dominant kernel, from one ncu
-# capture of this bench's own command (cold L2: ncu flushes the caches before
+# capture of an RK stage of the same case (cold L2: ncu flushes the caches before
 # each captured launch). Keyed by (workload, precision, kernel).
 DRAM_TRAFFIC = {
-    ("cylinder2d", "fp32", "k_update"): 42937856 + 190976,
-    ("cylinder2d", "fp32", "k_flux"): 48100000 + 670000,
+    ("cylinder2d", "fp32", "k_update"): 41364992 + 6144,
+    ("cylinder2d", "fp32", "k_flux"): 47312128 + 81408,
     # the 384x256x96 wake is too large for a full capture: its figure is the
     # 192x128x48 capture
     # scaled by the cells (x8), the traffic being at the algorithmic bytes,
     # which grow in proportion
-    ("cylinder3d_small", "fp32", "k_flux"): 270532096 + 54157824,
-    ("cylinder3d", "fp32", "k_flux"): 8 * (270532096 + 54157824),
-    ("cylinder2d", "fp64", "k_flux"): 95838720 + 8762112,
+    ("cylinder3d_small", "fp32", "k_flux"): 263294720 + 55037184,
+    ("cylinder3d", "fp32", "k_flux"): 8 * (263294720 + 55037184),
+    ("cylinder2d", "fp64", "k_flux"): 152877056 + 13607168,
 }
 
 # FP64 pipe thread-instructions per cell of one launch of each kernel of the
@@ -124,7 +124,7 @@ DRAM_TRAFFIC = {
 # cells) on the 768x512 cylinder, M1, viscous; the update also derives the next
 # stage's primitives and boundary ghosts (no preparation kernel).
 FP64_INST_PER_CELL = {
-    "cylinder2d": {"k_prep": 0.0, "k_grad": 0.0, "k_vis": 45.00, "k_flux": 156.22, "k_update": 42.67},
+    "cylinder2d": {"k_prep": 0.0, "k_grad": 0.0, "k_vis": 43.00, "k_flux": 122.17, "k_update": 36.39},
 }
 # FP64 pipe instruction rate: the measured DFMA rate (FP64_PEAK_TFLOPS counts
 # an FMA as two operations) in instructions per second.
