@@ -23,7 +23,7 @@ geometry) with its own value, e2e, roofline and speed-up over FP64;
 FP64 state after --accuracy-steps time steps (all cells and 72 probes at
 r = 50 D); ``wake3d`` -- the 3D cylinder wake (384x256x96, 9.4M hex cells)
 device-timed in both precisions, the HBM-bound case; ``batch64`` -- the
-64-case batched sweep (15.5M cells, one persistent kernel per RK stage) with
+64-case batched sweep (15.5M cells, one fused kernel per RK stage) with
 its roofline, e2e and the plain FP64 path on the same cases; ``serve`` -- a
 30-second Poisson stream of solve requests into the request server (p50 /
 p99, throughput, against the same stream served one request at a time on the
@@ -705,7 +705,7 @@ def run_gpu(args):
 
 BATCH_DESC = ("64-case batched sweep: quad grids and jittered triangulations of [-10,10]^2, cells log-uniform "
               "16k-1M, isentropic vortex beta U(1,5), M U(0.1,0.6), M1/M2 at random, rkOrder 5, seed 20261203; "
-              "FP32-bulk, one persistent kernel per RK stage")
+              "FP32-bulk, one fused kernel per RK stage")
 
 
 def _build_sweep(n_cases: int, seed: int):

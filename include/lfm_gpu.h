@@ -493,7 +493,7 @@ int lfm_batch_autotune(lfm_batch* b, int trial_steps, lfm_batch_tuning* chosen);
  * Reports barrier failures; numeric state is left to lfm_batch_sync and
  * lfm_batch_case_status. */
 int lfm_batch_bench(lfm_batch* b, int nsteps, size_t flush_bytes, float* ms);
-/* Kernel launches per time step (one per RK stage). */
+/* Kernel launches per time step: per RK stage one, or one per phase (lfm_batch_tuning.phased). */
 int lfm_batch_launches_per_step(const lfm_batch* b, int* launches);
 /* Failure-detection test aid, no reference counterpart: every grid barrier of
  * the persistent stage kernel then waits for extra_arrivals blocks more than

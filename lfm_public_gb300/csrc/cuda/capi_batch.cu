@@ -857,6 +857,14 @@ extern "C" int lfm_batch_autotune(lfm_batch* b, int trial_steps, lfm_batch_tunin
 
 extern "C" int lfm_batch_launches_per_step(const lfm_batch* b, int* launches) {
     if (!b || !launches) return lfm::setError(LFM_ERR_INVALID, "null argument");
-    *launches = b->rkOrder;
+    // phased stages: [grad + vis] | flux | update (a preparation phase runs in the
+    // first step after restored states only); fused and persistent ones: one
+    bool fused = b->untuned && b->barrierExtra == 0, gradVis = false;
+    for (const Slot& sl : b->slots)
+        if (sl.used) {
+            fused = fused && sl.fusable;
+            gradVis = gradVis || sl.needGradVis;
+        }
+    *launches = b->rkOrder * (b->tune.phased && !fused ? 2 + (gradVis ? 1 : 0) : 1);
     return LFM_OK;
 }

@@ -46,3 +46,20 @@ def test_plain_and_general_phases_give_the_same_bits(dims, shape):
     for s, h, c in zip(slots, chs, cs):
         assert np.array_equal(b.get_state(s), _single(h, 7, c.delta_t)), c.name
     b.close()
+
+
+def test_launches_per_step():
+    """Fused stages are one kernel, phased ones one per phase, persistent ones one."""
+    vortex, viscous = cases.vortex_case(n=9, solver=0), _cyl(12, 8, 1, 0)
+    vh, ch = N.CaseHandle.from_case(vortex), N.CaseHandle.from_case(viscous)
+    b = N.Batch(arena_bytes=16 << 20, max_cases=4)
+    b.add(vh, vortex.delta_t)
+    assert b.launches_per_step() == 5
+    s = b.add(ch, viscous.delta_t)
+    assert b.launches_per_step() == 15
+    b.remove(s)
+    b.set_tuning(128, 1, 0, 1, 1)
+    assert b.launches_per_step() == 10
+    b.set_tuning(128, 1, 0, 1, 0)
+    assert b.launches_per_step() == 5
+    b.close()
