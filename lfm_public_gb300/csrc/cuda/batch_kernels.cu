@@ -226,7 +226,7 @@ __device__ __forceinline__ void fused_item(const BatchCase& bc, int stage, int i
 // A stage of a batch whose cases can all do flux and update at once
 // (CaseLayout::fusable) and have current primitives: one phase, no barrier, so stages follow one another as programmatic dependents (each loads
 // its first tile's case before it waits for the stage before).
-// 768 threads per SM (80 registers, 28 bytes spilled) beat 512 without spills
+// 768 threads per SM (80 registers, 56 bytes spilled) beat 512 without spills
 // and 1024 (64, 120 bytes): 143, 150 and 149 us a step of eight cases.
 template <int BLOCK>
 __global__ void __launch_bounds__(BLOCK, BLOCK > 256 ? 1 : 768 / BLOCK) k_batch_fused(const __grid_constant__ BatchArgs b,
