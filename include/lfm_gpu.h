@@ -414,6 +414,12 @@ int lfm_tiles_stats(const lfm_solver_desc* d, int tile_cells, int max_local, int
 int lfm_selftest_fp_convert(int64_t n, const uint32_t* f32_bits, const uint64_t* f64_bits, uint64_t* f64_of_f32,
                             uint32_t* f32_of_f64);
 
+/* Diagnostic: whether state transfers have kernels read and write the host
+ * memory [p, p + bytes) where it lies (1), or go through the copy calls (0):
+ * the former for page-locked memory that is aligned for doubles and page-locked
+ * to its end. Nothing at p is accessed. */
+int lfm_selftest_kernel_range(const void* p, size_t bytes);
+
 /* ---- batch engine: many cases, a few kernels per RK stage -----------------
  *
  * No single reference call corresponds: the reference advances one case per

@@ -196,6 +196,7 @@ def load_library(path: str = LIB_PATH) -> C.CDLL:
         "lfm_partitioned_get_state": ([vp, C.c_int, _dp], C.c_int),
         "lfm_partitioned_step": ([vp, C.c_int, C.c_double], C.c_int),
         "lfm_partitioned_sync": ([vp], C.c_int),
+        "lfm_selftest_kernel_range": ([vp, C.c_size_t], C.c_int),
         "lfm_selftest_fp_convert": ([C.c_int64, C.POINTER(C.c_uint32), C.POINTER(C.c_uint64), C.POINTER(C.c_uint64),
                                      C.POINTER(C.c_uint32)], C.c_int),
         "lfm_batch_create": ([C.POINTER(BatchOpts), C.POINTER(vp)], C.c_int),

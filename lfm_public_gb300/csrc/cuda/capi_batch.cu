@@ -535,7 +535,7 @@ namespace {
 int enqueueBatchSet(lfm_batch* b, int slot, const double* q) {
     Slot& sl = b->slots[(size_t)slot];
     const size_t bytes = (size_t)sl.nq * sl.nc * sizeof(double);
-    const double* direct = lfm::dev::kernel_address(q);
+    const double* direct = lfm::dev::kernel_address(q, bytes);
     if (!direct) {
         int rc = ensureStage(b, bytes);
         if (rc) return rc;
@@ -553,7 +553,7 @@ int enqueueBatchSet(lfm_batch* b, int slot, const double* q) {
 int enqueueBatchGet(lfm_batch* b, int slot, double* q) {
     const Slot& sl = b->slots[(size_t)slot];
     const size_t bytes = (size_t)sl.nq * sl.nc * sizeof(double);
-    double* direct = lfm::dev::kernel_address(q);
+    double* direct = lfm::dev::kernel_address(q, bytes);
     if (!direct) {
         int rc = ensureStage(b, bytes);
         if (rc) return rc;
@@ -589,10 +589,11 @@ int enqueueBatchStates(lfm_batch* b, int n, const int* slots, const double* cons
     for (int i = 0; i < n; ++i) {
         if (!q[i]) continue;
         const Slot& sl = b->slots[(size_t)slots[i]];
-        double* direct = lfm::dev::kernel_address(q[i]);
+        const size_t bytes = (size_t)sl.nq * sl.nc * sizeof(double);
+        double* direct = lfm::dev::kernel_address(q[i], bytes);
         if (!direct) {
             staged.push_back(i);
-            most = std::max(most, (size_t)sl.nq * sl.nc * sizeof(double));
+            most = std::max(most, bytes);
             continue;
         }
         m.slot[count] = slots[i];

@@ -103,10 +103,11 @@ struct lfm_solver {
     int* flagHost = nullptr;
     // lfm_solver_advance between page-locked host states as one graph (copy
     // in, conversion, primitives, steps, conversion, copy out, flag), kept
-    // for the pointers and step count it was captured with
+    // for the pointers (the host's and those its kernels use) and step count it
+    // was captured with
     cudaGraphExec_t advGraph = nullptr;
-    const double* advIn = nullptr;
-    double* advOut = nullptr;
+    const double *advIn = nullptr, *advInAt = nullptr;
+    double *advOut = nullptr, *advOutAt = nullptr;
     int advSteps = 0;
 };
 
@@ -838,11 +839,11 @@ int enqueueSetState(lfm_solver* s, const double* q) {
     // of the ghosts that the update keeps, and clears the non-finite flag: the
     // per-stage preparation covers the other ghosts and halos
     const size_t nc = (size_t)s->nc;
-    const double* direct = lfm::dev::kernel_address(q);
+    const size_t bytes = (size_t)s->nq * nc * sizeof(double);
+    const double* direct = lfm::dev::kernel_address(q, bytes);
     if (s->precision == LFM_FP32_BULK) {   // stored as q - q_ref
         if (!direct)
-            LFM_CUDA(cudaMemcpyAsync(s->stage, q, (size_t)s->nq * nc * sizeof(double), cudaMemcpyHostToDevice,
-                                     s->stream));
+            LFM_CUDA(cudaMemcpyAsync(s->stage, q, bytes, cudaMemcpyHostToDevice, s->stream));
         lfm::dev::launch_set_state32(s->a32, direct ? direct : s->stage, s->nc, s->stream);
     } else {
         if (!direct)   // rows of nc values into rows of nt
@@ -862,12 +863,12 @@ int enqueueGetState(lfm_solver* s, double* q) {
     if (s->precision == LFM_FP32_BULK) {   // stored as q - q_ref
         lfm::dev::QOffset qo;
         for (int v = 0; v < 5; ++v) qo.v[v] = s->qRef[v];
-        double* direct = lfm::dev::kernel_address(q);
+        const size_t bytes = (size_t)s->nq * s->nc * sizeof(double);
+        double* direct = lfm::dev::kernel_address(q, bytes);
         lfm::dev::launch_offset_rows(direct ? direct : s->stage, s->nc, s->q, s->nt, s->nc, s->nq, qo, 1.0, s->stream);
         LFM_CUDA(cudaGetLastError());
         if (direct) return LFM_OK;
-        LFM_CUDA(cudaMemcpyAsync(q, s->stage, (size_t)s->nq * s->nc * sizeof(double), cudaMemcpyDeviceToHost,
-                                 s->stream));
+        LFM_CUDA(cudaMemcpyAsync(q, s->stage, bytes, cudaMemcpyDeviceToHost, s->stream));
     } else {
         LFM_CUDA(cudaMemcpy2DAsync(q, (size_t)s->nc * sizeof(double), s->q, (size_t)s->nt * sizeof(double),
                                    (size_t)s->nc * sizeof(double), (size_t)s->nq, cudaMemcpyDeviceToHost,
@@ -900,9 +901,11 @@ namespace {
 
 // The whole advance between page-locked host states as one graph launch
 // (device work only; the host-side state flags are set as the enqueued path
-// leaves them). Captured once per (q_in, q_out, nsteps).
-int advanceGraph(lfm_solver* s, const double* qIn, int nsteps, double dt, double* qOut) {
-    if (!(s->advGraph && s->advIn == qIn && s->advOut == qOut && s->advSteps == nsteps)) {
+// leaves them). Captured once per (q_in, q_out, their kernel addresses inAt and
+// outAt, nsteps).
+int advanceGraph(lfm_solver* s, const double* qIn, const double* inAt, int nsteps, double dt, double* qOut, double* outAt) {
+    if (!(s->advGraph && s->advIn == qIn && s->advOut == qOut && s->advInAt == inAt && s->advOutAt == outAt &&
+          s->advSteps == nsteps)) {
         if (s->advGraph) cudaGraphExecDestroy(s->advGraph);
         s->advGraph = nullptr;
         cudaGraph_t g = nullptr;
@@ -929,6 +932,8 @@ int advanceGraph(lfm_solver* s, const double* qIn, int nsteps, double dt, double
         if (e != cudaSuccess) return cudaFail(e, "cudaGraphInstantiate");
         s->advIn = qIn;
         s->advOut = qOut;
+        s->advInAt = inAt;
+        s->advOutAt = outAt;
         s->advSteps = nsteps;
     }
     const int rc = setStep(s, dt);
@@ -951,8 +956,12 @@ extern "C" int lfm_solver_advance(lfm_solver* s, const double* q_in, int nsteps,
     if (!s || nsteps < 0) return lfm::setError(LFM_ERR_INVALID, "bad argument");
     LFM_CUDA(cudaSetDevice(s->device));
     int rc = LFM_OK;
-    if (q_in && q_out && nsteps > 0 && s->rkOrder > 0 && lfm::dev::kernel_address(q_in) && lfm::dev::kernel_address(q_out))
-        return advanceGraph(s, q_in, nsteps, dt, q_out);
+    const size_t bytes = (size_t)s->nq * s->nc * sizeof(double);
+    if (q_in && q_out && nsteps > 0 && s->rkOrder > 0) {
+        const double* in = lfm::dev::kernel_address(q_in, bytes);
+        double* out = in ? lfm::dev::kernel_address(q_out, bytes) : nullptr;
+        if (in && out) return advanceGraph(s, q_in, in, nsteps, dt, q_out, out);
+    }
     if (q_in && (rc = enqueueSetState(s, q_in))) return rc;
     if (nsteps > 0 && (rc = lfm_solver_step(s, nsteps, dt))) return rc;
     if (q_out && (rc = enqueueGetState(s, q_out))) return rc;

@@ -1,4 +1,9 @@
 // Device kernels of the explicit finite-volume time step (see solver_kernels.cuh).
+#include <cuda.h>
+
+#include <cstdint>
+
+#include "lfm_gpu.h"
 #include "solver_device.cuh"
 #include "solver_launch.h"
 
@@ -619,13 +624,31 @@ void launch_prep_residual64(const Args<double>& a, const double* q, int64_t stri
     else k_prep_residual64<3><<<nb, 128, 0, st>>>(a, q, stride, vRows, gradRows, cellGrad);
 }
 
-double* kernel_address(const double* p) {
+double* kernel_address(const double* p, size_t bytes) {
+    // a copy engine takes any address, a kernel's loads only aligned ones
+    if (reinterpret_cast<uintptr_t>(p) % alignof(double) != 0) return nullptr;
     cudaPointerAttributes at{};
     if (cudaPointerGetAttributes(&at, p) != cudaSuccess) {
         cudaGetLastError();
         return nullptr;
     }
-    return at.type == cudaMemoryTypeHost ? static_cast<double*>(at.devicePointer) : nullptr;
+    if (at.type != cudaMemoryTypeHost || !at.devicePointer) return nullptr;
+    // what is page-locked and mapped ends with its allocation or registration
+    static const auto attribute = [] {
+        void* f = nullptr;
+        cudaDriverEntryPointQueryResult found;
+        if (cudaGetDriverEntryPointByVersion("cuPointerGetAttribute", &f, 12000, cudaEnableDefault, &found) != cudaSuccess)
+            cudaGetLastError();
+        return reinterpret_cast<CUresult (*)(void*, CUpointer_attribute, CUdeviceptr)>(f);
+    }();
+    const CUdeviceptr d = reinterpret_cast<CUdeviceptr>(at.devicePointer);
+    CUdeviceptr start = 0;
+    size_t size = 0;
+    if (!attribute || attribute(&start, CU_POINTER_ATTRIBUTE_RANGE_START_ADDR, d) != CUDA_SUCCESS ||
+        attribute(&size, CU_POINTER_ATTRIBUTE_RANGE_SIZE, d) != CUDA_SUCCESS)
+        return nullptr;
+    if (d < start || d - start > size || bytes > size - (size_t)(d - start)) return nullptr;
+    return static_cast<double*>(at.devicePointer);
 }
 
 // ---------------------------------------------------------------------------
@@ -843,3 +866,7 @@ void launch_halo_gather_cells(float* dst, int first, int words, int nh, const in
 
 }  // namespace dev
 }  // namespace lfm
+
+extern "C" int lfm_selftest_kernel_range(const void* p, size_t bytes) {
+    return lfm::dev::kernel_address(static_cast<const double*>(p), bytes) ? 1 : 0;
+}

@@ -102,12 +102,14 @@ void launch_prep_residual64(const Args<double>& a, const double* q, int64_t stri
                             cudaStream_t st);
 void launch_prep_residual32(const Args<float>& a, const double* q, int64_t stride, int vWords, int gradWords, int cellGrad,
                             cudaStream_t st);
-// The address at which kernels read and write page-locked host memory p, or null
-// for other memory. A state in page-locked memory is read and written by the
+// The address at which kernels read and write the page-locked host memory
+// [p, p + bytes), or null for other memory, for a p that is not aligned for
+// doubles and for a range that is not page-locked to its end: the copy calls serve
+// those. A state in page-locked memory is read and written by the
 // kernels that convert it: the C2C link moves it at the copy engines' rate, and
 // the stream does not change between engine and kernels, which costs a batch
 // of eight cases about 30 us a case.
-double* kernel_address(const double* p);
+double* kernel_address(const double* p, size_t bytes);
 // A new FP64 state from an absolute one (or from the stored rows, stride nt).
 void launch_set_state64(const Args<double>& a, const double* q, int64_t stride, cudaStream_t st);
 // A new FP32-bulk state from an absolute one: q', the cells' primitives and
