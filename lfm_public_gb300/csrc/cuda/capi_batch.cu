@@ -10,6 +10,7 @@
 // whose kernels read the case table and tile lists from device memory, so
 // admissions and removals between steps only rewrite those tables.
 #include <algorithm>
+#include <cstdint>
 #include <cstring>
 #include <map>
 #include <string>
@@ -573,11 +574,22 @@ namespace {
 // The states of several cases in or out (null entries skipped): those in
 // page-locked memory by one kernel per kBatchStates cases, which copies all at
 // once; the others one after another through the staging buffer, sized before
-// anything is enqueued.
+// anything is enqueued. The kernel's entries run side by side, so it is launched
+// before an entry that writes what one of them writes (a slot given a second
+// state, a host range read into twice): the last entry wins, as in the separate
+// calls.
 int enqueueBatchStates(lfm_batch* b, int n, const int* slots, const double* const* q, bool set) {
+    auto bytesOf = [&](int i) {
+        const Slot& sl = b->slots[(size_t)slots[i]];
+        return (size_t)sl.nq * sl.nc * sizeof(double);
+    };
     size_t most = 0;
-    std::vector<int> staged;
+    for (int i = 0; i < n; ++i)
+        if (q[i] && !lfm::dev::kernel_address(q[i], bytesOf(i))) most = std::max(most, bytesOf(i));
+    int rc;
+    if (most && (rc = ensureStage(b, most))) return rc;
     lfm::dev::BatchStates m{};
+    int entry[lfm::dev::kBatchStates];
     int count = 0, maxCells = 0;
     auto flush = [&]() -> int {
         if (count > 0)
@@ -585,28 +597,30 @@ int enqueueBatchStates(lfm_batch* b, int n, const int* slots, const double* cons
         count = maxCells = 0;
         return LFM_OK;
     };
-    int rc;
+    auto again = [&](int i) {   // writes what a pending entry writes
+        const auto at = [&](int k) { return reinterpret_cast<uintptr_t>(q[k]); };
+        for (int k = 0; k < count; ++k) {
+            const int e = entry[k];
+            if (set ? slots[e] == slots[i] : at(e) < at(i) + bytesOf(i) && at(i) < at(e) + bytesOf(e)) return true;
+        }
+        return false;
+    };
     for (int i = 0; i < n; ++i) {
         if (!q[i]) continue;
-        const Slot& sl = b->slots[(size_t)slots[i]];
-        const size_t bytes = (size_t)sl.nq * sl.nc * sizeof(double);
-        double* direct = lfm::dev::kernel_address(q[i], bytes);
+        if (again(i) && (rc = flush())) return rc;
+        double* direct = lfm::dev::kernel_address(q[i], bytesOf(i));
         if (!direct) {
-            staged.push_back(i);
-            most = std::max(most, bytes);
+            rc = set ? enqueueBatchSet(b, slots[i], q[i]) : enqueueBatchGet(b, slots[i], const_cast<double*>(q[i]));
+            if (rc) return rc;
             continue;
         }
         m.slot[count] = slots[i];
         m.q[count] = direct;
-        maxCells = std::max(maxCells, sl.nc);
+        entry[count] = i;
+        maxCells = std::max(maxCells, b->slots[(size_t)slots[i]].nc);
         if (++count == lfm::dev::kBatchStates && (rc = flush())) return rc;
     }
-    if ((rc = flush())) return rc;
-    if (!staged.empty() && (rc = ensureStage(b, most))) return rc;
-    for (int i : staged)
-        if ((rc = set ? enqueueBatchSet(b, slots[i], q[i]) : enqueueBatchGet(b, slots[i], const_cast<double*>(q[i]))))
-            return rc;
-    return LFM_OK;
+    return flush();
 }
 
 }  // namespace
