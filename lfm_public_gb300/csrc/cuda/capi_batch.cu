@@ -124,12 +124,15 @@ void dropGraphs(lfm_batch* b) {
 
 int rebuildTiles(lfm_batch* b) {
     // a step whose cases are all fusable and have current primitives is fused
-    bool lean = (b->untuned || !b->tune.phased) && b->barrierExtra == 0, plain = true;
+    // (a batch without cases has none to fuse)
+    bool any = false, lean = (b->untuned || !b->tune.phased) && b->barrierExtra == 0, plain = true;
     for (const Slot& sl : b->slots)
         if (sl.used) {
+            any = true;
             lean = lean && sl.fusable && sl.primsValid;
             plain = plain && sl.plain;
         }
+    lean = lean && any;
     const int tileSize = b->tune.block * b->tune.items_per_thread;
     std::vector<BatchTile> tl[kBatchPhases];
     for (int s = 0; s < (int)b->slots.size(); ++s) {
