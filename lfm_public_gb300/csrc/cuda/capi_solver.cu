@@ -1855,6 +1855,7 @@ extern "C" int lfm_solver_autotune(lfm_solver* s, double dt, int trial_steps, si
     // state is q - q_ref: a round trip through the absolute state would not
     // keep its bits)
     LFM_CUDA(cudaStreamSynchronize(s->stream));
+    untile(s);   // the current primitives in a32.prim, which is what is copied
     int rc = ensurePrims(s);
     if (rc) return rc;
     const size_t qBytes = (size_t)s->nq * (size_t)s->nt * sizeof(double);
