@@ -506,8 +506,9 @@ int lfm_batch_launches_per_step(const lfm_batch* b, int* launches);
  * its grid has (0: normal operation). With extra_arrivals > 0 no barrier is
  * ever reached: each block gives up after its bounded wait (about a second),
  * the kernel returns, and lfm_batch_sync reports LFM_ERR_CUDA; the batch's
- * case states are then undefined. Affects the persistent launch mode only
- * (lfm_batch_tuning.phased = 0). */
+ * case states are then undefined. A batch whose launch shape was not chosen
+ * (lfm_batch_set_tuning, lfm_batch_autotune) runs the persistent kernel
+ * meanwhile; one that was given phased launches has no barriers to affect. */
 int lfm_batch_debug_barrier(lfm_batch* b, int extra_arrivals);
 
 /* ---- request server: continuous batching of solve requests ---------------

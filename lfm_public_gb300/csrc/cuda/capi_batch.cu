@@ -122,6 +122,11 @@ void dropGraphs(lfm_batch* b) {
         }
 }
 
+// Whether a stage that is not fused runs one kernel per phase. Barrier arrivals
+// beyond the grid's (lfm_batch_debug_barrier) need the kernel that has barriers,
+// unless the phased launches were asked for.
+bool phasedStages(const lfm_batch* b) { return b->tune.phased && !(b->untuned && b->barrierExtra > 0); }
+
 int rebuildTiles(lfm_batch* b) {
     // a step whose cases are all fusable and have current primitives is fused
     // (a batch without cases has none to fuse)
@@ -169,7 +174,7 @@ int rebuildTiles(lfm_batch* b) {
     // a phased or fused step's grids follow the tiles
     bool changed = realloc || variant != b->variant || plain != b->plain;
     for (int ph = 0; ph < kBatchPhases; ++ph) {
-        changed = changed || ((b->tune.phased || lean) && n[ph] != b->nTiles[ph]);
+        changed = changed || ((phasedStages(b) || lean) && n[ph] != b->nTiles[ph]);
         b->nTiles[ph] = n[ph];
     }
     if (changed)
@@ -203,10 +208,10 @@ int captureStep(lfm_batch* b, bool cooperative, cudaGraphExec_t* out) {
     LFM_CUDA(cudaStreamBeginCapture(b->stream, cudaStreamCaptureModeThreadLocal));
     cudaError_t le = cudaMemsetAsync(b->dCtl, 0, sizeof(BatchCtl), b->stream);
     for (int k = 0; k < b->rkOrder && le == cudaSuccess; ++k)
-        le = b->lean          ? lfm::dev::launch_batch_fused(args, k, b->tune.block, shape, b->stream)
-             : b->tune.phased ? lfm::dev::launch_batch_phased(args, k, b->tune.block, b->variant, shape, b->stream)
-                         : lfm::dev::launch_batch_stage(args, k, b->tune.block, b->variant, b->grid, cooperative,
-                                                        b->stream);
+        le = b->lean           ? lfm::dev::launch_batch_fused(args, k, b->tune.block, shape, b->stream)
+             : phasedStages(b) ? lfm::dev::launch_batch_phased(args, k, b->tune.block, b->variant, shape, b->stream)
+                               : lfm::dev::launch_batch_stage(args, k, b->tune.block, b->variant, b->grid, cooperative,
+                                                              b->stream);
     cudaError_t e = cudaStreamEndCapture(b->stream, &g);
     if (le != cudaSuccess || e != cudaSuccess) {
         if (g) cudaGraphDestroy(g);
@@ -246,7 +251,7 @@ int ensureGraph(lfm_batch* b) {
     bool& stale = b->graphStale[b->lean ? 1 : 0][b->parity];
     if (*graph && !stale) return LFM_OK;
     stale = true;   // until its capture has succeeded
-    if (b->tune.phased || b->lean) {   // no co-residency needed
+    if (phasedStages(b) || b->lean) {   // no co-residency needed
         const int rc = captureStep(b, false, graph);
         if (rc == LFM_OK) stale = false;
         return rc;
@@ -883,6 +888,6 @@ extern "C" int lfm_batch_launches_per_step(const lfm_batch* b, int* launches) {
             fused = fused && sl.fusable;
             gradVis = gradVis || sl.needGradVis;
         }
-    *launches = b->rkOrder * (b->tune.phased && !fused ? 2 + (gradVis ? 1 : 0) : 1);
+    *launches = b->rkOrder * (phasedStages(b) && !fused ? 2 + (gradVis ? 1 : 0) : 1);
     return LFM_OK;
 }
