@@ -419,25 +419,26 @@ __device__ __forceinline__ CellGhosts cell_ghosts(const Args<T>& a, int c) {
 }
 
 // f(j, kind) for each of them: the first two, then (a cell with more boundary
-// faces) the others in entry order.
+// faces) the others in entry order, told by their place among the cell's ghost
+// entries -- not by their numbers: faces may share a ghost.
 template <typename T, int D, class F>
 __device__ __forceinline__ void for_ghosts(const Args<T>& a, int c, const CellGhosts& g, F f) {
-    int left = g.count;
+    int e = 0, seen = 0;   // entries passed, ghosts among them
 #pragma unroll 1
-    for (int k = 0; left > 0; ++k) {
+    for (int k = 0; k < g.count; ++k) {
         int j = k == 0 ? g.j[0] : g.j[1], kind = k == 0 ? g.kind[0] : g.kind[1];
         if (k >= 2) {
-            j = entry_cell<T, D>(a, c, k - 2);
-            if (j < a.nc || j >= a.nc + a.ng || j == g.j[0] || j == g.j[1]) continue;
+            do {
+                j = entry_cell<T, D>(a, c, e++);
+                if (j >= a.nc && j < a.nc + a.ng) ++seen;
+            } while (j >= 0 && seen <= k);
+            if (j < 0) return;   // past the last entry
             kind = a.gKind[j - a.nc];
         }
         f(j, kind);
-        --left;
     }
 }
 
-// FP64 path: the states and primitives of the boundary ghosts of cell c from
-// its conservative state qc (those k_prep computes for the next stage).
 // FP64 path: state and primitives of ghost g into the stored arrays.
 template <int D>
 __device__ __forceinline__ void ghost64(const Args<double>& a, int g, int kind, const GhostIn<D>& in) {
@@ -453,6 +454,8 @@ __device__ __forceinline__ void ghost64(const Args<double>& a, int g, int kind, 
     if (a.primC) a.prim[(D + 2) * nt + t] = sqrt(a.gamma * o.R);
 }
 
+// FP64 path: the states and primitives of the boundary ghosts of cell c from
+// its conservative state qc (those k_prep computes for the next stage).
 template <int D>
 __device__ __forceinline__ void ghosts_of64(const Args<double>& a, int c, const CellGhosts& g, const double* qc) {
     const GhostIn<D> in = ghost_in<double, D>(a, qc);
