@@ -93,9 +93,15 @@ struct CaseLayout {
         prim = add((size_t)lfm::dev::primRows<float>(d->dim) * nt * 4);
         // As in the single-case solver, evaluating each face twice pays where
         // the flux is short (2D inviscid M1 / M2): a stage then is one phase
-        // without a grid barrier. The second primitive buffer takes the space
-        // the second copy of the face lists took.
-        fusable = D == 2 && !lfm::setup::needVis(d) && !ausm && lfm::setup::ellFits(d);
+        // without a grid barrier. The second primitive buffer takes the space that
+        // rows of single values and a second copy of the face lists would: callers
+        // size arenas by that footprint, and no case may outgrow it (one of mostly
+        // isolated cells would, with far more ghosts than cells).
+        const size_t one = roundUp(nf), fours = roundUp(nf * 4), eights = roundUp(nf * 8);
+        const size_t rows = 4 * eights + 5 * fours + one + roundUp(nc * 8) + roundUp((nc + 1) * 4) + 2 * roundUp(ne * 4);
+        const size_t parts = 2 * roundUp(nf * 16) + roundUp(nc * 16);
+        const size_t second = roundUp((size_t)lfm::dev::primRows<float>(d->dim) * nt * 4);
+        fusable = D == 2 && !lfm::setup::needVis(d) && !ausm && lfm::setup::ellFits(d) && parts + second <= rows;
         prim1 = fusable ? add((size_t)lfm::dev::primRows<float>(d->dim) * nt * 4) : npos();
         V = lfm::setup::needVis(d) ? add((size_t)lfm::dev::visStride32(d->dim, false) * nt * 4) : npos();
         grad = ausm ? add((size_t)lfm::dev::gradStride32(d->dim) * nt * 4) : npos();
@@ -103,8 +109,9 @@ struct CaseLayout {
         fG0 = add(nf * 16);
         fG1 = add(nf * 16);
         this->d = ausm ? add(D * nf * 4) : npos();
-        dinv = add(nf * 4);
-        dnorm = add(D * nf * 4);
+        // the two-point gradients of viscous boundary faces
+        dinv = d->mu != 0.0 ? add(nf * 4) : npos();
+        dnorm = d->mu != 0.0 ? add(D * nf * 4) : npos();
         fP = D == 3 ? add(nf * 4) : npos();   // 2D: in fG1
         fN = D == 3 ? add(nf * 4) : npos();
         volInv32 = add(nc * 4);

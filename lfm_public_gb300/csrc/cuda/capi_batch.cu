@@ -69,8 +69,10 @@ std::vector<unsigned char> packCase(const lfm_solver_desc* d, const CaseLayout& 
         for (size_t c = 0; c < nc; ++c) row[c] = (d->q0 ? d->q0[v * nc + c] : 0.0) - qRef[v];
     }
     if (L.d != CaseLayout::npos()) conv(L.d, d->d, D * nf);
-    conv(L.dinv, d->dmag_inv, nf);
-    conv(L.dnorm, d->dnorm, D * nf);
+    if (L.dinv != CaseLayout::npos()) {
+        conv(L.dinv, d->dmag_inv, nf);
+        conv(L.dnorm, d->dnorm, D * nf);
+    }
     lfm::setup::DescIndex ix(d);
     for (size_t f = 0; f < nf; ++f) {
         const int n = lfm::setup::flaggedN(d, f);
