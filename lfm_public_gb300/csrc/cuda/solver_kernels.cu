@@ -266,7 +266,11 @@ __global__ void __launch_bounds__(kFaceThreads<D>) k_flux(Args<T> a) {
     }
     const T cRpsi = a.prim[(D + 1) * nt + i], aRpsi = a.prim[(D + 1) * nt + j];
     const T dR = aRpsi - cRpsi;
-    T rhs[NQ];
+    // The convective rhs of a momentum component is -(cm cphi + cp S), the
+    // energy's -(ea eb + ec ed). They are added to the viscous sum last, largest
+    // product last, as one FMA each: the viscous terms then round at their own
+    // size, and a momentum component rounds once at the size of p S.
+    T cm[D], cphi, cp, ea, eb, ec, ed, mass;
 
     if (SCH == kSchemeM1) {
         // One_rk_step_M1's Kurganov-Tadmor flux (src/cfd_v0.cpp:2588-2675)
@@ -293,13 +297,16 @@ __global__ void __launch_bounds__(kFaceThreads<D>) k_flux(Args<T> a) {
             u2 += m[k] * m[k];
         }
         const T phi = mS * rinv;                          // u_f . S
-        const T gh2 = T(2) * (T)a.gh;
-        const T p = rho * Rpsi;
-        rhs[0] = -mS;
+        mass = -mS;
+        cphi = phi;
+        cp = rho * Rpsi;
 #pragma unroll
-        for (int k = 0; k < D; ++k) rhs[k + 1] = -(m[k] * phi + p * S[k]);
-        // mS (gh Rpsi + |u|^2 / 2) with mS Rpsi = phi p and mS |u|^2 = phi |m|^2 / rho
-        rhs[D + 1] = -(T(0.5) * phi) * (gh2 * p + u2 * rinv);
+        for (int k = 0; k < D; ++k) cm[k] = m[k];
+        // mS (gh Rpsi + |u|^2 / 2) with mS |u|^2 = phi |m|^2 / rho
+        ea = T(0.5) * phi;
+        eb = u2 * rinv;
+        ec = mS;
+        ed = (T)a.gh * Rpsi;
     } else {
         // Pirozzoli kinetic-energy-preserving mid-point flux (src/cfd_v0.cpp:1966-2023)
         // on the sums of the two sides: rho u.S = (m_P + m_N).S / 2 and
@@ -346,7 +353,7 @@ __global__ void __launch_bounds__(kFaceThreads<D>) k_flux(Args<T> a) {
             const T ct = pos_part(-cdiv * rsqrt64(cdiv * cdiv + ccurl + T(4e-2)));
             const T nt_ = pos_part(-ndiv * rsqrt64(ndiv * ndiv + ncurl + T(4e-2)));
             const T theta = T(0.5) * (ct + nt_);
-            const T cp = qi[0] * cRpsi, np = qj[0] * aRpsi;   // p = rho R psi
+            const T pi = qi[0] * cRpsi, pj = qj[0] * aRpsi;   // p = rho R psi
             T gri[D], grj[D], gpi[D], gpj[D];
 #pragma unroll
             for (int y = 0; y < D; ++y) {
@@ -357,7 +364,7 @@ __global__ void __launch_bounds__(kFaceThreads<D>) k_flux(Args<T> a) {
             }
             T rhoPos, rhoNeg, pPos, pNeg;
             minmod_pair<D>(qi[0], qj[0], gri, grj, d, w, wN, rhoPos, rhoNeg);
-            minmod_pair<D>(cp, np, gpi, gpj, d, w, wN, pPos, pNeg);
+            minmod_pair<D>(pi, pj, gpi, gpj, d, w, wN, pPos, pNeg);
             const T sc = rcp64(a.smag[f] * cavg);
             const T MPos = unPos * sc, MNeg = unNeg * sc;
             const T Msq = T(0.5) * (MPos * MPos + MNeg * MNeg);
@@ -374,10 +381,14 @@ __global__ void __launch_bounds__(kFaceThreads<D>) k_flux(Args<T> a) {
         }
         const T hphi = T(0.5) * mS2 * rcp64(rho2);   // u_f . S / 2
         const T mS = T(0.5) * mS2;
-        rhs[0] = -mS;
+        mass = -mS;
+        cphi = hphi;
+        cp = pavg;
 #pragma unroll
-        for (int k = 0; k < D; ++k) rhs[k + 1] = -(m2[k] * hphi + pavg * S[k]);
-        rhs[D + 1] = -(T(0.5) * mS) * H2;
+        for (int k = 0; k < D; ++k) cm[k] = m2[k];
+        ea = eb = T(0);
+        ec = T(0.5) * mS;
+        ed = H2;
     }
 
     // Viscous face terms (src/cfd_v0.cpp:2682-2796). With mu == 0 every term
@@ -396,6 +407,9 @@ __global__ void __launch_bounds__(kFaceThreads<D>) k_flux(Args<T> a) {
     // operations less took the flux of the 768 x 512 M1 cylinder from 583 to
     // 459 us a step, of the 97 x 61 x 23 M2 wake from 484 to 390 (GB300).
     const T mu = (T)a.mu;
+    T vis[D], visE = T(0);
+#pragma unroll
+    for (int x = 0; x < D; ++x) vis[x] = T(0);
     if (mu != T(0)) {
         T g[D][D];
         if (!ghost) {
@@ -411,8 +425,7 @@ __global__ void __launch_bounds__(kFaceThreads<D>) k_flux(Args<T> a) {
                 ei += a.V[(D * D + D + x) * nt + i] * S[x];
                 ej += a.V[(D * D + D + x) * nt + j] * S[x];
             }
-            rhs[D + 1] += wN * ej;
-            rhs[D + 1] += w * ei;
+            visE = interp2(w, wN, ei, ej);
         } else {
             // explicit two-point gradients on physical boundaries
             const T dinv = a.dinv[f];
@@ -431,12 +444,12 @@ __global__ void __launch_bounds__(kFaceThreads<D>) k_flux(Args<T> a) {
             stress<T, D>(g, mu, tau);
 #pragma unroll
             for (int x = 0; x < D; ++x) eV += dotv<T, D>(Uf, tau[x]) * S[x];
-            rhs[D + 1] += eV;
+            visE = eV;
         }
         const T ml = a.ml[f];
 #pragma unroll
         for (int x = 0; x < D; ++x) {
-            T r = rhs[x + 1] + g[x][x] * a.mSK[x * nf + f];
+            T r = g[x][x] * a.mSK[x * nf + f];
             T off = T(0);   // the trace without g[x][x]
             bool any = false;
 #pragma unroll
@@ -448,9 +461,9 @@ __global__ void __launch_bounds__(kFaceThreads<D>) k_flux(Args<T> a) {
                 any = true;
             }
             r += off * a.mT[x * nf + f];
-            rhs[x + 1] = r + ml * (aU[x] - cU[x]);
+            vis[x] = r + ml * (aU[x] - cU[x]);
         }
-        rhs[D + 1] += a.kl[f] * dR;
+        visE += a.kl[f] * dR;
         // Smagorinsky LES: the face tauMC also interpolates the cells' SGS
         // stress (boundary faces keep the laminar two-point one, as in the
         // reference)
@@ -462,10 +475,15 @@ __global__ void __launch_bounds__(kFaceThreads<D>) k_flux(Args<T> a) {
                 for (int y = 0; y < D; ++y)
                     s += interp(w, a.V[(kVisRows<D> + x * D + y) * nt + i], a.V[(kVisRows<D> + x * D + y) * nt + j]) *
                          S[y];
-                rhs[x + 1] += s;
+                vis[x] += s;
             }
         }
     }
+    T rhs[NQ];
+    rhs[0] = mass;
+#pragma unroll
+    for (int k = 0; k < D; ++k) rhs[k + 1] = fma(-cp, S[k], fma(-cm[k], cphi, vis[k]));
+    rhs[D + 1] = fma(-ec, ed, SCH == kSchemeM1 ? fma(-ea, eb, visE) : visE);
 #pragma unroll
     for (int v = 0; v < NQ; ++v) a.flux[v * nf + f] = rhs[v];
 }
