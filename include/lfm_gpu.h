@@ -414,6 +414,18 @@ int lfm_tiles_stats(const lfm_solver_desc* d, int tile_cells, int max_local, int
 int lfm_selftest_fp_convert(int64_t n, const uint32_t* f32_bits, const uint64_t* f64_bits, uint64_t* f64_of_f32,
                             uint32_t* f32_of_f64);
 
+/* Diagnostic: one of the FP64 kernels' own functions on the device over n
+ * argument tuples (host arrays, in [arguments][n]):
+ *   0  reciprocal            x
+ *   1  reciprocal root       x
+ *   2  positive part         x
+ *   3  x >= 1 (0 or 1)       x
+ *   4  half the difference of the AUSM+ pressure polynomials   M, alpha
+ *   5  limited face value from P   P, N, gradient of P [2], of N [2], d [2], w
+ *   6  the same from N
+ */
+int lfm_selftest_fp64(int fn, int64_t n, const double* in, double* out);
+
 /* Diagnostic: whether state transfers have kernels read and write the host
  * memory [p, p + bytes) where it lies (1), or go through the copy calls (0):
  * the former for page-locked memory that is aligned for doubles and page-locked

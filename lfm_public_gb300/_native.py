@@ -196,6 +196,7 @@ def load_library(path: str = LIB_PATH) -> C.CDLL:
         "lfm_partitioned_get_state": ([vp, C.c_int, _dp], C.c_int),
         "lfm_partitioned_step": ([vp, C.c_int, C.c_double], C.c_int),
         "lfm_partitioned_sync": ([vp], C.c_int),
+        "lfm_selftest_fp64": ([C.c_int, C.c_int64, _dp, _dp], C.c_int),
         "lfm_selftest_kernel_range": ([vp, C.c_size_t], C.c_int),
         "lfm_selftest_fp_convert": ([C.c_int64, C.POINTER(C.c_uint32), C.POINTER(C.c_uint64), C.POINTER(C.c_uint64),
                                      C.POINTER(C.c_uint32)], C.c_int),
@@ -834,3 +835,16 @@ def selftest_fp_convert(f32_bits: np.ndarray, f64_bits: np.ndarray):
     if rc != 0:
         raise LfmError(rc, "conversion self-test failed to run")
     return o64, o32
+
+
+FP64_FUNCTIONS = {"rcp": 0, "rsqrt": 1, "pos_part": 2, "atleast1": 3, "p5half": 4, "limited_p": 5, "limited_n": 6}
+
+
+def selftest_fp64(fn: str, *args: np.ndarray) -> np.ndarray:
+    """One of the FP64 kernels' own functions (lfm_selftest_fp64) on the device."""
+    a = np.ascontiguousarray(np.stack(np.broadcast_arrays(*args)), dtype=np.float64)
+    out = np.empty(a.shape[1], dtype=np.float64)
+    rc = load_library().lfm_selftest_fp64(FP64_FUNCTIONS[fn], out.size, _ptr(a, C.c_double), _ptr(out, C.c_double))
+    if rc != 0:
+        raise LfmError(rc, "FP64 self-test failed to run")
+    return out

@@ -885,6 +885,56 @@ void launch_halo_gather_cells(float* dst, int first, int words, int nh, const in
 }  // namespace dev
 }  // namespace lfm
 
+// ---------------------------------------------------------------------------
+// Self-test of the FP64 path's own arithmetic (lfm_selftest_fp64).
+// ---------------------------------------------------------------------------
+namespace {
+
+// Inputs a function takes (lfm_selftest_fp64), 0: no such function.
+int selftest_inputs(int fn) {
+    static const int n[] = {1, 1, 1, 1, 2, 9, 9};
+    return fn >= 0 && fn < (int)(sizeof(n) / sizeof(n[0])) ? n[fn] : 0;
+}
+
+__global__ void k_selftest_fp64(int fn, int64_t n, const double* in, double* out) {
+    using namespace lfm::dev;
+    const int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
+    if (i >= n) return;
+    auto x = [&](int k) { return in[k * n + i]; };
+    switch (fn) {
+        case 0: out[i] = rcp64(x(0)); break;
+        case 1: out[i] = rsqrt64(x(0)); break;
+        case 2: out[i] = pos_part(x(0)); break;
+        case 3: out[i] = atleast1(x(0)) ? 1.0 : 0.0; break;
+        case 4: out[i] = p5half(x(0), x(1)); break;
+        default: {
+            const double gP[2] = {x(2), x(3)}, gN[2] = {x(4), x(5)}, d[2] = {x(6), x(7)};
+            double fromP, fromN;
+            minmod_pair<2>(x(0), x(1), gP, gN, d, x(8), 1.0 - x(8), fromP, fromN);
+            out[i] = fn == 5 ? fromP : fromN;
+        }
+    }
+}
+
+}  // namespace
+
+extern "C" int lfm_selftest_fp64(int fn, int64_t n, const double* in, double* out) {
+    const int rows = selftest_inputs(fn);
+    if (rows == 0 || n <= 0 || !in || !out) return LFM_ERR_INVALID;
+    double *di = nullptr, *dout = nullptr;
+    cudaError_t e = cudaMalloc(&di, (size_t)rows * (size_t)n * sizeof(double));
+    if (e == cudaSuccess) e = cudaMalloc(&dout, (size_t)n * sizeof(double));
+    if (e == cudaSuccess) e = cudaMemcpy(di, in, (size_t)rows * (size_t)n * sizeof(double), cudaMemcpyHostToDevice);
+    if (e == cudaSuccess) {
+        k_selftest_fp64<<<(unsigned)((n + 255) / 256), 256>>>(fn, n, di, dout);
+        e = cudaGetLastError();
+    }
+    if (e == cudaSuccess) e = cudaMemcpy(out, dout, (size_t)n * sizeof(double), cudaMemcpyDeviceToHost);
+    cudaFree(di);
+    cudaFree(dout);
+    return e == cudaSuccess ? LFM_OK : LFM_ERR_CUDA;
+}
+
 extern "C" int lfm_selftest_kernel_range(const void* p, size_t bytes) {
     return lfm::dev::kernel_address(static_cast<const double*>(p), bytes) ? 1 : 0;
 }
