@@ -62,17 +62,14 @@ inline bool needVis(const lfm_solver_desc* d) { return d->mu != 0.0 || d->solver
 // 32-bit device index arrays of a description.
 struct DescIndex {
     std::vector<int> fP, fN, cfOff, cfList, cfNbr, gCell, gKind, gFace;
-    std::vector<double> lapc;   // |delta| / |d| per face
 
     explicit DescIndex(const lfm_solver_desc* d) {
         const size_t nf = (size_t)d->n_faces, nc = (size_t)d->n_cells, ng = (size_t)d->n_ghosts;
         fP.resize(nf);
         fN.resize(nf);
-        lapc.resize(nf);
         for (size_t f = 0; f < nf; ++f) {
             fP[f] = (int)d->face_p[f];
             fN[f] = (int)d->face_n[f];
-            lapc[f] = d->delta_mag[f] * d->dmag_inv[f];
         }
         cfOff.resize(nc + 1);
         for (size_t c = 0; c <= nc; ++c) cfOff[c] = (int)d->cell_face_offsets[c];

@@ -93,7 +93,7 @@ __device__ __forceinline__ void item(const BatchCase& bc, int stage, int i, Sync
     } else {
         const int first = stage == 0;
         const bool res = bc.residuals && first;
-        update32<D, true, PLAIN ? kEntriesEll : kEntriesEither>(a, i, bc.rkA[stage], bc.rkB[stage], bc.dt32, first, res, sync);
+        update32<D, PLAIN ? kEntriesEll : kEntriesEither>(a, i, bc.rkA[stage], bc.rkB[stage], bc.dt32, first, res, sync);
     }
 }
 
@@ -218,9 +218,9 @@ __device__ __forceinline__ void fused_item(const BatchCase& bc, int stage, int i
     const int first = stage == 0;
     const bool res = bc.residuals && first;
     if (bc.scheme == kSchemeM1)
-        fluxupdate32<2, kSchemeM1, false, true, true>(bc.a, i, bc.rkA[stage], bc.rkB[stage], bc.dt32, first, res);
+        fluxupdate32<2, kSchemeM1, false, true>(bc.a, i, bc.rkA[stage], bc.rkB[stage], bc.dt32, first, res);
     else
-        fluxupdate32<2, kSchemeM2, false, true, true>(bc.a, i, bc.rkA[stage], bc.rkB[stage], bc.dt32, first, res);
+        fluxupdate32<2, kSchemeM2, false, true>(bc.a, i, bc.rkA[stage], bc.rkB[stage], bc.dt32, first, res);
 }
 
 // A stage of a batch whose cases can all do flux and update at once

@@ -191,7 +191,7 @@ int buildArgs(lfm_solver* s, const lfm_solver_desc* d, Args<T>& a, const int* fP
     a.smagC = nullptr;
     a.wN = nullptr;
     a.mS = a.mK = a.mT = a.mSK = a.kK = a.ml = a.kl = nullptr;
-    a.S = a.w = a.smag = a.d = a.K = a.lapc = a.dmag = nullptr;
+    a.S = a.w = a.smag = a.d = a.K = a.dmag = nullptr;
     a.cfSoN = nullptr;
     a.cellSoW = nullptr;
     constexpr bool fp64 = sizeof(T) == sizeof(double);
@@ -230,8 +230,10 @@ int buildArgs(lfm_solver* s, const lfm_solver_desc* d, Args<T>& a, const int* fP
     if (s->scheme == LFM_SOLVER_M2AUSM) {   // read by its reconstruction only
         if ((rc = uploadAs<T>(s, &p, d->d, D * nf))) return rc;
         a.d = p;
-        if ((rc = uploadAs<T>(s, &p, d->smag, nf))) return rc;
-        a.smag = p;
+        if (fp64) {
+            if ((rc = uploadAs<T>(s, &p, d->smag, nf))) return rc;
+            a.smag = p;
+        }
     }
     if ((rc = uploadAs<T>(s, &p, d->sponge, (size_t)s->nc))) return rc;
     a.sponge = p;
@@ -754,10 +756,9 @@ int createSolver(const lfm_solver_desc* d, const lfm_solver_opts* opts, cudaStre
         s->tile.block = tiles.tileCells <= 128 ? 128 : 256;
         s->tiled = true;
     }
-    // fused flux + update stages: FP32-bulk single cases whose update writes
-    // the ghosts (no processor halos, laminar, no tile stages)
-    if (s->precision == LFM_FP32_BULK && !tiled && s->nh == 0 && !d->smag_c && s->a32.cellGhosts &&
-        fluxUpdateOption(s)) {
+    // fused flux + update stages: FP32-bulk single cases without processor
+    // halos, LES terms and tile stages
+    if (s->precision == LFM_FP32_BULK && !tiled && s->nh == 0 && !d->smag_c && fluxUpdateOption(s)) {
         if ((rc = devAlloc(s, &s->prim1, (size_t)lfm::dev::primRows<float>(s->D) * nt))) return fail(rc);
         s->fluxUpdate = true;
     }
@@ -1400,10 +1401,9 @@ extern "C" int lfm_solver_bench(lfm_solver* s, int nsteps, double dt, size_t flu
 
 extern "C" int lfm_solver_launches_per_step(const lfm_solver* s, int* launches) {
     if (!s || !launches) return lfm::setError(LFM_ERR_INVALID, "bad argument");
-    // preparation: the update writes the cells' and (cellGhosts) the ghosts'
-    // primitives, so only halos remain
-    const bool fused = s->precision == LFM_FP32_BULK ? s->a32.cellGhosts != nullptr : s->a64.cellGhosts != nullptr;
-    const bool prep = !fused || s->nh > 0;
+    // preparation: the update writes the cells' and the ghosts' primitives, so
+    // only halos remain
+    const bool prep = s->nh > 0;
     *launches = s->tiled ? s->rkOrder
                          : s->rkOrder * ((prep ? 1 : 0) + (s->fluxUpdate ? 1 : 2) + (s->needGrad ? 1 : 0) +
                                          (s->needVis ? 1 : 0));

@@ -66,11 +66,10 @@ __global__ void __launch_bounds__(256) k_probe(const double* q, int64_t nt, QOff
 // (src/cfd_v0.cpp:3180-3240). The reference's ghost cells hold, after a
 // step, the boundary state of the last stage's starting state. The ghost
 // state here is (ghost mode):
-//   kGhostStored -- the stored one (FP64 path: written by the last stage),
 //   kGhostFresh  -- the boundary state of the current state (no stage run),
 //   kGhostUndo   -- the boundary state of q' - B dq, the last stage's
 //                   starting state recovered from its update q' += B dq
-//                   (FP32-bulk path, which stores no ghost states).
+//                   (the stored ghosts are those of the next stage).
 template <typename T, int D>
 __global__ void __launch_bounds__(128) k_force_terms(const Args<T> a, QOffset qo, const double* gS, const double* gD,
                                                      int mode, double Blast, double* terms) {
@@ -83,7 +82,7 @@ __global__ void __launch_bounds__(128) k_force_terms(const Args<T> a, QOffset qo
     load_state<D>(a.q, nt, qo, cell, qc);
     if (mode == kGhostFresh) {
         ghost_bc<T, D>(a, g, qc, qg);
-    } else if (mode == kGhostUndo) {
+    } else {
         double qs[D + 2];
 #pragma unroll
         for (int v = 0; v < D + 2; ++v)
@@ -91,8 +90,6 @@ __global__ void __launch_bounds__(128) k_force_terms(const Args<T> a, QOffset qo
                                         __dmul_rn(Blast, (double)a.dq[(size_t)v * a.nc + cell])),
                               qo.v[v]);
         ghost_bc<T, D>(a, g, qs, qg);
-    } else {
-        load_state<D>(a.q, nt, qo, a.nc + g, qg);
     }
     const double r = qc[0];
     double Uvec[D], Umag = 0.0;

@@ -466,7 +466,7 @@ __device__ __forceinline__ void ghosts_of64(const Args<double>& a, int c, const 
 // RK update (src/cfd_v0.cpp:2800-2822). The rhs are summed in ascending face
 // order (the order in which the reference's scatter reaches the cell); the
 // sum is the cell residual RES. PRIM: the cell also writes the next stage's
-// primitives from the registers it holds, and (a.cellGhosts) the next stage's
+// primitives from the registers it holds, and the next stage's
 // states and primitives of its boundary ghosts -- a ghost depends on its
 // interior cell only -- so that no preparation pass runs between the stages.
 template <typename T, int D, bool RES, bool PRIM = false, class Sync = NoWait>
@@ -480,7 +480,7 @@ __device__ __forceinline__ void update_cell(const Args<T>& a, int c, double Ak, 
 #pragma unroll
     for (int k = 0; k < W; ++k) code[k] = e0 + k < e1 ? a.cfList[e0 + k] : kEllPad;
     const double vi = a.volInv[c], sg = a.sponge[c];
-    const bool ghosts = PRIM && a.cellGhosts && a.cellGhosts[c];
+    const bool ghosts = PRIM && a.cellGhosts[c];
     CellGhosts gh;
     sync();
     double qv[NQ], dq[NQ];

@@ -333,12 +333,12 @@ __device__ __forceinline__ void prep32(const Args<float>& a, int t) {
 // q' = q' + B dq (one FP64 FMA per component), so rounding does not build up
 // over the steps. The sponge pulls q towards q_ref:
 // dt sigma (q_ref - q) = -dt sigma q'.
-// GH: the cell also writes the next stage's state of its boundary ghosts
+// The cell also writes the next stage's state of its boundary ghosts
 // (a ghost depends on its interior cell only), so no preparation pass over
 // the ghosts is needed; the values are those prep32 computes.
 // ---------------------------------------------------------------------------
-// ghosts_of32: the FP64 states and FP32 primitives of the boundary ghosts of
-// cell c from its perturbation state qp (those prep32 computes).
+// ghosts_of32: the FP32 primitives of the boundary ghosts of cell c, from FP64
+// states formed from its perturbation state qp (those prep32 computes).
 template <int D>
 __device__ __forceinline__ void ghosts_of32(const Args<float>& a, int c, const CellGhosts& g, const double* qp,
                                             float* dst) {
@@ -396,17 +396,17 @@ struct CellIn32 {
     double qp[D + 2];   // q'
     float dq[D + 2];
     float vi, sg;       // 1/V, sponge sigma
-    int ghosts;         // it has boundary faces (GH)
+    int ghosts;         // it has boundary faces
     CellGhosts gh;
 };
 
-template <int D, bool GH, class Sync = NoWait>
+template <int D, class Sync = NoWait>
 __device__ __forceinline__ void load_cell32(const Args<float>& a, int c, int first, CellIn32<D>& in,
                                             Sync sync = Sync()) {
     const size_t nt = (size_t)a.nt, nc = (size_t)a.nc;
     in.vi = a.volInv32[c];
     in.sg = a.sponge[c];
-    in.ghosts = GH ? a.cellGhosts[c] : 0;
+    in.ghosts = a.cellGhosts[c];
     sync();
 #pragma unroll
     for (int v = 0; v < D + 2; ++v) {
@@ -417,7 +417,7 @@ __device__ __forceinline__ void load_cell32(const Args<float>& a, int c, int fir
 
 // apply32: the update of cell c from its rhs sum and its loaded values
 // (see update32).
-template <int D, bool GH>
+template <int D>
 __device__ __forceinline__ void apply32(const Args<float>& a, int c, const float* sum, const CellIn32<D>& in,
                                         double Ak, double Bk, float dt32, int first, bool res) {
     constexpr int NQ = D + 2;
@@ -442,23 +442,23 @@ __device__ __forceinline__ void apply32(const Args<float>& a, int c, const float
     }
     if (!finite) atomicOr(a.flag, 1);
     prims32<D>(a, c, qn, a.primW);
-    if (GH && in.ghosts) ghosts_of32<D>(a, c, in.gh, qn, a.primW);
+    if (in.ghosts) ghosts_of32<D>(a, c, in.gh, qn, a.primW);
 }
 
 // ELL: the fixed-width table, the face list, or (the batch, one copy of whose
 // code serves every case) whichever the case has.
 enum Entries32 { kEntriesList, kEntriesEll, kEntriesEither };
-template <int D, bool GH, Entries32 ELL, class Sync = NoWait>
+template <int D, Entries32 ELL, class Sync = NoWait>
 __device__ __forceinline__ void update32(const Args<float>& a, int c, double Ak, double Bk, float dt32, int first,
                                          bool res, Sync sync = Sync()) {
     constexpr int W = kEllWidth<D>;
     int code[ELL != kEntriesList ? W : 1];
     if (ELL == kEntriesEll || (ELL == kEntriesEither && a.cfEll)) load_ell<D>(a.cfEll, c, code);
     CellIn32<D> in;
-    load_cell32<D, GH>(a, c, first, in, sync);
+    load_cell32<D>(a, c, first, in, sync);
     float sum[D + 2];
     auto ghosts = [&] {
-        if (GH && in.ghosts) in.gh = cell_ghosts<float, D>(a, c);
+        if (in.ghosts) in.gh = cell_ghosts<float, D>(a, c);
     };
     if (ELL == kEntriesEll || (ELL == kEntriesEither && a.cfEll)) {
         gather32_ell<D>(a, code, sum, ghosts);
@@ -466,12 +466,11 @@ __device__ __forceinline__ void update32(const Args<float>& a, int c, double Ak,
         ghosts();
         gather32<D>(a, c, sum);
     }
-    apply32<D, GH>(a, c, sum, in, Ak, Bk, dt32, first, res);
+    apply32<D>(a, c, sum, in, Ak, Bk, dt32, first, res);
 }
 
 // A new state: q' = q - q_ref of cell c from a caller's absolute state q
-// ([nq][stride] doubles), its primitives and, where the update keeps them
-// (a.cellGhosts), its boundary ghosts' -- the values the preparation pass
+// ([nq][stride] doubles), its primitives and its boundary ghosts' -- the values the preparation pass
 // derives from the stored q', from registers.
 template <int D>
 __device__ __forceinline__ void set_state32(const Args<float>& a, const double* q, int64_t stride, int c) {
@@ -482,7 +481,7 @@ __device__ __forceinline__ void set_state32(const Args<float>& a, const double* 
         a.q[(size_t)v * a.nt + c] = qp[v];
     }
     prims32<D>(a, c, qp, a.prim);
-    if (a.cellGhosts && a.cellGhosts[c]) ghosts_of32<D>(a, c, cell_ghosts<float, D>(a, c), qp, a.prim);
+    if (a.cellGhosts[c]) ghosts_of32<D>(a, c, cell_ghosts<float, D>(a, c), qp, a.prim);
 }
 
 // Calls f(code, o, S, w) for every face entry of cell c in ascending face
@@ -927,7 +926,7 @@ __device__ __forceinline__ void flux32_cell(const Args<float>& a, int c, Sync sy
 // stage's primitives go to a.primW, the other of two buffers (the cells of
 // this launch still read a.prim). The cell's own values are read once.
 // ---------------------------------------------------------------------------
-template <int D, int SCH, bool VIS, bool GH, bool ELL, class Sync = NoWait>
+template <int D, int SCH, bool VIS, bool ELL, class Sync = NoWait>
 __device__ __forceinline__ void fluxupdate32(const Args<float>& a, int c, double Ak, double Bk, float dt32, int first,
                                              bool res, Sync sync = Sync()) {
     constexpr int NQ = D + 2;
@@ -936,10 +935,10 @@ __device__ __forceinline__ void fluxupdate32(const Args<float>& a, int c, double
     constexpr bool needV = VIS || SCH == kSchemeAUSM;
     float Vc[needV ? kVisVec<D> : 1];
     auto own_values = [&] {
-        load_cell32<D, GH>(a, c, first, in, sync);
+        load_cell32<D>(a, c, first, in, sync);
         load_prim<D>(a, c, self);
         if constexpr (needV) load_vis<D, false>(a, c, Vc);
-        if (GH && in.ghosts) in.gh = cell_ghosts<float, D>(a, c);
+        if (in.ghosts) in.gh = cell_ghosts<float, D>(a, c);
     };
     float sum[NQ];
 #pragma unroll
@@ -986,7 +985,7 @@ __device__ __forceinline__ void fluxupdate32(const Args<float>& a, int c, double
 #pragma unroll
         for (int v = 0; v < NQ; ++v) sum[v] += own ? r[v] : neg_bits(r[v]);
     });
-    apply32<D, GH>(a, c, sum, in, Ak, Bk, dt32, first, res);
+    apply32<D>(a, c, sum, in, Ak, Bk, dt32, first, res);
 }
 
 }  // namespace dev

@@ -43,7 +43,7 @@ __global__ void __launch_bounds__(256) k_prep(Args<T> a, int first) {
 
 // A new state: the rows of the stored state from the caller's q ([nq][stride];
 // the stored rows themselves after a copy, stride nt), the cells' primitives
-// and (a.cellGhosts) their boundary ghosts' states and primitives, and a clear
+// and their boundary ghosts' states and primitives, and a clear
 // non-finite flag.
 template <int D>
 __global__ void __launch_bounds__(256) k_set_state64(const __grid_constant__ Args<double> a, const double* q,
@@ -58,7 +58,7 @@ __global__ void __launch_bounds__(256) k_set_state64(const __grid_constant__ Arg
         a.q[(size_t)v * a.nt + c] = qv[v];
     }
     prims64<D>(a, c, qv);
-    if (a.cellGhosts && a.cellGhosts[c]) ghosts_of64<D>(a, c, cell_ghosts<double, D>(a, c), qv);
+    if (a.cellGhosts[c]) ghosts_of64<D>(a, c, cell_ghosts<double, D>(a, c), qv);
 }
 
 void launch_set_state64(const Args<double>& a, const double* q, int64_t stride, cudaStream_t st) {
@@ -490,7 +490,7 @@ __global__ void __launch_bounds__(kFaceThreads<D>) k_flux(Args<T> a) {
 
 // ---------------------------------------------------------------------------
 // k_update: gather, sponge, RK update (update_cell, solver_device.cuh), then
-// the next stage's primitives of the cell and, with a.cellGhosts, the states
+// the next stage's primitives of the cell and the states
 // and primitives of its boundary ghosts.
 // ---------------------------------------------------------------------------
 template <typename T, int D, bool RES>
@@ -571,20 +571,15 @@ __global__ void __launch_bounds__(256) k_cfl(const double* q, QOffset qo, int nt
     }
 }
 
-__global__ void __launch_bounds__(256) k_reduce_final(const double* partial, int n, int mode, double* out) {
+// The sum of the block results of k_res_sq.
+__global__ void __launch_bounds__(256) k_sum_final(const double* partial, int n, double* out) {
     __shared__ double sh[256];
-    double v = (mode == 0) ? 0.0 : (mode == 1 ? 100.0 : 0.0);
-    for (int k = threadIdx.x; k < n; k += blockDim.x) {
-        const double o = partial[k];
-        v = (mode == 0) ? fmax(v, o) : (mode == 1 ? fmin(v, o) : v + o);
-    }
+    double v = 0.0;
+    for (int k = threadIdx.x; k < n; k += blockDim.x) v = v + partial[k];
     sh[threadIdx.x] = v;
     __syncthreads();
     for (int s = blockDim.x / 2; s > 0; s >>= 1) {
-        if (threadIdx.x < s) {
-            const double o = sh[threadIdx.x + s];
-            sh[threadIdx.x] = (mode == 0) ? fmax(sh[threadIdx.x], o) : (mode == 1 ? fmin(sh[threadIdx.x], o) : sh[threadIdx.x] + o);
-        }
+        if (threadIdx.x < s) sh[threadIdx.x] = sh[threadIdx.x] + sh[threadIdx.x + s];
         __syncthreads();
     }
     if (threadIdx.x == 0) *out = sh[0];
@@ -683,9 +678,9 @@ template <typename T, int D, bool LES>
 void launch_fp64(const Args<T>& a, const StageConfig& s, int which, cudaStream_t st) {
     switch (which) {
         case 0: {
-            // the update keeps the cells' and (a.cellGhosts) the ghosts'
-            // primitives current: only halos remain, unless the state is new
-            const int first = s.fullPrep ? 0 : (a.cellGhosts ? a.nc + a.ng : a.nc);
+            // the update keeps the cells' and the ghosts' primitives
+            // current: only halos remain, unless all are stale
+            const int first = s.fullPrep ? 0 : a.nc + a.ng;
             if (a.nt > first) launch_kernel_pdl(s.pdl && a.pdl, k_prep<T, D>, blocks(a.nt - first, 256), 256, st, a, first);
             break;
         }
@@ -753,7 +748,7 @@ void launch_set_step(StepDt* step, double dt, cudaStream_t st) { k_set_step<<<1,
 void launch_res_sum(const double* res, int nc, double* partial, double* out, cudaStream_t st) {
     const unsigned nb = blocks(nc, 256);
     k_res_sq<<<nb, 256, 0, st>>>(res, nc, partial);
-    k_reduce_final<<<1, 256, 0, st>>>(partial, (int)nb, 2, out);
+    k_sum_final<<<1, 256, 0, st>>>(partial, (int)nb, out);
 }
 
 // The constants of the FP64 path, each the value its kernels would otherwise

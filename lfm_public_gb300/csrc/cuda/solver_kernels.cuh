@@ -101,7 +101,6 @@ struct Args {
     const T* dnorm;           // D x nf
     const T* dmag;            // |delta|
     const T* K;               // D x nf
-    const T* lapc;            // |delta| / |d| per face
     const T* wN;              // FP64 path: 1 - w per face (the linear weight of N)
     // FP64 path, mu != 0: the viscous face constants (D x nf, ml and kl nf)
     const T* mS;              // mu S
@@ -125,8 +124,8 @@ struct Args {
                               // v_c cellSoW_c + sum over entries of v_across cfSoN)
     const T* smagC;           // Smagorinsky LES: the constant each cell's tauMC is built with
                               // (V then holds D x D more rows: its SGS stress), or null
-    const uint8_t* cellGhosts;  // boundary faces of each cell
-                                // (its update writes their ghosts' primitives), or null
+    const uint8_t* cellGhosts;  // per cell: has boundary faces (its update writes their
+                                // ghosts' primitives)
     const int* fOwn;          // FP32-bulk cell-centred flux: nc + 1 offsets, the flux faces that
                               // cell c owns (is P of) are fOwn[c] .. fOwn[c + 1] - 1 (the faces
                               // are stored by owner); null where the face-per-thread kernel runs
@@ -136,7 +135,7 @@ struct Args {
                               // faces (the gathers then go through cfOff / cfList / cfNbr)
     const int* cfEllN;        // FP32-bulk, with cfEll: the cfNbr entries likewise, padded with -1
     const float4* fG0;        // FP32-bulk: face geometry in 16-byte parts (solver_fp32.cuh); S, w, K,
-    const float4* fG1;        // lapc and fGhost are then null, fN carries the boundary flag
+    const float4* fG1;        // dmag and fGhost are then null, fN carries the boundary flag
     // ghosts
     const int* gCell;
     const int* gKind;

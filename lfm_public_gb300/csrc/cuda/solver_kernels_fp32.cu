@@ -17,9 +17,8 @@ constexpr int kCellThreads = 128;
 template <int SCH>
 constexpr int kFaceThreads = SCH == kSchemeAUSM ? 64 : 128;
 
-// Primitives of cells, ghosts and halos [first, a.nt): first = 0 after a new
-// state; once the update kernels keep the cells' current, first = nc (ghosts
-// and halos), or nc + ng (halos only) when the update also writes the ghosts.
+// Primitives of cells, ghosts and halos [first, a.nt): first = 0 where all are
+// stale, else nc + ng (halos only: the update keeps the others current).
 template <int D>
 __global__ void __launch_bounds__(256) k_prep32(const __grid_constant__ Args<float> a, int first) {
     const int t = first + LFM_GLOBAL_ID();
@@ -67,18 +66,18 @@ __global__ void __launch_bounds__(kCellThreads, 768 / kCellThreads) k_flux32_cel
 template <int D>
 constexpr int kSpreadCells = D == 2 ? 1 << 20 : 1 << 18;
 
-template <int D, bool RES, bool GH, bool ELL>
+template <int D, bool RES, bool ELL>
 __device__ __forceinline__ void update_thread(const Args<float>& a, double Ak, double Bk, int first) {
-    const bool spread = GH && a.nc <= kSpreadCells<D>;
+    const bool spread = a.nc <= kSpreadCells<D>;
     const int c = spread ? (int)(((threadIdx.x >> 5) * gridDim.x + blockIdx.x) << 5) + (int)(threadIdx.x & 31u)
                          : (int)LFM_GLOBAL_ID();
-    if (c < a.nc) update32<D, GH, ELL ? kEntriesEll : kEntriesList>(a, c, Ak, Bk, a.step->dt32, first, RES, PdlWait{a.pdl});
+    if (c < a.nc) update32<D, ELL ? kEntriesEll : kEntriesList>(a, c, Ak, Bk, a.step->dt32, first, RES, PdlWait{a.pdl});
 }
 
-template <int D, bool RES, bool GH, bool ELL>
+template <int D, bool RES, bool ELL>
 __global__ void __launch_bounds__(kCellThreads) k_update32(const __grid_constant__ Args<float> a, double Ak, double Bk,
                                                             int first) {
-    update_thread<D, RES, GH, ELL>(a, Ak, Bk, first);
+    update_thread<D, RES, ELL>(a, Ak, Bk, first);
 }
 
 // Fused flux + update (fluxupdate32): one thread per cell, cells mapped as
@@ -87,7 +86,7 @@ template <int D, int SCH, bool VIS, bool RES, bool ELL>
 __global__ void __launch_bounds__(kCellThreads) k_fluxupdate32(const __grid_constant__ Args<float> a, double Ak, double Bk,
                                                                 int first) {
     const int c = (int)(((threadIdx.x >> 5) * gridDim.x + blockIdx.x) << 5) + (int)(threadIdx.x & 31u);
-    if (c < a.nc) fluxupdate32<D, SCH, VIS, true, ELL>(a, c, Ak, Bk, a.step->dt32, first, RES, PdlWait{a.pdl});
+    if (c < a.nc) fluxupdate32<D, SCH, VIS, ELL>(a, c, Ak, Bk, a.step->dt32, first, RES, PdlWait{a.pdl});
 }
 
 template <int D, int SCH, bool VIS, bool ELL>
@@ -111,13 +110,8 @@ void launch_fluxupdate32_scheme(const Args<float>& a, const StageConfig& s, cuda
 template <int D, bool ELL>
 void launch_update32(const Args<float>& a, const StageConfig& s, cudaStream_t st) {
     const unsigned nb = (unsigned)((a.nc + kCellThreads - 1) / kCellThreads);   // a 32-cell chunk per warp
-    if (a.cellGhosts) {
-        if (s.withRes) launch_kernel_pdl(s.pdl && a.pdl, k_update32<D, true, true, ELL>, nb, kCellThreads, st, a, s.A, s.B, s.first);
-        else launch_kernel_pdl(s.pdl && a.pdl, k_update32<D, false, true, ELL>, nb, kCellThreads, st, a, s.A, s.B, s.first);
-    } else {
-        if (s.withRes) launch_kernel_pdl(s.pdl && a.pdl, k_update32<D, true, false, ELL>, nb, kCellThreads, st, a, s.A, s.B, s.first);
-        else launch_kernel_pdl(s.pdl && a.pdl, k_update32<D, false, false, ELL>, nb, kCellThreads, st, a, s.A, s.B, s.first);
-    }
+    if (s.withRes) launch_kernel_pdl(s.pdl && a.pdl, k_update32<D, true, ELL>, nb, kCellThreads, st, a, s.A, s.B, s.first);
+    else launch_kernel_pdl(s.pdl && a.pdl, k_update32<D, false, ELL>, nb, kCellThreads, st, a, s.A, s.B, s.first);
 }
 
 template <int D>
@@ -163,7 +157,7 @@ template <int D>
 void launch_fp32(const Args<float>& a, const StageConfig& s, int which, cudaStream_t st) {
     switch (which) {
         case 0: {
-            const int first = s.fullPrep ? 0 : (a.cellGhosts ? a.nc + a.ng : a.nc);
+            const int first = s.fullPrep ? 0 : a.nc + a.ng;
             // not as a dependent: few blocks of FP64 work, crowded when released early
             if (a.nt > first) launch_kernel_pdl(false, k_prep32<D>, nblocks(a.nt - first, 256), 256, st, a, first);
             break;

@@ -86,9 +86,8 @@ template <>
 void launch_kernel<float>(const Args<float>& a, const StageConfig& s, int which, cudaStream_t st);
 // FP32-bulk kernels (perturbation form).
 void launch_kernel_fp32(const Args<float>& a, const StageConfig& s, int which, cudaStream_t st);
-// FP32-bulk fused flux + update of every cell (laminar, a.cellGhosts set): the
-// face rhs evaluated by the cells themselves; the next stage's primitives go
-// to a.primW, which must not be a.prim.
+// FP32-bulk fused flux + update of every cell (laminar): the face rhs
+// evaluated by the cells themselves; the next stage's primitives go to a.primW, which must not be a.prim.
 void launch_fluxupdate32(const Args<float>& a, const StageConfig& s, cudaStream_t st);
 // Staged flux kernel: for M1 / M2 without the LES terms; configure sets the
 // kernel's shared-memory limit (outside graph capture) and fs.grid, fs.smem.
@@ -113,7 +112,7 @@ double* kernel_address(const double* p, size_t bytes);
 // A new FP64 state from an absolute one (or from the stored rows, stride nt).
 void launch_set_state64(const Args<double>& a, const double* q, int64_t stride, cudaStream_t st);
 // A new FP32-bulk state from an absolute one: q', the cells' primitives and
-// (with a.cellGhosts) their boundary ghosts' states and primitives.
+// their boundary ghosts' primitives.
 void launch_set_state32(const Args<float>& a, const double* q, int64_t stride, cudaStream_t st);
 
 // Rows of the per-cell primitive array: FP64 keeps 1/rho, u[D], R psi, c;
@@ -165,7 +164,7 @@ void launch_stats(int D, const double* q, int64_t nt, QOffset qo, int nc, double
                   double* rms, cudaStream_t st);
 void launch_probe(int D, const double* q, int64_t nt, QOffset qo, const int* cells, int n, double gm1, double pInf,
                   double* out, cudaStream_t st);
-enum { kGhostStored = 0, kGhostFresh = 1, kGhostUndo = 2 };
+enum { kGhostFresh = 0, kGhostUndo = 1 };
 template <typename T>
 void launch_forces(const Args<T>& a, QOffset qo, const double* gS, const double* gD, const int* gPatch, int mode,
                    double Blast, const int* patches, int nPatches, double* terms, double* fp, double* fv,

@@ -95,11 +95,11 @@ __global__ void __launch_bounds__(256) k_tile_stage(const __grid_constant__ Args
     __syncthreads();
     for (int lc = threadIdx.x; lc < td.nA; lc += blockDim.x) {
         CellIn32<D> in;
-        load_cell32<D, true>(g, td.c0 + lc, first, in);
+        load_cell32<D>(g, td.c0 + lc, first, in);
         if (in.ghosts) in.gh = cell_ghosts<float, D>(g, td.c0 + lc);
         float sum[R::Q];
         gather32<D>(a, lc, sum);
-        apply32<D, true>(g, td.c0 + lc, sum, in, Ak, Bk, g.step->dt32, first, RES);
+        apply32<D>(g, td.c0 + lc, sum, in, Ak, Bk, g.step->dt32, first, RES);
     }
 }
 
