@@ -101,6 +101,11 @@ struct Args {
     const T* dnorm;           // D x nf
     const T* dmag;            // |delta|
     const T* K;               // D x nf
+    // (Here and not at the end: the batch's kernels hold an Args in shared memory, and
+    // the members' offsets decide which pairs they load as 16 bytes. With every
+    // later one 8 bytes nearer the fused stage spilled 76 bytes for 56, and a batch
+    // of 2.5M cells took 733 us a step for 704.)
+    int* flag;                // error flag (non-finite state)
     const T* wN;              // FP64 path: 1 - w per face (the linear weight of N)
     // FP64 path, mu != 0: the viscous face constants (D x nf, ml and kl nf)
     const T* mS;              // mu S
@@ -155,8 +160,6 @@ struct Args {
     // the primitives include the sound speed (read by M2AUSM only)
     int primC;
     const StepDt* step;       // single cases: the time step, set before the step's kernels
-    // error flag (non-finite state)
-    int* flag;
     // the step's kernels are launched as programmatic dependents (pdl_pays)
     int pdl;
 };
