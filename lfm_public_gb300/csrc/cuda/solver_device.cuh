@@ -419,23 +419,24 @@ __device__ __forceinline__ CellGhosts cell_ghosts(const Args<T>& a, int c) {
 }
 
 // f(j, kind) for each of them: the first two, then (a cell with more boundary
-// faces) the others in entry order, told by their place among the cell's ghost
-// entries -- not by their numbers: faces may share a ghost.
+// faces) the others in entry order. Faces may share a ghost, so that fewer than
+// `count` are left: the walk ends with the entries. (Telling them by their place
+// among the ghosts passed takes two counters more, and the batch's update phases
+// spilled 8 bytes more.)
 template <typename T, int D, class F>
 __device__ __forceinline__ void for_ghosts(const Args<T>& a, int c, const CellGhosts& g, F f) {
-    int e = 0, seen = 0;   // entries passed, ghosts among them
+    int left = g.count;
 #pragma unroll 1
-    for (int k = 0; k < g.count; ++k) {
+    for (int k = 0; left > 0; ++k) {
         int j = k == 0 ? g.j[0] : g.j[1], kind = k == 0 ? g.kind[0] : g.kind[1];
         if (k >= 2) {
-            do {
-                j = entry_cell<T, D>(a, c, e++);
-                if (j >= a.nc && j < a.nc + a.ng) ++seen;
-            } while (j >= 0 && seen <= k);
-            if (j < 0) return;   // past the last entry
+            j = entry_cell<T, D>(a, c, k - 2);
+            if (j < 0) break;   // past the last entry
+            if (j < a.nc || j >= a.nc + a.ng || j == g.j[0] || j == g.j[1]) continue;
             kind = a.gKind[j - a.nc];
         }
         f(j, kind);
+        --left;
     }
 }
 
