@@ -593,9 +593,15 @@ int enqueueBatchStates(lfm_batch* b, int n, const int* slots, const double* cons
         const Slot& sl = b->slots[(size_t)slots[i]];
         return (size_t)sl.nq * sl.nc * sizeof(double);
     };
+    double* first[lfm::dev::kBatchStates];   // of the first entries, which are as a rule all
+    auto direct = [&](int i) { return lfm::dev::kernel_address(q[i], bytesOf(i)); };
     size_t most = 0;
-    for (int i = 0; i < n; ++i)
-        if (q[i] && !lfm::dev::kernel_address(q[i], bytesOf(i))) most = std::max(most, bytesOf(i));
+    for (int i = 0; i < n; ++i) {
+        if (!q[i]) continue;
+        double* at = direct(i);
+        if (!at) most = std::max(most, bytesOf(i));
+        if (i < lfm::dev::kBatchStates) first[i] = at;
+    }
     int rc;
     if (most && (rc = ensureStage(b, most))) return rc;
     lfm::dev::BatchStates m{};
@@ -608,24 +614,25 @@ int enqueueBatchStates(lfm_batch* b, int n, const int* slots, const double* cons
         return LFM_OK;
     };
     auto again = [&](int i) {   // writes what a pending entry writes
-        const auto at = [&](int k) { return reinterpret_cast<uintptr_t>(q[k]); };
+        const auto host = [&](int k) { return reinterpret_cast<uintptr_t>(q[k]); };
         for (int k = 0; k < count; ++k) {
             const int e = entry[k];
-            if (set ? slots[e] == slots[i] : at(e) < at(i) + bytesOf(i) && at(i) < at(e) + bytesOf(e)) return true;
+            if (set ? slots[e] == slots[i] : host(e) < host(i) + bytesOf(i) && host(i) < host(e) + bytesOf(e))
+                return true;
         }
         return false;
     };
     for (int i = 0; i < n; ++i) {
         if (!q[i]) continue;
         if (again(i) && (rc = flush())) return rc;
-        double* direct = lfm::dev::kernel_address(q[i], bytesOf(i));
-        if (!direct) {
+        double* at = i < lfm::dev::kBatchStates ? first[i] : direct(i);
+        if (!at) {
             rc = set ? enqueueBatchSet(b, slots[i], q[i]) : enqueueBatchGet(b, slots[i], const_cast<double*>(q[i]));
             if (rc) return rc;
             continue;
         }
         m.slot[count] = slots[i];
-        m.q[count] = direct;
+        m.q[count] = at;
         entry[count] = i;
         maxCells = std::max(maxCells, b->slots[(size_t)slots[i]].nc);
         if (++count == lfm::dev::kBatchStates && (rc = flush())) return rc;

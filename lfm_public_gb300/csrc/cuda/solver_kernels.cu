@@ -640,28 +640,29 @@ void launch_prep_residual64(const Args<double>& a, const double* q, int64_t stri
 double* kernel_address(const double* p, size_t bytes) {
     // a copy engine takes any address, a kernel's loads only aligned ones
     if (reinterpret_cast<uintptr_t>(p) % alignof(double) != 0) return nullptr;
-    cudaPointerAttributes at{};
-    if (cudaPointerGetAttributes(&at, p) != cudaSuccess) {
-        cudaGetLastError();
-        return nullptr;
-    }
-    if (at.type != cudaMemoryTypeHost || !at.devicePointer) return nullptr;
-    // what is page-locked and mapped ends with its allocation or registration
-    static const auto attribute = [] {
+    // One query for all that is asked (a batch asks for every state it moves);
+    // what is page-locked and mapped ends with its allocation or registration.
+    static const auto query = [] {
         void* f = nullptr;
         cudaDriverEntryPointQueryResult found;
-        if (cudaGetDriverEntryPointByVersion("cuPointerGetAttribute", &f, 12000, cudaEnableDefault, &found) != cudaSuccess)
+        if (cudaGetDriverEntryPointByVersion("cuPointerGetAttributes", &f, 12000, cudaEnableDefault, &found) !=
+            cudaSuccess) {
             cudaGetLastError();
-        return reinterpret_cast<CUresult (*)(void*, CUpointer_attribute, CUdeviceptr)>(f);
+            f = nullptr;
+        }
+        return reinterpret_cast<CUresult (*)(unsigned, CUpointer_attribute*, void**, CUdeviceptr)>(f);
     }();
-    const CUdeviceptr d = reinterpret_cast<CUdeviceptr>(at.devicePointer);
-    CUdeviceptr start = 0;
+    CUpointer_attribute what[] = {CU_POINTER_ATTRIBUTE_MEMORY_TYPE, CU_POINTER_ATTRIBUTE_IS_MANAGED,
+                                  CU_POINTER_ATTRIBUTE_DEVICE_POINTER, CU_POINTER_ATTRIBUTE_RANGE_START_ADDR,
+                                  CU_POINTER_ATTRIBUTE_RANGE_SIZE};
+    unsigned type = 0, managed = 0;
+    CUdeviceptr d = 0, start = 0;
     size_t size = 0;
-    if (!attribute || attribute(&start, CU_POINTER_ATTRIBUTE_RANGE_START_ADDR, d) != CUDA_SUCCESS ||
-        attribute(&size, CU_POINTER_ATTRIBUTE_RANGE_SIZE, d) != CUDA_SUCCESS)
-        return nullptr;
+    void* into[] = {&type, &managed, &d, &start, &size};   // zeros where p is unknown to the driver
+    if (!query || query(5, what, into, reinterpret_cast<CUdeviceptr>(p)) != CUDA_SUCCESS) return nullptr;
+    if (type != CU_MEMORYTYPE_HOST || managed || d == 0) return nullptr;
     if (d < start || d - start > size || bytes > size - (size_t)(d - start)) return nullptr;
-    return static_cast<double*>(at.devicePointer);
+    return reinterpret_cast<double*>(d);
 }
 
 // ---------------------------------------------------------------------------
