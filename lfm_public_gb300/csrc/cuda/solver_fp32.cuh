@@ -652,9 +652,10 @@ __device__ __forceinline__ float p5diff_dd(float a, float b, float alpha) {
 // VIS = false compiles the viscous terms out (for callers that know mu = 0).
 // EARLYV loads the viscous rows of both cells together with the primitives, so
 // the gathers overlap instead of following one another: the stand-alone flux
-// kernel (3D flux 4.05 -> 3.43 ms per step on the 9.4M-cell wake, whose
-// gathers come from HBM; 2 % in 2D, whose gathers hit L2). The fused kernels,
-// whose registers other phases already fill, keep the late loads.
+// kernel (measured with rows of single values in place of the 16-byte parts: 3D
+// flux 4.05 -> 3.43 ms per step on the 9.4M-cell wake, whose gathers come from
+// HBM; 2 % in 2D, whose gathers hit L2). The batch's kernels, whose registers
+// other code already fills, keep the late loads.
 //
 // face_rhs32_core takes the face's geometry and both cells' primitives as
 // values and loadV(Vi, Vj), which fills their viscous rows; `a` gives the

@@ -45,9 +45,9 @@ __global__ void __launch_bounds__(kFaceThreads<SCH>) k_flux32(const __grid_const
 }
 
 // Cell-centred form (flux32_cell): one thread per cell over the faces it
-// owns. 3D at three blocks per SM (80 registers; the cell keeps its own 23
-// rows across its faces): the 9.4M-cell wake's flux 3.42 -> 3.27 ms per step;
-// at four blocks per SM it spills (3.66 ms).
+// owns, at 768 threads per SM (80 registers; the cell keeps its own 23 values
+// across its faces, 3D spills 24 bytes). Off by default: fluxCellOption gives
+// both sides' measurements.
 template <int D, int SCH>
 __global__ void __launch_bounds__(kCellThreads, 768 / kCellThreads) k_flux32_cell(const __grid_constant__ Args<float> a) {
     const int c = LFM_GLOBAL_ID();

@@ -34,7 +34,8 @@ struct FluxStaging {
 //              134k cells 641.0 632.8 | 171k 794.5 772.0
 //   FP32 2D      2k cells  36.8  34.7 |  46k  57.2  49.9 | 135k 73.7 67.5
 //   FP32 3D      5k cells  61.4  53.2 |  51k  81.9  83.9 | 83k 98.2 99.9 | 134k 118.7 116.7 | 171k 147.4 137.1
-// (viscous but for the FP64 2D M1 sizes below 100k).
+// (viscous but for the FP64 2D M1 sizes below 100k). FP32 3D from 50k to 100k
+// cells is even, within the timer's unit, and goes with the sizes around it.
 inline bool pdl_pays(bool fp64, int D, int scheme, int nc) {
     if (!fp64 || nc >= 131072) return true;
     if (D == 3) return nc <= 8192;
