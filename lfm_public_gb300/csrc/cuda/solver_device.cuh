@@ -203,7 +203,7 @@ __device__ __forceinline__ double rsqrt64(double x) {
 // case of a quotient too large to form (minmod_interp's 1000; 0 / 0 counts as one)
 // is told by the exponents. With the sensor's and the Mach numbers' divisions replaced alike
 // the M2AUSM flux of a 331 x 217 cylinder took 413 us a step where it took 681,
-// and 306 with the comparisons on the integer pipe, the sensor's roots by
+// and 301 with the comparisons on the integer pipe, the sensor's roots by
 // rsqrt64 and the pressure polynomials by p5half (GB300).
 template <int D>
 __device__ __forceinline__ void minmod_pair(double cp, double ap, const double* gradP, const double* gradN,
@@ -481,7 +481,9 @@ __device__ __forceinline__ void update_cell(const Args<T>& a, int c, double Ak, 
 #pragma unroll
     for (int k = 0; k < W; ++k) code[k] = e0 + k < e1 ? a.cfList[e0 + k] : kEllPad;
     const double vi = a.volInv[c], sg = a.sponge[c];
-    const bool ghosts = PRIM && a.cellGhosts[c];
+    // (ng > 0 first: a uniform branch around the load, without which the 2D kernel
+    // keeps 79 registers for 72, six blocks an SM for seven)
+    const bool ghosts = PRIM && a.ng > 0 && a.cellGhosts[c];
     CellGhosts gh;
     sync();
     double qv[NQ], dq[NQ];

@@ -15,11 +15,19 @@ namespace dev {
 // boundary cell's ghost work holds few threads. Measured on GB300, us a step at
 // 256, 128 and 64 threads: update, 48 x 48 vortex 39.9, 27.7, 29.3, 768 x 512
 // cylinder 168.2, 160.6, 159.1, 192 x 128 x 48 wake 836, 792, 756; flux of the
-// cylinder at 256, 128, 64 461, 451, 451, of the wake 2974, 3001, 3001.
+// cylinder 442, 432, 431, of the 331 x 217 M2AUSM cylinder 307, 301, 301, of the
+// 97 x 61 x 23 wake 360, 358, 360, of the 384 x 256 x 96 wake 22117, 22097, 22101.
 template <int D>
 constexpr int kCellThreads = D == 2 ? 128 : 64;
 template <int D>
 constexpr int kFaceThreads = D == 2 ? 128 : 256;
+// Blocks per SM that the flux has to fit (0: whatever does): 56 registers in 2D
+// without M2AUSM (with 64 a 50k-cell M2 vortex, whose kernels overlap (pdl_pays),
+// took 102 us a step for 72, with the LES stress 217 for 168), and with the LES
+// stress in 3D 80, with M2AUSM 128, which it exceeds by a few otherwise.
+template <int D, int SCH, bool LES>
+constexpr int kFluxBlocks = D == 2 ? (SCH != kSchemeAUSM ? 9 : 0)
+                                   : (!LES ? 0 : SCH == kSchemeAUSM ? 2 : 3);
 
 // ---------------------------------------------------------------------------
 // k_prep: ghost states and per-cell primitives of entries [first, nt). The
@@ -239,7 +247,7 @@ __global__ void __launch_bounds__(kCellThreads<D>) k_vis(Args<T> a) {
 // k_flux: rhs of one face.
 // ---------------------------------------------------------------------------
 template <typename T, int D, int SCH, bool LES>
-__global__ void __launch_bounds__(kFaceThreads<D>) k_flux(Args<T> a) {
+__global__ void __launch_bounds__(kFaceThreads<D>, kFluxBlocks<D, SCH, LES>) k_flux(Args<T> a) {
     const int f = LFM_GLOBAL_ID();
     if (f >= a.nf) return;
     constexpr int NQ = D + 2;
@@ -409,9 +417,10 @@ __global__ void __launch_bounds__(kFaceThreads<D>) k_flux(Args<T> a) {
     //   heat: k/R (K.gR + |delta|/|d| d(R psi)) + sigmaU . S
     // The heat flux and sigmaU.S of each side are summed before they are
     // interpolated (10 instead of 12 operations in 2D). The kernel is bound by
-    // the FP64 pipe, and loads are not: seven constants more per face and 14
-    // operations less took the flux of the 768 x 512 M1 cylinder from 583 to
-    // 459 us a step, of the 97 x 61 x 23 M2 wake from 484 to 390 (GB300).
+    // the FP64 pipe, and loads are not: seven constants more per face, the
+    // convective products joined by FMAs and in all 18 operations less took the flux
+    // of the 768 x 512 M1 cylinder from 580 to 431 us a step, of the 97 x 61 x 23 M2
+    // wake from 483 to 359 (GB300).
     const T mu = (T)a.mu;
     T vis[D], visE = T(0);
 #pragma unroll
