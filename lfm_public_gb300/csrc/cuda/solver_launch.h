@@ -25,21 +25,26 @@ struct FluxStaging {
 // first; one with fewer blocks than the chip holds at once is crowded onto part
 // of the SMs, and FP64 work then waits for their FP64 pipes, while a larger one
 // fills every SM anyway and a smaller one finds idle SMs. FP32 kernels wait for
-// loads, which crowded SMs serve as well. Measured on GB300, us a step without
-// and with (one unit of the timer is 2 us):
-//   FP64 2D M1   2k cells  45.0  38.8 |  36k  69.6  61.4 | 51k  88.0  79.8 | 58k  86.0 112.6
-//               81k cells 116.7 124.7 | 101k 239.6 253.9 | 135k 296.9 293.3 | 144k 325.6 311.2
-//   FP64 2D M2AUSM 15k cells 9 % less | 22k 255.9 243.7 | 33k 305.1 341.9 | 135k 932.8 932.3
-//   FP64 3D      5k cells 135.1 124.9 |  10k 137.2 151.5 | 61k 330.1 391.1 | 117k 579.0 581.1
-//              134k cells 641.0 632.8 | 171k 794.5 772.0
+// loads, which crowded SMs serve as well. Where the line lies depends on the blocks
+// an SM holds: with the 2D update at 79 registers (6 blocks) for 72 (7) 47k cells
+// took 90 us in place of 72. Measured on GB300, us a step without and with (one unit
+// of the timer is 2 us):
+//   FP64 2D M1   2k cells  44.9  38.8 |  36k  65.5  59.3 | 51.5k 83.9 75.7 | 52.0k 83.9 94.1
+//             65.5k cells  96.2 114.6 |  81k 112.6 118.7 | viscous 51.2k 151.5 139.2
+//             52.1k 151.5 178.8 | 101k 240.6 253.9 | 135k 295.9 294.8 | 144k 319.4 309.2
+//   FP64 2D M2AUSM 15k cells 163.8 153.5 | 24.1k 215.0 206.8 | 24.6k 215.0 249.8 | 33k 251.9 292.2
+//              135k cells 749.0 750.5
+//   FP64 3D      5k cells 133.1 122.8 | 8.1k 133.1 126.9 | 10k 133.1 147.4 | 61k 323.6 384.9
+//              117k cells 560.1 563.1 | 134k 624.6 616.4 | 171k 773.1 747.6
+//   FP64 3D M2AUSM 6.0k cells 235.5 227.3 | 6.8k 237.5 307.1
 //   FP32 2D      2k cells  36.8  34.7 |  46k  57.2  49.9 | 135k 73.7 67.5
 //   FP32 3D      5k cells  61.4  53.2 |  51k  81.9  83.9 | 83k 98.2 99.9 | 134k 118.7 116.7 | 171k 147.4 137.1
-// (viscous but for the FP64 2D M1 sizes below 100k). FP32 3D from 50k to 100k
-// cells is even, within the timer's unit, and goes with the sizes around it.
+// FP32 3D from 50k to 100k cells is even, within the timer's unit, and goes with the
+// sizes around it.
 inline bool pdl_pays(bool fp64, int D, int scheme, int nc) {
     if (!fp64 || nc >= 131072) return true;
-    if (D == 3) return nc <= 8192;
-    return nc <= (scheme == kSchemeAUSM ? 24576 : 53248);
+    if (D == 3) return nc <= (scheme == kSchemeAUSM ? 6000 : 8192);
+    return nc <= (scheme == kSchemeAUSM ? 24192 : 51200);
 }
 
 // Launches k, with `pdl` as a programmatic dependent of the stream's previous

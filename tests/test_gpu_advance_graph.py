@@ -11,8 +11,13 @@ from tests.test_gpu_dependent_launch import SHAPES, _cylinder
 pytestmark = pytest.mark.gpu
 
 
+# on either side of the sizes at which FP64 steps change to dependent launches
+LINES = [(256, 200, 1, 0), (257, 200, 1, 1), (192, 126, 1, 2), (192, 127, 1, 2), (30, 20, 10, 2), (31, 20, 10, 2),
+         (32, 16, 16, 0), (33, 16, 16, 0), (512, 256, 1, 0), (512, 255, 1, 0)]
+
+
 @pytest.mark.parametrize("precision", [N.LFM_FP64, N.LFM_FP32_BULK])
-@pytest.mark.parametrize("shape", [*SHAPES, None], ids=lambda s: "x".join(map(str, s)) if s else "vortex")
+@pytest.mark.parametrize("shape", [*SHAPES, *LINES, None], ids=lambda s: "x".join(map(str, s)) if s else "vortex")
 def test_advance_graph_gives_the_steps_bits(shape, precision):
     torch = pytest.importorskip("torch")
     case = _cylinder(*shape) if shape else cases.vortex_case(n=67, ny=41, solver=0)
