@@ -115,7 +115,7 @@ DRAM_TRAFFIC = {
     # which grow in proportion
     ("cylinder3d_small", "fp32", "k_flux"): 263294720 + 55037184,
     ("cylinder3d", "fp32", "k_flux"): 8 * (263294720 + 55037184),
-    ("cylinder2d", "fp64", "k_flux"): 152877056 + 13607168,
+    ("cylinder2d", "fp64", "k_flux"): 152876800 + 13403648,
 }
 
 # FP64 pipe thread-instructions per cell of one launch of each kernel of the
@@ -124,7 +124,7 @@ DRAM_TRAFFIC = {
 # cells) on the 768x512 cylinder, M1, viscous; the update also derives the next
 # stage's primitives and boundary ghosts (no preparation kernel).
 FP64_INST_PER_CELL = {
-    "cylinder2d": {"k_prep": 0.0, "k_grad": 0.0, "k_vis": 43.00, "k_flux": 122.17, "k_update": 36.39},
+    "cylinder2d": {"k_prep": 0.0, "k_grad": 0.0, "k_vis": 43.00, "k_flux": 118.16, "k_update": 36.39},
 }
 # FP64 pipe instruction rate: the measured DFMA rate (FP64_PEAK_TFLOPS counts
 # an FMA as two operations) in instructions per second.
