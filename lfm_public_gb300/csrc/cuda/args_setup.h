@@ -103,21 +103,16 @@ inline bool ellFits(const lfm_solver_desc* d) {
     return true;
 }
 
-// Fixed-width tables of the face entries and the cells across them
-// (Args::cfEll, cfEllN), [n_cells][W] each.
-inline void packEll(const lfm_solver_desc* d, int* ell, int* ellN) {
-    const size_t W = (size_t)(d->dim == 2 ? dev::kEllWidth<2> : dev::kEllWidth<3>);
-    for (size_t c = 0; c < (size_t)d->n_cells; ++c) {
-        size_t at = c * W;
-        for (int64_t e = d->cell_face_offsets[c]; e < d->cell_face_offsets[c + 1]; ++e, ++at) {
-            const int64_t f = d->cell_faces[e];
-            const bool own = d->cell_face_sign[e] > 0;
-            ell[at] = own ? (int)f : ~(int)f;
-            ellN[at] = (int)(own ? d->face_n[f] : d->face_p[f]);
-        }
-        for (; at < (c + 1) * W; ++at) {
-            ell[at] = dev::kEllPad;
-            ellN[at] = -1;
+// Fixed-width tables (Args::cfEll, cfEllN), [n_cells][W] each, of the face lists
+// and the cells across (cfOff, cfList, cfNbr: in order, where another walk over
+// the description would gather from its faces once more).
+inline void packEll(int dim, size_t nc, const int* cfOff, const int* cfList, const int* cfNbr, int* ell, int* ellN) {
+    const int W = dim == 2 ? dev::kEllWidth<2> : dev::kEllWidth<3>;
+    for (size_t c = 0; c < nc; ++c, ell += W, ellN += W) {
+        const int e0 = cfOff[c], n = cfOff[c + 1] - e0;
+        for (int k = 0; k < W; ++k) {
+            ell[k] = k < n ? cfList[e0 + k] : dev::kEllPad;
+            ellN[k] = k < n ? cfNbr[e0 + k] : -1;
         }
     }
 }

@@ -83,7 +83,7 @@ std::vector<unsigned char> packCase(const lfm_solver_desc* d, const CaseLayout& 
     conv(L.volInv32, d->vol_inv, nc);
     conv(L.sponge, d->sponge, nc);
     if (L.cfEll != CaseLayout::npos()) {
-        lfm::setup::packEll(d, i32(L.cfEll), i32(L.cfEllN));
+        lfm::setup::packEll(d->dim, nc, ix.cfOff.data(), ix.cfList.data(), ix.cfNbr.data(), i32(L.cfEll), i32(L.cfEllN));
     } else {
         std::memcpy(i32(L.cfOff), ix.cfOff.data(), (nc + 1) * 4);
         std::memcpy(i32(L.cfList), ix.cfList.data(), ix.cfList.size() * 4);
