@@ -656,16 +656,11 @@ int createSolver(const lfm_solver_desc* d, const lfm_solver_opts* opts, cudaStre
     for (int f = 0; f < s->nf; ++f)   // ghosts only (halos follow them)
         if (fN[(size_t)f] >= s->nc && fN[(size_t)f] < s->nc + s->ng) gFace[(size_t)(fN[(size_t)f] - s->nc)] = f;
     std::vector<int> sOff = toInt(d->cell_s_offsets, nc + 1);
-    int *dP = nullptr, *dN, *dOff, *dList, *dNbr = nullptr, *dGC, *dGK, *dGF;
+    int *dP, *dN, *dOff, *dList, *dNbr, *dGC, *dGK, *dGF;
     uint8_t* dG = nullptr;
-    // FP32-bulk: fixed-width tables in place of the neighbour list where every cell
-    // fits them (and no tiles are cut, whose update reads the list), and in 2D a
-    // face's P in its geometry
-    const bool fp32 = s->precision == LFM_FP32_BULK;
-    const bool ellFits = fp32 && lfm::setup::ellFits(d);
-    if (!(fp32 && s->D == 2) && (rc = upload(s, &dP, fP.data(), nf))) return fail(rc);
+    if ((rc = upload(s, &dP, fP.data(), nf))) return fail(rc);
     std::vector<int> fNf;   // FP32-bulk: with the boundary flag in the top bit
-    if (fp32) {
+    if (s->precision == LFM_FP32_BULK) {
         fNf.resize(nf);
         for (size_t f = 0; f < nf; ++f) fNf[f] = lfm::setup::flaggedN(d, f);
     }
@@ -673,7 +668,7 @@ int createSolver(const lfm_solver_desc* d, const lfm_solver_opts* opts, cudaStre
     if (s->precision == LFM_FP64 && (rc = upload(s, &dG, d->face_ghost, nf))) return fail(rc);
     if ((rc = upload(s, &dOff, cfOff.data(), nc + 1))) return fail(rc);
     if ((rc = upload(s, &dList, cfList.data(), ne))) return fail(rc);
-    if ((!ellFits || tileCellsOption() > 0) && (rc = upload(s, &dNbr, cfNbr.data(), ne))) return fail(rc);
+    if ((rc = upload(s, &dNbr, cfNbr.data(), ne))) return fail(rc);
     if ((rc = upload(s, &dGC, gCell.data(), (size_t)s->ng))) return fail(rc);
     if ((rc = upload(s, &dGK, gKind.data(), (size_t)s->ng))) return fail(rc);
     if ((rc = upload(s, &dGF, gFace.data(), (size_t)s->ng))) return fail(rc);
@@ -714,7 +709,7 @@ int createSolver(const lfm_solver_desc* d, const lfm_solver_opts* opts, cudaStre
         if (s->precision == LFM_FP32_BULK) s->a32.cellGhosts = dCG;
         else s->a64.cellGhosts = dCG;
     }
-    if (ellFits && !tiled) {
+    if (s->precision == LFM_FP32_BULK && !tiled && lfm::setup::ellFits(d)) {
         // the fixed-width tables of a cell's faces and the cells across them
         const size_t W = (size_t)(s->D == 2 ? lfm::dev::kEllWidth<2> : lfm::dev::kEllWidth<3>);
         std::vector<int> ell(W * nc), ellN(W * nc);
